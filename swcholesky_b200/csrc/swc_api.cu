@@ -12,6 +12,7 @@
 
 #include "../../include/swcholesky_b200.h"
 #include "swc_engine.h"
+#include "swc_front.h"
 
 #include "swc_handle.h"
 
@@ -418,6 +419,10 @@ int swc_plan_stats(int n, const int *c, const int *r, const size_t *lC, const in
     return fail(SWC_INVALID_INPUT, err);
   if (!swc::check_scatter_plan(n, Ls, H, P, swc::plan_candidate(plan), err))
     return fail(SWC_INVALID_INPUT, err);
+  swc::FrontPlan FP;
+  swc::build_front_plan(n, c, r, Ls, prunePtr, pruneSet, H, P, swc::plan_candidate(plan), FP);
+  if (!swc::check_front_plan(n, Ls, H, P, FP, err)) return fail(SWC_INVALID_INPUT, err);
+  if (FP.ok) P.launches = FP.launches;
   swc::SolvePlan SP;
   swc::build_solve_plan(n, Ls, H, SP);
   if (!swc::check_solve_plan(n, Ls, H, SP, err)) return fail(SWC_INVALID_INPUT, err);

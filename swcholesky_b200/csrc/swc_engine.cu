@@ -10,6 +10,7 @@
 #include <tuple>
 
 #include "swc_engine.h"
+#include "swc_front.h"
 
 namespace swc {
 
@@ -174,6 +175,7 @@ void Engine::release() {
   for (void *p : ptrs)
     if (p) cudaFree(p);
   release_adjoint();
+  release_front();
   d_super_ = d_Ls_ = d_Ap_ = d_Ai_ = nullptr;
   d_rowptr_ = d_xptr_ = nullptr;
   d_upd_ptr_ = d_upd_ = nullptr;
@@ -1174,7 +1176,8 @@ bool Engine::analyze(int n, const int *c, const int *r, const int64_t *lC, const
                      const int64_t *Li_ptr, const int *blockSet, int supNo,
                      const int *prunePtr, const int *pruneSet, std::string &err) {
   cudaSetDevice(device_);
-  if (!kernels_configure(err) || !update_tc_configure(err) || !scatter_tc_configure(err))
+  if (!kernels_configure(err) || !update_tc_configure(err) || !scatter_tc_configure(err) ||
+      !front_configure(err))
     return false;
   HostSym H;
   Plan P;
@@ -1185,6 +1188,10 @@ bool Engine::analyze(int n, const int *c, const int *r, const int64_t *lC, const
   const std::vector<int64_t> &rowptr = H.rowptr, &xptr = H.xptr;
   const int64_t nls = H.nls, xsize = H.xsize, nnz = H.nnz;
   const int nprune = H.nprune;
+
+  std::shared_ptr<FrontPlan> FP = std::make_shared<FrontPlan>();
+  build_front_plan(n, c, r, Ls, prunePtr, pruneSet, H, P, tuning_, *FP);
+  if (FP->ok) P.launches = FP->launches;
 
   // ---- solve plan: levels of the supernodal etree, per-level task lists ----
   SolvePlan SP;
@@ -1320,7 +1327,61 @@ bool Engine::analyze(int n, const int *c, const int *r, const int64_t *lC, const
   kmirror_len_ = kmirror_layout(H.super, H.rowptr, h_xk_);
   hsym_ = H;
   h_Ls_.assign(Ls, Ls + nls);
+  front_ = FP;
 
+  return true;
+}
+
+void Engine::release_front() {
+  void *ptrs[] = {d_fchild_ptr_, d_fchild_, d_fn1_, d_frel_, d_fapos_, d_fwarp_, d_fcta_, d_fsmall_,
+                  d_fext_end_, d_fsch_end_, d_fext_, d_fsch_, d_fext_pairs_, d_fsch_pairs_,
+                  d_fcb_off_, d_cb_};
+  for (void *p : ptrs)
+    if (p) cudaFree(p);
+  d_fchild_ptr_ = d_fchild_ = d_fn1_ = d_frel_ = d_fapos_ = d_fwarp_ = d_fcta_ = d_fsmall_ = nullptr;
+  d_fext_end_ = d_fsch_end_ = nullptr;
+  d_fext_ = d_fsch_ = d_fext_pairs_ = d_fsch_pairs_ = nullptr;
+  d_fcb_off_ = nullptr;
+  d_cb_ = nullptr;
+  front_.reset();
+  front_dev_.reset();
+  front_ready_ = front_tried_ = false;
+}
+
+// The multifrontal plan's tables and the contribution blocks on the device, on the first FP64
+// factorization of a structure; without the memory for them the left-looking kernels stay.
+bool Engine::prepare_front(std::string &err) {
+  if (front_tried_ || !front_ || !front_->ok) return true;
+  front_tried_ = true;
+  const FrontPlan &F = *front_;
+  cudaStream_t st = stream_;
+  if (cudaMalloc(&d_cb_, sizeof(double) * std::max<int64_t>(F.cb_len, 1)) != cudaSuccess) {
+    cudaGetLastError();
+    d_cb_ = nullptr;
+    return true;
+  }
+  if (!(upload(d_fchild_ptr_, F.child_ptr.data(), F.child_ptr.size(), st, err) &&
+        upload(d_fchild_, F.child.data(), F.child.size(), st, err) &&
+        upload(d_fn1_, F.child_n1.data(), F.child_n1.size(), st, err) &&
+        upload(d_frel_, F.rel.data(), F.rel.size(), st, err) &&
+        upload(d_fapos_, F.apos.data(), F.apos.size(), st, err) &&
+        upload(d_fwarp_, F.warp_list.data(), F.warp_list.size(), st, err) &&
+        upload(d_fcta_, F.cta_list.data(), F.cta_list.size(), st, err) &&
+        upload(d_fsmall_, F.small_list.data(), F.small_list.size(), st, err) &&
+        upload(d_fext_, F.ext_tasks.data(), F.ext_tasks.size(), st, err) &&
+        upload(d_fext_end_, F.ext_end.data(), F.ext_end.size(), st, err) &&
+        upload(d_fext_pairs_, F.ext_pairs.data(), F.ext_pairs.size(), st, err) &&
+        upload(d_fsch_, F.sch_tasks.data(), F.sch_tasks.size(), st, err) &&
+        upload(d_fsch_end_, F.sch_end.data(), F.sch_end.size(), st, err) &&
+        upload(d_fsch_pairs_, F.sch_pairs.data(), F.sch_pairs.size(), st, err) &&
+        upload(d_fcb_off_, F.cb_off.data(), F.cb_off.size(), st, err)))
+    return false;
+  if (cudaStreamSynchronize(st) != cudaSuccess) { err = "device upload: front plan"; return false; }
+  front_dev_ = std::make_shared<FrontDev>(
+      FrontDev{d_fchild_ptr_, d_fchild_, d_fn1_, d_frel_, d_fapos_, d_fcb_off_, d_cb_});
+  if (!F.warp_list.empty()) fwarp_ctas_ = front_warp_walk_ctas((int)F.warp_list.size());
+  if (!F.cta_list.empty()) fcta_ctas_ = front_cta_walk_ctas(F.cta_smem, (int)F.cta_list.size());
+  front_ready_ = true;
   return true;
 }
 
@@ -1359,22 +1420,37 @@ void Engine::launch_all(std::vector<std::pair<int, cudaEvent_t>> *prof, int prec
   cudaMemsetAsync(dL_, 0, sizeof(double) * xsize_, st);
   launch_init_status(d_status_, st);
   mark(-1, 1);
-  if (scatter && !plan_.asm_tasks.empty()) {
+  const bool front = prec == 0 && front_ready_;   // multifrontal
+  const FrontPlan *FP = front_.get();
+  if ((scatter || front) && !plan_.asm_tasks.empty()) {
     mark(K_ASSEMBLE, 1);
     launch_assemble(sym_, d_asm_, (int)plan_.asm_tasks.size(), st);
     mark(-1, 1);
   }
-  if (!plan_.tiny_list.empty() || !plan_.persist_list.empty())
+  if (front ? !FP->warp_list.empty() || !FP->cta_list.empty()
+            : !plan_.tiny_list.empty() || !plan_.persist_list.empty())
     cudaMemsetAsync(d_qctr_, 0, sizeof(int) * (nsuper_ + 2), st);
   if (d_dense_ver_) cudaMemsetAsync(d_dense_ver_, 0, sizeof(int) * dense_ver_len_, st);
-  if (!plan_.tiny_list.empty()) {
+  if (front && !FP->warp_list.empty()) {
+    mark(K_SMALL, 1);
+    launch_front_warp_walk(sym_, *front_dev_, d_fwarp_, (int)FP->warp_list.size(), fwarp_ctas_, d_qctr_,
+                           d_qctr_ + 1 + nsuper_, st);
+    mark(-1, 1);
+  }
+  if (front && !FP->cta_list.empty()) {
+    mark(K_SMALL, 1);
+    launch_front_cta_walk(sym_, *front_dev_, d_fcta_, (int)FP->cta_list.size(), FP->cta_smem,
+                          fcta_ctas_, d_qctr_, st);
+    mark(-1, 1);
+  }
+  if (!front && !plan_.tiny_list.empty()) {
     mark(K_SMALL, 1);
     launch_factor_tiny_persist(sym_, d_upd_lbub_, d_tiny_, (int)plan_.tiny_list.size(), tiny_ctas_,
                                d_qctr_,
                                d_qctr_ + 1 + nsuper_, st);
     mark(-1, 1);
   }
-  if (!plan_.persist_list.empty()) {
+  if (!front && !plan_.persist_list.empty()) {
     mark(K_SMALL, 1);
     launch_factor_small_persist(sym_, d_upd_lbub_, d_persist_, (int)plan_.persist_list.size(),
                                 plan_.persist_smem, persist_ctas_, d_qctr_, st);
@@ -1384,19 +1460,41 @@ void Engine::launch_all(std::vector<std::pair<int, cudaEvent_t>> *prof, int prec
     // the wave's small supernodes read only earlier waves' panels and write only their own,
     // so they run beside the wave's tiled work (updates and dense steps) on a second
     // stream, joined before the next wave (whose updates and supernodes read them)
-    const bool side = !prof && W.small_cnt > 0 && W.big_cnt > 0;
+    const FrontWave *FWv = front ? &FP->waves[&W - plan_.waves.data()] : nullptr;
+    const int small_cnt = front ? FWv->small_cnt : W.small_cnt;
+    const bool side = !prof && small_cnt > 0 && W.big_cnt > 0;
+    auto launch_small = [&](cudaStream_t on) {
+      if (front)
+        launch_front_small(sym_, *front_dev_, d_fsmall_ + FWv->small_off, small_cnt, FWv->small_smem, on);
+      else
+        launch_factor_small(sym_, d_upd_lbub_, d_small_ + W.small_off, W.small_cnt, W.small_smem, on);
+    };
     if (side) {
       cudaEventRecord(ev_sfork_, st);
       cudaStreamWaitEvent(small_stream_, ev_sfork_, 0);
-      launch_factor_small(sym_, d_upd_lbub_, d_small_ + W.small_off, W.small_cnt, W.small_smem,
-                          small_stream_);
+      launch_small(small_stream_);
       cudaEventRecord(ev_sjoin_, small_stream_);
     } else {
-      mark(K_SMALL, W.small_cnt);
-      launch_factor_small(sym_, d_upd_lbub_, d_small_ + W.small_off, W.small_cnt, W.small_smem, st);
-      mark(-1, W.small_cnt);
+      mark(K_SMALL, small_cnt);
+      launch_small(st);
+      mark(-1, small_cnt);
     }
-    if (scatter) {
+    // the end of the wave: its small supernodes joined, then (multifrontal) the tiles of its
+    // contribution blocks
+    auto finish_wave = [&]() {
+      if (side) cudaStreamWaitEvent(st, ev_sjoin_, 0);
+      if (!front) return;
+      mark(K_UPDATE, FWv->sch_cnt);
+      launch_front_schur(sym_, *front_dev_, d_fsch_ + FWv->sch_off, d_fsch_end_ + FWv->sch_off,
+                         d_fsch_pairs_, FWv->sch_cnt, st);
+      mark(-1, FWv->sch_cnt);
+    };
+    if (front) {
+      mark(K_ASSEMBLE, FWv->ext_cnt);
+      launch_front_extend(sym_, *front_dev_, d_fext_ + FWv->ext_off, d_fext_end_ + FWv->ext_off,
+                          d_fext_pairs_, FWv->ext_cnt, st);
+      mark(-1, FWv->ext_cnt);
+    } else if (scatter) {
       mark(K_UPDATE, W.scs_cnt);
       launch_scatter_small(sym_, d_sc_small_ + W.scs_off, W.scs_cnt, sc_cols, st);
       mark(-1, W.scs_cnt);
@@ -1424,7 +1522,7 @@ void Engine::launch_all(std::vector<std::pair<int, cudaEvent_t>> *prof, int prec
                            d_dense_toff_, d_dense_ver_ + plan_.waves.size(), d_dense_ver_ + wave,
                            st);
       mark(-1, 1);
-      if (side) cudaStreamWaitEvent(st, ev_sjoin_, 0);
+      finish_wave();
       continue;
     }
     mark(K_PANEL, W.big_cnt);
@@ -1474,7 +1572,7 @@ void Engine::launch_all(std::vector<std::pair<int, cudaEvent_t>> *prof, int prec
         syrk(W, (int)j);
       }
     }
-    if (side) cudaStreamWaitEvent(st, ev_sjoin_, 0);
+    finish_wave();
   }
 }
 
@@ -1526,7 +1624,7 @@ int Engine::factor(const double *values, bool values_on_device, int *info, std::
   if (prec < 0 || prec > 2) { err = "unknown precision mode"; return -1; }
   if (!dL_) { err = "factor before analyze"; return -1; }
   cudaSetDevice(device_);
-  if (!set_mode(prec, err)) return -1;
+  if (!set_mode(prec, err) || (prec == 0 && !prepare_front(err))) return -1;
   cudaStream_t st = stream_;
   // values always reach the kernels through d_Ax_, so a captured graph stays valid
   cudaError_t e = cudaMemcpyAsync(d_Ax_, values, sizeof(double) * nnz_,
@@ -1561,7 +1659,7 @@ int Engine::factor_profiled(const double *values, bool values_on_device, int *in
   if (prec < 0 || prec > 2) { err = "unknown precision mode"; return -1; }
   if (!dL_) { err = "factor before analyze"; return -1; }
   cudaSetDevice(device_);
-  if (!set_mode(prec, err)) return -1;
+  if (!set_mode(prec, err) || (prec == 0 && !prepare_front(err))) return -1;
   cudaStream_t st = stream_;
   cudaError_t e = cudaMemcpyAsync(d_Ax_, values, sizeof(double) * nnz_,
                                   values_on_device ? cudaMemcpyDeviceToDevice

@@ -246,6 +246,8 @@ void build_solve_plan(int n, const int *Ls, const HostSym &H, SolvePlan &SP);
 bool check_solve_plan(int n, const int *Ls, const HostSym &H, const SolvePlan &SP,
                       std::string &err);
 
+struct FrontPlan;     // multifrontal FP64 factorization (swc_front.h)
+struct FrontDev;
 struct AdjointPlan;   // reverse-sweep schedule of the adjoint (swc_adjoint.cu)
 
 class Engine {
@@ -330,6 +332,20 @@ class Engine {
   void release();
   void launch_all(std::vector<std::pair<int, cudaEvent_t>> *prof = nullptr, int prec = 0);
   bool set_mode(int prec, std::string &err);
+  // multifrontal FP64 factorization: the contribution blocks are allocated on first use; when
+  // the structure or the memory does not allow it, the left-looking kernels are used
+  std::shared_ptr<FrontPlan> front_;
+  std::shared_ptr<FrontDev> front_dev_;
+  bool front_ready_ = false, front_tried_ = false;
+  int *d_fchild_ptr_ = nullptr, *d_fchild_ = nullptr, *d_fn1_ = nullptr, *d_frel_ = nullptr;
+  int *d_fapos_ = nullptr, *d_fwarp_ = nullptr, *d_fcta_ = nullptr, *d_fsmall_ = nullptr;
+  int *d_fext_end_ = nullptr, *d_fsch_end_ = nullptr;
+  int4 *d_fext_ = nullptr, *d_fsch_ = nullptr, *d_fext_pairs_ = nullptr, *d_fsch_pairs_ = nullptr;
+  int64_t *d_fcb_off_ = nullptr;
+  double *d_cb_ = nullptr;
+  int fwarp_ctas_ = 0, fcta_ctas_ = 0;
+  bool prepare_front(std::string &err);
+  void release_front();
   int finish(int *info, std::string &err);
   int64_t h2d_bytes_ = 0, d2h_bytes_ = 0;
   int wait_budget_ = kDefaultWaitBudget;

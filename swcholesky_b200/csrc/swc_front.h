@@ -1,0 +1,107 @@
+// Multifrontal FP64 factorization: plan (host) and launches.
+//
+// Every supernode s passes ONE dense contribution block to its parent in the supernodal
+// elimination tree: CB_s = (contribution blocks of s's children, at s's off-diagonal rows)
+// - L_rs L_rs^T, over the r = m - w off-diagonal rows of s (lower triangle, column-major,
+// leading dimension r).  A front is assembled from A and the two or three blocks of its
+// children instead of from every descendant that touches it (the prune set: up to hundreds
+// of narrow panels per supernode, each located by its own row search), and every product is
+// a dense one over contiguous rows.  Blocks are added in child order: no atomics, and the
+// factor is reproducible bit for bit.  Against the left-looking kernels (B200, ms per
+// factorization): 5-point grids 20 x 20 0.50 -> 0.13, 100 x 100 1.81 -> 0.42; 7-point grids
+// 41 x 37 x 43 5.43 -> 3.41, 60^3 24.7 -> 16.3 (the descendants' updates 16.3 -> 6.4);
+// 3-unknown 27-point grid 24 x 23 x 22 5.56 -> 3.60.  The blocks alive at once take about as
+// much memory as L; the left-looking kernels remain for handles that cannot have it, for prune
+// sets that are not the complete descendant lists, and for the mixed modes.
+#pragma once
+#include <cuda_runtime.h>
+
+#include <cstdint>
+#include <string>
+#include <vector>
+
+#include "swc_engine.h"
+
+namespace swc {
+
+// Fronts done by one warp: padded panel of at most FRONT_WARP_ELEMS doubles, at most
+// FRONT_WARP_R off-diagonal rows.
+constexpr int FRONT_WARP_ELEMS = 1280;
+constexpr int FRONT_WARP_M = 128;
+constexpr int FRONT_KIDS = 4;   // children whose row maps are held at a time
+
+// Padded front in shared memory: the w columns padded to a multiple of 8 (identity), the
+// off-diagonal rows below them, and a leading dimension of 4 mod 16 doubles, with which the
+// 8x8 DMMA operand loads meet no bank conflict.
+__host__ __device__ inline int front_wp(int w) { return (w + 7) & ~7; }
+__host__ __device__ inline int front_ld(int w, int m) {
+  const int rows = front_wp(w) + ((m - w + 7) & ~7);
+  return rows + ((4 - rows) & 15);
+}
+inline int64_t front_smem(int w, int64_t m) {
+  return 8LL * front_wp(w) * front_ld(w, (int)m) + 8 * 64 + 2LL * FRONT_KIDS * ((m + 3) & ~3LL);
+}
+
+// Device view of the plan.
+struct FrontDev {
+  const int *child_ptr, *child;   // children of each supernode, in increasing order
+  const int *child_n1;            // per supernode: its rows that are columns of its parent
+  const int *rel;                 // per off-diagonal row (at rowptr[s] - super[s]): position in
+                                  // the parent's row list
+  const int *apos;                // per entry of A: position in its column's row list (-1: none)
+  const int64_t *cb_off;          // per supernode: its contribution block in cb
+  double *cb;
+};
+
+struct FrontWave {
+  int small_off = 0, small_cnt = 0, small_smem = 0;
+  int ext_off = 0, ext_cnt = 0;    // tiles of tiled panels that receive children's blocks
+  int sch_off = 0, sch_cnt = 0;    // tiles of contribution blocks
+};
+
+struct FrontPlan {
+  bool ok = false;                 // the structure allows it (see build_front_plan)
+  std::vector<int> child_ptr, child, child_n1, rel, apos;
+  std::vector<int64_t> cb_off;
+  int64_t cb_len = 0;              // doubles of contribution blocks alive at once
+  std::vector<int> warp_list;      // fronts of the warp walk, in level order
+  std::vector<int> cta_list;       // fronts of the CTA walk, in level order
+  int cta_smem = 0;
+  std::vector<int> small_list;     // per wave; ~s: its contribution block is formed by tiles
+  std::vector<FrontWave> waves;
+  std::vector<int4> ext_tasks, sch_tasks;   // (s, r0, c0, first pair)
+  std::vector<int> ext_end, sch_end;        // one past the last pair
+  std::vector<int4> ext_pairs, sch_pairs;   // (child, a0, b0, na | nb << 16)
+  int launches = 0;
+};
+
+// Derives the multifrontal plan of an analysed structure.  P.ok stays false, and the
+// left-looking kernels are used, when the prune sets are not exactly the descendants that
+// touch each supernode or a child's rows are not among its parent's.
+void build_front_plan(int n, const int *c, const int *r, const int *Ls, const int *prunePtr,
+                      const int *pruneSet, const HostSym &H, const Plan &P, const Tuning &T,
+                      FrontPlan &F);
+
+// Host check of a multifrontal plan: every front factored once, after its children; every
+// entry of every child's block added once (to the panel by the front's own launch or by a
+// panel tile, to the parent's block likewise); every block tile formed once; the shared memory
+// of every launch sufficient; no two blocks alive in one place.  False with a message on the
+// first violation (true for a plan that is not ok).
+bool check_front_plan(int n, const int *Ls, const HostSym &H, const Plan &P, const FrontPlan &F,
+                      std::string &err);
+
+bool front_configure(std::string &err);
+int front_cta_walk_ctas(int smem, int count);
+int front_warp_walk_ctas(int count);
+void launch_front_warp_walk(const DevSym &S, const FrontDev &F, const int *order, int count,
+                            int ctas, int *qctr, int *qhead, cudaStream_t st);
+void launch_front_cta_walk(const DevSym &S, const FrontDev &F, const int *order, int count,
+                           int smem, int ctas, int *qctr, cudaStream_t st);
+void launch_front_small(const DevSym &S, const FrontDev &F, const int *list, int count, int smem,
+                        cudaStream_t st);
+void launch_front_extend(const DevSym &S, const FrontDev &F, const int4 *tasks, const int *end,
+                         const int4 *pairs, int count, cudaStream_t st);
+void launch_front_schur(const DevSym &S, const FrontDev &F, const int4 *tasks, const int *end,
+                        const int4 *pairs, int count, cudaStream_t st);
+
+}  // namespace swc
