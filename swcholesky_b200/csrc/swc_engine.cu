@@ -164,7 +164,7 @@ void Engine::release() {
   void *ptrs[] = {d_super_, d_Ls_, d_Ap_, d_Ai_, d_rowptr_, d_xptr_, d_upd_ptr_, d_upd_, d_upd_lbub_,
                   d_Ax_, dL_, d_status_, d_small_, d_big_, d_asm_, d_panel_, d_upd_tasks_,
                   d_syrk_, d_pairs_, d_upd_end_, d_dinv_, d_dinv_off_, d_diag_,
-                  d_slist_, d_cptr_, d_cidx_, d_flags_, d_fchain_, d_bchain_, d_scontrib_, d_sgather_, d_csr_rp_, d_csr_ci_,
+                  d_slist_, d_cptr_, d_cidx_, d_flags_, d_fchain_, d_bchain_, d_scontrib_, d_sgather_, d_c8_tasks_, d_g8_tasks_, d_csr_rp_, d_csr_ci_,
                   d_csr_map_,
                   d_csr_val_, d_contrib_, d_work_, d_norms_, d_persist_, d_qctr_, d_npart_,
                   d_tiny_, d_dense_tasks_, d_dense_toff_, d_dense_ver_, d_swarp_,
@@ -194,7 +194,7 @@ void Engine::release() {
   d_slist_ = d_cptr_ = d_cidx_ = d_flags_ = nullptr;
   d_swarp_ = nullptr;
   d_fchain_ = d_bchain_ = nullptr;
-  d_scontrib_ = d_sgather_ = nullptr;
+  d_scontrib_ = d_sgather_ = d_c8_tasks_ = d_g8_tasks_ = nullptr;
   d_csr_rp_ = d_csr_ci_ = d_csr_map_ = nullptr;
   d_csr_val_ = d_contrib_ = d_work_ = d_norms_ = nullptr;
   d_persist_ = d_qctr_ = d_tiny_ = nullptr;
@@ -214,8 +214,10 @@ void Engine::release() {
   d_npart_ = nullptr;
   persist_ctas_ = 0;
   release_solve_graphs();
-  if (d_sx_) cudaFree(d_sx_);
-  d_sx_ = nullptr;
+  for (double **p : {&d_sx_, &d_x8_, &d_c8_}) {
+    if (*p) cudaFree(*p);
+    *p = nullptr;
+  }
   work_nrhs_ = 0;
   for (int k = 0; k < 3; ++k) {
     if (graph_exec_[k]) cudaGraphExecDestroy(graph_exec_[k]);
@@ -959,6 +961,21 @@ void build_solve_plan(int n, const int *Ls, const HostSym &H, SolvePlan &SP) {
     SP.chain_off.push_back((int)SP.fchain.size());
     SP.contrib_off.push_back((int)SP.contrib_tasks.size());
     SP.gather_off.push_back((int)SP.gather_tasks.size());
+    SP.c8_off.push_back((int)SP.c8_tasks.size());
+    SP.g8_off.push_back((int)SP.g8_tasks.size());
+    {
+      int64_t nt = 0;
+      for (int s : bylev[l])
+        if (H.dinv_off[s] >= 0) nt += (rowptr[s + 1] - rowptr[s] - (super[s + 1] - super[s]) + 127) / 128;
+      const bool split = nt < SOLVE8_FULL_TASKS;
+      SP.c8_split.push_back(split);
+      for (int s : bylev[l]) {
+        if (H.dinv_off[s] < 0) continue;
+        const int w = super[s + 1] - super[s], m = (int)(rowptr[s + 1] - rowptr[s]);
+        for (int r0 = w; r0 < m; r0 += split ? 32 : 128) SP.c8_tasks.push_back(make_int2(s, r0));
+        for (int j0 = 0; j0 < w && m > w; j0 += SOLVE_GATHER_COLS) SP.g8_tasks.push_back(make_int2(s, j0));
+      }
+    }
     std::vector<int2> narrow, wide;
     // 128-row tasks of 8 warps for the wide supernodes only when the level has enough of
     // them to fill the GPU; otherwise 32-row tasks of 32 warps (more, shorter CTAs)
@@ -1002,6 +1019,8 @@ void build_solve_plan(int n, const int *Ls, const HostSym &H, SolvePlan &SP) {
   SP.chain_off.push_back((int)SP.fchain.size());
   SP.contrib_off.push_back((int)SP.contrib_tasks.size());
   SP.gather_off.push_back((int)SP.gather_tasks.size());
+  SP.c8_off.push_back((int)SP.c8_tasks.size());
+  SP.g8_off.push_back((int)SP.g8_tasks.size());
   SP.contrib_len = nls - n;
   // column contribution lists: off-diagonal row a of supernode d (a >= w_d) feeds column
   // Ls[a] through contribution (rowptr[d] - super[d]) + (a - w_d)
@@ -1169,6 +1188,22 @@ bool check_solve_plan(int n, const int *Ls, const HostSym &H, const SolvePlan &S
       if (level[p] <= level[s]) return bad("a parent not in a later level");
     }
   }
+  // eight right-hand sides: the tiled supernodes' rows and column groups, each once, in order
+  for (int l = 0; l < nl; ++l) {
+    const int span = SP.c8_split[l] ? 32 : 128;
+    int c = SP.c8_off[l], g = SP.g8_off[l];
+    for (int k = SP.chain_off[l]; k < SP.chain_off[l + 1]; ++k) {
+      if (SP.fchain[k].y != 0) continue;
+      const int s = SP.fchain[k].x, w = super[s + 1] - super[s], m = (int)(rowptr[s + 1] - rowptr[s]);
+      for (int r0 = w; r0 < m; r0 += span, ++c)
+        if (c >= SP.c8_off[l + 1] || SP.c8_tasks[c].x != s || SP.c8_tasks[c].y != r0)
+          return bad("contribution tasks of eight right-hand sides");
+      for (int j0 = 0; j0 < w && m > w; j0 += SOLVE_GATHER_COLS, ++g)
+        if (g >= SP.g8_off[l + 1] || SP.g8_tasks[g].x != s || SP.g8_tasks[g].y != j0)
+          return bad("gather tasks of eight right-hand sides");
+    }
+    if (c != SP.c8_off[l + 1] || g != SP.g8_off[l + 1]) return bad("tasks of eight right-hand sides left over");
+  }
   return check_solve_tasks(n, Ls, H, SP, level, by_warp, err);
 }
 
@@ -1196,7 +1231,7 @@ bool Engine::analyze(int n, const int *c, const int *r, const int64_t *lC, const
   // ---- solve plan: levels of the supernodal etree, per-level task lists ----
   SolvePlan SP;
   build_solve_plan(n, Ls, H, SP);
-  if (!solve_configure(SP.max_w, err)) return false;
+  if (!solve_configure(SP.max_w, err) || !solve8_configure(err)) return false;
   // ---- full CSR of the symmetric matrix for residuals: entry -> index into A2 values ----
   std::vector<int> csr_rp(n + 1, 0), csr_ci, csr_map;
   {
@@ -1265,6 +1300,8 @@ bool Engine::analyze(int n, const int *c, const int *r, const int64_t *lC, const
             upload(d_fchain_, SP.fchain.data(), SP.fchain.size(), st, err) &&
             upload(d_bchain_, SP.bchain.data(), SP.bchain.size(), st, err) &&
             upload(d_scontrib_, SP.contrib_tasks.data(), SP.contrib_tasks.size(), st, err) &&
+            upload(d_c8_tasks_, SP.c8_tasks.data(), SP.c8_tasks.size(), st, err) &&
+            upload(d_g8_tasks_, SP.g8_tasks.data(), SP.g8_tasks.size(), st, err) &&
             upload(d_sgather_, SP.gather_tasks.data(), SP.gather_tasks.size(), st, err) &&
             upload(d_csr_rp_, csr_rp.data(), csr_rp.size(), st, err) &&
             upload(d_csr_ci_, csr_ci.data(), csr_ci.size(), st, err) &&
@@ -1747,21 +1784,23 @@ double *Engine::staging(size_t doubles, std::string &err) {
 bool Engine::ensure_work(int nrhs, std::string &err) {
   if (nrhs <= work_nrhs_) return true;
   release_solve_graphs();   // they hold the old buffers
-  if (d_sx_) cudaFree(d_sx_);
-  d_sx_ = nullptr;
-  if (d_contrib_) cudaFree(d_contrib_);
-  if (d_work_) cudaFree(d_work_);
-  if (d_norms_) cudaFree(d_norms_);
+  for (double **p : {&d_sx_, &d_x8_, &d_c8_, &d_contrib_, &d_work_, &d_norms_, &d_npart_}) {
+    if (*p) cudaFree(*p);
+    *p = nullptr;
+  }
   if (h_norms_) cudaFreeHost(h_norms_);
-  if (d_npart_) cudaFree(d_npart_);
-  d_contrib_ = d_work_ = d_norms_ = h_norms_ = d_npart_ = nullptr;
-  cudaError_t e = cudaMalloc(&d_contrib_, sizeof(double) * std::max<int64_t>(splan_.contrib_len, 1) * nrhs);
+  h_norms_ = nullptr;
+  // one vector, and (several right-hand sides) eight interleaved ones with their contributions
+  const size_t clen = (size_t)std::max<int64_t>(splan_.contrib_len, 1);
+  cudaError_t e = cudaMalloc(&d_contrib_, sizeof(double) * clen);
+  if (e == cudaSuccess) e = cudaMalloc(&d_sx_, sizeof(double) * (size_t)n_);
+  if (e == cudaSuccess && nrhs > 1) e = cudaMalloc(&d_x8_, sizeof(double) * 8 * (size_t)n_);
+  if (e == cudaSuccess && nrhs > 1) e = cudaMalloc(&d_c8_, sizeof(double) * 8 * clen);
   // work: r, d, p, q vectors (4 * n * nrhs) + row sums
   if (e == cudaSuccess) e = cudaMalloc(&d_work_, sizeof(double) * ((size_t)4 * n_ * nrhs + n_));
   if (e == cudaSuccess) e = cudaMalloc(&d_norms_, sizeof(double) * 8 * (nrhs + 1));
   if (e == cudaSuccess) e = cudaMallocHost(&h_norms_, sizeof(double) * 8 * (nrhs + 1));
   if (e == cudaSuccess) e = cudaMalloc(&d_npart_, sizeof(double) * norm_scratch_doubles(nrhs));
-  if (e == cudaSuccess) e = cudaMalloc(&d_sx_, sizeof(double) * (size_t)n_ * nrhs);
   if (e != cudaSuccess) {
     err = std::string("solve workspace: ") + cudaGetErrorString(e);
     work_nrhs_ = 0;
@@ -1772,44 +1811,66 @@ bool Engine::ensure_work(int nrhs, std::string &err) {
 }
 
 void Engine::release_solve_graphs() {
-  for (auto &g : solve_graphs_) cudaGraphExecDestroy(g.second);
-  solve_graphs_.clear();
+  for (cudaGraphExec_t &g : solve_graph_) {
+    if (g) cudaGraphExecDestroy(g);
+    g = nullptr;
+  }
 }
 
-// The solve of nrhs right-hand sides held in d_sx_ as one CUDA graph (its launch sequence
-// and buffers are fixed by the structure and nrhs); captured on first use, nullptr when the
-// capture fails (the caller then launches directly).
-cudaGraphExec_t Engine::solve_graph(int nrhs) {
-  for (auto &g : solve_graphs_)
-    if (g.first == nrhs) return g.second;
+// The solve of the vector in d_sx_, or of the eight interleaved ones in d_x8_, as one CUDA
+// graph (its launch sequence and buffers are fixed by the structure); captured on first use,
+// nullptr when the capture fails (the caller then launches directly).
+cudaGraphExec_t Engine::solve_graph(bool eight) {
+  cudaGraphExec_t &exec = solve_graph_[eight];
+  if (exec) return exec;
   cudaStream_t st = stream_;
   cudaGraph_t graph = nullptr;
-  cudaGraphExec_t exec = nullptr;
   if (cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal) != cudaSuccess) return nullptr;
-  run_solve_with(d_sx_, nrhs, d_contrib_);
+  if (eight) run_solve8(d_x8_);
+  else run_solve_with(d_sx_, 1, d_contrib_);
   cudaError_t e = cudaStreamEndCapture(st, &graph);
   if (e == cudaSuccess) e = cudaGraphInstantiate(&exec, graph, 0);
   if (graph) cudaGraphDestroy(graph);
   if (e != cudaSuccess) {
     cudaGetLastError();
-    return nullptr;
+    exec = nullptr;
   }
-  solve_graphs_.emplace_back(nrhs, exec);
   return exec;
 }
 
-// x := (L L^T)^{-1} x for device x (n x nrhs): the solve graph on a copy of x in d_sx_,
-// or direct launches without graphs.
+void Engine::run_solve8(double *x8) {
+  cudaMemsetAsync(d_flags_, 0, sizeof(int) * std::max<int64_t>(nflags_, 1), stream_);
+  const Solve8Dev D{d_slist_, d_swarp_, d_cptr_, d_cidx_, d_fchain_, d_bchain_, d_c8_tasks_,
+                    d_g8_tasks_, d_flags_};
+  launch_solve8(sym_, splan_, D, x8, d_c8_, stream_);
+}
+
+// x := (L L^T)^{-1} x for device x (n x nrhs), eight right-hand sides at a time (a single one
+// by the kernels for one vector): the solve graph on a copy of x, or direct launches without
+// graphs.  The caller clears status[2] once: a wait that times out stays recorded whatever
+// solves follow.
 void Engine::run_solve(double *x, int nrhs) {
-  cudaGraphExec_t g = use_graph_ ? solve_graph(nrhs) : nullptr;
-  if (!g) {
-    run_solve_with(x, nrhs, d_contrib_);
-    return;
+  for (int r0 = 0; r0 < nrhs; r0 += 8) {
+    const int nr = std::min(8, nrhs - r0);
+    double *xr = x + (size_t)r0 * n_;
+    if (nr == 1) {
+      cudaGraphExec_t g = use_graph_ ? solve_graph(false) : nullptr;
+      if (!g) {
+        run_solve_with(xr, 1, d_contrib_);
+      } else {
+        const size_t bytes = sizeof(double) * (size_t)n_;
+        cudaMemcpyAsync(d_sx_, xr, bytes, cudaMemcpyDeviceToDevice, stream_);
+        cudaGraphLaunch(g, stream_);
+        cudaMemcpyAsync(xr, d_sx_, bytes, cudaMemcpyDeviceToDevice, stream_);
+      }
+    } else {
+      launch_pack8(n_, nr, xr, d_x8_, stream_);
+      cudaGraphExec_t g = use_graph_ ? solve_graph(true) : nullptr;
+      if (g) cudaGraphLaunch(g, stream_);
+      else run_solve8(d_x8_);
+      launch_unpack8(n_, nr, d_x8_, xr, stream_);
+    }
   }
-  const size_t bytes = sizeof(double) * (size_t)n_ * nrhs;
-  cudaMemcpyAsync(d_sx_, x, bytes, cudaMemcpyDeviceToDevice, stream_);
-  cudaGraphLaunch(g, stream_);
-  cudaMemcpyAsync(x, d_sx_, bytes, cudaMemcpyDeviceToDevice, stream_);
 }
 
 // Forward then backward supernodal solve, level by level, with the contribution scratch
@@ -1826,7 +1887,6 @@ void Engine::run_solve_with(double *x, int nrhs, double *contrib) {
   const int64_t cs = std::max<int64_t>(SP.contrib_len, 1);
   const int base = 0;
   cudaMemsetAsync(d_flags_, 0, sizeof(int) * std::max<int64_t>(nflags_, 1), st);
-  cudaMemsetAsync(d_status_ + 2, 0, sizeof(int), st);
   for (int l = 0; l < nl; ++l) {
     launch_fwd_warp(sym_, d_swarp_ + SP.warp_off[l], SP.warp_off[l + 1] - SP.warp_off[l], x,
                     contrib, d_cptr_, d_cidx_, n_, nrhs, cs, st);
@@ -1870,6 +1930,7 @@ bool Engine::solve(const double *b, double *x, int nrhs, std::string &err) {
   if (!ensure_work(nrhs, err)) return false;
   cudaError_t e = cudaSuccess;
   if (x != b) e = cudaMemcpyAsync(x, b, sizeof(double) * n_ * nrhs, cudaMemcpyDeviceToDevice, stream_);
+  if (e == cudaSuccess) e = cudaMemsetAsync(d_status_ + 2, 0, sizeof(int), stream_);
   if (e != cudaSuccess) { err = std::string("solve: ") + cudaGetErrorString(e); return false; }
   run_solve(x, nrhs);
   e = cudaStreamSynchronize(stream_);
@@ -1893,6 +1954,7 @@ bool Engine::refine(const double *b, double *x, int nrhs, double tol, int maxit,
     if (e != cudaSuccess) { err = std::string("refine: ") + cudaGetErrorString(e); return false; }
     return true;
   };
+  cudaMemsetAsync(d_status_ + 2, 0, sizeof(int), st);
   // ||A||_inf
   launch_rowabs(n_, d_csr_rp_, d_csr_val_, rows, st);
   launch_norms(n_, 1, rows, nullptr, d_norms_, d_npart_, st);
@@ -1997,6 +2059,7 @@ bool Engine::solve_in_scratch(const double *b, double *x, int nrhs, double *scra
   cudaStream_t st = stream_;
   cudaError_t e = cudaSuccess;
   if (x != b) e = cudaMemcpyAsync(x, b, sizeof(double) * n_ * nrhs, cudaMemcpyDeviceToDevice, st);
+  if (e == cudaSuccess) e = cudaMemsetAsync(d_status_ + 2, 0, sizeof(int), st);
   if (e != cudaSuccess) { err = std::string("solve: ") + cudaGetErrorString(e); return false; }
   run_solve_with(x, nrhs, scratch);
   e = cudaStreamSynchronize(st);

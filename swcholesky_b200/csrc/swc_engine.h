@@ -195,10 +195,27 @@ struct SolvePlan {
   std::vector<int2> contrib_tasks;
   std::vector<int> gather_off;      // (s, j0) tasks of level l
   std::vector<int2> gather_tasks;
+  // several right-hand sides at a time: the tiled supernodes' tasks of level l
+  std::vector<int> c8_off, c8_split;  // (s, r0) contribution tasks: 128 rows, or (c8_split[l]) 32
+  std::vector<int2> c8_tasks;
+  std::vector<int> g8_off;            // (s, j0) gather tasks, 16 columns
+  std::vector<int2> g8_tasks;
   int max_w = 0;
   int64_t contrib_len = 0;          // off-diagonal rows in total (one contribution each)
   std::vector<int> cptr, cidx;      // per column: contributions it receives (CSR)
 };
+
+// Solves of up to eight right-hand sides at a time, vectors interleaved by eight (swc_solve8.cu)
+struct Solve8Dev {
+  const int *list, *warp_list, *cptr, *cidx;
+  const int2 *fchain, *bchain, *c8_tasks, *g8_tasks;
+  int *flags;   // the chained blocks' counters, zeroed before the solve
+};
+bool solve8_configure(std::string &err);
+void launch_pack8(int n, int nr, const double *x, double *x8, cudaStream_t st);
+void launch_unpack8(int n, int nr, const double *x8, double *x, cudaStream_t st);
+void launch_solve8(const DevSym &S, const SolvePlan &SP, const Solve8Dev &D, double *x8, double *c8,
+                   cudaStream_t st);
 
 // Result of a refined solve, per right-hand side.
 struct RefineInfo {
@@ -405,8 +422,11 @@ class Engine {
   int2 *d_fchain_ = nullptr, *d_bchain_ = nullptr;
   int64_t nflags_ = 0;
   double *d_sx_ = nullptr;                                         // solve graphs' vectors
-  std::vector<std::pair<int, cudaGraphExec_t>> solve_graphs_;      // per nrhs
-  cudaGraphExec_t solve_graph(int nrhs);
+  double *d_x8_ = nullptr, *d_c8_ = nullptr;                       // the same, interleaved by eight
+  int2 *d_c8_tasks_ = nullptr, *d_g8_tasks_ = nullptr;
+  cudaGraphExec_t solve_graph_[2] = {nullptr, nullptr};            // one vector; eight
+  cudaGraphExec_t solve_graph(bool eight);
+  void run_solve8(double *x8);
   void release_solve_graphs();
   int2 *d_scontrib_ = nullptr, *d_sgather_ = nullptr;
   int *d_csr_rp_ = nullptr, *d_csr_ci_ = nullptr, *d_csr_map_ = nullptr;

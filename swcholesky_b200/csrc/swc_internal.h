@@ -70,6 +70,9 @@ constexpr int SOLVE_NARROW_W = 64;   // contribution tasks of supernodes this na
 constexpr int SOLVE_WARP_W = 32;
 constexpr int SOLVE_WARP_ROWS = 256;
 constexpr int SOLVE_WARP_LEVEL_MIN = 4096;
+// Several right-hand sides: contribution tasks of 128 rows on levels with at least one per SM,
+// else 32-row tasks whose warps split the columns.
+constexpr int SOLVE8_FULL_TASKS = 148;
 
 // Size classes of the executor (the B200 counterpart of the reference's triple queue,
 // cholesky/tripleQueue.c:17-170): a supernode whose whole panel fits in shared memory is

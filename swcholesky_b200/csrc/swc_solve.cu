@@ -8,6 +8,7 @@
 #include <cstdint>
 
 #include "swc_engine.h"
+#include "swc_chain.h"
 
 namespace swc {
 
@@ -409,50 +410,6 @@ __global__ void __launch_bounds__(ST) k_bwd_diag(DevSym S, const int *list, doub
 // bounded: after the poll budget in status[4] a waiter records a timeout in status[2] and
 // stops waiting.
 constexpr int CHAIN_WARPS = ST / 32;
-__device__ __forceinline__ int ld_acquire(const int *p) {
-  int v;
-  asm volatile("ld.acquire.gpu.global.s32 %0, [%1];\n" : "=r"(v) : "l"(p));
-  return v;
-}
-__device__ __forceinline__ void red_release_add(int *p, int v) {
-  asm volatile("red.release.gpu.global.add.s32 [%0], %1;\n" ::"l"(p), "r"(v) : "memory");
-}
-
-// Lane u < nf polls the counter at flag + dir * u (no sleep between polls: a hop between
-// clusters is on the chain's critical path) until the first one has reached `target`;
-// returns how many consecutive counters from the first have reached it (1 .. nf), or 0
-// after a timeout (its own, or one another block recorded).  A batch is never held back
-// by a block that is not finished yet.
-__device__ int warp_wait_prefix(const int *flag, int dir, int nf, int target, int *status) {
-  const long long budget = wait_budget(status);
-  long long it = 0;
-  const int lane = threadIdx.x & 31;
-  bool mine = lane < nf && ld_acquire(flag + dir * lane) >= target;
-  int n = 0;
-  for (;;) {
-    const unsigned done = __ballot_sync(0xffffffffu, mine);
-    n = min(nf, __ffs(~done) - 1);
-    if (n > 0) break;
-    if (++it > budget || ((it & 31) == 0 && *(volatile int *)&status[2])) {
-      if (lane == 0) atomicExch(&status[2], 1);
-      break;
-    }
-    if (lane < nf && !mine) mine = ld_acquire(flag + dir * lane) >= target;
-  }
-  __syncwarp();   // the lanes' later loads are ordered after the polling lanes' acquires
-  return n;
-}
-
-template <int N>
-__device__ __forceinline__ void stage_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N)); }
-// an empty cp.async group (keeps one group per ring step)
-__device__ __forceinline__ void stage_commit() { asm volatile("cp.async.commit_group;\n" ::); }
-__device__ __forceinline__ void cp8(double *dst, const double *src, bool in) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(
-                   (unsigned)__cvta_generic_to_shared(dst)),
-               "l"(src), "r"(in ? 8 : 0));
-}
-
 // ---- chained dense solves with the diagonal block of a tiled-class supernode -----------
 // One CTA per 64-row block k of the diagonal block; block k consumes the solved blocks
 // c < k (forward) or c > k (backward) as they arrive and applies its own block through the
@@ -499,36 +456,6 @@ struct ChainCluster {
   unsigned long long bar[CHAIN_CL];
 };
 
-__device__ __forceinline__ uint32_t chain_rank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;\n" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;\n" ::
-                   : "memory");
-}
-__device__ __forceinline__ uint32_t smem_addr(const void *p) {
-  return (uint32_t)__cvta_generic_to_shared(p);
-}
-// address of the same shared-memory location in the CTA of cluster rank `rank`
-__device__ __forceinline__ uint32_t cluster_addr(const void *p, uint32_t rank) {
-  uint32_t r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(r) : "r"(smem_addr(p)), "r"(rank));
-  return r;
-}
-__device__ __forceinline__ void chain_cluster_init(ChainCluster &cc) {
-  if (threadIdx.x == 0) {
-    for (int j = 0; j < CHAIN_CL; ++j) {
-      const uint32_t b = smem_addr(&cc.bar[j]);
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(b) : "memory");
-      asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(b), "r"(TB * 8)
-                   : "memory");
-    }
-    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
-  }
-  cluster_sync_all();
-}
 // Lane l (holding element `row` of this block's solution when (l & 3) == 0; every lane of
 // quad l >> 2 holds it) sends it to the later ranks me+1 .. last of its cluster, the four
 // lanes of a quad to different ranks.
@@ -539,31 +466,6 @@ __device__ __forceinline__ void chain_send(ChainCluster &cc, int me, int last, i
                  "d"(val), "r"(cluster_addr(&cc.bar[me], q))
                  : "memory");
 }
-// Every lane waits (bounded) for slot j's 512 bytes; false after a timeout (its own, or
-// one another block recorded) in any lane.
-__device__ bool warp_chain_recv(ChainCluster &cc, int j, int *status) {
-  const uint32_t b = smem_addr(&cc.bar[j]);
-  const long long budget = wait_budget(status);
-  long long it = 0;
-  int ok = 1;
-  for (;;) {
-    uint32_t done;
-    asm volatile(
-        "{\n\t.reg .pred P1;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 P1, [%1], 0;\n\t"
-        "selp.b32 %0, 1, 0, P1;\n\t}\n"
-        : "=r"(done)
-        : "r"(b)
-        : "memory");
-    if (done) break;
-    if (++it > budget || ((it & 31) == 0 && *(volatile int *)&status[2])) {
-      atomicExch(&status[2], 1);
-      ok = 0;
-      break;
-    }
-  }
-  return __all_sync(0xffffffffu, ok) != 0;
-}
-
 // Sum over the lanes of a[i] (this lane's part of row 8w + i): the total of row
 // 8w + ((lane >> 2) & 7), in every lane of the quad.
 __device__ __forceinline__ double warp_rows8(double (&a)[8], int lane) {
@@ -602,7 +504,7 @@ __global__ void __launch_bounds__(ST, NS == CHAIN_NS_SMALL ? 2 : 1) k_fwd_chain(
   extern __shared__ double csm[];
   __shared__ double vs[TB], part[CHAIN_WARPS][TB];
   __shared__ ChainCluster cc;
-  chain_cluster_init(cc);
+  cluster_bars_init(cc.bar, CHAIN_CL, TB * 8);
   const int me = (int)chain_rank();
   if ((int)blockIdx.x < count) {
     const int s = tasks[blockIdx.x].x, k = tasks[blockIdx.x].y;
@@ -670,7 +572,7 @@ __global__ void __launch_bounds__(ST, NS == CHAIN_NS_SMALL ? 2 : 1) k_fwd_chain(
       const double *xc;                  // x_c(8w + q) at xc[q]
       if (c >= cfirst) {   // from the cluster
         const int j = me - (k - c);
-        if (!warp_chain_recv(cc, j, S.status)) { ok = false; break; }
+        if (!warp_bar_recv(&cc.bar[j], S.status)) { ok = false; break; }
         xc = &cc.yin[j][w8];
       } else {             // from global memory, a batch of finished blocks at a time
         if (c >= xb0 + nbt) {
@@ -730,7 +632,7 @@ __global__ void __launch_bounds__(ST, NS == CHAIN_NS_SMALL ? 2 : 1) k_bwd_chain(
   extern __shared__ double csm[];
   __shared__ double vs[TB];
   __shared__ ChainCluster cc;
-  chain_cluster_init(cc);
+  cluster_bars_init(cc.bar, CHAIN_CL, TB * 8);
   const int me = (int)chain_rank();
   if ((int)blockIdx.x < count) {
     const int s = tasks[blockIdx.x].x, k = tasks[blockIdx.x].y;
@@ -791,7 +693,7 @@ __global__ void __launch_bounds__(ST, NS == CHAIN_NS_SMALL ? 2 : 1) k_bwd_chain(
       double x0, x1;
       if (c <= clast) {   // from the cluster
         const int j = me - (c - k);
-        if (!warp_chain_recv(cc, j, S.status)) { ok = false; break; }
+        if (!warp_bar_recv(&cc.bar[j], S.status)) { ok = false; break; }
         x0 = cc.yin[j][lane];
         x1 = cc.yin[j][lane + 32];
       } else {            // from global memory, a batch of blocks c, c - 1, .. at a time
@@ -852,14 +754,25 @@ __global__ void __launch_bounds__(256) k_spmv(int n, const int *rp, const int *c
   const int sub = threadIdx.x & 7;
   const bool ok = row < n;
   const int p0 = ok ? rp[row] : 0, p1 = ok ? rp[row + 1] : 0;
-  for (int r = 0; r < nrhs; ++r) {
-    const double *xr = x + (size_t)r * n;
-    double acc = 0.0;
-    for (int p = p0 + sub; p < p1; p += 8) acc = fma(val[p], xr[ci[p]], acc);
-    acc += __shfl_xor_sync(0xffffffffu, acc, 4);
-    acc += __shfl_xor_sync(0xffffffffu, acc, 2);
-    acc += __shfl_xor_sync(0xffffffffu, acc, 1);
-    if (ok && sub == 0) y[(size_t)r * n + row] = acc;
+  // four vectors per pass over the matrix
+  for (int r0 = 0; r0 < nrhs; r0 += 4) {
+    const int nr = min(4, nrhs - r0);
+    const double *xr = x + (size_t)r0 * n;
+    double acc[4] = {0.0, 0.0, 0.0, 0.0};
+    for (int p = p0 + sub; p < p1; p += 8) {
+      const double v = val[p];
+      const int c = ci[p];
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (u < nr) acc[u] = fma(v, xr[(size_t)u * n + c], acc[u]);
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      acc[u] += __shfl_xor_sync(0xffffffffu, acc[u], 4);
+      acc[u] += __shfl_xor_sync(0xffffffffu, acc[u], 2);
+      acc[u] += __shfl_xor_sync(0xffffffffu, acc[u], 1);
+      if (ok && sub == 0 && u < nr) y[(size_t)(r0 + u) * n + row] = acc[u];
+    }
   }
 }
 
