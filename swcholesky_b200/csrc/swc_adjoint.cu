@@ -4,21 +4,25 @@
 //
 // log det A.  d log det A = tr(A^{-1} dA), so the gradient is A^{-1} on the pattern of A,
 // times 2 off the diagonal.  A^{-1} is computed on the whole pattern of L (the selected
-// inverse Z) by a reverse sweep over the elimination tree, root to leaves, that retraces the
-// factorization's POTRF / TRSM / SYRK steps backwards.  Per column block K of a supernode
-// (at most 64 columns; a wide supernode is a chain of such blocks) with the rows R of L
-// below it:
-//     U    = L_RK L_KK^{-1}                  recomputed from L (the factorization stores no
-//                                            intermediate panels)
-//     Z_RK = -Z_RR U                         Z_RR: symmetric, gathered from the ancestors
+// inverse) by a reverse sweep over the elimination tree, root to leaves, that retraces the
+// factorization's POTRF / TRSM / SYRK steps backwards.  Per column block K (a small supernode,
+// or 64 columns of a wide one) with the rows R of L below it:
+//     U    = L_RK L_KK^{-1}
+//     Z_RK = -Z_RR U
 //     Z_KK = L_KK^{-T} L_KK^{-1} - U^T Z_RK
 // (Takahashi, Fagan and Chin, 1973; the supernodal form of the reverse-mode Cholesky of
-// Murray, "Differentiation of the Cholesky decomposition", 2016).  Z_RR is inside the
-// ancestors' stored pattern: for rows i >= j of R, row i belongs to the row list of the
-// supernode holding column j (row lists are closed under the elimination).  Its entries are
-// located through position tables built once per structure: for every off-diagonal row run
-// of a supernode that falls into one ancestor (a "segment"), the positions of the
-// supernode's later rows in that ancestor's row list.
+// Murray, "Differentiation of the Cholesky decomposition", 2016).
+//
+// The sweep is multifrontal: every supernode with children holds A^{-1} on its whole front (all
+// rows of its panel squared, both triangles, column-major, leading dimension m), whose block
+// over the off-diagonal rows is copied from the parent's front through the child's row map
+// (rows are contained in the parent's).  Z_RR is then contiguous, so every product is a dense
+// one; a front lives until its children are done, in an arena placed at analysis.  Supernodes
+// without children keep only their panel.  Small supernodes take one kernel per level (a warp
+// or a CTA each, everything in shared memory but Z_RR, which is read once from the parent's
+// front); wide ones 64-column steps of three launches with 64x64 DMMA tiles.  Against the sweep
+// it replaces (one 64-row FMA tile per column block and row block, Z_RR gathered entry by
+// entry from all ancestors): see the launch code below.
 //
 // Functions of x = A^{-1} b.  With lam = A^{-1} (df/dx):
 //     df/dA_ij = -(lam_i x_j + lam_j x_i)  (i != j),   -lam_i x_i  (i == j).
@@ -35,94 +39,255 @@
 #include <vector>
 
 #include "swc_engine.h"
+#include "swc_front.h"
+#include "swc_tile.h"
 
 namespace swc {
 
 namespace {
 
-constexpr int AT = 256;       // threads of the tile kernels (4x4 register micro-tiles)
-constexpr int AKC = 16;       // rows of R per gathered chunk
-constexpr int ALD = TB + 1;   // padded row of a 64-wide shared tile
-constexpr int64_t OWN = INT64_MIN;  // location code: the row belongs to the unit's own supernode
-
 struct AdjDev {
-  const int4 *units;         // (supernode J, first column offset c0, width w, off = c0 + w)
-  const int64_t *tinv_off;   // per unit: offset of its w x w inverse in tinv
-  const int2 *tasks;         // (unit, x0): 64-row block of R starting at R index x0
-  const int *rowseg;         // per Ls position of an off-diagonal row: its segment
-  const int *seg_t;          // segment: first off-diagonal row index inside its supernode
-  const int *seg_S;          //          ancestor supernode holding the segment's columns
-  const int64_t *seg_tbl;    //          offset of its position list in tbl
-  const int *tbl;            // positions in the ancestor's row list
-  double *Z;                 // selected inverse, same layout as L
-  double *U;                 // L_RK L_KK^{-1}, same layout as L
-  double *tinv;              // L_KK^{-1} per unit, column-major w x w
-  double *P;                 // per task of the current wave: U(X,:)^T (Z_RR U)(X,:), 64 x 64
+  const int *parent, *rel, *apos;   // the tree (swc_front.h)
+  const int64_t *zoff;              // per supernode: its front (or panel) in Z
+  const char *kids;                 // per supernode: has children (a whole front is kept)
+  double *Z;
+  double *UT;                       // per task of the current step: U^T, 64 x rows, see utoff
+  double *P;                        // per task: U(X,:)^T (Z_RR U)(X,:), 64 x 64
+  double *grad;                     // per entry of A
 };
-
-__device__ __forceinline__ int lbound_a(const int *a, int len, int key) {
-  int lo = 0, hi = len;
-  while (lo < hi) {
-    int mid = (lo + hi) >> 1;
-    if (a[mid] < key) lo = mid + 1; else hi = mid;
-  }
-  return lo;
-}
 
 __device__ __forceinline__ int nrows_of(const DevSym &S, int s) {
   return (int)(S.rowptr[s + 1] - S.rowptr[s]);
 }
 
-// L_KK^{-1} of every unit (one CTA of 64 threads per unit; thread c forms column c by
-// forward substitution, all threads walking the rows in lock step).
-constexpr int TINV_SMEM = 2 * TB * ALD * 8 + TB * 8;
-__global__ void __launch_bounds__(TB) k_adj_tinv(DevSym S, AdjDev A) {
-  extern __shared__ double sm[];
-  double *T = sm, *X = sm + TB * ALD, *rd = X + TB * ALD;
-  const int4 u = A.units[blockIdx.x];
-  const int J = u.x, c0 = u.y, w = u.z;
-  const int ns = nrows_of(S, J);
-  const double *Lb = S.L + S.xptr[J] + (size_t)c0 * ns + c0;
-  const int c = threadIdx.x;
-  for (int idx = c; idx < w * w; idx += TB) {
-    const int col = idx / w, row = idx - col * w;
-    T[row * ALD + col] = row >= col ? Lb[(size_t)col * ns + row] : 0.0;
-  }
-  __syncthreads();
-  if (c < w) rd[c] = 1.0 / T[c * ALD + c];
-  __syncthreads();
-  if (c < w) {
-    for (int i = 0; i < w; ++i) {
-      double acc = (i == c) ? 1.0 : 0.0;
-      for (int k = c; k < i; ++k) acc -= T[i * ALD + k] * X[k * ALD + c];
-      X[i * ALD + c] = i >= c ? acc * rd[i] : 0.0;
-    }
-  }
-  __syncthreads();
-  double *out = A.tinv + A.tinv_off[blockIdx.x];
-  for (int idx = c; idx < w * w; idx += TB) {
-    const int col = idx / w, row = idx - col * w;
-    out[idx] = X[row * ALD + col];
-  }
+// ---- small supernodes: NW warps each.  In shared memory: the padded panel (front layout, see
+// front_ld), in which U replaces L_RK; Y = Z_RR U; T = L_KK^{-1}.  y_global: the two panels do
+// not fit, Y is read back from Z_RK = -Y (its scratch of 64 doubles per warp stays).
+constexpr int ZW_W = 16, ZW_WARPS = 2;            // warp variant: width limit, warps per CTA
+constexpr int ZW_SLICE = (2 * FRONT_WARP_ELEMS + ZW_W * (ZW_W + 4)) * 8 + FRONT_WARP_M * 4;
+constexpr int ZC_T = 256, ZC_W = ZC_T / 32;
+constexpr int ADJ_SMEM_MAX = 220 * 1024;
+
+template <int NW>
+__device__ __forceinline__ void zsync() {
+  if (NW == 1) __syncwarp(); else __syncthreads();
 }
 
-// U(X, :) = L_RK(X, :) L_KK^{-1} for one 64-row block X of R.
+template <int NW>
+__device__ void adj_small_body(const DevSym &S, const AdjDev &A, int s, double *Pm, double *Y, double *T,
+                               int *rel, bool y_global) {
+  constexpr int NTH = 32 * NW;
+  const int t = NW == 1 ? (int)(threadIdx.x & 31) : (int)threadIdx.x;
+  const int lane = t & 31, warp = t >> 5, g = lane >> 2, kq = lane & 3;
+  const int f = S.super[s], w = S.super[s + 1] - f;
+  const int m = nrows_of(S, s), r = m - w;
+  const int wp = front_wp(w), ld = front_ld(w, m), pad = wp - w, nk = wp >> 3, nr8 = (r + 7) >> 3;
+  const int ldt = adj_ldt(w);
+  const double *Ls = S.L + S.xptr[s];
+  double *Z = A.Z + A.zoff[s];
+  const bool front = A.kids[s] != 0;
+  // the panel (upper triangle, padding: zeros; padded diagonal: ones) and the row map
+  for (int e = t; e < wp * ld; e += NTH) {
+    const int j = e / ld, i = e - j * ld;
+    double v = i == j && j >= w ? 1.0 : 0.0;
+    const int row = i < wp ? i : i - pad;
+    if (j < w && (i < wp ? i < w && i >= j : row < m)) v = Ls[(size_t)j * m + row];
+    Pm[e] = v;
+  }
+  for (int e = t; e < wp * ldt; e += NTH) T[e] = 0.0;
+  const int *grel = A.rel + (S.rowptr[s] - f);
+  for (int i = t; i < r; i += NTH) rel[i] = grel[i];
+  zsync<NW>();
+  // inverses of the 8x8 diagonal blocks: lane j of eight forms column j by forward substitution
+  for (int c = t; c < wp; c += NTH) {
+    const int b0 = c & ~7, j = c & 7;
+    double x[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      double acc = i == j ? 1.0 : 0.0;
+#pragma unroll
+      for (int k = 0; k < i; ++k)
+        if (k >= j) acc = fma(-Pm[(b0 + k) * ld + b0 + i], x[k], acc);
+      x[i] = i >= j ? acc / Pm[(b0 + i) * ld + b0 + i] : 0.0;
+      T[c * ldt + b0 + i] = x[i];
+    }
+  }
+  zsync<NW>();
+  // T_ik = -T_ii sum_{k <= j < i} L_ij T_jk, a block column per warp (scratch: 64 doubles of Y)
+  double *Ww = Y + warp * 64;
+  for (int k = warp; k < nk; k += NW)
+    for (int i = k + 1; i < nk; ++i) {
+      double a[2] = {0.0, 0.0};
+      for (int j = k; j < i; ++j)
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+          dmma(a, Pm[(8 * j + 4 * h + kq) * ld + 8 * i + g], T[(8 * k + g) * ldt + 8 * j + 4 * h + kq]);
+      Ww[(2 * kq) * 8 + g] = a[0];
+      Ww[(2 * kq + 1) * 8 + g] = a[1];
+      __syncwarp();
+      double c[2] = {0.0, 0.0};
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+        dmma(c, neg(T[(8 * i + 4 * h + kq) * ldt + 8 * i + g]), Ww[g * 8 + 4 * h + kq]);
+      T[(8 * k + 2 * kq) * ldt + 8 * i + g] = c[0];
+      T[(8 * k + 2 * kq + 1) * ldt + 8 * i + g] = c[1];
+      __syncwarp();
+    }
+  zsync<NW>();
+  // U = L_RK T in place (a block row per warp; output block columns in increasing order only
+  // read input block columns at or after them)
+  for (int ib = warp; ib < nr8; ib += NW) {
+    double *row = Pm + wp + 8 * ib;
+    for (int n = 0; n < nk; ++n) {
+      double c[2] = {0.0, 0.0};
+      for (int k = 8 * n; k < wp; k += 4) dmma(c, row[(k + kq) * ld + g], T[(8 * n + g) * ldt + k + kq]);
+      __syncwarp();
+      row[(8 * n + 2 * kq) * ld + g] = c[0];
+      row[(8 * n + 2 * kq + 1) * ld + g] = c[1];
+      __syncwarp();
+    }
+  }
+  zsync<NW>();
+  // Y = Z_RR U, Z_RR read from the parent's front and, for a front of its own, written to it
+  if (r > 0) {
+    const int p = A.parent[s], mp = nrows_of(S, p);
+    const double *Zp = A.Z + A.zoff[p];
+    for (int ib = warp; ib < nr8; ib += NW) {
+      const int i = 8 * ib + g;
+      const bool iin = i < r;
+      const double *zrow = Zp + (iin ? rel[i] : 0);
+      double *own = Z + (size_t)w * m + w + i;
+      for (int n0 = 0; n0 < nk; n0 += 4) {
+        double c[4][2];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) c[q][0] = c[q][1] = 0.0;
+        for (int k0 = 0; k0 < r; k0 += 16) {
+          double a[4];
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            const int k = k0 + 4 * u + kq;
+            a[u] = iin && k < r ? zrow[(size_t)rel[k] * mp] : 0.0;
+          }
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            const int k = k0 + 4 * u + kq;
+            if (front && n0 == 0 && iin && k < r) own[(size_t)k * m] = a[u];
+            if (k0 + 4 * u < r)
+#pragma unroll
+              for (int q = 0; q < 4; ++q)
+                if (n0 + q < nk)
+                  dmma(c[q], a[u], Pm[(8 * (n0 + q) + g) * ld + wp + min(k, 8 * nr8 - 1)]);
+          }
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          if (n0 + q < nk) {
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+              const int col = 8 * (n0 + q) + 2 * kq + e;
+              if (!y_global) Y[col * ld + wp + 8 * ib + g] = c[q][e];
+              if (iin && col < w) {   // Z_RK = -Y
+                Z[(size_t)col * m + w + i] = -c[q][e];
+                if (front) Z[(size_t)(w + i) * m + col] = -c[q][e];
+              }
+            }
+          }
+      }
+    }
+  }
+  zsync<NW>();
+  // Z_KK = T^T T + U^T Y, lower 8x8 blocks
+  int blk = 0;
+  for (int a = 0; a < nk; ++a)
+    for (int b = 0; b <= a; ++b, ++blk) {
+      if (blk % NW != warp) continue;
+      double c[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
+      for (int k = 8 * a; k < wp; k += 4)
+        dmma(c[0], T[(8 * a + g) * ldt + k + kq], T[(8 * b + g) * ldt + k + kq]);
+      for (int k = 0; k < 8 * nr8; k += 8)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int row = k + 4 * h + kq, col = 8 * b + g;
+          const double y = !y_global ? Y[col * ld + wp + row]
+                           : (row < r && col < w) ? -Z[(size_t)col * m + w + row] : 0.0;
+          dmma(c[h], Pm[(8 * a + g) * ld + wp + row], y);
+        }
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int i = 8 * a + g, j = 8 * b + 2 * kq + e;
+        if (i < w && j <= i) {
+          const double v = c[0][e] + c[1][e];
+          Z[(size_t)j * m + i] = v;
+          Z[(size_t)i * m + j] = v;
+        }
+      }
+    }
+  zsync<NW>();
+  // gradient of the entries of A in the supernode's columns
+  for (int j = warp; j < w; j += NW)
+    for (int p = S.Ap[f + j] + lane; p < S.Ap[f + j + 1]; p += 32) {
+      const int pos = A.apos[p];
+      if (pos < 0) { atomicExch(&S.status[1], 1); A.grad[p] = 0.0; continue; }
+      A.grad[p] = Z[(size_t)j * m + pos] * (pos == j ? 1.0 : 2.0);
+    }
+  zsync<NW>();
+}
+
+__global__ void __launch_bounds__(ZC_T) k_adj_small(DevSym S, AdjDev A, const int *list) {
+  extern __shared__ double zsm[];
+  const int e = list[blockIdx.x], s = e < 0 ? ~e : e;   // ~s: y_global
+  const int w = S.super[s + 1] - S.super[s], m = nrows_of(S, s);
+  const int pe = front_wp(w) * front_ld(w, m);
+  const int ye = e < 0 ? ZC_W * 64 : max(pe, ZC_W * 64);
+  adj_small_body<ZC_W>(S, A, s, zsm, zsm + pe, zsm + pe + ye,
+                       reinterpret_cast<int *>(zsm + pe + ye + front_wp(w) * adj_ldt(w)), e < 0);
+}
+
+__global__ void __launch_bounds__(ZW_WARPS * 32) k_adj_warp(DevSym S, AdjDev A, const int *list, int count) {
+  extern __shared__ double zsm[];
+  const int q = blockIdx.x * ZW_WARPS + (threadIdx.x >> 5);
+  if (q >= count) return;
+  double *P = reinterpret_cast<double *>(reinterpret_cast<unsigned char *>(zsm) +
+                                         (size_t)(threadIdx.x >> 5) * ZW_SLICE);
+  double *Y = P + FRONT_WARP_ELEMS, *T = Y + FRONT_WARP_ELEMS;
+  adj_small_body<1>(S, A, list[q], P, Y, T, reinterpret_cast<int *>(T + ZW_W * (ZW_W + 4)), false);
+}
+
+// ---- wide supernodes ----------------------------------------------------------------------
+
+// The block over the off-diagonal rows, from the parent's front: task = (s, i0, j0).
+__global__ void __launch_bounds__(256) k_adj_copy(DevSym S, AdjDev A, const int4 *tasks) {
+  const int4 tk = tasks[blockIdx.x];
+  const int s = tk.x, w = S.super[s + 1] - S.super[s], m = nrows_of(S, s), r = m - w;
+  const int p = A.parent[s], mp = nrows_of(S, p);
+  const int *rel = A.rel + (S.rowptr[s] - S.super[s]);
+  const int i = tk.y + (threadIdx.x & 63);
+  if (i >= r) return;
+  const double *src = A.Z + A.zoff[p] + rel[i];
+  double *dst = A.Z + A.zoff[s] + (size_t)w * m + w + i;
+#pragma unroll 4
+  for (int j = tk.z + (threadIdx.x >> 6); j < min(r, tk.z + TB); j += 4)
+    dst[(size_t)j * m] = src[(size_t)rel[j] * mp];
+}
+
+// task = (s, column block b, first row x0 of R, task index of x0 = 0): rows x0 .. x0 + 63 of
+// U = L_RK T with T the inverse of the diagonal block the factorization stored; U^T at
+// UT + 4096 * (first task) + row * 64.
+constexpr int ALD = TB + 1;
 constexpr int U_SMEM = 2 * TB * ALD * 8;
-__global__ void __launch_bounds__(AT) k_adj_u(DevSym S, AdjDev A, const int2 *tasks) {
-  extern __shared__ double sm[];
-  double *Lx = sm, *Ti = sm + TB * ALD;
-  const int2 tk = tasks[blockIdx.x];
-  const int4 u = A.units[tk.x];
-  const int J = u.x, c0 = u.y, w = u.z, off = u.w;
-  const int ns = nrows_of(S, J);
-  const int m = ns - off, x0 = tk.y;
-  const int nrow = min(TB, m - x0);
-  const size_t base = S.xptr[J] + (size_t)c0 * ns + off + x0;
-  const double *ti = A.tinv + A.tinv_off[tk.x];
-  for (int idx = threadIdx.x; idx < TB * TB; idx += AT) {
-    const int col = idx >> 6, row = idx & (TB - 1);
-    Lx[row * ALD + col] = (row < nrow && col < w) ? S.L[base + (size_t)col * ns + row] : 0.0;
-    Ti[row * ALD + col] = (row < w && col < w) ? ti[col * w + row] : 0.0;
+__global__ void __launch_bounds__(256) k_adj_u(DevSym S, AdjDev A, const int4 *tasks) {
+  extern __shared__ double zsm[];
+  double *Lx = zsm, *Ti = zsm + TB * ALD;   // [row][k], [k][col]
+  const int4 tk = tasks[blockIdx.x];
+  const int s = tk.x, c0 = tk.y * TB, x0 = tk.z;
+  const int m = nrows_of(S, s), w = min(TB, S.super[s + 1] - S.super[s] - c0), off = c0 + w;
+  const int nrow = min(TB, m - off - x0);
+  const double *Lb = S.L + S.xptr[s] + (size_t)c0 * m + off + x0;
+  const double *ti = S.dinv + ((size_t)S.dinv_off[s] + tk.y) * (TB * TB);
+  for (int e = threadIdx.x; e < TB * TB; e += 256) {
+    const int c = e >> 6, q = e & (TB - 1);
+    Lx[q * ALD + c] = (q < nrow && c < w) ? Lb[(size_t)c * m + q] : 0.0;
+    Ti[q * ALD + c] = (q < w && c < w) ? ti[e] : 0.0;
   }
   __syncthreads();
   const int r0 = (threadIdx.x >> 4) * 4, cc0 = (threadIdx.x & 15) * 4;
@@ -138,140 +303,82 @@ __global__ void __launch_bounds__(AT) k_adj_u(DevSym S, AdjDev A, const int2 *ta
 #pragma unroll
       for (int j = 0; j < 4; ++j) acc[i][j] = fma(a[i], b[j], acc[i][j]);
   }
+  double *UT = A.UT + (size_t)tk.w * (TB * TB) + (size_t)x0 * TB;
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+    if (r0 + i < nrow)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) UT[(size_t)(r0 + i) * TB + cc0 + j] = acc[i][j];
+}
+
+// The same rows of Z_RK = -Z_RR U (DMMA, K = all rows of R) and their share of U^T Z_RR U.
+constexpr int ZRK_SMEM = (2 * TB * ALD > 2 * STAGE ? 2 * TB * ALD : 2 * STAGE) * 8;
+__global__ void __launch_bounds__(MT, 2) k_adj_zrk(DevSym S, AdjDev A, const int4 *tasks) {
+  extern __shared__ double zsm[];
+  const int4 tk = tasks[blockIdx.x];
+  const int s = tk.x, c0 = tk.y * TB, x0 = tk.z;
+  const int m = nrows_of(S, s), w = min(TB, S.super[s + 1] - S.super[s] - c0), off = c0 + w;
+  const int mr = m - off, nrow = min(TB, mr - x0);
+  double *Z = A.Z + A.zoff[s];
+  const double *UT = A.UT + (size_t)tk.w * (TB * TB);
+  TileAcc acc;
+  acc.zero();
+  dmma_tile_product(Z + (size_t)off * m + off + x0, m, nrow, UT, TB, w, mr, zsm, acc);
+  __syncthreads();
+  double *ys = zsm, *ux = zsm + TB * ALD;   // [row][column]
 #pragma unroll
   for (int i = 0; i < 4; ++i)
 #pragma unroll
     for (int j = 0; j < 4; ++j)
-      if (r0 + i < nrow && cc0 + j < w) A.U[base + (size_t)(cc0 + j) * ns + r0 + i] = acc[i][j];
-}
-
-// Location of column j of Z_RR (j: index into R = rows off.. of J's row list, as the
-// smaller index of a lower-triangle entry): the column's base offset in Z and the code that
-// turns the row index i into a position (OWN: position off + i in J's list; else an offset
-// into tbl).
-__device__ __forceinline__ void locate(const DevSym &S, const AdjDev &A, int J, int off, int own,
-                                       int ns, int j, int64_t &cb, int64_t &to) {
-  if (j < own) {
-    cb = S.xptr[J] + (int64_t)(off + j) * ns;
-    to = OWN;
-  } else {
-    const int64_t q = S.rowptr[J] + off + j;
-    const int sg = A.rowseg[q];
-    const int Sa = A.seg_S[sg];
-    cb = S.xptr[Sa] + (int64_t)(S.Ls[q] - S.super[Sa]) * nrows_of(S, Sa);
-    to = A.seg_tbl[sg] - A.seg_t[sg] - own;
-  }
-}
-
-// Z_RK(X, :) = -(Z_RR U)(X, :) for one 64-row block X of R, and the block's share of
-// U^T Z_RR U (for Z_KK), written to the wave's P scratch.
-constexpr int ZRK_SMEM = 2 * TB * 8 + 2 * AKC * 8 + TB * (AKC + 1) * 8 + AKC * ALD * 8 +
-                         2 * TB * ALD * 8;
-__global__ void __launch_bounds__(AT) k_adj_zrk(DevSym S, AdjDev A, const int2 *tasks) {
-  extern __shared__ double sm[];
-  int64_t *xcb = reinterpret_cast<int64_t *>(sm), *xto = xcb + TB;
-  int64_t *bcb = xto + TB, *bto = bcb + AKC;
-  double *zt = reinterpret_cast<double *>(bto + AKC);   // [x][b], ld AKC + 1
-  double *uc = zt + TB * (AKC + 1);                      // [b][c], ld ALD
-  double *ys = uc + AKC * ALD, *ux = ys + TB * ALD;      // [x][c], ld ALD
-  const int2 tk = tasks[blockIdx.x];
-  const int4 u = A.units[tk.x];
-  const int J = u.x, c0 = u.y, w = u.z, off = u.w;
-  const int ns = nrows_of(S, J);
-  const int wJ = S.super[J + 1] - S.super[J];
-  const int own = wJ - off;
-  const int m = ns - off, x0 = tk.y;
-  const int nrow = min(TB, m - x0);
-  const size_t ubase = S.xptr[J] + (size_t)c0 * ns + off;   // + col * ns + R index
-  const int tid = threadIdx.x;
-  if (tid < TB && tid < nrow) locate(S, A, J, off, own, ns, x0 + tid, xcb[tid], xto[tid]);
-  const int r0 = (tid >> 4) * 4, cc0 = (tid & 15) * 4;
-  double acc[4][4] = {};
-  for (int b0 = 0; b0 < m; b0 += AKC) {
-    __syncthreads();
-    if (tid < AKC && b0 + tid < m) locate(S, A, J, off, own, ns, b0 + tid, bcb[tid], bto[tid]);
-    for (int idx = tid; idx < AKC * TB; idx += AT) {
-      const int b = idx >> 6, c = idx & (TB - 1);
-      uc[b * ALD + c] = (b0 + b < m && c < w) ? A.U[ubase + (size_t)c * ns + b0 + b] : 0.0;
-    }
-    __syncthreads();
-    for (int idx = tid; idx < AKC * TB; idx += AT) {
-      const int b = idx >> 6, x = idx & (TB - 1);
-      const int ix = x0 + x, ib = b0 + b;
-      double v = 0.0;
-      if (x < nrow && ib < m) {
-        int64_t cb, to;
-        int i;
-        if (ix >= ib) { cb = bcb[b]; to = bto[b]; i = ix; }
-        else { cb = xcb[x]; to = xto[x]; i = ib; }
-        const int64_t pos = (to == OWN) ? (int64_t)(off + i) : (int64_t)A.tbl[to + i];
-        v = A.Z[cb + pos];
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int r = acc_row(i), c = acc_col(j, e);
+        ys[r * ALD + c] = (r < nrow && c < w) ? acc.v[i][j][e] : 0.0;
       }
-      zt[x * (AKC + 1) + b] = v;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int b = 0; b < AKC; ++b) {
-      double a[4], bb[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) a[i] = zt[(r0 + i) * (AKC + 1) + b];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) bb[j] = uc[b * ALD + cc0 + j];
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = fma(a[i], bb[j], acc[i][j]);
-    }
-  }
-  // Z_RK(X, :) = -Y; stage Y and U(X, :) for the Z_KK share
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int r = r0 + i, c = cc0 + j;
-      const bool ok = r < nrow && c < w;
-      if (ok) A.Z[ubase + (size_t)c * ns + x0 + r] = -acc[i][j];
-      ys[r * ALD + c] = ok ? acc[i][j] : 0.0;
-    }
-  for (int idx = tid; idx < TB * TB; idx += AT) {
-    const int c = idx >> 6, r = idx & (TB - 1);
-    ux[r * ALD + c] = (r < nrow && c < w) ? A.U[ubase + (size_t)c * ns + x0 + r] : 0.0;
+  for (int e = threadIdx.x; e < TB * TB; e += MT) {
+    const int r = e >> 6, c = e & (TB - 1);
+    ux[r * ALD + c] = (r < nrow && c < w) ? UT[(size_t)(x0 + r) * TB + c] : 0.0;
   }
   __syncthreads();
-  double p[4][4] = {};
-  for (int r = 0; r < nrow; ++r) {
-    double a[4], bb[4];
+  for (int e = threadIdx.x; e < TB * TB; e += MT) {
+    const int c = e >> 6, r = e & (TB - 1);
+    if (c < w && r < nrow) Z[(size_t)(c0 + c) * m + off + x0 + r] = -ys[r * ALD + c];
+  }
+  for (int e = threadIdx.x; e < TB * TB; e += MT) {
+    const int r = e >> 6, c = e & (TB - 1);
+    if (c < w && r < nrow) Z[(size_t)(off + x0 + r) * m + c0 + c] = -ys[r * ALD + c];
+  }
+  // U(X)^T Y(X), 4 x 8 entries per thread
+  const int i0 = (threadIdx.x >> 3) * 4, j0 = (threadIdx.x & 7) * 8;
+  double p[4][8] = {};
+  for (int k = 0; k < nrow; ++k) {
+    double a[4], b[8];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) a[i] = ux[r * ALD + r0 + i];
+    for (int i = 0; i < 4; ++i) a[i] = ux[k * ALD + i0 + i];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) bb[j] = ys[r * ALD + cc0 + j];
+    for (int j = 0; j < 8; ++j) b[j] = ys[k * ALD + j0 + j];
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
-      for (int j = 0; j < 4; ++j) p[i][j] = fma(a[i], bb[j], p[i][j]);
+      for (int j = 0; j < 8; ++j) p[i][j] = fma(a[i], b[j], p[i][j]);
   }
-  double *P = A.P + (size_t)blockIdx.x * TB * TB;
+  double *P = A.P + (size_t)blockIdx.x * (TB * TB);
 #pragma unroll
   for (int i = 0; i < 4; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) P[(size_t)(cc0 + j) * TB + r0 + i] = p[i][j];
+    for (int j = 0; j < 8; ++j) P[(i0 + i) * TB + j0 + j] = p[i][j];
 }
 
-// Z_KK = L_KK^{-T} L_KK^{-1} + sum over the unit's row blocks of U^T Z_RR U (lower part).
-constexpr int ZKK_SMEM = TB * ALD * 8;
-__global__ void __launch_bounds__(AT) k_adj_zkk(DevSym S, AdjDev A, const int *wave_units,
-                                                const int *ut_begin, const int *ut_end,
-                                                int task_base) {
-  extern __shared__ double sm[];
-  double *Ti = sm;
-  const int ui = wave_units[blockIdx.x];
-  const int4 u = A.units[ui];
-  const int J = u.x, c0 = u.y, w = u.z;
-  const int ns = nrows_of(S, J);
-  const double *ti = A.tinv + A.tinv_off[ui];
-  for (int idx = threadIdx.x; idx < TB * TB; idx += AT) {
-    const int col = idx >> 6, row = idx & (TB - 1);
-    Ti[row * ALD + col] = (row < w && col < w) ? ti[col * w + row] : 0.0;
+// Z_KK = T^T T + the row blocks' shares.  unit = (s, column block, first task, tasks).
+__global__ void __launch_bounds__(256) k_adj_zkk(DevSym S, AdjDev A, const int4 *units) {
+  __shared__ double Ti[TB * ALD];   // [k][col]
+  const int4 un = units[blockIdx.x];
+  const int s = un.x, c0 = un.y * TB;
+  const int m = nrows_of(S, s), w = min(TB, S.super[s + 1] - S.super[s] - c0);
+  const double *ti = S.dinv + ((size_t)S.dinv_off[s] + un.y) * (TB * TB);
+  for (int e = threadIdx.x; e < TB * TB; e += 256) {
+    const int c = e >> 6, k = e & (TB - 1);
+    Ti[k * ALD + c] = (k < w && c < w) ? ti[e] : 0.0;
   }
   __syncthreads();
   const int r0 = (threadIdx.x >> 4) * 4, cc0 = (threadIdx.x & 15) * 4;
@@ -287,21 +394,37 @@ __global__ void __launch_bounds__(AT) k_adj_zkk(DevSym S, AdjDev A, const int *w
 #pragma unroll
       for (int j = 0; j < 4; ++j) acc[i][j] = fma(a[i], b[j], acc[i][j]);
   }
-  for (int t = ut_begin[ui]; t < ut_end[ui]; ++t) {
-    const double *P = A.P + (size_t)(t - task_base) * TB * TB;
+  for (int t = un.z; t < un.z + un.w; ++t) {
+    const double *P = A.P + (size_t)t * (TB * TB);
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
-      for (int j = 0; j < 4; ++j) acc[i][j] += P[(size_t)(cc0 + j) * TB + r0 + i];
+      for (int j = 0; j < 4; ++j) acc[i][j] += P[(r0 + i) * TB + cc0 + j];
   }
-  double *Zb = A.Z + S.xptr[J] + (size_t)c0 * ns + c0;
+  double *Z = A.Z + A.zoff[s] + (size_t)c0 * m + c0;
 #pragma unroll
   for (int i = 0; i < 4; ++i)
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const int r = r0 + i, c = cc0 + j;
-      if (r < w && c < w && r >= c) Zb[(size_t)c * ns + r] = acc[i][j];
+      if (r < w && c <= r) {
+        Z[(size_t)c * m + r] = acc[i][j];
+        Z[(size_t)r * m + c] = acc[i][j];
+      }
     }
+}
+
+// Gradient of the entries of A in a wide supernode's columns: one warp per (s, column).
+__global__ void k_adj_grad(DevSym S, AdjDev A, const int2 *cols, int count) {
+  const int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  if (t >= count) return;
+  const int s = cols[t].x, j = cols[t].y, c = j - S.super[s];
+  const double *col = A.Z + A.zoff[s] + (size_t)c * nrows_of(S, s);
+  for (int p = S.Ap[j] + lane; p < S.Ap[j + 1]; p += 32) {
+    const int pos = A.apos[p];
+    if (pos < 0) { atomicExch(&S.status[1], 1); A.grad[p] = 0.0; continue; }
+    A.grad[p] = col[pos] * (pos == c ? 1.0 : 2.0);
+  }
 }
 
 // Supernode holding column j.
@@ -333,23 +456,6 @@ __global__ void __launch_bounds__(256) k_logdet(DevSym S, double *partial) {
   if (threadIdx.x == 0) partial[blockIdx.x] = red[0];
 }
 
-// grad[p] = d log det A / d Ax[p] = Z_ij (2 - delta_ij); one warp per column.
-__global__ void k_logdet_grad(DevSym S, const double *Z, double *grad) {
-  const int j = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (j >= S.n) return;
-  const int s = snode_of(S, j);
-  const int64_t rb = S.rowptr[s];
-  const int m = (int)(S.rowptr[s + 1] - rb);
-  const double *col = Z + S.xptr[s] + (size_t)(j - S.super[s]) * m;
-  for (int p = S.Ap[j] + lane; p < S.Ap[j + 1]; p += 32) {
-    const int i = S.Ai[p];
-    const int pos = lbound_a(S.Ls + rb, m, i);
-    grad[p] = (pos < m && S.Ls[rb + pos] == i) ? col[pos] * (i == j ? 1.0 : 2.0) : 0.0;
-    if (!(pos < m && S.Ls[rb + pos] == i)) atomicExch(&S.status[1], 1);
-  }
-}
-
 // grad[p] = -(lam_i x_j + lam_j x_i) for i != j, -lam_i x_i on the diagonal.
 __global__ void k_solve_grad(DevSym S, const double *x, const double *lam, double *grad) {
   const int j = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -366,111 +472,114 @@ __global__ void k_solve_grad(DevSym S, const double *x, const double *lam, doubl
 
 // ---------------------------------------------------------------------------------------
 
+// Reverse sweep: waves by decreasing level.
 struct AdjointPlan {
-  bool ready = false;
-  std::vector<int4> units;
-  std::vector<int64_t> tinv_off;
-  std::vector<int> wave_unit_off, wave_units;   // units of wave v (root side first)
-  std::vector<int> wave_task_off;
-  std::vector<int2> tasks;                      // grouped by wave
-  std::vector<int> ut_begin, ut_end;            // per unit: its tasks
-  int max_wave_tasks = 0;
-  std::vector<int> rowseg, seg_t, seg_S, tbl;
-  std::vector<int64_t> seg_tbl;
+  struct Step { int task_off, task_cnt, unit_off, unit_cnt; };   // one 64-column step of a wave
+  struct AdjWave {
+    int warp_off, warp_cnt, cta_off, cta_cnt, cta_smem, copy_off, copy_cnt;
+    std::vector<Step> steps;
+  };
+  std::vector<AdjWave> waves;
+  std::vector<int> warp_list, cta_list, parent;
+  std::vector<int4> copies, tasks, units;
+  std::vector<char> kids;
+  std::vector<int64_t> zoff;
+  int64_t z_len = 0;
+  int max_tasks = 0;
 };
 
-bool Engine::prepare_adjoint(std::string &err) {
-  if (adj_ && adj_->ready) return true;
-  if (!adj_) adj_.reset(new AdjointPlan);
-  AdjointPlan &AP = *adj_;
-  const std::vector<int> &super = hsym_.super;
-  const std::vector<int64_t> &rowptr = hsym_.rowptr;
-  const int ns_ = nsuper_;
-  std::vector<int> col2sup(n_);
-  for (int s = 0; s < ns_; ++s)
-    for (int j = super[s]; j < super[s + 1]; ++j) col2sup[j] = s;
-  // segments and position tables
-  AP.rowseg.assign(h_Ls_.size(), -1);
-  for (int J = 0; J < ns_; ++J) {
-    const int wJ = super[J + 1] - super[J];
-    const int64_t rb = rowptr[J], re = rowptr[J + 1];
-    int64_t q = rb + wJ;
-    while (q < re) {
-      const int Sa = col2sup[h_Ls_[q]];
-      int64_t qe = q;
-      while (qe < re && col2sup[h_Ls_[qe]] == Sa) ++qe;
-      const int sg = (int)AP.seg_t.size();
-      AP.seg_t.push_back((int)(q - rb - wJ));
-      AP.seg_S.push_back(Sa);
-      AP.seg_tbl.push_back((int64_t)AP.tbl.size());
-      const int *ls = h_Ls_.data() + rowptr[Sa];
-      const int lsn = (int)(rowptr[Sa + 1] - rowptr[Sa]);
-      int pos = 0;
-      for (int64_t t = q; t < re; ++t) {
-        pos = (int)(std::lower_bound(ls + pos, ls + lsn, h_Ls_[t]) - ls);
-        if (pos >= lsn || ls[pos] != h_Ls_[t]) {
-          err = "adjoint: row list not closed under the elimination (invalid structure)";
-          return false;
-        }
-        AP.tbl.push_back(pos);
+static void build_adjoint_plan(const HostSym &H, const Plan &P, const FrontPlan &F, AdjointPlan &AP) {
+  const std::vector<int> &super = H.super;
+  const int ns = (int)super.size() - 1, nlev = (int)P.waves.size();
+  auto width = [&](int s) { return super[s + 1] - super[s]; };
+  auto rows = [&](int s) { return (int)(H.rowptr[s + 1] - H.rowptr[s]); };
+  std::vector<int> level(ns, 0);
+  AP.parent.assign(ns, -1);
+  AP.kids.assign(ns, 0);
+  AP.zoff.assign(ns, 0);
+  for (int s = 0; s < ns; ++s)
+    for (int q = F.child_ptr[s]; q < F.child_ptr[s + 1]; ++q) {
+      AP.parent[F.child[q]] = s;
+      AP.kids[s] = 1;
+      level[s] = std::max(level[s], level[F.child[q]] + 1);
+    }
+  std::vector<std::vector<int>> by_level(nlev);
+  std::vector<char> tiled(ns, 0);
+  for (int s : P.big_list) tiled[s] = 1;
+  for (int s = 0; s < ns; ++s) by_level[level[s]].push_back(s);
+  FrontArena A;
+  auto len = [&](int s) {
+    return ((int64_t)rows(s) * (AP.kids[s] || tiled[s] ? rows(s) : width(s)) + 15) & ~(int64_t)15;
+  };
+  std::vector<int> left(ns, 0);   // children not done yet
+  for (int s = 0; s < ns; ++s) left[s] = F.child_ptr[s + 1] - F.child_ptr[s];
+  AP.waves.resize(nlev);
+  for (int v = 0; v < nlev; ++v) {
+    const std::vector<int> &here = by_level[nlev - 1 - v];
+    AdjointPlan::AdjWave &W = AP.waves[v];
+    W.warp_off = (int)AP.warp_list.size();
+    W.cta_off = (int)AP.cta_list.size();
+    W.copy_off = (int)AP.copies.size();
+    W.cta_smem = 0;
+    int fit = 0, maxnb = 0;
+    auto warp_fits = [&](int s) {
+      const int w = width(s), m = rows(s);
+      return !tiled[s] && w <= ZW_W && m <= FRONT_WARP_M && front_wp(w) * front_ld(w, m) <= FRONT_WARP_ELEMS;
+    };
+    for (int s : here) fit += warp_fits(s);
+    for (int s : here) {
+      const int w = width(s), m = rows(s);
+      AP.zoff[s] = A.take(len(s));
+      if (tiled[s]) {
+        for (int j0 = 0; j0 < m - w; j0 += TB)
+          for (int i0 = 0; i0 < m - w; i0 += TB) AP.copies.push_back(make_int4(s, i0, j0, 0));
+        maxnb = std::max(maxnb, (w + TB - 1) / TB);
+      } else if (fit >= FRONT_WARP_LEVEL_MIN && warp_fits(s)) {
+        AP.warp_list.push_back(s);
+      } else {
+        const bool y_global = adj_small_smem(w, m, false) > ADJ_SMEM_MAX;
+        AP.cta_list.push_back(y_global ? ~s : s);
+        W.cta_smem = std::max<int>(W.cta_smem, (int)adj_small_smem(w, m, y_global));
       }
-      for (int64_t t = q; t < qe; ++t) AP.rowseg[t] = sg;
-      q = qe;
+    }
+    W.warp_cnt = (int)AP.warp_list.size() - W.warp_off;
+    W.cta_cnt = (int)AP.cta_list.size() - W.cta_off;
+    W.copy_cnt = (int)AP.copies.size() - W.copy_off;
+    for (int t = 0; t < maxnb; ++t) {   // last column block first
+      AdjointPlan::Step st{(int)AP.tasks.size(), 0, (int)AP.units.size(), 0};
+      for (int s : here) {
+        if (!tiled[s]) continue;
+        const int w = width(s), b = (w + TB - 1) / TB - 1 - t;
+        if (b < 0) continue;
+        const int first = (int)AP.tasks.size() - st.task_off, mr = rows(s) - std::min(w, (b + 1) * TB);
+        for (int x0 = 0; x0 < mr; x0 += TB) AP.tasks.push_back(make_int4(s, b, x0, first));
+        AP.units.push_back(make_int4(s, b, first, (int)AP.tasks.size() - st.task_off - first));
+      }
+      st.task_cnt = (int)AP.tasks.size() - st.task_off;
+      st.unit_cnt = (int)AP.units.size() - st.unit_off;
+      AP.max_tasks = std::max(AP.max_tasks, st.task_cnt);
+      W.steps.push_back(st);
+    }
+    // a front is read by its children only: free it once the last one is done
+    for (int s : here) {
+      if (!AP.kids[s]) A.give(AP.zoff[s], len(s));
+      const int p = AP.parent[s];
+      if (p >= 0 && --left[p] == 0) A.give(AP.zoff[p], len(p));
     }
   }
-  // units (64-column blocks) and their levels, root side first
-  std::vector<int> ufirst(ns_ + 1, 0);
-  for (int J = 0; J < ns_; ++J) ufirst[J + 1] = ufirst[J] + (super[J + 1] - super[J] + TB - 1) / TB;
-  const int nunits = ufirst[ns_];
-  AP.units.resize(nunits);
-  AP.tinv_off.assign(nunits + 1, 0);
-  std::vector<int> ulev(nunits), top(ns_);
-  int nlev = 0;
-  for (int J = ns_ - 1; J >= 0; --J) {
-    const int wJ = super[J + 1] - super[J];
-    const int64_t m = rowptr[J + 1] - rowptr[J];
-    const int nb = ufirst[J + 1] - ufirst[J];
-    int t = 0;
-    if (m > wJ) {
-      const int p = col2sup[h_Ls_[rowptr[J] + wJ]];
-      t = top[p] + (ufirst[p + 1] - ufirst[p]);   // one past the parent's last unit level
-    }
-    top[J] = t;
-    for (int b = 0; b < nb; ++b) {
-      const int c0 = b * TB, w = std::min(TB, wJ - c0);
-      const int u = ufirst[J] + b;
-      AP.units[u] = make_int4(J, c0, w, c0 + w);
-      ulev[u] = t + (nb - 1 - b);
-      nlev = std::max(nlev, ulev[u] + 1);
-    }
+  AP.z_len = A.end();
+}
+
+bool Engine::prepare_adjoint(std::string &err) {
+  if (adj_) return true;
+  if (!front_ || !front_->closed) {
+    err = "adjoint: row list not closed under the elimination (invalid structure)";
+    return false;
   }
-  for (int u = 0; u < nunits; ++u)
-    AP.tinv_off[u + 1] = AP.tinv_off[u] + (int64_t)AP.units[u].z * AP.units[u].z;
-  std::vector<std::vector<int>> bylev(nlev);
-  for (int u = 0; u < nunits; ++u) bylev[ulev[u]].push_back(u);
-  AP.ut_begin.assign(nunits, 0);
-  AP.ut_end.assign(nunits, 0);
-  AP.wave_unit_off.clear();
-  AP.wave_units.clear();
-  AP.wave_task_off.clear();
-  AP.tasks.clear();
-  AP.max_wave_tasks = 0;
-  for (int l = 0; l < nlev; ++l) {
-    AP.wave_unit_off.push_back((int)AP.wave_units.size());
-    AP.wave_task_off.push_back((int)AP.tasks.size());
-    for (int u : bylev[l]) {
-      AP.wave_units.push_back(u);
-      const int J = AP.units[u].x;
-      const int m = (int)(rowptr[J + 1] - rowptr[J]) - AP.units[u].w;
-      AP.ut_begin[u] = (int)AP.tasks.size();
-      for (int x0 = 0; x0 < m; x0 += TB) AP.tasks.push_back(make_int2(u, x0));
-      AP.ut_end[u] = (int)AP.tasks.size();
-    }
-    AP.max_wave_tasks = std::max(AP.max_wave_tasks, (int)AP.tasks.size() - AP.wave_task_off.back());
-  }
-  AP.wave_unit_off.push_back((int)AP.wave_units.size());
-  AP.wave_task_off.push_back((int)AP.tasks.size());
-  // device copies and scratch
+  if (!prepare_tree(err)) return false;
+  std::shared_ptr<AdjointPlan> plan = std::make_shared<AdjointPlan>();
+  AdjointPlan &AP = *plan;
+  build_adjoint_plan(hsym_, plan_, *front_, AP);
   cudaStream_t st = stream_;
   cudaError_t e = cudaSuccess;
   auto up = [&](auto *&dst, const auto &v) {
@@ -478,61 +587,60 @@ bool Engine::prepare_adjoint(std::string &err) {
     if (e != cudaSuccess) return;
     e = cudaMalloc(&dst, sizeof(T) * std::max<size_t>(v.size(), 1));
     if (e == cudaSuccess && !v.empty())
-      e = cudaMemcpyAsync(dst, v.data(), sizeof(T) * v.size(), cudaMemcpyHostToDevice, st);
+      e = cudaMemcpyAsync(const_cast<typename std::remove_const<T>::type *>(dst), v.data(), sizeof(T) * v.size(),
+                          cudaMemcpyHostToDevice, st);
   };
-  up(d_adj_units_, AP.units);
-  up(d_adj_tinv_off_, AP.tinv_off);
+  up(d_adj_parent_, AP.parent);
+  up(d_adj_kids_, AP.kids);
+  up(d_adj_zoff_, AP.zoff);
+  up(d_adj_warp_, AP.warp_list);
+  up(d_adj_cta_, AP.cta_list);
+  up(d_adj_copies_, AP.copies);
   up(d_adj_tasks_, AP.tasks);
-  up(d_adj_wave_units_, AP.wave_units);
-  up(d_adj_ut_begin_, AP.ut_begin);
-  up(d_adj_ut_end_, AP.ut_end);
-  up(d_adj_rowseg_, AP.rowseg);
-  up(d_adj_seg_t_, AP.seg_t);
-  up(d_adj_seg_S_, AP.seg_S);
-  up(d_adj_seg_tbl_, AP.seg_tbl);
-  up(d_adj_tbl_, AP.tbl);
-  if (e == cudaSuccess) e = cudaMalloc(&d_adj_Z_, sizeof(double) * std::max<int64_t>(xsize_, 1));
-  if (e == cudaSuccess) e = cudaMalloc(&d_adj_U_, sizeof(double) * std::max<int64_t>(xsize_, 1));
-  if (e == cudaSuccess)
-    e = cudaMalloc(&d_adj_tinv_, sizeof(double) * std::max<int64_t>(AP.tinv_off[nunits], 1));
-  if (e == cudaSuccess)
-    e = cudaMalloc(&d_adj_P_, sizeof(double) * TB * TB * std::max(AP.max_wave_tasks, 1));
-  if (e == cudaSuccess) e = cudaMalloc(&d_adj_partial_, sizeof(double) * LD_BLOCKS);
+  up(d_adj_units_, AP.units);
+  const size_t scratch = sizeof(double) * TB * TB * std::max(AP.max_tasks, 1);
+  if (e == cudaSuccess) e = cudaMalloc(&d_adj_Z_, sizeof(double) * std::max<int64_t>(AP.z_len, 1));
+  if (e == cudaSuccess) e = cudaMalloc(&d_adj_UT_, scratch);
+  if (e == cudaSuccess) e = cudaMalloc(&d_adj_P_, scratch);
+  if (e == cudaSuccess) e = cudaMalloc(&d_adj_grad_, sizeof(double) * std::max<int64_t>(nnz_, 1));
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_adj_tinv, cudaFuncAttributeMaxDynamicSharedMemorySize, TINV_SMEM);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_adj_small, cudaFuncAttributeMaxDynamicSharedMemorySize, ADJ_SMEM_MAX);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_adj_warp, cudaFuncAttributeMaxDynamicSharedMemorySize, ZW_WARPS * ZW_SLICE);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_adj_u, cudaFuncAttributeMaxDynamicSharedMemorySize, U_SMEM);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_adj_zrk, cudaFuncAttributeMaxDynamicSharedMemorySize, ZRK_SMEM);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_adj_zkk, cudaFuncAttributeMaxDynamicSharedMemorySize, ZKK_SMEM);
   if (e != cudaSuccess) {
+    release_adjoint();
     err = std::string("adjoint setup: ") + cudaGetErrorString(e);
     return false;
   }
-  AP.ready = true;
+  adj_ = plan;
   return true;
 }
 
 void Engine::release_adjoint() {
-  void *bufs[] = {d_adj_units_, d_adj_tinv_off_, d_adj_tasks_, d_adj_wave_units_, d_adj_ut_begin_,
-                  d_adj_ut_end_, d_adj_rowseg_, d_adj_seg_t_, d_adj_seg_S_, d_adj_seg_tbl_,
-                  d_adj_tbl_, d_adj_Z_, d_adj_U_, d_adj_tinv_, d_adj_P_, d_adj_partial_};
+  void *bufs[] = {d_adj_parent_, d_adj_kids_, d_adj_zoff_, d_adj_warp_, d_adj_cta_, d_adj_copies_,
+                  d_adj_tasks_, d_adj_units_, d_adj_Z_, d_adj_UT_, d_adj_P_, d_adj_grad_, d_adj_partial_};
   for (void *p : bufs)
     if (p) cudaFree(p);
-  d_adj_units_ = nullptr;
-  d_adj_tinv_off_ = nullptr;
-  d_adj_tasks_ = nullptr;
-  d_adj_wave_units_ = d_adj_ut_begin_ = d_adj_ut_end_ = d_adj_rowseg_ = nullptr;
-  d_adj_seg_t_ = d_adj_seg_S_ = d_adj_tbl_ = nullptr;
-  d_adj_seg_tbl_ = nullptr;
-  d_adj_Z_ = d_adj_U_ = d_adj_tinv_ = d_adj_P_ = d_adj_partial_ = nullptr;
+  if (adj_graph_) cudaGraphExecDestroy(adj_graph_);
+  adj_graph_ = nullptr;
+  d_adj_parent_ = d_adj_warp_ = d_adj_cta_ = nullptr;
+  d_adj_kids_ = nullptr;
+  d_adj_zoff_ = nullptr;
+  d_adj_copies_ = d_adj_tasks_ = d_adj_units_ = nullptr;
+  d_adj_Z_ = d_adj_UT_ = d_adj_P_ = d_adj_grad_ = d_adj_partial_ = nullptr;
   adj_.reset();
 }
 
 bool Engine::logdet(double *out, std::string &err) {
   cudaSetDevice(device_);
-  if (!prepare_adjoint(err)) return false;
-  k_logdet<<<LD_BLOCKS, 256, 0, stream_>>>(sym_, d_adj_partial_);
+  cudaError_t e = cudaSuccess;
+  if (!d_adj_partial_) e = cudaMalloc(&d_adj_partial_, sizeof(double) * LD_BLOCKS);
   double part[LD_BLOCKS];
-  cudaError_t e = cudaMemcpyAsync(part, d_adj_partial_, sizeof(part), cudaMemcpyDeviceToHost, stream_);
+  if (e == cudaSuccess) {
+    k_logdet<<<LD_BLOCKS, 256, 0, stream_>>>(sym_, d_adj_partial_);
+    e = cudaMemcpyAsync(part, d_adj_partial_, sizeof(part), cudaMemcpyDeviceToHost, stream_);
+  }
   if (e == cudaSuccess) e = cudaStreamSynchronize(stream_);
   if (e != cudaSuccess) {
     err = std::string("logdet: ") + cudaGetErrorString(e);
@@ -544,55 +652,60 @@ bool Engine::logdet(double *out, std::string &err) {
   return true;
 }
 
-bool Engine::selected_inverse(std::string &err) {
-  cudaSetDevice(device_);
-  if (!prepare_adjoint(err)) return false;
+// The reverse sweep's launches (fixed by the structure), gradient into d_adj_grad_.
+void Engine::run_adjoint() {
   const AdjointPlan &AP = *adj_;
-  AdjDev A;
-  A.units = d_adj_units_;
-  A.tinv_off = d_adj_tinv_off_;
-  A.tasks = d_adj_tasks_;
-  A.rowseg = d_adj_rowseg_;
-  A.seg_t = d_adj_seg_t_;
-  A.seg_S = d_adj_seg_S_;
-  A.seg_tbl = d_adj_seg_tbl_;
-  A.tbl = d_adj_tbl_;
-  A.Z = d_adj_Z_;
-  A.U = d_adj_U_;
-  A.tinv = d_adj_tinv_;
-  A.P = d_adj_P_;
   cudaStream_t st = stream_;
-  cudaMemsetAsync(d_adj_Z_, 0, sizeof(double) * xsize_, st);
-  const int nunits = (int)AP.units.size();
-  if (nunits > 0) k_adj_tinv<<<nunits, TB, TINV_SMEM, st>>>(sym_, A);
-  const int nw = (int)AP.wave_unit_off.size() - 1;
-  for (int v = 0; v < nw; ++v) {
-    const int t0 = AP.wave_task_off[v], nt = AP.wave_task_off[v + 1] - t0;
-    const int u0 = AP.wave_unit_off[v], nu = AP.wave_unit_off[v + 1] - u0;
-    if (nt > 0) {
-      k_adj_u<<<nt, AT, U_SMEM, st>>>(sym_, A, d_adj_tasks_ + t0);
-      k_adj_zrk<<<nt, AT, ZRK_SMEM, st>>>(sym_, A, d_adj_tasks_ + t0);
+  const AdjDev A{d_adj_parent_, d_frel_, d_fapos_, d_adj_zoff_, d_adj_kids_,
+                 d_adj_Z_,      d_adj_UT_, d_adj_P_, d_adj_grad_};
+  for (size_t v = 0; v < AP.waves.size(); ++v) {
+    const AdjointPlan::AdjWave &W = AP.waves[v];
+    if (W.copy_cnt > 0) k_adj_copy<<<W.copy_cnt, 256, 0, st>>>(sym_, A, d_adj_copies_ + W.copy_off);
+    if (W.cta_cnt > 0) k_adj_small<<<W.cta_cnt, ZC_T, W.cta_smem, st>>>(sym_, A, d_adj_cta_ + W.cta_off);
+    if (W.warp_cnt > 0)
+      k_adj_warp<<<(W.warp_cnt + ZW_WARPS - 1) / ZW_WARPS, ZW_WARPS * 32, ZW_WARPS * ZW_SLICE, st>>>(
+          sym_, A, d_adj_warp_ + W.warp_off, W.warp_cnt);
+    for (const AdjointPlan::Step &t : W.steps) {
+      if (t.task_cnt > 0) {
+        k_adj_u<<<t.task_cnt, 256, U_SMEM, st>>>(sym_, A, d_adj_tasks_ + t.task_off);
+        k_adj_zrk<<<t.task_cnt, MT, ZRK_SMEM, st>>>(sym_, A, d_adj_tasks_ + t.task_off);
+      }
+      if (t.unit_cnt > 0) k_adj_zkk<<<t.unit_cnt, 256, 0, st>>>(sym_, A, d_adj_units_ + t.unit_off);
     }
-    if (nu > 0)
-      k_adj_zkk<<<nu, AT, ZKK_SMEM, st>>>(sym_, A, d_adj_wave_units_ + u0, d_adj_ut_begin_,
-                                          d_adj_ut_end_, t0);
+    const Wave &B = plan_.waves[AP.waves.size() - 1 - v];
+    if (B.asm_cnt > 0)
+      k_adj_grad<<<(B.asm_cnt * 32 + 255) / 256, 256, 0, st>>>(sym_, A, d_asm_ + B.asm_off, B.asm_cnt);
   }
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) {
-    err = std::string("adjoint sweep: ") + cudaGetErrorString(e);
-    return false;
-  }
-  return true;
 }
 
 bool Engine::logdet_grad(double *grad, std::string &err) {
-  if (!selected_inverse(err)) return false;
+  cudaSetDevice(device_);
+  if (!prepare_adjoint(err)) return false;
   cudaStream_t st = stream_;
   cudaMemsetAsync(d_status_ + 1, 0, sizeof(int), st);
-  const int blocks = (int)(((int64_t)n_ * 32 + 255) / 256);
-  k_logdet_grad<<<blocks, 256, 0, st>>>(sym_, d_adj_Z_, grad);
+  cudaError_t e = cudaSuccess;
+  if (use_graph_ && !adj_graph_) {
+    cudaGraph_t g = nullptr;
+    e = cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal);
+    if (e == cudaSuccess) {
+      run_adjoint();
+      e = cudaStreamEndCapture(st, &g);
+    }
+    if (e == cudaSuccess) e = cudaGraphInstantiate(&adj_graph_, g, 0);
+    if (g) cudaGraphDestroy(g);
+    if (e != cudaSuccess) {
+      adj_graph_ = nullptr;
+      err = std::string("logdet gradient: ") + cudaGetErrorString(e);
+      return false;
+    }
+  }
+  if (adj_graph_) e = cudaGraphLaunch(adj_graph_, st);
+  else run_adjoint();
+  if (e == cudaSuccess) e = cudaGetLastError();
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(grad, d_adj_grad_, sizeof(double) * nnz_, cudaMemcpyDeviceToDevice, st);
   int flag = 0;
-  cudaError_t e = cudaMemcpyAsync(&flag, d_status_ + 1, sizeof(int), cudaMemcpyDeviceToHost, st);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(&flag, d_status_ + 1, sizeof(int), cudaMemcpyDeviceToHost, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   if (e != cudaSuccess) {
     err = std::string("logdet gradient: ") + cudaGetErrorString(e);

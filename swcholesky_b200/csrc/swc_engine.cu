@@ -1385,6 +1385,20 @@ void Engine::release_front() {
   front_ready_ = front_tried_ = false;
 }
 
+bool Engine::prepare_tree(std::string &err) {
+  if (d_frel_) return true;
+  const FrontPlan &F = *front_;
+  cudaStream_t st = stream_;
+  if (!(upload(d_fchild_ptr_, F.child_ptr.data(), F.child_ptr.size(), st, err) &&
+        upload(d_fchild_, F.child.data(), F.child.size(), st, err) &&
+        upload(d_fn1_, F.child_n1.data(), F.child_n1.size(), st, err) &&
+        upload(d_fapos_, F.apos.data(), F.apos.size(), st, err) &&
+        upload(d_frel_, F.rel.data(), F.rel.size(), st, err)))
+    return false;
+  if (cudaStreamSynchronize(st) != cudaSuccess) { err = "device upload: elimination tree"; return false; }
+  return true;
+}
+
 // The multifrontal plan's tables and the contribution blocks on the device, on the first FP64
 // factorization of a structure; without the memory for them the left-looking kernels stay.
 bool Engine::prepare_front(std::string &err) {
@@ -1397,12 +1411,7 @@ bool Engine::prepare_front(std::string &err) {
     d_cb_ = nullptr;
     return true;
   }
-  if (!(upload(d_fchild_ptr_, F.child_ptr.data(), F.child_ptr.size(), st, err) &&
-        upload(d_fchild_, F.child.data(), F.child.size(), st, err) &&
-        upload(d_fn1_, F.child_n1.data(), F.child_n1.size(), st, err) &&
-        upload(d_frel_, F.rel.data(), F.rel.size(), st, err) &&
-        upload(d_fapos_, F.apos.data(), F.apos.size(), st, err) &&
-        upload(d_fwarp_, F.warp_list.data(), F.warp_list.size(), st, err) &&
+  if (!(prepare_tree(err) && upload(d_fwarp_, F.warp_list.data(), F.warp_list.size(), st, err) &&
         upload(d_fcta_, F.cta_list.data(), F.cta_list.size(), st, err) &&
         upload(d_fsmall_, F.small_list.data(), F.small_list.size(), st, err) &&
         upload(d_fext_, F.ext_tasks.data(), F.ext_tasks.size(), st, err) &&

@@ -321,8 +321,6 @@ class Engine {
   // Adjoint (swc_adjoint.cu), on the current factor; device pointers, grad has one entry
   // per stored nonzero of A.
   bool logdet(double *out, std::string &err);
-  bool selected_inverse(std::string &err);   // Z = A^{-1} on the pattern of L
-  const double *selected_inverse_ptr() const { return d_adj_Z_; }
   bool logdet_grad(double *grad, std::string &err);
   bool solve_grad(const double *x, const double *lam, double *grad, std::string &err);
 
@@ -337,13 +335,13 @@ class Engine {
   std::shared_ptr<AdjointPlan> adj_;
   HostSym hsym_;
   std::vector<int> h_Ls_;
-  int4 *d_adj_units_ = nullptr;
-  int64_t *d_adj_tinv_off_ = nullptr, *d_adj_seg_tbl_ = nullptr;
-  int2 *d_adj_tasks_ = nullptr;
-  int *d_adj_wave_units_ = nullptr, *d_adj_ut_begin_ = nullptr, *d_adj_ut_end_ = nullptr;
-  int *d_adj_rowseg_ = nullptr, *d_adj_seg_t_ = nullptr, *d_adj_seg_S_ = nullptr;
-  int *d_adj_tbl_ = nullptr;
-  double *d_adj_Z_ = nullptr, *d_adj_U_ = nullptr, *d_adj_tinv_ = nullptr, *d_adj_P_ = nullptr;
+  int *d_adj_parent_ = nullptr, *d_adj_warp_ = nullptr, *d_adj_cta_ = nullptr;
+  char *d_adj_kids_ = nullptr;
+  int64_t *d_adj_zoff_ = nullptr;
+  int4 *d_adj_copies_ = nullptr, *d_adj_tasks_ = nullptr, *d_adj_units_ = nullptr;
+  double *d_adj_Z_ = nullptr, *d_adj_UT_ = nullptr, *d_adj_P_ = nullptr, *d_adj_grad_ = nullptr;
+  cudaGraphExec_t adj_graph_ = nullptr;
+  void run_adjoint();
   double *d_adj_partial_ = nullptr;
 
   void release();
@@ -361,6 +359,7 @@ class Engine {
   int64_t *d_fcb_off_ = nullptr;
   double *d_cb_ = nullptr;
   int fwarp_ctas_ = 0, fcta_ctas_ = 0;
+  bool prepare_tree(std::string &err);   // the tree's tables (also the adjoint's)
   bool prepare_front(std::string &err);
   void release_front();
   int finish(int *info, std::string &err);

@@ -17,6 +17,7 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <map>
 #include <string>
 #include <vector>
 
@@ -29,6 +30,9 @@ namespace swc {
 constexpr int FRONT_WARP_ELEMS = 1280;
 constexpr int FRONT_WARP_M = 128;
 constexpr int FRONT_KIDS = 4;   // children whose row maps are held at a time
+// Fronts of the warp kernels sit on levels of at least this many of them: below, a CTA per front
+// finishes the level sooner than warps that leave the SMs idle.
+constexpr int FRONT_WARP_LEVEL_MIN = 1024;
 
 // Padded front in shared memory: the w columns padded to a multiple of 8 (identity), the
 // off-diagonal rows below them, and a leading dimension of 4 mod 16 doubles, with which the
@@ -41,6 +45,26 @@ __host__ __device__ inline int front_ld(int w, int m) {
 inline int64_t front_smem(int w, int64_t m) {
   return 8LL * front_wp(w) * front_ld(w, (int)m) + 8 * 64 + 2LL * FRONT_KIDS * ((m + 3) & ~3LL);
 }
+
+// The adjoint's small fronts: padded panel, a second one (at least 64 doubles per warp), the
+// inverse of the diagonal block (leading dimension 4 mod 16), the row map.
+__host__ __device__ inline int adj_ldt(int w) { return front_wp(w) + ((4 - front_wp(w)) & 15); }
+inline int64_t adj_small_smem(int w, int64_t m, bool y_global) {
+  const int64_t pe = (int64_t)front_wp(w) * front_ld(w, (int)m);
+  return 8 * (pe + (pe > 512 && !y_global ? pe : 512) + (int64_t)front_wp(w) * adj_ldt(w)) + 4 * (m + 1);
+}
+
+// First-fit placement of blocks that live over a range of waves.
+class FrontArena {
+ public:
+  int64_t take(int64_t len);
+  void give(int64_t at, int64_t len);
+  int64_t end() const { return end_; }
+
+ private:
+  std::map<int64_t, int64_t> free_;
+  int64_t end_ = 0;
+};
 
 // Device view of the plan.
 struct FrontDev {
@@ -60,7 +84,8 @@ struct FrontWave {
 };
 
 struct FrontPlan {
-  bool ok = false;                 // the structure allows it (see build_front_plan)
+  bool closed = false;             // the tree below holds: children's rows among the parent's
+  bool ok = false;                 // the factorization allows it (see build_front_plan)
   std::vector<int> child_ptr, child, child_n1, rel, apos;
   std::vector<int64_t> cb_off;
   int64_t cb_len = 0;              // doubles of contribution blocks alive at once

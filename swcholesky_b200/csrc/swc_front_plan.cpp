@@ -9,9 +9,6 @@ namespace swc {
 
 namespace {
 
-// Fronts of the warp walk sit on levels of at least this many of them: below, a CTA per front
-// finishes the level sooner than warps that leave the SMs idle.
-constexpr int FRONT_WARP_LEVEL_MIN = 1024;
 // Largest contribution block a walk's CTA forms by itself, and a level launch's; larger ones
 // go to 64x64 tiles over the whole GPU.
 constexpr int FRONT_WALK_R = 512;
@@ -44,49 +41,41 @@ bool prune_sets_complete(const int *Ls, const int *prunePtr, const int *pruneSet
   return true;
 }
 
-// First-fit placement of blocks that live over a range of waves.
-class Arena {
- public:
-  int64_t take(int64_t len) {
-    for (auto it = free_.begin(); it != free_.end(); ++it)
-      if (it->second >= len) {
-        const int64_t at = it->first, rest = it->second - len;
-        free_.erase(it);
-        if (rest) free_[at + len] = rest;
-        return at;
-      }
-    const int64_t at = end_;
-    end_ += len;
-    return at;
-  }
-  void give(int64_t at, int64_t len) {
-    auto it = free_.emplace(at, len).first;
-    auto nx = std::next(it);
-    if (nx != free_.end() && it->first + it->second == nx->first) {
-      it->second += nx->second;
-      free_.erase(nx);
-    }
-    if (it != free_.begin()) {
-      auto pv = std::prev(it);
-      if (pv->first + pv->second == it->first) {
-        pv->second += it->second;
-        free_.erase(it);
-      }
-    }
-  }
-  int64_t end() const { return end_; }
-
- private:
-  std::map<int64_t, int64_t> free_;
-  int64_t end_ = 0;
-};
-
 struct Tile {
   int4 task;
   std::vector<int4> pairs;
 };
 
 }  // namespace
+
+int64_t FrontArena::take(int64_t len) {
+  for (auto it = free_.begin(); it != free_.end(); ++it)
+    if (it->second >= len) {
+      const int64_t at = it->first, rest = it->second - len;
+      free_.erase(it);
+      if (rest) free_[at + len] = rest;
+      return at;
+    }
+  const int64_t at = end_;
+  end_ += len;
+  return at;
+}
+
+void FrontArena::give(int64_t at, int64_t len) {
+  auto it = free_.emplace(at, len).first;
+  auto nx = std::next(it);
+  if (nx != free_.end() && it->first + it->second == nx->first) {
+    it->second += nx->second;
+    free_.erase(nx);
+  }
+  if (it != free_.begin()) {
+    auto pv = std::prev(it);
+    if (pv->first + pv->second == it->first) {
+      pv->second += it->second;
+      free_.erase(it);
+    }
+  }
+}
 
 void build_front_plan(int n, const int *c, const int *r, const int *Ls, const int *prunePtr,
                       const int *pruneSet, const HostSym &H, const Plan &P, const Tuning &T,
@@ -100,7 +89,6 @@ void build_front_plan(int n, const int *c, const int *r, const int *Ls, const in
   std::vector<int> col2sup(n);
   for (int s = 0; s < ns; ++s)
     for (int j = super[s]; j < super[s + 1]; ++j) col2sup[j] = s;
-  if (!prune_sets_complete(Ls, prunePtr, pruneSet, H, col2sup)) return;
 
   // tree, the children's positions in their parent, levels
   std::vector<int> parent(ns, -1), level(ns, 0);
@@ -146,6 +134,9 @@ void build_front_plan(int n, const int *c, const int *r, const int *Ls, const in
       for (int i = 0; i < m; ++i) at[rs[i]] = -1;
     }
   }
+
+  F.closed = true;
+  if (!prune_sets_complete(Ls, prunePtr, pruneSet, H, col2sup)) return;
 
   // classes
   std::vector<char> tiled(ns, 0);
@@ -269,7 +260,7 @@ void build_front_plan(int n, const int *c, const int *r, const int *Ls, const in
   // contribution blocks: a block lives from its supernode's wave (the walks': from the start)
   // to the end of its parent's wave (the walks': the end of the walks)
   F.cb_off.assign(ns, 0);
-  Arena A;
+  FrontArena A;
   auto len = [&](int s) {
     const int64_t rr = rows(s) - width(s);
     return (rr * rr + 15) & ~(int64_t)15;
