@@ -20,9 +20,10 @@
 // one; a front lives until its children are done, in an arena placed at analysis.  Supernodes
 // without children keep only their panel.  Small supernodes take one kernel per level (a warp
 // or a CTA each, everything in shared memory but Z_RR, which is read once from the parent's
-// front); wide ones 64-column steps of three launches with 64x64 DMMA tiles.  Against the sweep
-// it replaces (one 64-row FMA tile per column block and row block, Z_RR gathered entry by
-// entry from all ancestors): see the launch code below.
+// front); wide ones 64-column steps of three launches with 64x64 DMMA tiles.  Bound: the chain of
+// steps from the root (22 of them for a 320 x 310 5-point grid, about 45 us each), then the
+// small fronts' latency.  Against a sweep of 64-row FMA tiles per column block with Z_RR
+// gathered entry by entry from all ancestors, that grid's gradient takes 1.3 ms, not 4.4 (B200).
 //
 // Functions of x = A^{-1} b.  With lam = A^{-1} (df/dx):
 //     df/dA_ij = -(lam_i x_j + lam_j x_i)  (i != j),   -lam_i x_i  (i == j).
@@ -273,47 +274,47 @@ __global__ void __launch_bounds__(256) k_adj_copy(DevSym S, AdjDev A, const int4
 // task = (s, column block b, first row x0 of R, task index of x0 = 0): rows x0 .. x0 + 63 of
 // U = L_RK T with T the inverse of the diagonal block the factorization stored; U^T at
 // UT + 4096 * (first task) + row * 64.
-constexpr int ALD = TB + 1;
-constexpr int U_SMEM = 2 * TB * ALD * 8;
-__global__ void __launch_bounds__(256) k_adj_u(DevSym S, AdjDev A, const int4 *tasks) {
+// T(k, c) of the diagonal block at ti (column-major as the factorization stored it), as [k][c].
+__device__ __forceinline__ void load_tinv(double *Ts, const double *ti, int w) {
+#pragma unroll 8
+  for (int e = threadIdx.x; e < TB * TB; e += MT) {
+    const int c = e >> 6, k = e & (TB - 1);
+    Ts[k * LDS + c] = (k < w && c < w) ? ti[e] : 0.0;
+  }
+}
+
+constexpr int TT_SMEM = 2 * TB * LDS * 8;   // two 64x64 operands
+static_assert(2 * TB * LDS >= 2 * STAGE, "the product's stages fit");
+__global__ void __launch_bounds__(MT) k_adj_u(DevSym S, AdjDev A, const int4 *tasks) {
   extern __shared__ double zsm[];
-  double *Lx = zsm, *Ti = zsm + TB * ALD;   // [row][k], [k][col]
+  double *Ts = zsm, *Lx = zsm + TB * LDS;   // [k][column], [k][row]
   const int4 tk = tasks[blockIdx.x];
   const int s = tk.x, c0 = tk.y * TB, x0 = tk.z;
   const int m = nrows_of(S, s), w = min(TB, S.super[s + 1] - S.super[s] - c0), off = c0 + w;
   const int nrow = min(TB, m - off - x0);
   const double *Lb = S.L + S.xptr[s] + (size_t)c0 * m + off + x0;
-  const double *ti = S.dinv + ((size_t)S.dinv_off[s] + tk.y) * (TB * TB);
-  for (int e = threadIdx.x; e < TB * TB; e += 256) {
-    const int c = e >> 6, q = e & (TB - 1);
-    Lx[q * ALD + c] = (q < nrow && c < w) ? Lb[(size_t)c * m + q] : 0.0;
-    Ti[q * ALD + c] = (q < w && c < w) ? ti[e] : 0.0;
+  load_tinv(Ts, S.dinv + ((size_t)S.dinv_off[s] + tk.y) * (TB * TB), w);
+#pragma unroll 8
+  for (int e = threadIdx.x; e < TB * TB; e += MT) {
+    const int k = e >> 6, q = e & (TB - 1);
+    Lx[k * LDS + q] = (q < nrow && k < w) ? Lb[(size_t)k * m + q] : 0.0;
   }
   __syncthreads();
-  const int r0 = (threadIdx.x >> 4) * 4, cc0 = (threadIdx.x & 15) * 4;
-  double acc[4][4] = {};
-  for (int k = 0; k < w; ++k) {
-    double a[4], b[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) a[i] = Lx[(r0 + i) * ALD + k];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) b[j] = Ti[k * ALD + cc0 + j];
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) acc[i][j] = fma(a[i], b[j], acc[i][j]);
-  }
+  TileAcc acc;   // U^T: rows are columns of the block
+  acc.zero();
+  dmma_tile_smem(Ts, Lx, TB, acc);
   double *UT = A.UT + (size_t)tk.w * (TB * TB) + (size_t)x0 * TB;
 #pragma unroll
   for (int i = 0; i < 4; ++i)
-    if (r0 + i < nrow)
 #pragma unroll
-      for (int j = 0; j < 4; ++j) UT[(size_t)(r0 + i) * TB + cc0 + j] = acc[i][j];
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+      for (int e = 0; e < 2; ++e)
+        if (acc_col(j, e) < nrow) UT[(size_t)acc_col(j, e) * TB + acc_row(i)] = acc.v[i][j][e];
 }
 
 // The same rows of Z_RK = -Z_RR U (DMMA, K = all rows of R) and their share of U^T Z_RR U.
-constexpr int ZRK_SMEM = (2 * TB * ALD > 2 * STAGE ? 2 * TB * ALD : 2 * STAGE) * 8;
-__global__ void __launch_bounds__(MT, 2) k_adj_zrk(DevSym S, AdjDev A, const int4 *tasks) {
+__global__ void __launch_bounds__(MT, 3) k_adj_zrk(DevSym S, AdjDev A, const int4 *tasks) {
   extern __shared__ double zsm[];
   const int4 tk = tasks[blockIdx.x];
   const int s = tk.x, c0 = tk.y * TB, x0 = tk.z;
@@ -325,7 +326,7 @@ __global__ void __launch_bounds__(MT, 2) k_adj_zrk(DevSym S, AdjDev A, const int
   acc.zero();
   dmma_tile_product(Z + (size_t)off * m + off + x0, m, nrow, UT, TB, w, mr, zsm, acc);
   __syncthreads();
-  double *ys = zsm, *ux = zsm + TB * ALD;   // [row][column]
+  double *ys = zsm, *ux = zsm + TB * LDS;   // [row][column]
 #pragma unroll
   for (int i = 0; i < 4; ++i)
 #pragma unroll
@@ -333,85 +334,68 @@ __global__ void __launch_bounds__(MT, 2) k_adj_zrk(DevSym S, AdjDev A, const int
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
         const int r = acc_row(i), c = acc_col(j, e);
-        ys[r * ALD + c] = (r < nrow && c < w) ? acc.v[i][j][e] : 0.0;
+        ys[r * LDS + c] = (r < nrow && c < w) ? acc.v[i][j][e] : 0.0;
       }
+#pragma unroll 8
   for (int e = threadIdx.x; e < TB * TB; e += MT) {
     const int r = e >> 6, c = e & (TB - 1);
-    ux[r * ALD + c] = (r < nrow && c < w) ? UT[(size_t)(x0 + r) * TB + c] : 0.0;
+    ux[r * LDS + c] = (r < nrow && c < w) ? UT[(size_t)(x0 + r) * TB + c] : 0.0;
   }
   __syncthreads();
   for (int e = threadIdx.x; e < TB * TB; e += MT) {
     const int c = e >> 6, r = e & (TB - 1);
-    if (c < w && r < nrow) Z[(size_t)(c0 + c) * m + off + x0 + r] = -ys[r * ALD + c];
+    if (c < w && r < nrow) Z[(size_t)(c0 + c) * m + off + x0 + r] = -ys[r * LDS + c];
   }
   for (int e = threadIdx.x; e < TB * TB; e += MT) {
     const int r = e >> 6, c = e & (TB - 1);
-    if (c < w && r < nrow) Z[(size_t)(off + x0 + r) * m + c0 + c] = -ys[r * ALD + c];
+    if (c < w && r < nrow) Z[(size_t)(off + x0 + r) * m + c0 + c] = -ys[r * LDS + c];
   }
-  // U(X)^T Y(X), 4 x 8 entries per thread
-  const int i0 = (threadIdx.x >> 3) * 4, j0 = (threadIdx.x & 7) * 8;
-  double p[4][8] = {};
-  for (int k = 0; k < nrow; ++k) {
-    double a[4], b[8];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) a[i] = ux[k * ALD + i0 + i];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) b[j] = ys[k * ALD + j0 + j];
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-      for (int j = 0; j < 8; ++j) p[i][j] = fma(a[i], b[j], p[i][j]);
-  }
+  acc.zero();   // U(X)^T Y(X)
+  dmma_tile_smem(ux, ys, (nrow + 3) & ~3, acc);
   double *P = A.P + (size_t)blockIdx.x * (TB * TB);
 #pragma unroll
   for (int i = 0; i < 4; ++i)
 #pragma unroll
-    for (int j = 0; j < 8; ++j) P[(i0 + i) * TB + j0 + j] = p[i][j];
+    for (int j = 0; j < 4; ++j)
+      *reinterpret_cast<double2 *>(P + acc_row(i) * TB + acc_col(j, 0)) =
+          make_double2(acc.v[i][j][0], acc.v[i][j][1]);
 }
 
 // Z_KK = T^T T + the row blocks' shares.  unit = (s, column block, first task, tasks).
-__global__ void __launch_bounds__(256) k_adj_zkk(DevSym S, AdjDev A, const int4 *units) {
-  __shared__ double Ti[TB * ALD];   // [k][col]
+__global__ void __launch_bounds__(MT) k_adj_zkk(DevSym S, AdjDev A, const int4 *units) {
+  extern __shared__ double zsm[];
   const int4 un = units[blockIdx.x];
   const int s = un.x, c0 = un.y * TB;
   const int m = nrows_of(S, s), w = min(TB, S.super[s + 1] - S.super[s] - c0);
-  const double *ti = S.dinv + ((size_t)S.dinv_off[s] + un.y) * (TB * TB);
-  for (int e = threadIdx.x; e < TB * TB; e += 256) {
-    const int c = e >> 6, k = e & (TB - 1);
-    Ti[k * ALD + c] = (k < w && c < w) ? ti[e] : 0.0;
-  }
+  load_tinv(zsm, S.dinv + ((size_t)S.dinv_off[s] + un.y) * (TB * TB), w);
   __syncthreads();
-  const int r0 = (threadIdx.x >> 4) * 4, cc0 = (threadIdx.x & 15) * 4;
-  double acc[4][4] = {};
-  for (int k = 0; k < w; ++k) {
-    double a[4], b[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) a[i] = Ti[k * ALD + r0 + i];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) b[j] = Ti[k * ALD + cc0 + j];
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) acc[i][j] = fma(a[i], b[j], acc[i][j]);
-  }
+  TileAcc acc;
+  acc.zero();
+  dmma_tile_smem(zsm, zsm, TB, acc);
   for (int t = un.z; t < un.z + un.w; ++t) {
     const double *P = A.P + (size_t)t * (TB * TB);
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
-      for (int j = 0; j < 4; ++j) acc[i][j] += P[(r0 + i) * TB + cc0 + j];
+      for (int j = 0; j < 4; ++j) {
+        const double2 p = *reinterpret_cast<const double2 *>(P + acc_row(i) * TB + acc_col(j, 0));
+        acc.v[i][j][0] += p.x;
+        acc.v[i][j][1] += p.y;
+      }
   }
   double *Z = A.Z + A.zoff[s] + (size_t)c0 * m + c0;
 #pragma unroll
   for (int i = 0; i < 4; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int r = r0 + i, c = cc0 + j;
-      if (r < w && c <= r) {
-        Z[(size_t)c * m + r] = acc[i][j];
-        Z[(size_t)r * m + c] = acc[i][j];
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int r = acc_row(i), c = acc_col(j, e);
+        if (r < w && c <= r) {
+          Z[(size_t)c * m + r] = acc.v[i][j][e];
+          Z[(size_t)r * m + c] = acc.v[i][j][e];
+        }
       }
-    }
 }
 
 // Gradient of the entries of A in a wide supernode's columns: one warp per (s, column).
@@ -606,8 +590,8 @@ bool Engine::prepare_adjoint(std::string &err) {
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_adj_small, cudaFuncAttributeMaxDynamicSharedMemorySize, ADJ_SMEM_MAX);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_adj_warp, cudaFuncAttributeMaxDynamicSharedMemorySize, ZW_WARPS * ZW_SLICE);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_adj_u, cudaFuncAttributeMaxDynamicSharedMemorySize, U_SMEM);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_adj_zrk, cudaFuncAttributeMaxDynamicSharedMemorySize, ZRK_SMEM);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_adj_u, cudaFuncAttributeMaxDynamicSharedMemorySize, TT_SMEM);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_adj_zrk, cudaFuncAttributeMaxDynamicSharedMemorySize, TT_SMEM);
   if (e != cudaSuccess) {
     release_adjoint();
     err = std::string("adjoint setup: ") + cudaGetErrorString(e);
@@ -667,10 +651,10 @@ void Engine::run_adjoint() {
           sym_, A, d_adj_warp_ + W.warp_off, W.warp_cnt);
     for (const AdjointPlan::Step &t : W.steps) {
       if (t.task_cnt > 0) {
-        k_adj_u<<<t.task_cnt, 256, U_SMEM, st>>>(sym_, A, d_adj_tasks_ + t.task_off);
-        k_adj_zrk<<<t.task_cnt, MT, ZRK_SMEM, st>>>(sym_, A, d_adj_tasks_ + t.task_off);
+        k_adj_u<<<t.task_cnt, MT, TT_SMEM, st>>>(sym_, A, d_adj_tasks_ + t.task_off);
+        k_adj_zrk<<<t.task_cnt, MT, TT_SMEM, st>>>(sym_, A, d_adj_tasks_ + t.task_off);
       }
-      if (t.unit_cnt > 0) k_adj_zkk<<<t.unit_cnt, 256, 0, st>>>(sym_, A, d_adj_units_ + t.unit_off);
+      if (t.unit_cnt > 0) k_adj_zkk<<<t.unit_cnt, MT, TB * LDS * 8, st>>>(sym_, A, d_adj_units_ + t.unit_off);
     }
     const Wave &B = plan_.waves[AP.waves.size() - 1 - v];
     if (B.asm_cnt > 0)

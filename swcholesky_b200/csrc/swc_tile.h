@@ -123,6 +123,25 @@ __device__ __forceinline__ void dmma_tile_product(const double *__restrict__ Pa,
   }
 }
 
+// acc += A B^T of operands in shared memory ([k][row] and [k][column], leading dimension LDS),
+// K a multiple of 4, by the same four warps.
+__device__ __forceinline__ void dmma_tile_smem(const double *As, const double *Bs, int K, TileAcc &acc) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int wr = (warp >> 1) * 32, wc = (warp & 1) * 32;
+  const int kq = lane & 3, g = lane >> 2;
+  for (int k4 = 0; k4 < K; k4 += 4) {
+    double a[4], b[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) a[i] = As[(k4 + kq) * LDS + wr + 8 * i + g];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) b[j] = Bs[(k4 + kq) * LDS + wc + 8 * j + g];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) dmma(acc.v[i][j], a[i], b[j]);
+  }
+}
+
 // Sign flip through the integer pipe (FP64 arithmetic outside the tensor cores is slow).
 __device__ __forceinline__ double neg(double x) {
   return __longlong_as_double(__double_as_longlong(x) ^ (long long)0x8000000000000000ULL);
