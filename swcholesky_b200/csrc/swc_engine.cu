@@ -1370,12 +1370,14 @@ bool Engine::analyze(int n, const int *c, const int *r, const int64_t *lC, const
 }
 
 void Engine::release_front() {
-  void *ptrs[] = {d_fchild_ptr_, d_fchild_, d_fn1_, d_frel_, d_fapos_, d_fwarp_, d_fcta_, d_fsmall_,
+  void *ptrs[] = {d_frel_, d_fapos_, d_fppos_, d_fkids_, d_fwarp_, d_fcta_, d_fsmall_,
                   d_fext_end_, d_fsch_end_, d_fext_, d_fsch_, d_fext_pairs_, d_fsch_pairs_,
                   d_fcb_off_, d_cb_};
   for (void *p : ptrs)
     if (p) cudaFree(p);
-  d_fchild_ptr_ = d_fchild_ = d_fn1_ = d_frel_ = d_fapos_ = d_fwarp_ = d_fcta_ = d_fsmall_ = nullptr;
+  d_frel_ = d_fapos_ = d_fppos_ = nullptr;
+  d_fkids_ = nullptr;
+  d_fwarp_ = d_fcta_ = d_fsmall_ = nullptr;
   d_fext_end_ = d_fsch_end_ = nullptr;
   d_fext_ = d_fsch_ = d_fext_pairs_ = d_fsch_pairs_ = nullptr;
   d_fcb_off_ = nullptr;
@@ -1389,10 +1391,7 @@ bool Engine::prepare_tree(std::string &err) {
   if (d_frel_) return true;
   const FrontPlan &F = *front_;
   cudaStream_t st = stream_;
-  if (!(upload(d_fchild_ptr_, F.child_ptr.data(), F.child_ptr.size(), st, err) &&
-        upload(d_fchild_, F.child.data(), F.child.size(), st, err) &&
-        upload(d_fn1_, F.child_n1.data(), F.child_n1.size(), st, err) &&
-        upload(d_fapos_, F.apos.data(), F.apos.size(), st, err) &&
+  if (!(upload(d_fapos_, F.apos.data(), F.apos.size(), st, err) &&
         upload(d_frel_, F.rel.data(), F.rel.size(), st, err)))
     return false;
   if (cudaStreamSynchronize(st) != cudaSuccess) { err = "device upload: elimination tree"; return false; }
@@ -1411,9 +1410,11 @@ bool Engine::prepare_front(std::string &err) {
     d_cb_ = nullptr;
     return true;
   }
-  if (!(prepare_tree(err) && upload(d_fwarp_, F.warp_list.data(), F.warp_list.size(), st, err) &&
-        upload(d_fcta_, F.cta_list.data(), F.cta_list.size(), st, err) &&
-        upload(d_fsmall_, F.small_list.data(), F.small_list.size(), st, err) &&
+  if (!(prepare_tree(err) && upload(d_fwarp_, F.warp_desc.data(), F.warp_desc.size(), st, err) &&
+        upload(d_fcta_, F.cta_desc.data(), F.cta_desc.size(), st, err) &&
+        upload(d_fsmall_, F.small_desc.data(), F.small_desc.size(), st, err) &&
+        upload(d_fkids_, F.kids.data(), F.kids.size(), st, err) &&
+        upload(d_fppos_, F.ppos.data(), F.ppos.size(), st, err) &&
         upload(d_fext_, F.ext_tasks.data(), F.ext_tasks.size(), st, err) &&
         upload(d_fext_end_, F.ext_end.data(), F.ext_end.size(), st, err) &&
         upload(d_fext_pairs_, F.ext_pairs.data(), F.ext_pairs.size(), st, err) &&
@@ -1424,7 +1425,7 @@ bool Engine::prepare_front(std::string &err) {
     return false;
   if (cudaStreamSynchronize(st) != cudaSuccess) { err = "device upload: front plan"; return false; }
   front_dev_ = std::make_shared<FrontDev>(
-      FrontDev{d_fchild_ptr_, d_fchild_, d_fn1_, d_frel_, d_fapos_, d_fcb_off_, d_cb_});
+      FrontDev{d_fkids_, d_frel_, d_fppos_, d_fcb_off_, d_cb_});
   if (!F.warp_list.empty()) fwarp_ctas_ = front_warp_walk_ctas((int)F.warp_list.size());
   if (!F.cta_list.empty()) fcta_ctas_ = front_cta_walk_ctas(F.cta_smem, (int)F.cta_list.size());
   front_ready_ = true;

@@ -265,6 +265,8 @@ bool check_solve_plan(int n, const int *Ls, const HostSym &H, const SolvePlan &S
 
 struct FrontPlan;     // multifrontal FP64 factorization (swc_front.h)
 struct FrontDev;
+struct FrontDesc;
+struct FrontChild;
 struct AdjointPlan;   // reverse-sweep schedule of the adjoint (swc_adjoint.cu)
 
 class Engine {
@@ -352,8 +354,9 @@ class Engine {
   std::shared_ptr<FrontPlan> front_;
   std::shared_ptr<FrontDev> front_dev_;
   bool front_ready_ = false, front_tried_ = false;
-  int *d_fchild_ptr_ = nullptr, *d_fchild_ = nullptr, *d_fn1_ = nullptr, *d_frel_ = nullptr;
-  int *d_fapos_ = nullptr, *d_fwarp_ = nullptr, *d_fcta_ = nullptr, *d_fsmall_ = nullptr;
+  int *d_frel_ = nullptr, *d_fapos_ = nullptr, *d_fppos_ = nullptr;
+  FrontChild *d_fkids_ = nullptr;
+  FrontDesc *d_fwarp_ = nullptr, *d_fcta_ = nullptr, *d_fsmall_ = nullptr;
   int *d_fext_end_ = nullptr, *d_fsch_end_ = nullptr;
   int4 *d_fext_ = nullptr, *d_fsch_ = nullptr, *d_fext_pairs_ = nullptr, *d_fsch_pairs_ = nullptr;
   int64_t *d_fcb_off_ = nullptr;

@@ -15,7 +15,13 @@ namespace swc {
 
 namespace {
 
-constexpr int FT = 256, FW = FT / 32;       // CTA fronts: threads, warps
+constexpr int FT = 256, FW = FT / 32;       // CTA fronts: threads, warps (largest)
+// Walks of at least this many fronts use CTAs of 128 threads, three to an SM, others one of 256:
+// long walks are bound by how many fronts are in flight (60^3 7-point grid, 5,900 fronts:
+// 15.58 against 15.81 ms), short ones by each front's latency (100 x 100 5-point grid, 1,221
+// fronts: 319 against 390 us).
+constexpr int FRONT_MANY = 2048;
+constexpr int ET = 256;                     // extend-add tiles
 constexpr int WW = 4;                       // warp fronts: warps per CTA
 constexpr int WARP_SLICE = FRONT_WARP_ELEMS * 8 + 64 * 8 + FRONT_KIDS * FRONT_WARP_M * 2;
 constexpr int WARP_SMEM = WW * WARP_SLICE;
@@ -25,202 +31,185 @@ __device__ __forceinline__ void group_sync() {
   if (NW == 1) __syncwarp(); else __syncthreads();
 }
 
-// The whole factorization of one small front s in shared memory by NW warps:
-//   assembly of A and of the children's blocks into the padded panel P, Cholesky by 8-column
-//   blocks (the 8x8 diagonal blocks by one warp with their inverses, everything else 8x8x4
-//   DMMA products), the panel to L, and the contribution block
-//   CB_s = (children's blocks) - L_rs L_rs^T to global memory unless cb_by_tiles.
-// Bound: latency (the chain of 8x8 pivots blocks, then barriers); a front of 16 columns and 50
-// rows takes a few microseconds.  T: 64 doubles (inverse of the current diagonal block), inv:
-// FRONT_KIDS row maps of m entries.
+// The whole factorization of one small front in shared memory by NW warps:
+//   row maps of the children (up to FRONT_KIDS at a time), the padded panel P gathered from the
+//   children's blocks through them, A's entries, the panel's Cholesky (chol_panel), the panel to
+//   L, and the contribution block CB = (children's blocks) - L_rs L_rs^T to global memory
+//   (unless d.cb < 0).
+// Bound: latency.  A front passes four dependent global loads (its children's descriptors,
+// their row maps, their blocks; A's entries beside them), the chain of pivots and seven or so
+// barriers; the loads of a phase are issued together, several per thread.  sc: 64 doubles per
+// warp, inv: FRONT_KIDS row maps of m entries (inv[k * mm + i]: child k's index of row i, or -1).
 template <int NW>
-__device__ void front_body(const DevSym &S, const FrontDev &F, int s, bool cb_by_tiles, double *P,
-                           double *T, short *inv) {
+__device__ __forceinline__ void build_maps(const FrontDev &F, int q0, int kids, int w, int m, int mm,
+                                           short *inv, const double *(&cb)[FRONT_KIDS],
+                                           int (&rc)[FRONT_KIDS]) {
+  constexpr int NTH = 32 * NW;
+  const int t = NW == 1 ? (int)(threadIdx.x & 31) : (int)threadIdx.x;
+  int64_t rel[FRONT_KIDS];
+#pragma unroll
+  for (int k = 0; k < FRONT_KIDS; ++k) {
+    cb[k] = nullptr;
+    rc[k] = 0;
+    rel[k] = 0;
+    if (k < kids) {
+      const FrontChild c = F.child[q0 + k];
+      rc[k] = c.rc;
+      rel[k] = c.rel;
+      cb[k] = F.cb + c.cb;
+    }
+  }
+  for (int i = t; i < kids * mm; i += NTH) inv[i] = -1;
+  group_sync<NW>();
+#pragma unroll
+  for (int k = 0; k < FRONT_KIDS; ++k)
+    for (int i = t; i < rc[k]; i += NTH) inv[k * mm + F.rel[rel[k] + i]] = (short)i;
+  group_sync<NW>();
+}
+
+template <int NW>
+__device__ void front_body(const DevSym &S, const FrontDev &F, const FrontDesc &d, double *P, double *sc,
+                           short *inv) {
   constexpr int NTH = 32 * NW;
   const int t = NW == 1 ? (int)(threadIdx.x & 31) : (int)threadIdx.x;
   const int lane = t & 31, warp = t >> 5, g = lane >> 2, kq = lane & 3;
-  const int f = S.super[s], w = S.super[s + 1] - f;
-  const int64_t rb = S.rowptr[s];
-  const int m = (int)(S.rowptr[s + 1] - rb), r = m - w;
-  const int wp = front_wp(w), ld = front_ld(w, m), pad = wp - w;
+  const int w = d.w, m = d.m, r = m - w;
+  const int wp = front_wp(w), ld = front_ld(w, m), pad = wp - w, mm = (m + 3) & ~3;
   const int nrb = (wp + ((r + 7) & ~7)) >> 3, nkb = wp >> 3;   // 8-row / 8-column blocks
-  const int ch0 = F.child_ptr[s], ch1 = F.child_ptr[s + 1];
+  const double *cb[FRONT_KIDS];
+  int rc[FRONT_KIDS];
+  int kids = min(FRONT_KIDS, d.ch1 - d.ch0);
+  build_maps<NW>(F, d.ch0, kids, w, m, mm, inv, cb, rc);
 
-  for (int i = t; i < wp * ld; i += NTH) P[i] = 0.0;
-  group_sync<NW>();
-  if (t < pad) P[(w + t) * ld + w + t] = 1.0;
-  // A: one warp per column (front row i at i, or i + pad below the padded columns)
-  for (int j = warp; j < w; j += NW)
-    for (int p = S.Ap[f + j] + lane; p < S.Ap[f + j + 1]; p += 32) {
-      const int pos = F.apos[p];
-      if (pos >= 0) P[j * ld + (pos < w ? pos : pos + pad)] = S.Ax[p];
-      else atomicExch(&S.status[1], 1);
-    }
-  group_sync<NW>();
-  // children's blocks, the columns that are columns of s
-  for (int q = ch0; q < ch1; ++q) {
-    const int c = F.child[q];
-    const int64_t ro = S.rowptr[c] - S.super[c];
-    const int rc = (int)(S.rowptr[c + 1] - S.rowptr[c]) - (S.super[c + 1] - S.super[c]);
-    const int n1 = F.child_n1[c];
-    const int *rel = F.rel + ro;
-    const double *cb = F.cb + F.cb_off[c];
-    for (int j = warp; j < n1; j += NW) {
-      const int pj = rel[j];
-      for (int i = j + lane; i < rc; i += 32) {
-        const int pi = rel[i];
-        P[pj * ld + (pi < w ? pi : pi + pad)] += cb[(size_t)j * rc + i];
+  // the panel from the children's blocks (padded diagonal: ones), four entries per thread at a time
+  for (int q0 = d.ch0;;) {
+    const bool first = q0 == d.ch0;
+    for (int e0 = t; e0 < wp * ld; e0 += 4 * NTH) {
+      double v[4][FRONT_KIDS];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int e = e0 + u * NTH, j = e / ld, i = e - j * ld;
+        const int row = i < wp ? i : i - pad;
+        const bool in = e < wp * ld && j < w && (i < wp ? i < w && i >= j : row < m);
+#pragma unroll
+        for (int k = 0; k < FRONT_KIDS; ++k) {
+          v[u][k] = 0.0;
+          if (k < kids) {
+            const int pi = in ? inv[k * mm + row] : -1, pj = in ? inv[k * mm + j] : -1;
+            v[u][k] = ld_if(cb[k] + (int64_t)pj * rc[k] + pi, pi >= 0 && pj >= 0);
+          }
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int e = e0 + u * NTH;
+        if (e < wp * ld) {
+          const int j = e / ld;
+          double x = first ? (j >= w && e == j * ld + j ? 1.0 : 0.0) : P[e];
+#pragma unroll
+          for (int k = 0; k < FRONT_KIDS; ++k) x += v[u][k];
+          P[e] = x;
+        }
       }
     }
+    q0 += FRONT_KIDS;
+    if (q0 >= d.ch1) break;
     group_sync<NW>();
+    kids = min(FRONT_KIDS, d.ch1 - q0);
+    build_maps<NW>(F, q0, kids, w, m, mm, inv, cb, rc);
   }
+  group_sync<NW>();
+  for (int p = d.a0 + t; p < d.a1; p += NTH) {
+    const int pos = F.ppos[p];
+    if (pos >= 0) P[pos] += S.Ax[p];
+    else atomicExch(&S.status[1], 1);
+  }
+  group_sync<NW>();
 
-  // Cholesky of the panel by 8-column blocks; warp 0 factors the next diagonal block while the
-  // others update the rest
-  if (warp == 0) potrf8_inv8(P, ld, T, S.status, f, w);
-  group_sync<NW>();
-  for (int kb = 0; kb < nkb; ++kb) {
-    const int k0 = 8 * kb;
-    // rows below: X = B L_kk^{-T}, four row blocks of a warp interleaved
-    for (int ib0 = kb + 1 + 4 * warp; ib0 < nrb; ib0 += 4 * NW) {
-      double c[4][2];
-#pragma unroll
-      for (int q = 0; q < 4; ++q) c[q][0] = c[q][1] = 0.0;
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const double b = T[(4 * h + kq) * 8 + g];
-#pragma unroll
-        for (int q = 0; q < 4; ++q)
-          if (ib0 + q < nrb) dmma(c[q], P[(k0 + 4 * h + kq) * ld + 8 * (ib0 + q) + g], b);
-      }
-      __syncwarp();
-#pragma unroll
-      for (int q = 0; q < 4; ++q)
-        if (ib0 + q < nrb) {
-          P[(k0 + 2 * kq) * ld + 8 * (ib0 + q) + g] = c[q][0];
-          P[(k0 + 2 * kq + 1) * ld + 8 * (ib0 + q) + g] = c[q][1];
-        }
-    }
-    group_sync<NW>();
-    if (kb + 1 >= nkb) break;
-    // trailing blocks (ib, jb), kb < jb <= ib: minus X_ib X_jb^T
-    auto update4 = [&](int jb, int ib0, int ib1) {   // row blocks ib0 .. min(ib0 + 4, ib1) - 1
-      double c[4][2];
-#pragma unroll
-      for (int q = 0; q < 4; ++q)
-        if (ib0 + q < ib1) {
-          c[q][0] = P[(8 * jb + 2 * kq) * ld + 8 * (ib0 + q) + g];
-          c[q][1] = P[(8 * jb + 2 * kq + 1) * ld + 8 * (ib0 + q) + g];
-        }
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const double b = neg(P[(k0 + 4 * h + kq) * ld + 8 * jb + g]);
-#pragma unroll
-        for (int q = 0; q < 4; ++q)
-          if (ib0 + q < ib1) dmma(c[q], P[(k0 + 4 * h + kq) * ld + 8 * (ib0 + q) + g], b);
-      }
-#pragma unroll
-      for (int q = 0; q < 4; ++q)
-        if (ib0 + q < ib1) {
-          P[(8 * jb + 2 * kq) * ld + 8 * (ib0 + q) + g] = c[q][0];
-          P[(8 * jb + 2 * kq + 1) * ld + 8 * (ib0 + q) + g] = c[q][1];
-        }
-    };
-    const int nb = kb + 1;
-    if (warp == 0) {
-      update4(nb, nb, nb + 1);
-      __syncwarp();
-      potrf8_inv8(P + 8 * nb * ld + 8 * nb, ld, T, S.status, f + 8 * nb, w - 8 * nb);
-    }
-    if (NW == 1 || warp > 0) {
-      const int u = NW == 1 ? 0 : warp - 1, nu = NW == 1 ? 1 : NW - 1;
-      int strip = 0;
-      for (int jb = nb; jb < nkb; ++jb)
-        for (int ib0 = jb == nb ? jb + 1 : jb; ib0 < nrb; ib0 += 4, ++strip)
-          if (strip % nu == u) update4(jb, ib0, nrb);
-    }
-    group_sync<NW>();
-  }
+  chol_panel<NW>(P, ld, nkb, nrb, sc, S.status, d.f, w);
 
   // the panel to L (upper triangle of the diagonal block: zeros, as stored by the reference)
-  double *dst = S.L + S.xptr[s];
+  double *dst = S.L + d.xoff;
   for (int j = warp; j < w; j += NW)
     for (int i = lane; i < m; i += 32)
       dst[(size_t)j * m + i] = i < j ? 0.0 : P[j * ld + (i < w ? i : i + pad)];
 
-  if (r == 0 || cb_by_tiles) return;
-  double *cbs = F.cb + F.cb_off[s];
+  if (r == 0 || d.cb < 0) return;
+  double *cbs = F.cb + d.cb;
   const int r8 = (r + 7) >> 3;
-  int q0 = ch0;
-  do {
-    // row maps of up to FRONT_KIDS children: inv[k * m + i] = the child's index of s's
-    // off-diagonal row i, or -1
-    const int kids = min(FRONT_KIDS, ch1 - q0);
-    for (int i = t; i < kids * r; i += NTH) inv[i] = -1;
-    group_sync<NW>();
-    const double *cbc[FRONT_KIDS];
-    int rc[FRONT_KIDS];
-#pragma unroll
-    for (int k = 0; k < FRONT_KIDS; ++k) {
-      cbc[k] = nullptr;
-      rc[k] = 0;
-      if (k < kids) {
-        const int c = F.child[q0 + k];
-        rc[k] = (int)(S.rowptr[c + 1] - S.rowptr[c]) - (S.super[c + 1] - S.super[c]);
-        cbc[k] = F.cb + F.cb_off[c];
-        const int *rel = F.rel + (S.rowptr[c] - S.super[c]);
-        for (int i = F.child_n1[c] + t; i < rc[k]; i += NTH) inv[k * r + rel[i] - w] = (short)i;
-      }
+  const bool many = d.ch1 - d.ch0 > FRONT_KIDS;
+  for (int q0 = d.ch0;;) {
+    const bool first = q0 == d.ch0;
+    if (many) {
+      kids = min(FRONT_KIDS, d.ch1 - q0);
+      group_sync<NW>();
+      build_maps<NW>(F, q0, kids, w, m, mm, inv, cb, rc);
     }
-    group_sync<NW>();
+    const short *im = inv + w;   // off-diagonal rows
     int strip = 0;
     for (int bj = 0; bj < r8; ++bj)
       for (int bi0 = bj; bi0 < r8; bi0 += 4, ++strip) {
         if (strip % NW != warp) continue;
+        // the children's entries first: in flight during the product
+        const int j0 = 8 * bj + 2 * kq;
+        double v[FRONT_KIDS][4][2], old[4][2];
+        int pj[FRONT_KIDS][2];
+#pragma unroll
+        for (int k = 0; k < FRONT_KIDS; ++k)
+#pragma unroll
+          for (int e = 0; e < 2; ++e) pj[k][e] = k < kids && j0 + e < r ? im[k * mm + j0 + e] : -1;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const int i = 8 * (bi0 + q) + g;
+#pragma unroll
+          for (int e = 0; e < 2; ++e)
+            old[q][e] = first ? 0.0 : ld_if(cbs + (size_t)(j0 + e) * r + i, i < r && j0 + e <= i);
+#pragma unroll
+          for (int k = 0; k < FRONT_KIDS; ++k) {
+            v[k][q][0] = v[k][q][1] = 0.0;
+            if (k < kids) {
+              const int pi = i < r ? im[k * mm + i] : -1;
+#pragma unroll
+              for (int e = 0; e < 2; ++e)
+                v[k][q][e] = ld_if(cb[k] + (int64_t)pj[k][e] * rc[k] + pi, pi >= 0 && pj[k][e] >= 0 && j0 + e <= i);
+            }
+          }
+        }
         double c[4][2];
 #pragma unroll
         for (int q = 0; q < 4; ++q) c[q][0] = c[q][1] = 0.0;
-        if (q0 == ch0) {
+        if (first)
           for (int k = 0; k < wp; k += 4) {
             const double b = neg(P[(k + kq) * ld + wp + 8 * bj + g]);
 #pragma unroll
             for (int q = 0; q < 4; ++q)
               if (bi0 + q < r8) dmma(c[q], P[(k + kq) * ld + wp + 8 * (bi0 + q) + g], b);
           }
-        }
-        const int j0 = 8 * bj + 2 * kq;
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
           const int i = 8 * (bi0 + q) + g;
 #pragma unroll
-          for (int e = 0; e < 2; ++e) {
-            const int j = j0 + e;
-            if (i < r && j <= i) {
-              double v = c[q][e];
-              if (q0 > ch0) v += cbs[(size_t)j * r + i];
+          for (int e = 0; e < 2; ++e)
+            if (i < r && j0 + e <= i) {
+              double x = c[q][e] + old[q][e];
 #pragma unroll
-              for (int k = 0; k < FRONT_KIDS; ++k)
-                if (k < kids) {
-                  const int pi = inv[k * r + i], pj = inv[k * r + j];
-                  if (pi >= 0 && pj >= 0) v += cbc[k][(size_t)pj * rc[k] + pi];
-                }
-              cbs[(size_t)j * r + i] = v;
+              for (int k = 0; k < FRONT_KIDS; ++k) x += v[k][q][e];
+              cbs[(size_t)(j0 + e) * r + i] = x;
             }
-          }
         }
       }
     q0 += FRONT_KIDS;
-    group_sync<NW>();
-  } while (q0 < ch1);
+    if (q0 >= d.ch1) break;
+  }
 }
 
-// Lane q waits (bounded by the poll budget) for the done flag of s's child q.
-__device__ __forceinline__ void wait_children(const DevSym &S, const FrontDev &F, int s,
+// Lane q waits (bounded by the poll budget) for the done flag of the front's child q.
+__device__ __forceinline__ void wait_children(const DevSym &S, const FrontDev &F, const FrontDesc &d,
                                               const int *done) {
   const long long budget = wait_budget(S.status);
   bool timed_out = false;
-  for (int q = F.child_ptr[s] + (int)(threadIdx.x & 31); q < F.child_ptr[s + 1] && !timed_out; q += 32) {
-    const int *flag = done + F.child[q];
+  for (int q = d.ch0 + (int)(threadIdx.x & 31); q < d.ch1 && !timed_out; q += 32) {
+    const int *flag = done + F.child[q].s;
     long long it = 0;
     while (ld_acquire_k(flag) == 0) {
       if (++it > budget) {
@@ -228,48 +217,60 @@ __device__ __forceinline__ void wait_children(const DevSym &S, const FrontDev &F
         timed_out = true;
         break;
       }
-      __nanosleep(32);
+      if (it > 64) __nanosleep(32);
     }
   }
 }
 
 // The fronts of the bottom of the tree (a set closed under descendants) in one persistent
 // launch: CTAs take fronts from a device queue in level order, wait for the fronts' children
-// (acquire on their done flags), factor and publish their own flag (release).  A CTA only
-// waits for fronts taken before its own, so the walk progresses whatever the number of
-// resident CTAs.  qctr[0]: queue head, qctr[1 + s]: done flags, zeroed before the launch.
-__global__ void __launch_bounds__(FT) k_front_cta_walk(DevSym S, FrontDev F, const int *order,
-                                                       int count, int *qctr) {
+// (acquire on their done flags), factor and publish their own flag (release).  A CTA takes its
+// next front, and loads its descriptor, while it works on the current one.  The unfinished
+// front that comes first in the order is being worked on (its CTA has no earlier one left) and
+// its children are finished, so the walk progresses whatever the number of resident CTAs.
+// qctr[0]: queue head, qctr[1 + s]: done flags, zeroed before the launch.
+template <int T>
+__global__ void __launch_bounds__(T, T == 128 ? 3 : 1) k_front_cta_walk(DevSym S, FrontDev F,
+                                                                       const FrontDesc *order, int count,
+                                                                       int *qctr) {
   extern __shared__ double fsm[];
-  __shared__ int item;
+  __shared__ FrontDesc desc[2];
+  __shared__ int item[2];
   int *done = qctr + 1;
-  for (;;) {
-    if (threadIdx.x == 0) item = atomicAdd(qctr, 1);
+  if (threadIdx.x == 0) {
+    const int i = atomicAdd(qctr, 1);
+    item[0] = i;
+    if (i < count) desc[0] = order[i];
+  }
+  __syncthreads();
+  for (int b = 0; item[b] < count; b ^= 1) {
+    const FrontDesc d = desc[b];
+    int next = 0;
+    if (threadIdx.x == T - 32) next = atomicAdd(qctr, 1);
+    if (threadIdx.x < 32) wait_children(S, F, d, done);
     __syncthreads();
-    const int idx = item;
-    if (idx >= count) break;
-    const int s = order[idx];
-    if (threadIdx.x < 32) wait_children(S, F, s, done);
-    __syncthreads();
-    front_body<FW>(S, F, s, false, fsm + 64, fsm, reinterpret_cast<short *>(
-        fsm + 64 + front_wp(S.super[s + 1] - S.super[s]) *
-                       front_ld(S.super[s + 1] - S.super[s], (int)(S.rowptr[s + 1] - S.rowptr[s]))));
+    double *P = fsm + (T / 32) * 64;
+    front_body<T / 32>(S, F, d, P, fsm, reinterpret_cast<short *>(P + front_wp(d.w) * front_ld(d.w, d.m)));
+    if (threadIdx.x == T - 32) {
+      item[b ^ 1] = next;
+      if (next < count) desc[b ^ 1] = order[next];
+    }
     __syncthreads();
     if (threadIdx.x == 0) {
       __threadfence();
-      st_release_k(done + s, 1);
+      st_release_k(done + d.s, 1);
     }
   }
 }
 
 // The same at warp granularity, for the crowded levels of tiny fronts.
-__global__ void __launch_bounds__(WW * 32) k_front_warp_walk(DevSym S, FrontDev F, const int *order,
+__global__ void __launch_bounds__(WW * 32) k_front_warp_walk(DevSym S, FrontDev F, const FrontDesc *order,
                                                              int count, int *qctr, int *qhead) {
   extern __shared__ double fsm[];
   const int lane = threadIdx.x & 31;
-  double *T = reinterpret_cast<double *>(reinterpret_cast<unsigned char *>(fsm) +
-                                         (size_t)(threadIdx.x >> 5) * WARP_SLICE);
-  double *P = T + 64;
+  double *sc = reinterpret_cast<double *>(reinterpret_cast<unsigned char *>(fsm) +
+                                          (size_t)(threadIdx.x >> 5) * WARP_SLICE);
+  double *P = sc + 64;
   short *inv = reinterpret_cast<short *>(P + FRONT_WARP_ELEMS);
   int *done = qctr + 1;
   for (;;) {
@@ -277,25 +278,24 @@ __global__ void __launch_bounds__(WW * 32) k_front_warp_walk(DevSym S, FrontDev 
     if (lane == 0) idx = atomicAdd(qhead, 1);
     idx = __shfl_sync(0xffffffffu, idx, 0);
     if (idx >= count) break;
-    const int s = order[idx];
-    wait_children(S, F, s, done);
+    const FrontDesc d = order[idx];
+    wait_children(S, F, d, done);
     __syncwarp();
-    front_body<1>(S, F, s, false, P, T, inv);
+    front_body<1>(S, F, d, P, sc, inv);
     __syncwarp();
     if (lane == 0) {
       __threadfence();
-      st_release_k(done + s, 1);
+      st_release_k(done + d.s, 1);
     }
   }
 }
 
 // One CTA per small front of a level.
-__global__ void __launch_bounds__(FT) k_front_small(DevSym S, FrontDev F, const int *list) {
+__global__ void __launch_bounds__(FT) k_front_small(DevSym S, FrontDev F, const FrontDesc *list) {
   extern __shared__ double fsm[];
-  const int e = list[blockIdx.x], s = e < 0 ? ~e : e;
-  const int w = S.super[s + 1] - S.super[s], m = (int)(S.rowptr[s + 1] - S.rowptr[s]);
-  front_body<FW>(S, F, s, e < 0, fsm + 64, fsm,
-                 reinterpret_cast<short *>(fsm + 64 + front_wp(w) * front_ld(w, m)));
+  const FrontDesc d = list[blockIdx.x];
+  double *P = fsm + FW * 64;
+  front_body<FW>(S, F, d, P, fsm, reinterpret_cast<short *>(P + front_wp(d.w) * front_ld(d.w, d.m)));
 }
 
 // Children's blocks into one 64x64 tile: row maps of up to FRONT_KIDS pairs at a time.  Pair
@@ -335,7 +335,7 @@ __device__ __forceinline__ void load_pair_maps(const DevSym &S, const FrontDev &
 // Extend-add into the panels of tiled supernodes: task = (s, r0, c0, first pair), a 64x64 tile
 // of the panel that some child's block reaches.  Bound: memory (the blocks are read once and
 // the touched tiles read and written once).
-__global__ void __launch_bounds__(FT) k_front_extend(DevSym S, FrontDev F, const int4 *tasks,
+__global__ void __launch_bounds__(ET) k_front_extend(DevSym S, FrontDev F, const int4 *tasks,
                                                      const int *end, const int4 *pairs) {
   __shared__ PairMaps M;
   const int4 tk = tasks[blockIdx.x];
@@ -344,26 +344,29 @@ __global__ void __launch_bounds__(FT) k_front_extend(DevSym S, FrontDev F, const
   const int w = S.super[s + 1] - S.super[s], m = (int)(S.rowptr[s + 1] - S.rowptr[s]);
   double *Lt = S.L + S.xptr[s] + (size_t)c0 * m + r0;
   const int row = threadIdx.x & 63, cq = threadIdx.x >> 6;   // columns cq, cq + 4, ..
-  constexpr int NE = TB * TB / FT;
+  constexpr int NE = TB * TB / ET;
   double v[NE];
 #pragma unroll
   for (int e = 0; e < NE; ++e) {
     const int col = cq + 4 * e;
-    v[e] = (r0 + row < m && c0 + col < w && r0 + row >= c0 + col) ? Lt[(size_t)col * m + row] : 0.0;
+    v[e] = ld_if(Lt + (size_t)col * m + row, r0 + row < m && c0 + col < w && r0 + row >= c0 + col);
   }
   for (int q = tk.w; q < p_end; q += FRONT_KIDS) {
     const int kids = min(FRONT_KIDS, p_end - q);
     if (q > tk.w) __syncthreads();
-    load_pair_maps(S, F, pairs, q, kids, r0, c0, M, FT);
+    load_pair_maps(S, F, pairs, q, kids, r0, c0, M, ET);
     for (int k = 0; k < kids; ++k) {
       const int pi = M.ia[k][row];
       const double *cb = M.cb[k] + pi;
       const int ldc = M.ld[k];
+      double t[NE];
 #pragma unroll
       for (int e = 0; e < NE; ++e) {
         const int col = cq + 4 * e, pj = M.ib[k][col];
-        if (pi >= 0 && pj >= 0 && r0 + row >= c0 + col) v[e] += cb[(size_t)pj * ldc];
+        t[e] = ld_if(cb + (int64_t)pj * ldc, pi >= 0 && pj >= 0 && r0 + row >= c0 + col);
       }
+#pragma unroll
+      for (int e = 0; e < NE; ++e) v[e] += t[e];
     }
   }
 #pragma unroll
@@ -398,14 +401,19 @@ __global__ void __launch_bounds__(MT, 4) k_front_schur(DevSym S, FrontDev F, con
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         const int pi = M.ia[k][acc_row(i)];
+        double t[4][2];
 #pragma unroll
         for (int j = 0; j < 4; ++j)
 #pragma unroll
           for (int e = 0; e < 2; ++e) {
             const int pj = M.ib[k][acc_col(j, e)];
-            if (pi >= 0 && pj >= 0 && i0 + acc_row(i) >= j0 + acc_col(j, e))
-              acc.v[i][j][e] -= cb[(size_t)pj * ldc + pi];
+            t[j][e] = ld_if(cb + (int64_t)pj * ldc + pi,
+                            pi >= 0 && pj >= 0 && i0 + acc_row(i) >= j0 + acc_col(j, e));
           }
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+#pragma unroll
+          for (int e = 0; e < 2; ++e) acc.v[i][j][e] -= t[j][e];
       }
     }
   }
@@ -437,8 +445,10 @@ int resident_ctas(const void *fn, int threads, int smem) {
 }  // namespace
 
 bool front_configure(std::string &err) {
-  cudaError_t e = cudaFuncSetAttribute(k_front_cta_walk, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  cudaError_t e = cudaFuncSetAttribute(k_front_cta_walk<FT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        200 * 1024);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(k_front_cta_walk<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(k_front_small, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
   if (e == cudaSuccess)
@@ -453,28 +463,31 @@ bool front_configure(std::string &err) {
 }
 
 int front_cta_walk_ctas(int smem, int count) {
-  return std::max(1, std::min(count, resident_ctas((const void *)k_front_cta_walk, FT, smem)));
+  const int most = count >= FRONT_MANY ? resident_ctas((const void *)k_front_cta_walk<128>, 128, smem)
+                                       : resident_ctas((const void *)k_front_cta_walk<FT>, FT, smem);
+  return std::max(1, std::min(count, most));
 }
 int front_warp_walk_ctas(int count) {
   return std::max(1, std::min((count + WW - 1) / WW,
                               resident_ctas((const void *)k_front_warp_walk, WW * 32, WARP_SMEM)));
 }
-void launch_front_warp_walk(const DevSym &S, const FrontDev &F, const int *order, int count,
+void launch_front_warp_walk(const DevSym &S, const FrontDev &F, const FrontDesc *order, int count,
                             int ctas, int *qctr, int *qhead, cudaStream_t st) {
   if (count > 0)
     k_front_warp_walk<<<ctas, WW * 32, WARP_SMEM, st>>>(S, F, order, count, qctr, qhead);
 }
-void launch_front_cta_walk(const DevSym &S, const FrontDev &F, const int *order, int count,
+void launch_front_cta_walk(const DevSym &S, const FrontDev &F, const FrontDesc *order, int count,
                            int smem, int ctas, int *qctr, cudaStream_t st) {
-  if (count > 0) k_front_cta_walk<<<ctas, FT, smem, st>>>(S, F, order, count, qctr);
+  if (count >= FRONT_MANY) k_front_cta_walk<128><<<ctas, 128, smem, st>>>(S, F, order, count, qctr);
+  else if (count > 0) k_front_cta_walk<FT><<<ctas, FT, smem, st>>>(S, F, order, count, qctr);
 }
-void launch_front_small(const DevSym &S, const FrontDev &F, const int *list, int count, int smem,
+void launch_front_small(const DevSym &S, const FrontDev &F, const FrontDesc *list, int count, int smem,
                         cudaStream_t st) {
   if (count > 0) k_front_small<<<count, FT, smem, st>>>(S, F, list);
 }
 void launch_front_extend(const DevSym &S, const FrontDev &F, const int4 *tasks, const int *end,
                          const int4 *pairs, int count, cudaStream_t st) {
-  if (count > 0) k_front_extend<<<count, FT, 0, st>>>(S, F, tasks, end, pairs);
+  if (count > 0) k_front_extend<<<count, ET, 0, st>>>(S, F, tasks, end, pairs);
 }
 void launch_front_schur(const DevSym &S, const FrontDev &F, const int4 *tasks, const int *end,
                         const int4 *pairs, int count, cudaStream_t st) {

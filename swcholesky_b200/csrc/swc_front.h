@@ -43,7 +43,7 @@ __host__ __device__ inline int front_ld(int w, int m) {
   return rows + ((4 - rows) & 15);
 }
 inline int64_t front_smem(int w, int64_t m) {
-  return 8LL * front_wp(w) * front_ld(w, (int)m) + 8 * 64 + 2LL * FRONT_KIDS * ((m + 3) & ~3LL);
+  return 8LL * front_wp(w) * front_ld(w, (int)m) + 8 * 8 * 64 + 2LL * FRONT_KIDS * ((m + 3) & ~3LL);
 }
 
 // The adjoint's small fronts: padded panel, a second one (at least 64 doubles per warp), the
@@ -66,13 +66,25 @@ class FrontArena {
   int64_t end_ = 0;
 };
 
+// What a front's kernel needs to know, in one load each: the front (in list order), and its
+// children (in child_ptr order).
+struct __align__(16) FrontDesc {
+  int s, f, w, m;
+  int ch0, ch1, a0, a1;            // children, entries of A in its columns
+  int64_t xoff, cb;                // offsets in L and in the contribution blocks
+};
+struct __align__(16) FrontChild {
+  int s, rc, n1, pad;              // supernode, rows of its block, rows that are columns of the parent
+  int64_t rel, cb;                 // offsets of its row map and of its block
+};
+
 // Device view of the plan.
 struct FrontDev {
-  const int *child_ptr, *child;   // children of each supernode, in increasing order
-  const int *child_n1;            // per supernode: its rows that are columns of its parent
+  const FrontChild *child;
   const int *rel;                 // per off-diagonal row (at rowptr[s] - super[s]): position in
                                   // the parent's row list
-  const int *apos;                // per entry of A: position in its column's row list (-1: none)
+  const int *ppos;                // per entry of A in a small front: its place in the padded panel
+                                  // (-1: outside the pattern)
   const int64_t *cb_off;          // per supernode: its contribution block in cb
   double *cb;
 };
@@ -86,7 +98,11 @@ struct FrontWave {
 struct FrontPlan {
   bool closed = false;             // the tree below holds: children's rows among the parent's
   bool ok = false;                 // the factorization allows it (see build_front_plan)
-  std::vector<int> child_ptr, child, child_n1, rel, apos;
+  std::vector<int> child_ptr, child, child_n1, rel;
+  std::vector<int> apos;           // per entry of A: position in its column's row list (-1: none)
+  std::vector<int> ppos;           // see FrontDev
+  std::vector<FrontChild> kids;    // in child order
+  std::vector<FrontDesc> warp_desc, cta_desc, small_desc;
   std::vector<int64_t> cb_off;
   int64_t cb_len = 0;              // doubles of contribution blocks alive at once
   std::vector<int> warp_list;      // fronts of the warp walk, in level order
@@ -118,12 +134,12 @@ bool check_front_plan(int n, const int *Ls, const HostSym &H, const Plan &P, con
 bool front_configure(std::string &err);
 int front_cta_walk_ctas(int smem, int count);
 int front_warp_walk_ctas(int count);
-void launch_front_warp_walk(const DevSym &S, const FrontDev &F, const int *order, int count,
+void launch_front_warp_walk(const DevSym &S, const FrontDev &F, const FrontDesc *order, int count,
                             int ctas, int *qctr, int *qhead, cudaStream_t st);
-void launch_front_cta_walk(const DevSym &S, const FrontDev &F, const int *order, int count,
+void launch_front_cta_walk(const DevSym &S, const FrontDev &F, const FrontDesc *order, int count,
                            int smem, int ctas, int *qctr, cudaStream_t st);
-void launch_front_small(const DevSym &S, const FrontDev &F, const int *list, int count, int smem,
-                        cudaStream_t st);
+void launch_front_small(const DevSym &S, const FrontDev &F, const FrontDesc *list, int count, int smem,
+                        cudaStream_t st);   // cb < 0: the block is formed by tiles
 void launch_front_extend(const DevSym &S, const FrontDev &F, const int4 *tasks, const int *end,
                          const int4 *pairs, int count, cudaStream_t st);
 void launch_front_schur(const DevSym &S, const FrontDev &F, const int4 *tasks, const int *end,

@@ -41,11 +41,6 @@ bool prune_sets_complete(const int *Ls, const int *prunePtr, const int *pruneSet
   return true;
 }
 
-struct Tile {
-  int4 task;
-  std::vector<int4> pairs;
-};
-
 }  // namespace
 
 int64_t FrontArena::take(int64_t len) {
@@ -162,55 +157,64 @@ void build_front_plan(int n, const int *c, const int *r, const int *Ls, const in
   std::vector<std::vector<int>> by_level(nlev);
   for (int s = 0; s < ns; ++s) by_level[level[s]].push_back(s);
 
-  // tasks
-  std::vector<Tile> ext, sch;
+  // tasks: the tiles of s's list with origin o (positions o + 64 t of its rows; columns up to
+  // clim) and the pairs of children's rows that fall in each; tiles without pairs only if `all`
+  struct Run { int tile, start, count; };
+  std::vector<Run> run;
   std::vector<int> tile_of;
-  // the pairs of children's rows with the tiles of a grid with origin o (positions o + 64 t of
-  // s's row list; columns up to clim)
-  auto pairs_of = [&](int s, int o, int clim, std::vector<Tile> &tiles, bool all) {
+  std::vector<int4> tile_task;
+  std::vector<std::pair<int, int4>> items;
+  auto add_tiles = [&](int s, int o, int clim, bool all, std::vector<int4> &tasks, std::vector<int> &end,
+                       std::vector<int4> &pairs) {
     const int m = rows(s), nt = (m - o + TB - 1) / TB, nc = (clim - o + TB - 1) / TB;
     tile_of.assign((size_t)nt * nc, -1);
-    auto tile = [&](int a, int b) -> Tile & {
+    tile_task.clear();
+    items.clear();
+    auto tile = [&](int a, int b) {
       int &k = tile_of[(size_t)a * nc + b];
       if (k < 0) {
-        k = (int)tiles.size();
-        tiles.push_back(Tile{make_int4(s, a * TB, b * TB, 0), {}});
+        k = (int)tile_task.size();
+        tile_task.push_back(make_int4(s, a * TB, b * TB, 0));
       }
-      return tiles[k];
+      return k;
     };
     if (all)
       for (int b = 0; b < nc; ++b)
         for (int a = b; a < nt; ++a) tile(a, b);
-    struct Run { int tile, start, count; };
-    std::vector<Run> run;
     for (int q = F.child_ptr[s]; q < F.child_ptr[s + 1]; ++q) {
       const int d = F.child[q], rd = rows(d) - width(d);
       const int *rel = F.rel.data() + (rowptr[d] - super[d]);
       run.clear();
-      for (int i = (int)(std::lower_bound(rel, rel + rd, o) - rel); i < rd; ++i) {
-        const int tl = (rel[i] - o) / TB;
-        if (run.empty() || run.back().tile != tl) run.push_back({tl, i, 1});
-        else run.back().count++;
+      for (int i = (int)(std::lower_bound(rel, rel + rd, o) - rel); i < rd;) {
+        const int tl = (rel[i] - o) / TB, lim = o + (tl + 1) * TB;
+        int e = i + 1;
+        while (e < rd && rel[e] < lim) ++e;
+        run.push_back({tl, i, e - i});
+        i = e;
       }
-      for (const Run &cr : run) {
+      for (size_t x = 0; x < run.size(); ++x) {
+        const Run &cr = run[x];
         int nb = cr.count;   // columns below clim
         while (nb > 0 && rel[cr.start + nb - 1] >= clim) --nb;
         if (nb == 0) break;
-        for (const Run &rr : run)
-          if (rr.tile >= cr.tile)
-            tile(rr.tile, cr.tile).pairs.push_back(make_int4(d, rr.start, cr.start, rr.count | (nb << 16)));
+        for (size_t y = x; y < run.size(); ++y)
+          items.push_back({tile(run[y].tile, cr.tile),
+                           make_int4(d, run[y].start, cr.start, run[y].count | (nb << 16))});
       }
     }
-  };
-  auto flatten = [&](std::vector<Tile> &tiles, std::vector<int4> &tasks, std::vector<int> &end,
-                     std::vector<int4> &pairs) {
-    for (Tile &t : tiles) {
-      t.task.w = (int)pairs.size();
-      tasks.push_back(t.task);
-      pairs.insert(pairs.end(), t.pairs.begin(), t.pairs.end());
-      end.push_back((int)pairs.size());
+    // pairs grouped by tile, children in order
+    const size_t t0 = tasks.size(), p0 = pairs.size();
+    tasks.insert(tasks.end(), tile_task.begin(), tile_task.end());
+    end.resize(tasks.size(), 0);
+    for (const auto &it : items) ++end[t0 + it.first];
+    int at = (int)p0;
+    for (size_t t = t0; t < tasks.size(); ++t) {
+      tasks[t].w = at;
+      at += end[t];
+      end[t] = tasks[t].w;
     }
-    tiles.clear();
+    pairs.resize(at);
+    for (const auto &it : items) pairs[end[t0 + it.first]++] = it.second;
   };
   F.waves.resize(nlev);
   int launches = 2 + !P.big_list.empty();
@@ -229,7 +233,7 @@ void build_front_plan(int n, const int *c, const int *r, const int *Ls, const in
         F.cta_list.push_back(s);
         F.cta_smem = std::max<int>(F.cta_smem, (int)front_smem(w, m));
       } else if (tiled[s]) {
-        pairs_of(s, 0, w, ext, false);
+        add_tiles(s, 0, w, false, F.ext_tasks, F.ext_end, F.ext_pairs);
         if (m > w) by_width.push_back(s);
       } else {
         const bool by_tiles = m - w > FRONT_SMALL_R;
@@ -239,9 +243,7 @@ void build_front_plan(int n, const int *c, const int *r, const int *Ls, const in
       }
     }
     std::stable_sort(by_width.begin(), by_width.end(), [&](int a, int b) { return width(a) > width(b); });
-    for (int s : by_width) pairs_of(s, width(s), rows(s), sch, true);
-    flatten(ext, F.ext_tasks, F.ext_end, F.ext_pairs);
-    flatten(sch, F.sch_tasks, F.sch_end, F.sch_pairs);
+    for (int s : by_width) add_tiles(s, width(s), rows(s), true, F.sch_tasks, F.sch_end, F.sch_pairs);
     W.small_cnt = (int)F.small_list.size() - W.small_off;
     W.ext_cnt = (int)F.ext_tasks.size() - W.ext_off;
     W.sch_cnt = (int)F.sch_tasks.size() - W.sch_off;
@@ -279,6 +281,22 @@ void build_front_plan(int n, const int *c, const int *r, const int *Ls, const in
           A.give(F.cb_off[F.child[q]], len(F.child[q]));
   }
   F.cb_len = A.end();
+
+  // descriptors, and the entries of A of the small fronts in their padded panels
+  for (int d : F.child)
+    F.kids.push_back(FrontChild{d, rows(d) - width(d), F.child_n1[d], 0, rowptr[d] - super[d], F.cb_off[d]});
+  F.ppos = F.apos;
+  auto desc = [&](int s, bool by_tiles) {
+    const int w = width(s), ld = front_ld(w, rows(s)), pad = front_wp(w) - w;
+    for (int j = 0; j < w; ++j)
+      for (int p = c[super[s] + j]; p < c[super[s] + j + 1]; ++p)
+        if (F.apos[p] >= 0) F.ppos[p] = j * ld + (F.apos[p] < w ? F.apos[p] : F.apos[p] + pad);
+    return FrontDesc{s, super[s], w, rows(s), F.child_ptr[s], F.child_ptr[s + 1], c[super[s]], c[super[s + 1]],
+                     H.xptr[s], by_tiles ? -1 : F.cb_off[s]};
+  };
+  for (int s : F.warp_list) F.warp_desc.push_back(desc(s, false));
+  for (int s : F.cta_list) F.cta_desc.push_back(desc(s, false));
+  for (int e : F.small_list) F.small_desc.push_back(desc(e < 0 ? ~e : e, e < 0));
   F.ok = true;
 }
 

@@ -561,147 +561,17 @@ __global__ void __launch_bounds__(MT, 4) k_update_tiles(DevSym S, const int4 *ta
 //            the grouped updates of the later column blocks on a stream of their own.
 //   block 0 is factored by k_diag_step with step 0.
 
-// ---- one 64x64 diagonal block: POTRF and its inverse, blocked by 8 ----------------------
-// Every 8x8 block product runs on the tensor cores (DMMA); scalar FP64 work is limited to
-// the 8x8 diagonal pieces, done by one warp with shuffles.  D is a [column][row] shared
-// array with leading dimension DLD; E (the inverse, lower triangular) holds only its 36
-// lower 8x8 blocks, packed: block (bi, bk), bi >= bk, at (bi (bi + 1) / 2 + bk) * 64, each
-// block column-major.  128 threads (4 warps).
-// DLD = 68: the 8x8 DMMA operand loads (lane 4g + kq reads row g, column kq of a block)
-// hit 16 different bank pairs per half warp (68 = 4 mod 16); 65 gave four-way conflicts.
-constexpr int DLD = TB + 4;
-constexpr int E_ELEMS = 36 * 64;
-
-__device__ __forceinline__ int eix(int r, int c) {
-  const int bi = r >> 3, bk = c >> 3;
-  return ((bi * (bi + 1) / 2 + bk) << 6) + ((c & 7) << 3) + (r & 7);
-}
+// ---- one 64x64 diagonal block: POTRF (chol_panel) and its inverse (inverse64) -------------
+constexpr int DLD = LDS;   // leading dimension of its [column][row] arrays
 
 // c += A_blk * B_blk^T for 8x8 blocks of [column][row] arrays: A_blk = rows ar0..ar0+7,
 // columns ak0..ak0+7 of Am; B_blk = rows bn0..bn0+7, columns bk0..bk0+7 of Bm.
 __device__ __forceinline__ void mma8_abt(double (&c)[2], const double *Am, int ar0, int ak0,
-                                         const double *Bm, int bn0, int bk0, bool negate_a) {
+                                         const double *Bm, int bn0, int bk0) {
   const int lane = threadIdx.x & 31, g = lane >> 2, kq = lane & 3;
 #pragma unroll
-  for (int t = 0; t < 2; ++t) {
-    const double a = Am[(ak0 + 4 * t + kq) * DLD + ar0 + g];
-    const double b = Bm[(bk0 + 4 * t + kq) * DLD + bn0 + g];
-    dmma(c, negate_a ? neg(a) : a, b);
-  }
-}
-
-__device__ __forceinline__ void load8(double (&c)[2], const double *X, int r0, int c0) {
-  const int lane = threadIdx.x & 31, g = lane >> 2, kq = lane & 3;
-  c[0] = X[(c0 + 2 * kq) * DLD + r0 + g];
-  c[1] = X[(c0 + 2 * kq + 1) * DLD + r0 + g];
-}
-__device__ __forceinline__ void store8(const double (&c)[2], double *X, int r0, int c0, bool lower_only) {
-  const int lane = threadIdx.x & 31, g = lane >> 2, kq = lane & 3;
-#pragma unroll
-  for (int e = 0; e < 2; ++e)
-    if (!lower_only || g >= 2 * kq + e) X[(c0 + 2 * kq + e) * DLD + r0 + g] = c[e];
-}
-
-// D: bw x bw lower block padded to a multiple of 8 with identity.  Factors it in place
-// (right-looking over 8-column blocks) and leaves the inverses of its 8x8 diagonal blocks
-// in E.  Look-ahead: in the trailing update of step kb, warp 0 updates diagonal block kb+1
-// first and factors it while the other NW - 1 warps update the other blocks, so each step
-// costs one panel phase and one trailing phase (two barriers).  NW warps (32 NW threads).
-template <int NW>
-__device__ void potrf64_blocked(double *D, double *E, int bw, const DevSym &S, int gcol0) {
-  const int warp = threadIdx.x >> 5;
-  const int nbk = (bw + 7) >> 3;
-  if (warp == 0) potrf8_inv8(D, DLD, E, S.status, gcol0, bw);
-  __syncthreads();
-  for (int kb = 0; kb < nbk; ++kb) {
-    // panel below: X_ib = B_ib * T_kk^T (warp 0 gets ib = kb + 1)
-    for (int ib = kb + 1 + warp; ib < nbk; ib += NW) {
-      double c[2] = {0.0, 0.0};
-      const int lane = threadIdx.x & 31, g = lane >> 2, kq = lane & 3;
-#pragma unroll
-      for (int t = 0; t < 2; ++t)   // X_ib = B_ib T_kk^T
-        dmma(c, D[(8 * kb + 4 * t + kq) * DLD + 8 * ib + g], E[eix(8 * kb + g, 8 * kb + 4 * t + kq)]);
-      __syncwarp();
-      store8(c, D, 8 * ib, 8 * kb, false);
-    }
-    __syncthreads();
-    if (kb + 1 >= nbk) break;
-    // trailing update D_ib,jb -= X_ib X_jb^T for kb < jb <= ib
-    if (warp == 0) {
-      const int nb = kb + 1;
-      double c[2];
-      load8(c, D, 8 * nb, 8 * nb);
-      mma8_abt(c, D, 8 * nb, 8 * kb, D, 8 * nb, 8 * kb, true);
-      store8(c, D, 8 * nb, 8 * nb, true);
-      __syncwarp();
-      potrf8_inv8(D + 8 * nb * DLD + 8 * nb, DLD, E + eix(8 * nb, 8 * nb), S.status, gcol0 + 8 * nb,
-                  bw - 8 * nb);
-    } else if ((warp & 3) != 0) {
-      // blocks (ib, jb), kb < jb <= ib < nbk, except (kb+1, kb+1), in column order; the
-      // warps that do not share warp 0's scheduler (warp % 4 != 0: NU of them, rank u) take
-      // the blocks u, u + NU, .. and run them interleaved (independent DMMA chains: their
-      // latency, not their issue, bounds a short chain); warp 0's chain of pivots keeps its
-      // scheduler to itself
-      constexpr int NU = NW - NW / 4;
-      constexpr int MAXT = (27 + NU - 1) / NU;
-      const int u = warp - 1 - (warp >> 2);
-      const int nrem = nbk - kb - 1;                       // block rows/columns left
-      const int ntot = nrem * (nrem + 1) / 2 - 1;
-      double c[MAXT][2];
-      int bi[MAXT], bj[MAXT];
-#pragma unroll
-      for (int t = 0; t < MAXT; ++t) {
-        int idx = u + NU * t;
-        if (idx >= ntot) idx = -1;  // an unused slot: block (kb+1, kb+1), nothing stored
-        idx += 1;                   // skip (kb+1, kb+1), the first block of the order
-        int jj = 0;
-        while (idx >= nrem - jj) { idx -= nrem - jj; ++jj; }
-        bj[t] = 8 * (kb + 1 + jj);
-        bi[t] = bj[t] + 8 * idx;
-        load8(c[t], D, bi[t], bj[t]);
-      }
-#pragma unroll
-      for (int t = 0; t < MAXT; ++t)
-        if (u + NU * t < ntot) mma8_abt(c[t], D, bi[t], 8 * kb, D, bj[t], 8 * kb, true);
-#pragma unroll
-      for (int t = 0; t < MAXT; ++t)
-        if (u + NU * t < ntot) store8(c[t], D, bi[t], bj[t], bi[t] == bj[t]);
-    }
-    __syncthreads();
-  }
-}
-
-// Inverse of the factored block: off-diagonal 8x8 blocks T_ik = -T_ii sum_{j=k}^{i-1}
-// L_ij T_jk, one column block per warp (E holds T_kk on entry; W: 64 doubles per warp).
-template <int NW>
-__device__ void trtri64_blocked(const double *D, double *E, double *W, int bw) {
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, kq = lane & 3;
-  const int nbk = (bw + 7) >> 3;
-  double *Ww = W + warp * 64;
-  for (int k = warp; k < nbk; k += NW) {
-    for (int i = k + 1; i < nbk; ++i) {
-      double sacc[2] = {0.0, 0.0};
-      for (int j = k; j < i; ++j)   // sacc += L_ij T_jk
-#pragma unroll
-        for (int t = 0; t < 2; ++t)
-          dmma(sacc, D[(8 * j + 4 * t + kq) * DLD + 8 * i + g], E[eix(8 * j + 4 * t + kq, 8 * k + g)]);
-      // S (C layout) -> W[col * 8 + row], read back as the B operand of T_ii * S
-      Ww[(2 * kq) * 8 + g] = sacc[0];
-      Ww[(2 * kq + 1) * 8 + g] = sacc[1];
-      __syncwarp();
-      double c[2] = {0.0, 0.0};
-#pragma unroll
-      for (int t = 0; t < 2; ++t) {
-        const double a = neg(E[eix(8 * i + g, 8 * i + 4 * t + kq)]);
-        const double b = Ww[g * 8 + 4 * t + kq];
-        dmma(c, a, b);
-      }
-#pragma unroll
-      for (int e = 0; e < 2; ++e) E[eix(8 * i + g, 8 * k + 2 * kq + e)] = c[e];
-      __syncwarp();
-    }
-  }
-  __syncthreads();
+  for (int t = 0; t < 2; ++t)
+    dmma(c, Am[(ak0 + 4 * t + kq) * DLD + ar0 + g], Bm[(bk0 + 4 * t + kq) * DLD + bn0 + g]);
 }
 
 // Factor diagonal block c0/64 of supernode s in place (lower triangle only) and store its
@@ -711,8 +581,9 @@ __device__ void trtri64_blocked(const double *D, double *E, double *W, int bw) {
 // updated block never leaves the chip before its factorization; when the block is narrower
 // than 64 the tile's remaining rows are panel rows below it and go to L.
 // NW warps (upd needs NW = 4: the tile accumulator's layout), diag_smem(NW) bytes of
-// dynamic shared memory: E, W (NW x 64), then D.
-constexpr int diag_smem(int nw) { return (E_ELEMS + nw * 64 + TB * DLD) * 8; }
+// dynamic shared memory: E, the inverse's inner products, the warps' scratch, then D.
+constexpr int E_ELEMS = TB * DLD, W_ELEMS = 16 * 64;
+constexpr int diag_smem(int nw) { return (E_ELEMS + W_ELEMS + TB + nw * 64 + TB * DLD) * 8; }
 constexpr int diag_prev_smem(int nw) { return diag_smem(nw) + TB * DLD * 8; }   // + X
 constexpr int DIAG_SMEM = diag_smem(4);
 constexpr int DIAG_NW = 8;   // warps of the per-step diagonal-block kernel
@@ -724,7 +595,7 @@ template <int NW, bool PREV = false>
 __device__ void factor_diag_block(const DevSym &S, int s, int c0, double *smem,
                                   const TileAcc *upd) {
   constexpr int NTH = 32 * NW;
-  double *E = smem, *W = smem + E_ELEMS, *D = W + NW * 64;
+  double *E = smem, *W = smem + E_ELEMS, *rd = W + W_ELEMS, *sc = rd + TB, *D = sc + NW * 64;
   const int tid = threadIdx.x;
   const int f = S.super[s];
   const int w = S.super[s + 1] - f;
@@ -752,7 +623,6 @@ __device__ void factor_diag_block(const DevSym &S, int s, int c0, double *smem,
       if (PREV) Xs[(e >> 6) * DLD + (e & (TB - 1))] = xv[q];
     }
   }
-  for (int e = tid; e < E_ELEMS; e += blockDim.x) E[e] = 0.0;
   if (PREV) {
     __syncthreads();
     // tile -= X X^T over the lower 8x8 blocks (DMMA), block columns of the diagonal block
@@ -776,7 +646,7 @@ __device__ void factor_diag_block(const DevSym &S, int s, int c0, double *smem,
     for (int k0 = 0; k0 < TB; k0 += 8)
 #pragma unroll
       for (int q = 0; q < MAXB; ++q)
-        if (warp + NW * q < nblk) mma8_abt(acc[q], Xs, ar[q], k0, Xs, br[q], k0, false);
+        if (warp + NW * q < nblk) mma8_abt(acc[q], Xs, ar[q], k0, Xs, br[q], k0);
 #pragma unroll
     for (int q = 0; q < MAXB; ++q) {
       if (warp + NW * q >= nblk) continue;
@@ -809,17 +679,18 @@ __device__ void factor_diag_block(const DevSym &S, int s, int c0, double *smem,
     }
   }
   __syncthreads();
-  potrf64_blocked<NW>(D, E, bw, S, f + c0);
+  for (int c = tid; c < TB; c += blockDim.x) rd[c] = 1.0;   // the identity beyond the block
+  chol_panel<NW>(D, DLD, (bw + 7) >> 3, (bw + 7) >> 3, sc, S.status, f + c0, bw, rd);
   for (int e = tid; e < TB * TB; e += blockDim.x) {
     const int c = e >> 6, r = e & (TB - 1);
     if (c < bw && r < bw && r >= c) P[(size_t)(c0 + c) * m + c0 + r] = D[c * DLD + r];
   }
   {   // the inverse serves the TRSM of the rows below and the chained triangular solves
-    trtri64_blocked<NW>(D, E, W, bw);
+    inverse64<NW>(D, rd, E, W);
     double *T = S.dinv + ((size_t)S.dinv_off[s] + c0 / TB) * (TB * TB);
     for (int e = tid; e < TB * TB; e += blockDim.x) {
       const int c = e >> 6, r = e & (TB - 1);
-      T[e] = (c < bw && r < bw && r >= c) ? E[eix(r, c)] : 0.0;
+      T[e] = (c < bw && r < bw && r >= c) ? E[c * DLD + r] : 0.0;
     }
   }
 }
@@ -997,7 +868,7 @@ __device__ __forceinline__ bool dense_wait(const int *p, int need, int *status) 
   return true;
 }
 
-__global__ void __launch_bounds__(MT, 4) k_dense_persist(DevSym S, const int4 *tasks, int count,
+__global__ void __launch_bounds__(MT, 2) k_dense_persist(DevSym S, const int4 *tasks, int count,
                                                          const int *toff, int *ver, int *qhead) {
   extern __shared__ double dyn[];
   __shared__ int item, ok;

@@ -29,6 +29,17 @@ __device__ __forceinline__ void st_release_k(int *p, int v) {
   asm volatile("st.release.gpu.global.s32 [%0], %1;\n" ::"l"(p), "r"(v) : "memory");
 }
 
+// *p where ok, else 0: one predicated load.  A branch around a load that is summed at once makes
+// the warp wait for it before the next one; these are all in flight together.
+__device__ __forceinline__ double ld_if(const double *p, bool ok) {
+  double v;
+  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %2, 0;\n\tmov.f64 %0, 0d0000000000000000;\n\t"
+               "@q ld.global.f64 %0, [%1];\n\t}\n"
+               : "=d"(v)
+               : "l"(p), "r"((int)ok));
+  return v;
+}
+
 constexpr int KC = 16;
 
 // 64x64 FP64 tile product on the tensor cores (DMMA, mma.sync m8n8k4 .f64):
@@ -155,70 +166,220 @@ __device__ __forceinline__ int acc_col(int j, int e) {
   return ((threadIdx.x >> 5) & 1) * 32 + 8 * j + 2 * (threadIdx.x & 3) + e;
 }
 
-// Warp-level Cholesky of an 8x8 diagonal block (D points at its first entry, [column][row]
-// with leading dimension ld) and its inverse into T (8x8, column-major).  A pivot of one of
-// the first `real` columns that is <= 0 or NaN is reported (gcol: the block's first column).  Every lane factors the whole block in registers (broadcast loads of its 36
-// entries), so the chain of pivots is one reciprocal square root, one product and one
-// FMA per column with no shuffle on it; lane j < 8 then forms column j of the inverse by
-// forward substitution.
-__device__ __forceinline__ void potrf8_inv8(double *D, int ld, double *T, int *status, int gcol,
-                                            int real) {
-  const int lane = threadIdx.x & 31;
-  double a[8][8];
+// Cholesky of a panel in shared memory by NW = 1, 4 or 8 warps: P is [column][row] with
+// leading dimension ld, nkb 8-column blocks, nrb >= nkb 8-row blocks (padding: identity in the
+// diagonal blocks, zeros below).  The chain of pivots sets the time, so nothing else is on it:
+// each panel warp factors the 8x8 diagonal block by itself in registers (broadcast loads, no
+// shuffle, no barrier) and takes its own rows' columns along in the same instructions (32 rows
+// per warp, one per lane; further rows follow once the block is known).  One barrier per 8
+// columns is left, after which each panel warp updates its own rows and, privately, the next
+// diagonal block (8x8x4 DMMA).  Four panel warps, one per scheduler: with eight, two shared an
+// FP64 unit and the chain took 1.4 times as long.  With NW = 8 warps 4-7 update the columns
+// beyond the next block, beside the next pivots.  Panel warp p owns the row blocks congruent to
+// p mod NP.  sc: 64 doubles per warp.  A pivot of one of the first `real` columns that is <= 0
+// or NaN is reported in status[0] (gcol: the panel's first column).  rd (optional): the
+// reciprocals of the diagonal, one per column.
+template <int NW>
+__device__ __forceinline__ void chol_panel(double *P, int ld, int nkb, int nrb, double *sc, int *status,
+                                           int gcol, int real, double *rd = nullptr) {
+  constexpr int NP = NW == 1 ? 1 : 4;   // panel warps
+  const int lane = threadIdx.x & 31, warp = NW == 1 ? 0 : (int)(threadIdx.x >> 5);
+  const int g = lane >> 2, kq = lane & 3, sub = lane & 7, sb = lane >> 3;
+  sc += warp * 64;
+  // minus X_kb X_kb^T on the blocks (bi, bj), bj in [jlo, jhi), of the row blocks own, own + NP,
+  // .. (except the block (skip, skip)), two row blocks by two column blocks at a time
+  auto update = [&](int k0, int own, int jlo, int jhi, int skip) {
+    for (int i0 = own; i0 < nrb; i0 += 2 * NP)
+      for (int j0 = jlo; j0 < jhi && j0 <= i0 + NP; j0 += 2) {
+        double c[2][2][2];
+        bool on[2][2];
 #pragma unroll
-  for (int j = 0; j < 8; ++j)
+        for (int p = 0; p < 2; ++p)
 #pragma unroll
-    for (int i = j; i < 8; ++i) a[i][j] = D[j * ld + i];
-  double rinv[8];
-  int bad = 8;   // first column with a pivot <= 0 or NaN (reported after the chain)
-  double inv = rsqrt(a[0][0]);
+          for (int q = 0; q < 2; ++q) {
+            const int bi = i0 + p * NP, bj = j0 + q;
+            on[p][q] = bi < nrb && bj < jhi && bj <= bi && !(bi == skip && bj == skip);
+            if (on[p][q]) {
+              c[p][q][0] = P[(8 * bj + 2 * kq) * ld + 8 * bi + g];
+              c[p][q][1] = P[(8 * bj + 2 * kq + 1) * ld + 8 * bi + g];
+            }
+          }
 #pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    const double piv = a[j][j];
-    if (!(piv > 0.0) && j < bad) bad = j;
-    rinv[j] = inv;
-    a[j][j] = piv * inv;
-    // the chain first: the next pivot and its reciprocal square root, issued before the
-    // rest of the column's update, which runs under its latency
-    if (j + 1 < 8) {
-      a[j + 1][j] *= inv;
-      a[j + 1][j + 1] = fma(-a[j + 1][j], a[j + 1][j], a[j + 1][j + 1]);
+        for (int h = 0; h < 2; ++h) {
+          const int col = (k0 + 4 * h + kq) * ld + g;
+          double av[2], bv[2];
+#pragma unroll
+          for (int p = 0; p < 2; ++p) av[p] = i0 + p * NP < nrb ? P[col + 8 * (i0 + p * NP)] : 0.0;
+#pragma unroll
+          for (int q = 0; q < 2; ++q) bv[q] = j0 + q < jhi ? neg(P[col + 8 * (j0 + q)]) : 0.0;
+#pragma unroll
+          for (int p = 0; p < 2; ++p)
+#pragma unroll
+            for (int q = 0; q < 2; ++q)
+              if (on[p][q]) dmma(c[p][q], av[p], bv[q]);
+        }
+#pragma unroll
+        for (int p = 0; p < 2; ++p)
+#pragma unroll
+          for (int q = 0; q < 2; ++q)
+            if (on[p][q]) {
+              const int bi = i0 + p * NP, bj = j0 + q;
+              P[(8 * bj + 2 * kq) * ld + 8 * bi + g] = c[p][q][0];
+              P[(8 * bj + 2 * kq + 1) * ld + 8 * bi + g] = c[p][q][1];
+            }
+      }
+  };
+  if (NW > NP && warp >= NP) {   // trailing warps
+    for (int kb = 0; kb < nkb; ++kb) {
+      __syncthreads();
+      if (kb + 2 < nkb) update(8 * kb, kb + 2 + ((warp - kb - 2) & (NP - 1)), kb + 2, nkb, -1);
     }
-    const double inv_next = (j + 1 < 8) ? rsqrt(a[j + 1][j + 1]) : 0.0;
-#pragma unroll
-    for (int i = j + 2; i < 8; ++i) a[i][j] *= inv;
-#pragma unroll
-    for (int k = j + 1; k < 8; ++k)
-#pragma unroll
-      for (int i = k; i < 8; ++i)
-        if (!(k == j + 1 && i == j + 1)) a[i][k] = fma(-a[i][j], a[k][j], a[i][k]);
-    inv = inv_next;
+    __syncthreads();
+    return;
   }
-  if (lane == 0 && bad < 8 && bad < real) atomicMin(&status[0], gcol + bad + 1);
-  // every lane stores the same 36 values (one write per address; no lane-dependent index
-  // into a[][], which would move the array to local memory), once every lane has loaded them:
-  // the lanes of a warp need not run in step
-  __syncwarp();
+  for (int kb = 0; kb < nkb; ++kb) {
+    const int k0 = 8 * kb, nb = kb + 1;
+    const double *dg = kb == 0 ? P : sc;
+    const int ldd = kb == 0 ? ld : 8;
+    double a[8][8], rinv[8], x[8];
 #pragma unroll
-  for (int j = 0; j < 8; ++j)
+    for (int j = 0; j < 8; ++j)
 #pragma unroll
-    for (int i = j; i < 8; ++i) D[j * ld + i] = a[i][j];
-  // lane j < 8: column j of the inverse, 1/L(i,i) = rinv[i]
-  const int j = lane & 7;
-  double t[8];
+      for (int i = j; i < 8; ++i) a[i][j] = dg[j * ldd + i];
+    const int ib0 = nb + ((warp - nb) & (NP - 1));   // this warp's first row block below
+    int ib = ib0 + NP * sb;
+    double *row = P + k0 * ld + 8 * ib + sub;
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    double sacc = 0.0;
+    for (int j = 0; j < 8; ++j) x[j] = ib < nrb ? row[j * ld] : 0.0;
+    int bad = 8;
+    double inv = rsqrt(a[0][0]);
 #pragma unroll
-    for (int k = 0; k < i; ++k)
-      if (k >= j) sacc = fma(a[i][k], t[k], sacc);
-    t[i] = (i < j) ? 0.0 : ((i == j) ? rinv[i] : -sacc * rinv[i]);
+    for (int j = 0; j < 8; ++j) {
+      const double piv = a[j][j];
+      if (!(piv > 0.0) && j < bad) bad = j;
+      rinv[j] = inv;
+      a[j][j] = piv * inv;
+      // the chain first: the next pivot and its reciprocal square root
+      if (j + 1 < 8) {
+        a[j + 1][j] *= inv;
+        a[j + 1][j + 1] = fma(-a[j + 1][j], a[j + 1][j], a[j + 1][j + 1]);
+      }
+      const double inv_next = (j + 1 < 8) ? rsqrt(a[j + 1][j + 1]) : 0.0;
+#pragma unroll
+      for (int i = j + 2; i < 8; ++i) a[i][j] *= inv;
+#pragma unroll
+      for (int k = j + 1; k < 8; ++k)
+#pragma unroll
+        for (int i = k; i < 8; ++i)
+          if (!(k == j + 1 && i == j + 1)) a[i][k] = fma(-a[i][j], a[k][j], a[i][k]);
+      x[j] *= inv;
+#pragma unroll
+      for (int k = j + 1; k < 8; ++k) x[k] = fma(-x[j], a[k][j], x[k]);
+      inv = inv_next;
+    }
+    if (warp == 0 && lane == 0 && bad < 8 && k0 + bad < real) atomicMin(&status[0], gcol + k0 + bad + 1);
+    if (ib < nrb) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) row[j * ld] = x[j];
+    }
+    for (int ibc = ib0 + 4 * NP; ibc < nrb; ibc += 4 * NP) {   // rows beyond the first 32
+      ib += 4 * NP;
+      if (ib >= nrb) continue;
+      double *rw = P + k0 * ld + 8 * ib + sub;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) x[j] = rw[j * ld];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        x[j] *= rinv[j];
+#pragma unroll
+        for (int k = j + 1; k < 8; ++k) x[k] = fma(-x[j], a[k][j], x[k]);
+      }
+#pragma unroll
+      for (int j = 0; j < 8; ++j) rw[j * ld] = x[j];
+    }
+    if (NW == 1) __syncwarp(); else __syncthreads();
+    if (warp == (kb & (NP - 1))) {   // no warp reads the block any more
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+#pragma unroll
+        for (int i = j; i < 8; ++i) P[(k0 + j) * ld + k0 + i] = a[i][j];
+      if (rd && lane == 0)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) rd[k0 + j] = rinv[j];
+    }
+    if (nb >= nkb) break;
+    {
+      double c[2];   // the next diagonal block, updated privately
+      c[0] = P[(8 * nb + 2 * kq) * ld + 8 * nb + g];
+      c[1] = P[(8 * nb + 2 * kq + 1) * ld + 8 * nb + g];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const double v = P[(k0 + 4 * h + kq) * ld + 8 * nb + g];
+        dmma(c, v, neg(v));
+      }
+      sc[(2 * kq) * 8 + g] = c[0];
+      sc[(2 * kq + 1) * 8 + g] = c[1];
+    }
+    update(k0, ib0, nb, NW > NP ? nb + 1 : nkb, nb);
+    __syncwarp();
   }
-  if (lane < 8) {
+  if (NW == 1) __syncwarp(); else __syncthreads();
+}
+
+// Inverse of the 64x64 lower triangle D ([column][row], leading dimension LDS; rd: reciprocals of
+// its diagonal) into the lower 8x8 blocks of E (same layout), by doubling: the 8x8 diagonal
+// blocks by substitution, then T21 = -T22 (L21 T11) at 16, 32 and 64 columns, two products and
+// two barriers each (W: the inner product, 16 blocks of 64 doubles).
+template <int NW>
+__device__ __forceinline__ void inverse64(const double *D, const double *rd, double *E, double *W) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, kq = lane & 3;
+  if (tid < TB) {   // thread: one column of a diagonal block
+    const int b0 = tid & ~7, j = tid & 7;
+    double x[8];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) T[j * 8 + i] = t[i];
+    for (int i = 0; i < 8; ++i) x[i] = i == j ? 1.0 : 0.0;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      x[k] *= rd[b0 + k];
+#pragma unroll
+      for (int i = k + 1; i < 8; ++i) x[i] = fma(-D[(b0 + k) * LDS + b0 + i], x[k], x[i]);
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) E[tid * LDS + b0 + i] = x[i];
   }
-  __syncwarp();
+  __syncthreads();
+#pragma unroll
+  for (int h = 1; h <= 4; h *= 2) {
+    // tile t: pair t / h^2, block (i, k) of the pair's lower left part
+    for (int t = warp; t < 4 * h; t += NW) {
+      const int base = 2 * h * (t / (h * h)), i = (t % (h * h)) / h, k = t % h;
+      double c[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
+#pragma unroll
+      for (int j = 0; j < h; ++j)
+        if (j >= k)
+#pragma unroll
+          for (int u = 0; u < 2; ++u)
+            dmma(c[u], D[(8 * (base + j) + 4 * u + kq) * LDS + 8 * (base + h + i) + g],
+                 E[(8 * (base + k) + g) * LDS + 8 * (base + j) + 4 * u + kq]);
+      W[t * 64 + (2 * kq) * 8 + g] = c[0][0] + c[1][0];
+      W[t * 64 + (2 * kq + 1) * 8 + g] = c[0][1] + c[1][1];
+    }
+    __syncthreads();
+    for (int t = warp; t < 4 * h; t += NW) {
+      const int base = 2 * h * (t / (h * h)), i = (t % (h * h)) / h, k = t % h;
+      double c[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
+#pragma unroll
+      for (int j = 0; j < h; ++j)
+        if (j <= i)
+#pragma unroll
+          for (int u = 0; u < 2; ++u)
+            dmma(c[u], neg(E[(8 * (base + h + j) + 4 * u + kq) * LDS + 8 * (base + h + i) + g]),
+                 W[((t / (h * h)) * h * h + j * h + k) * 64 + g * 8 + 4 * u + kq]);
+      E[(8 * (base + k) + 2 * kq) * LDS + 8 * (base + h + i) + g] = c[0][0] + c[1][0];
+      E[(8 * (base + k) + 2 * kq + 1) * LDS + 8 * (base + h + i) + g] = c[0][1] + c[1][1];
+    }
+    __syncthreads();
+  }
 }
 
 }  // namespace
