@@ -564,30 +564,22 @@ bool Engine::prepare_adjoint(std::string &err) {
   std::shared_ptr<AdjointPlan> plan = std::make_shared<AdjointPlan>();
   AdjointPlan &AP = *plan;
   build_adjoint_plan(hsym_, plan_, *front_, AP);
-  cudaStream_t st = stream_;
+  TableUpload up;
+  up.add(d_adj_parent_, AP.parent);
+  up.add(d_adj_kids_, AP.kids);
+  up.add(d_adj_zoff_, AP.zoff);
+  up.add(d_adj_warp_, AP.warp_list);
+  up.add(d_adj_cta_, AP.cta_list);
+  up.add(d_adj_copies_, AP.copies);
+  up.add(d_adj_tasks_, AP.tasks);
+  up.add(d_adj_units_, AP.units);
+  if (!up.commit(mem_, tables_, stream_, err)) return false;
   cudaError_t e = cudaSuccess;
-  auto up = [&](auto *&dst, const auto &v) {
-    using T = typename std::remove_reference<decltype(v[0])>::type;
-    if (e != cudaSuccess) return;
-    e = cudaMalloc(&dst, sizeof(T) * std::max<size_t>(v.size(), 1));
-    if (e == cudaSuccess && !v.empty())
-      e = cudaMemcpyAsync(const_cast<typename std::remove_const<T>::type *>(dst), v.data(), sizeof(T) * v.size(),
-                          cudaMemcpyHostToDevice, st);
-  };
-  up(d_adj_parent_, AP.parent);
-  up(d_adj_kids_, AP.kids);
-  up(d_adj_zoff_, AP.zoff);
-  up(d_adj_warp_, AP.warp_list);
-  up(d_adj_cta_, AP.cta_list);
-  up(d_adj_copies_, AP.copies);
-  up(d_adj_tasks_, AP.tasks);
-  up(d_adj_units_, AP.units);
   const size_t scratch = sizeof(double) * TB * TB * std::max(AP.max_tasks, 1);
-  if (e == cudaSuccess) e = cudaMalloc(&d_adj_Z_, sizeof(double) * std::max<int64_t>(AP.z_len, 1));
-  if (e == cudaSuccess) e = cudaMalloc(&d_adj_UT_, scratch);
-  if (e == cudaSuccess) e = cudaMalloc(&d_adj_P_, scratch);
-  if (e == cudaSuccess) e = cudaMalloc(&d_adj_grad_, sizeof(double) * std::max<int64_t>(nnz_, 1));
-  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+  if (e == cudaSuccess) e = mem_.get(d_adj_Z_, sizeof(double) * std::max<int64_t>(AP.z_len, 1));
+  if (e == cudaSuccess) e = mem_.get(d_adj_UT_, scratch);
+  if (e == cudaSuccess) e = mem_.get(d_adj_P_, scratch);
+  if (e == cudaSuccess) e = mem_.get(d_adj_grad_, sizeof(double) * std::max<int64_t>(nnz_, 1));
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_adj_small, cudaFuncAttributeMaxDynamicSharedMemorySize, ADJ_SMEM_MAX);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_adj_warp, cudaFuncAttributeMaxDynamicSharedMemorySize, ZW_WARPS * ZW_SLICE);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_adj_u, cudaFuncAttributeMaxDynamicSharedMemorySize, TT_SMEM);
@@ -602,24 +594,20 @@ bool Engine::prepare_adjoint(std::string &err) {
 }
 
 void Engine::release_adjoint() {
-  void *bufs[] = {d_adj_parent_, d_adj_kids_, d_adj_zoff_, d_adj_warp_, d_adj_cta_, d_adj_copies_,
-                  d_adj_tasks_, d_adj_units_, d_adj_Z_, d_adj_UT_, d_adj_P_, d_adj_grad_, d_adj_partial_};
-  for (void *p : bufs)
-    if (p) cudaFree(p);
+  for (double **p : {&d_adj_Z_, &d_adj_UT_, &d_adj_P_, &d_adj_grad_, &d_adj_partial_}) mem_.put(*p);
   if (adj_graph_) cudaGraphExecDestroy(adj_graph_);
   adj_graph_ = nullptr;
   d_adj_parent_ = d_adj_warp_ = d_adj_cta_ = nullptr;
   d_adj_kids_ = nullptr;
   d_adj_zoff_ = nullptr;
   d_adj_copies_ = d_adj_tasks_ = d_adj_units_ = nullptr;
-  d_adj_Z_ = d_adj_UT_ = d_adj_P_ = d_adj_grad_ = d_adj_partial_ = nullptr;
   adj_.reset();
 }
 
 bool Engine::logdet(double *out, std::string &err) {
   cudaSetDevice(device_);
   cudaError_t e = cudaSuccess;
-  if (!d_adj_partial_) e = cudaMalloc(&d_adj_partial_, sizeof(double) * LD_BLOCKS);
+  if (!d_adj_partial_) e = mem_.get(d_adj_partial_, sizeof(double) * LD_BLOCKS);
   double part[LD_BLOCKS];
   if (e == cudaSuccess) {
     k_logdet<<<LD_BLOCKS, 256, 0, stream_>>>(sym_, d_adj_partial_);
@@ -668,7 +656,7 @@ bool Engine::logdet_grad(double *grad, std::string &err) {
   cudaStream_t st = stream_;
   cudaMemsetAsync(d_status_ + 1, 0, sizeof(int), st);
   cudaError_t e = cudaSuccess;
-  if (use_graph_ && !adj_graph_) {
+  if (use_graph_ && swept_ && !adj_graph_) {
     cudaGraph_t g = nullptr;
     e = cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal);
     if (e == cudaSuccess) {
@@ -685,6 +673,7 @@ bool Engine::logdet_grad(double *grad, std::string &err) {
   }
   if (adj_graph_) e = cudaGraphLaunch(adj_graph_, st);
   else run_adjoint();
+  swept_ = true;
   if (e == cudaSuccess) e = cudaGetLastError();
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(grad, d_adj_grad_, sizeof(double) * nnz_, cudaMemcpyDeviceToDevice, st);

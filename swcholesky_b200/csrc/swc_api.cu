@@ -417,10 +417,13 @@ int swc_plan_stats(int n, const int *c, const int *r, const size_t *lC, const in
   if (!swc::build_plan(n, c, r, lc.data(), Ls, lip.data(), blockSet, supNo, prunePtr, pruneSet,
                        H, P, err, swc::plan_candidate(plan)))
     return fail(SWC_INVALID_INPUT, err);
-  if (!swc::check_scatter_plan(n, Ls, H, P, swc::plan_candidate(plan), err))
-    return fail(SWC_INVALID_INPUT, err);
   swc::FrontPlan FP;
   swc::build_front_plan(n, c, r, Ls, prunePtr, pruneSet, H, P, swc::plan_candidate(plan), FP);
+  if (!swc::build_left_plan(Ls, prunePtr, pruneSet, H, P, err) ||
+      !swc::build_scatter_plan(n, Ls, H, &FP, P, swc::plan_candidate(plan), err))
+    return fail(SWC_INVALID_INPUT, err);
+  if (!swc::check_scatter_plan(n, Ls, H, P, swc::plan_candidate(plan), err))
+    return fail(SWC_INVALID_INPUT, err);
   if (!swc::check_front_plan(n, Ls, H, P, FP, err)) return fail(SWC_INVALID_INPUT, err);
   if (FP.ok) P.launches = FP.launches;
   swc::SolvePlan SP;

@@ -74,6 +74,7 @@ uint64_t fnv1a(uint64_t h, const void *data, size_t bytes) {
 bool Engine::segment_berr(const int64_t *d_seg, int nseg, const double *b, const double *x,
                           double *berr, std::string &err) {
   cudaSetDevice(device_);
+  refresh_csr();
   double *d_out = nullptr;
   cudaError_t e = cudaMalloc(&d_out, sizeof(double) * 3 * std::max(nseg, 1));
   std::vector<double> h(3 * (size_t)std::max(nseg, 1));

@@ -16,19 +16,6 @@ namespace swc {
 
 namespace {
 
-template <typename T>
-bool upload(T *&dst, const T *src, size_t count, cudaStream_t st, std::string &err) {
-  if (dst) { cudaFree(dst); dst = nullptr; }
-  size_t bytes = sizeof(T) * std::max<size_t>(count, 1);
-  cudaError_t e = cudaMalloc(&dst, bytes);
-  if (e == cudaSuccess && count) e = cudaMemcpyAsync(dst, src, sizeof(T) * count, cudaMemcpyHostToDevice, st);
-  if (e != cudaSuccess) {
-    err = std::string("device upload: ") + cudaGetErrorString(e);
-    return false;
-  }
-  return true;
-}
-
 bool small_class(int w, int64_t m, const Tuning &T) {
   return w <= std::min(T.small_max_w, SMALL_MAX_W) && m <= std::min(T.small_max_m, SMALL_MAX_M) &&
          (int64_t)w * m <= std::min(T.small_max_elems, SMALL_MAX_ELEMS);
@@ -126,6 +113,69 @@ bool build_update_pairs(int s, int f, int w, int m, const std::vector<int> &supe
 
 }  // namespace
 
+DeviceMemory::~DeviceMemory() {
+  for (Block &b : blocks_) cudaFree(b.p);
+}
+
+cudaError_t DeviceMemory::take(void **p, size_t bytes) {
+  bytes = std::max<size_t>((bytes + 255) & ~(size_t)255, 256);
+  Block *best = nullptr;
+  for (Block &b : blocks_)
+    if (!b.used && b.bytes >= bytes && b.bytes <= 2 * bytes + (1 << 16) && (!best || b.bytes < best->bytes))
+      best = &b;
+  if (best) {
+    best->used = true;
+    *p = best->p;
+    return cudaSuccess;
+  }
+  cudaError_t e = cudaMalloc(p, bytes);
+  if (e != cudaSuccess) {   // the free blocks may be what is missing
+    cudaGetLastError();
+    for (Block &b : blocks_) b.old = true;
+    sweep();
+    e = cudaMalloc(p, bytes);
+  }
+  if (e == cudaSuccess) blocks_.push_back({*p, bytes, true, false});
+  else *p = nullptr;
+  return e;
+}
+
+void DeviceMemory::give(void *p) {
+  for (Block &b : blocks_)
+    if (b.p == p) {
+      b.used = b.old = false;
+      return;
+    }
+}
+
+void DeviceMemory::age() {
+  for (Block &b : blocks_) b.old = !b.used;
+}
+
+void DeviceMemory::sweep() {
+  size_t k = 0;
+  for (Block &b : blocks_) {
+    if (!b.used && b.old) cudaFree(b.p);
+    else blocks_[k++] = b;
+  }
+  blocks_.resize(k);
+}
+
+bool TableUpload::commit(DeviceMemory &mem, std::vector<void *> &owned, cudaStream_t st, std::string &err) {
+  unsigned char *base = nullptr;
+  cudaError_t e = mem.get(base, bytes_);
+  if (e == cudaSuccess) owned.push_back(base);
+  for (const Slot &q : slots_)
+    if (e == cudaSuccess && q.len) e = cudaMemcpyAsync(base + q.at, q.src, q.len, cudaMemcpyHostToDevice, st);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+  if (e != cudaSuccess) {
+    err = std::string("device upload: ") + cudaGetErrorString(e);
+    return false;
+  }
+  for (const Slot &q : slots_) *q.dst = base + q.at;
+  return true;
+}
+
 Engine::Engine(int device) : device_(device) {
   cudaSetDevice(device_);
   const char *ng = getenv("SWC_NO_GRAPH");
@@ -161,19 +211,18 @@ Engine::~Engine() {
 }
 
 void Engine::release() {
-  void *ptrs[] = {d_super_, d_Ls_, d_Ap_, d_Ai_, d_rowptr_, d_xptr_, d_upd_ptr_, d_upd_, d_upd_lbub_,
-                  d_Ax_, dL_, d_status_, d_small_, d_big_, d_asm_, d_panel_, d_upd_tasks_,
-                  d_syrk_, d_pairs_, d_upd_end_, d_dinv_, d_dinv_off_, d_diag_,
-                  d_slist_, d_cptr_, d_cidx_, d_flags_, d_fchain_, d_bchain_, d_scontrib_, d_sgather_, d_c8_tasks_, d_g8_tasks_, d_csr_rp_, d_csr_ci_,
-                  d_csr_map_,
-                  d_csr_val_, d_contrib_, d_work_, d_norms_, d_persist_, d_qctr_, d_npart_,
-                  d_tiny_, d_dense_tasks_, d_dense_toff_, d_dense_ver_, d_swarp_,
-                  d_Lk_, d_xk_, d_xk16_, d_tmaps_, d_tc_pairs_, d_syrk_pairs_, d_syrk_end_,
-                  d_sc_tiles_, d_sc_base_, d_sc_coff_, d_sc_rel_, d_sc_relidx_, d_sc_maps_,
-                  d_sc_maps16_,
-                  d_sc_small_, d_sc_dense_};
-  for (void *p : ptrs)
-    if (p) cudaFree(p);
+  if (dL_) cudaDeviceSynchronize();   // nothing still reads the blocks given back
+  for (double **p : {&d_Ax_, &dL_, &d_dinv_, &d_csr_val_, &d_contrib_, &d_work_, &d_norms_, &d_npart_})
+    mem_.put(*p);
+  for (int **p : {&d_status_, &d_flags_, &d_qctr_, &d_dense_ver_}) mem_.put(*p);
+  if (reinterpret_cast<double *>(d_Lk_) == d_cb_) d_Lk_ = nullptr;
+  mem_.put(d_Lk_);
+  for (void *p : tables_) mem_.put(p);
+  tables_.clear();
+  csr_stale_ = false;
+  for (bool &b : ran_) b = false;
+  for (bool &b : solved_) b = false;
+  swept_ = false;
   release_adjoint();
   release_front();
   d_super_ = d_Ls_ = d_Ap_ = d_Ai_ = nullptr;
@@ -214,10 +263,7 @@ void Engine::release() {
   d_npart_ = nullptr;
   persist_ctas_ = 0;
   release_solve_graphs();
-  for (double **p : {&d_sx_, &d_x8_, &d_c8_}) {
-    if (*p) cudaFree(*p);
-    *p = nullptr;
-  }
+  for (double **p : {&d_sx_, &d_x8_, &d_c8_}) mem_.put(*p);
   work_nrhs_ = 0;
   for (int k = 0; k < 3; ++k) {
     if (graph_exec_[k]) cudaGraphExecDestroy(graph_exec_[k]);
@@ -344,6 +390,23 @@ static bool dense_order_ok(const int4 *tasks, int count, const std::vector<int> 
   return true;
 }
 
+// Relative indices the right-looking updates would take (see build_scatter_plan).
+static int64_t scatter_index_count(const int *Ls, const HostSym &H, const Plan &P, const std::vector<int> &col2sup) {
+  const int ns = (int)H.super.size() - 1;
+  std::vector<char> tiled(ns, 0);
+  for (int s : P.big_list) tiled[s] = 1;
+  int64_t total = 0;
+  for (int d = 0; d < ns; ++d) {
+    int last = -1;
+    for (int64_t q = H.rowptr[d] + (H.super[d + 1] - H.super[d]); q < H.rowptr[d + 1]; ++q) {
+      const int s = col2sup[Ls[q]];
+      if (s != last && tiled[s]) total += H.rowptr[d + 1] - q;
+      last = s;
+    }
+  }
+  return total;
+}
+
 bool build_plan(int n, const int *c, const int *r, const int64_t *lC, const int *Ls,
                 const int64_t *Li_ptr, const int *blockSet, int supNo, const int *prunePtr,
                 const int *pruneSet, HostSym &H, Plan &P, std::string &err, const Tuning &T) {
@@ -444,12 +507,10 @@ bool build_plan(int n, const int *c, const int *r, const int64_t *lC, const int 
   std::vector<std::vector<int>> by_level(nlev);
   for (int s = 0; s < supNo; ++s) by_level[level[s]].push_back(s);
   int launches = 2;
-  std::vector<TileWork> wave_tiles;
   for (int lv = 0; lv < nlev; ++lv) {
     Wave &W = P.waves[lv];
     W.small_off = (int)P.small_list.size();
     W.asm_off = (int)P.asm_tasks.size();
-    W.upd_off = (int)P.upd_tasks.size();
     std::vector<int> big;
     for (int s : by_level[lv]) {
       int w = super[s + 1] - super[s];
@@ -473,35 +534,14 @@ bool build_plan(int n, const int *c, const int *r, const int64_t *lC, const int 
     int maxnb = 0;
     for (int s : big) {
       int f = super[s], w = super[s + 1] - f;
-      int m = (int)(rowptr[s + 1] - rowptr[s]);
       for (int j = f; j < f + w; ++j) P.asm_tasks.push_back(make_int2(s, j));
-      if (prunePtr[s + 1] > prunePtr[s] &&
-          !build_update_pairs(s, f, w, m, super, rowptr, Ls, prunePtr, pruneSet, wave_tiles,
-                              err))
-        return false;
       maxnb = std::max(maxnb, (w + TB - 1) / TB);
     }
     W.asm_cnt = (int)P.asm_tasks.size() - W.asm_off;
-    // heaviest tiles first (shorter tail); ties keep supernode / tile order
-    std::stable_sort(wave_tiles.begin(), wave_tiles.end(),
-                     [](const TileWork &a, const TileWork &b) { return a.flops > b.flops; });
-    for (TileWork &tw : wave_tiles) {
-      tw.task.w = (int)P.upd_pairs.size();
-      P.upd_pairs.insert(P.upd_pairs.end(), tw.pairs.begin(), tw.pairs.end());
-      P.tc_pairs.insert(P.tc_pairs.end(), tw.tc.begin(), tw.tc.end());
-      P.upd_tasks.push_back(tw.task);
-      P.upd_end.push_back((int)P.upd_pairs.size());
-      P.work.flops[K_UPDATE] += tw.flops;
-      P.work.bytes[K_UPDATE] += tw.bytes;
-    }
-    wave_tiles.clear();
-    W.upd_cnt = (int)P.upd_tasks.size() - W.upd_off;
     for (int j = 0; j < maxnb; ++j) {
       W.panel_off.push_back((int)P.panel_tasks.size());
       W.syrk_off.push_back((int)P.syrk_tasks.size());
       W.diag_off.push_back((int)P.diag_list.size());
-      W.scd_off.push_back((int)P.sc_dense.size());
-      std::vector<ScTile> grouped;   // after the step's next-column tiles
       for (int s : big) {
         int w = super[s + 1] - super[s];
         int m = (int)(rowptr[s + 1] - rowptr[s]);
@@ -520,13 +560,6 @@ bool build_plan(int n, const int *c, const int *r, const int64_t *lC, const int 
           if (C == j + 1) first = j;
           else if ((C - 2 - j) % G == 0) first = std::max(0, j - G + 1);
           else continue;
-          if (T.scatter) {   // the same update as 128-row x one-column-block dense tiles
-            const int kc = c0 + bw - first * TB;
-            for (int r0 = cc == c0 + TB ? cc + TB : cc; r0 < m; r0 += 128)
-              (C == j + 1 ? P.sc_dense : grouped)
-                  .push_back(ScTile{s, r0, cc, (kc + 31) / 32, m, first * TB,
-                                    std::min(TB, w - cc), 1, 0, 0});
-          }
           for (int r0 = cc; r0 < m; r0 += TB)
             if (!(cc == c0 + TB && r0 == cc)) {   // next diagonal tile: the TRSM task's update
               // .w: the task's own index: its product (column blocks first..j) in syrk_pairs
@@ -542,11 +575,8 @@ bool build_plan(int n, const int *c, const int *r, const int64_t *lC, const int 
       W.panel_cnt.push_back((int)P.panel_tasks.size() - W.panel_off.back());
       W.syrk_cnt.push_back((int)P.syrk_tasks.size() - W.syrk_off.back());
       W.diag_cnt.push_back((int)P.diag_list.size() - W.diag_off.back());
-      W.scd_nc.push_back((int)P.sc_dense.size() - W.scd_off.back());
-      P.sc_dense.insert(P.sc_dense.end(), grouped.begin(), grouped.end());
-      W.scd_cnt.push_back((int)P.sc_dense.size() - W.scd_off.back());
     }
-    launches += (W.small_cnt > 0) + (W.asm_cnt > 0) + (W.upd_cnt > 0);
+    launches += (W.small_cnt > 0) + (W.asm_cnt > 0);
     int widest = 0;
     for (int s : big) widest = std::max(widest, super[s + 1] - super[s]);
     if (T.dense_dataflow && !big.empty() && (widest + TB - 1) / TB < (1 << 14)) {
@@ -579,107 +609,8 @@ bool build_plan(int n, const int *c, const int *r, const int64_t *lC, const int 
   }
   if (!P.persist_list.empty()) launches += 1;
   if (!P.tiny_list.empty()) launches += 1;
-  P.launches = launches;
-
-  // ---- right-looking updates of the split-TF32 mode: the contribution of every descendant
-  // d to tiled-class targets, C = B B^T over the rows of d from the first one whose column
-  // belongs to a tiled supernode, as 128x128 tiles of one dense product, launched in the
-  // level after d's own (every target sits on a later level) ----
-  if (T.scatter && !P.big_list.empty()) {
-    std::vector<char> tiled(supNo, 0);
-    for (int s : P.big_list) tiled[s] = 1;
-    std::vector<std::vector<ScTile>> by_wave(nlev);
-    std::vector<std::vector<int2>> small_by_wave(nlev);
-    P.sc_coff.assign(supNo, 0);
-    P.sc_used.assign(supNo, 0);
-    for (int d = 0; d < supNo; ++d) {
-      const int wd = super[d + 1] - super[d];
-      const int md = (int)(rowptr[d + 1] - rowptr[d]);
-      const int *rd = Ls + rowptr[d];
-      int c0 = wd;
-      while (c0 < md && !tiled[col2sup[rd[c0]]]) ++c0;
-      if (c0 == md) continue;
-      P.sc_coff[d] = (int64_t)P.sc_base.size() - c0;
-      for (int j = c0; j < md;) {
-        const int s = col2sup[rd[j]];
-        int je = j;
-        while (je < md && col2sup[rd[je]] == s) ++je;
-        if (!tiled[s]) {
-          P.sc_base.insert(P.sc_base.end(), (size_t)(je - j), (int64_t)-1);
-          P.sc_rel.insert(P.sc_rel.end(), (size_t)(je - j), 0);
-        } else {
-          // positions of rows j.. of d in the row list of s (contained in it: s is an
-          // ancestor of d)
-          const int *rs = Ls + rowptr[s];
-          const int ms = (int)(rowptr[s + 1] - rowptr[s]);
-          const int64_t rbase = (int64_t)P.sc_relidx.size() - j;
-          if ((int64_t)P.sc_relidx.size() + (md - j) > INT32_MAX) {
-            err = "relative indices of the right-looking updates exceed 2^31 entries";
-            return false;
-          }
-          int k = (int)(std::lower_bound(rs, rs + ms, rd[j]) - rs);
-          for (int i = j; i < md; ++i) {
-            while (k < ms && rs[k] < rd[i]) ++k;
-            if (k == ms || rs[k] != rd[i]) {
-              err = "row structure of a descendant is not contained in its ancestor's";
-              return false;
-            }
-            P.sc_relidx.push_back(k);
-          }
-          for (int q = j; q < je; ++q) {
-            P.sc_base.push_back(xptr[s] + (int64_t)(rd[q] - super[s]) * ms);
-            P.sc_rel.push_back((int)rbase);
-          }
-        }
-        j = je;
-      }
-      const int nk = (wd + 31) / 32, r = md - c0;
-      if (r <= 128 && (int64_t)wd * ((r + 31) & ~31) <= SC_SMALL_ELEMS) {
-        small_by_wave[level[d] + 1].push_back(make_int2(d, c0));   // FP64 on the CUDA cores
-        continue;
-      }
-      const int kcut = T.scatter_kmax > 0 ? std::max(1, T.scatter_kmax / 32) : nk;
-      for (int i0 = c0; i0 < md; i0 += 128)
-        for (int j0 = c0; j0 <= i0; j0 += 128) {
-          for (int kb = 0; kb < nk; kb += kcut)
-            by_wave[level[d] + 1].push_back(
-                ScTile{d, i0, j0, std::min(kcut, nk - kb), md, kb * 32, 128, 0, P.sc_coff[d], 0});
-          P.sc_flops += 2.0 * 128 * 128 * wd;
-        }
-      P.sc_used[d] |= 1;
-    }
-    // dense tiles of its own factorization: A operands through the 128-row maps, B through
-    // the 64-row maps
-    for (int s : P.big_list) P.sc_used[s] |= 3;
-    // every tile's supernode has the maps its loads use
-    for (const ScTile &t : P.sc_tiles)
-      if (!(P.sc_used[t.d] & 1)) { err = "internal: scatter tile without its tensor maps"; return false; }
-    for (const ScTile &t : P.sc_dense)
-      if ((P.sc_used[t.d] & 3) != 3) { err = "internal: dense tile without its tensor maps"; return false; }
-    // per level: larger K first (a shorter tail); one descendant's tiles stay together
-    int sc_launches = 0;
-    for (int lv = 0; lv < nlev; ++lv) {
-      std::vector<ScTile> &v = by_wave[lv];
-      std::stable_sort(v.begin(), v.end(),
-                       [](const ScTile &a, const ScTile &b) { return a.nk > b.nk; });
-      P.waves[lv].sc_off = (int)P.sc_tiles.size();
-      P.waves[lv].sc_cnt = (int)v.size();
-      P.sc_tiles.insert(P.sc_tiles.end(), v.begin(), v.end());
-      P.waves[lv].scs_off = (int)P.sc_small.size();
-      P.waves[lv].scs_cnt = (int)small_by_wave[lv].size();
-      P.sc_small.insert(P.sc_small.end(), small_by_wave[lv].begin(), small_by_wave[lv].end());
-      sc_launches += !v.empty() + !small_by_wave[lv].empty();
-    }
-    // one assemble launch up front instead of one per level; scatter instead of tile-owner
-    int asm_l = 0, upd_l = 0;
-    for (const Wave &W : P.waves) {
-      asm_l += W.asm_cnt > 0;
-      upd_l += W.upd_cnt > 0;
-    }
-    P.launches_scatter = launches - asm_l - upd_l + (asm_l > 0) + sc_launches;
-  } else {
-    P.launches_scatter = launches;
-  }
+  P.launches = launches;   // + one per wave with update tiles (build_left_plan)
+  P.launches_scatter = launches;
 
   // ---- algorithmic work per kernel class (one factorization) ----
   {
@@ -734,6 +665,7 @@ bool build_plan(int n, const int *c, const int *r, const int64_t *lC, const int 
       K.flops[K_SYRK] = K.bytes[K_SYRK] = 0.0;
     }
   }
+  H.xptr = xptr;
   H.dinv_off.assign(supNo, -1);
   H.ndinv = 0;
   for (int s : P.big_list) {
@@ -756,6 +688,215 @@ bool build_plan(int n, const int *c, const int *r, const int64_t *lC, const int 
       const int ub = (int)(std::lower_bound(b, e, H.super[t + 1]) - b) + wd;
       H.upd_lbub[q] = make_int2(lb, ub);
     }
+  P.sc_index_count = T.scatter ? scatter_index_count(Ls, H, P, col2sup) : 0;
+  if (P.sc_index_count > INT32_MAX) {
+    err = "relative indices of the right-looking updates exceed 2^31 entries";
+    return false;
+  }
+  return true;
+}
+
+// Left-looking update tiles of the tiled class (64x64 tiles and the descendants that touch
+// each), for structures without a multifrontal plan and for the tile-owner plans.
+bool build_left_plan(const int *Ls, const int *prunePtr, const int *pruneSet, const HostSym &H, Plan &P,
+                     std::string &err) {
+  std::vector<TileWork> tiles;
+  P.work.flops[K_UPDATE] = P.work.bytes[K_UPDATE] = 0.0;
+  for (Wave &W : P.waves) {
+    W.upd_off = (int)P.upd_tasks.size();
+    for (int k = W.big_off; k < W.big_off + W.big_cnt; ++k) {
+      const int s = P.big_list[k], f = H.super[s], w = H.super[s + 1] - f;
+      const int m = (int)(H.rowptr[s + 1] - H.rowptr[s]);
+      if (prunePtr[s + 1] > prunePtr[s] &&
+          !build_update_pairs(s, f, w, m, H.super, H.rowptr, Ls, prunePtr, pruneSet, tiles, err))
+        return false;
+    }
+    // heaviest tiles first (shorter tail); ties keep supernode / tile order
+    std::stable_sort(tiles.begin(), tiles.end(),
+                     [](const TileWork &a, const TileWork &b) { return a.flops > b.flops; });
+    for (TileWork &tw : tiles) {
+      tw.task.w = (int)P.upd_pairs.size();
+      P.upd_pairs.insert(P.upd_pairs.end(), tw.pairs.begin(), tw.pairs.end());
+      P.tc_pairs.insert(P.tc_pairs.end(), tw.tc.begin(), tw.tc.end());
+      P.upd_tasks.push_back(tw.task);
+      P.upd_end.push_back((int)P.upd_pairs.size());
+      P.work.flops[K_UPDATE] += tw.flops;
+      P.work.bytes[K_UPDATE] += tw.bytes;
+    }
+    tiles.clear();
+    W.upd_cnt = (int)P.upd_tasks.size() - W.upd_off;
+    P.launches += W.upd_cnt > 0;
+    P.launches_scatter += W.upd_cnt > 0;
+  }
+  P.left = true;
+  return true;
+}
+
+bool build_scatter_plan(int n, const int *Ls, const HostSym &H, const FrontPlan *tree, Plan &P,
+                        const Tuning &T, std::string &err) {
+  if (!T.scatter || P.big_list.empty()) return true;
+  if (tree && !tree->closed) tree = nullptr;
+  const std::vector<int> &super = H.super;
+  const std::vector<int64_t> &rowptr = H.rowptr, &xptr = H.xptr;
+  const int supNo = (int)super.size() - 1, nlev = (int)P.waves.size();
+  std::vector<int> col2sup(n), level(supNo, 0);
+  for (int s = 0; s < supNo; ++s)
+    for (int j = super[s]; j < super[s + 1]; ++j) col2sup[j] = s;
+  for (int s = 0; s < supNo; ++s) {
+    const int w = super[s + 1] - super[s];
+    if (rowptr[s + 1] - rowptr[s] > w) {
+      const int p = col2sup[Ls[rowptr[s] + w]];
+      level[p] = std::max(level[p], level[s] + 1);
+    }
+  }
+  std::vector<int> parent(supNo, -1), cur;
+  if (tree)
+    for (int s = 0; s < supNo; ++s)
+      for (int q = tree->child_ptr[s]; q < tree->child_ptr[s + 1]; ++q) parent[tree->child[q]] = s;
+  // the dense steps' trailing updates as 128-row x one-column-block tiles, each step's
+  // next-column ones first (the groups of the 64x64 tiles above)
+  const int G = std::max(1, T.dense_group);
+  for (Wave &W : P.waves) {
+    for (size_t j = 0; j < W.panel_off.size(); ++j) {
+      W.scd_off.push_back((int)P.sc_dense.size());
+      std::vector<ScTile> grouped;
+      for (int k = W.big_off; k < W.big_off + W.big_cnt; ++k) {
+        const int s = P.big_list[k], w = super[s + 1] - super[s];
+        const int m = (int)(rowptr[s + 1] - rowptr[s]), c0 = (int)j * TB;
+        if (c0 >= w) continue;
+        const int bw = std::min(TB, w - c0);
+        for (int cc = c0 + TB; cc < w; cc += TB) {
+          const int C = cc / TB, jj = (int)j;
+          int first;
+          if (C == jj + 1) first = jj;
+          else if ((C - 2 - jj) % G == 0) first = std::max(0, jj - G + 1);
+          else continue;
+          const int kc = c0 + bw - first * TB;
+          for (int r0 = C == jj + 1 ? cc + TB : cc; r0 < m; r0 += 128)
+            (C == jj + 1 ? P.sc_dense : grouped)
+                .push_back(ScTile{s, r0, cc, (kc + 31) / 32, m, first * TB, std::min(TB, w - cc), 1, 0, 0});
+        }
+      }
+      W.scd_nc.push_back((int)P.sc_dense.size() - W.scd_off.back());
+      P.sc_dense.insert(P.sc_dense.end(), grouped.begin(), grouped.end());
+      W.scd_cnt.push_back((int)P.sc_dense.size() - W.scd_off.back());
+    }
+  }
+  // ---- right-looking updates of the split-TF32 mode: the contribution of every descendant
+  // d to tiled-class targets, C = B B^T over the rows of d from the first one whose column
+  // belongs to a tiled supernode, as 128x128 tiles of one dense product, launched in the
+  // level after d's own (every target sits on a later level) ----
+    std::vector<char> tiled(supNo, 0);
+    for (int s : P.big_list) tiled[s] = 1;
+    std::vector<std::vector<ScTile>> by_wave(nlev);
+    std::vector<std::vector<int2>> small_by_wave(nlev);
+    P.sc_coff.assign(supNo, 0);
+    P.sc_used.assign(supNo, 0);
+    P.sc_relidx.reserve(P.sc_index_count);
+    P.sc_base.reserve(H.nls - n);
+    P.sc_rel.reserve(H.nls - n);
+    for (int d = 0; d < supNo; ++d) {
+      const int wd = super[d + 1] - super[d];
+      const int md = (int)(rowptr[d + 1] - rowptr[d]);
+      const int *rd = Ls + rowptr[d];
+      int c0 = wd;
+      while (c0 < md && !tiled[col2sup[rd[c0]]]) ++c0;
+      if (c0 == md) continue;
+      P.sc_coff[d] = (int64_t)P.sc_base.size() - c0;
+      // positions of d's rows in the row list of the ancestor at hand: from d's own map and the
+      // ancestors' (tree), else by a search
+      if (tree) cur.assign(tree->rel.begin() + (rowptr[d] - super[d]), tree->rel.begin() + (rowptr[d] - super[d]) + md - wd);
+      int anc = tree ? parent[d] : -1;
+      for (int j = tree ? wd : c0; j < md;) {
+        const int s = tree ? anc : col2sup[rd[j]];
+        int je = j;
+        if (tree)
+          while (je < md && cur[je - wd] < super[s + 1] - super[s]) ++je;
+        else
+          while (je < md && col2sup[rd[je]] == s) ++je;
+        if (je > c0 && !tiled[s]) {
+          P.sc_base.insert(P.sc_base.end(), (size_t)(je - j), (int64_t)-1);
+          P.sc_rel.insert(P.sc_rel.end(), (size_t)(je - j), 0);
+        } else if (je > c0 && je > j) {
+          // positions of rows j.. of d in the row list of s (contained in it: s is an
+          // ancestor of d)
+          const int *rs = Ls + rowptr[s];
+          const int ms = (int)(rowptr[s + 1] - rowptr[s]);
+          const int64_t rbase = (int64_t)P.sc_relidx.size() - j;
+          if ((int64_t)P.sc_relidx.size() + (md - j) > INT32_MAX) {
+            err = "relative indices of the right-looking updates exceed 2^31 entries";
+            return false;
+          }
+          if (tree) {
+            P.sc_relidx.insert(P.sc_relidx.end(), cur.begin() + (j - wd), cur.end());
+          } else {
+            int k = (int)(std::lower_bound(rs, rs + ms, rd[j]) - rs);
+            for (int i = j; i < md; ++i) {
+              while (k < ms && rs[k] < rd[i]) ++k;
+              if (k == ms || rs[k] != rd[i]) {
+                err = "row structure of a descendant is not contained in its ancestor's";
+                return false;
+              }
+              P.sc_relidx.push_back(k);
+            }
+          }
+          for (int q = j; q < je; ++q) {
+            P.sc_base.push_back(xptr[s] + (int64_t)(rd[q] - super[s]) * ms);
+            P.sc_rel.push_back((int)rbase);
+          }
+        }
+        j = je;
+        if (tree && j < md) {
+          const int ws = super[s + 1] - super[s];
+          const int *rel = tree->rel.data() + (rowptr[s] - super[s]);
+          for (int i = j; i < md; ++i) cur[i - wd] = rel[cur[i - wd] - ws];
+          anc = parent[s];
+        }
+      }
+      const int nk = (wd + 31) / 32, r = md - c0;
+      if (r <= 128 && (int64_t)wd * ((r + 31) & ~31) <= SC_SMALL_ELEMS) {
+        small_by_wave[level[d] + 1].push_back(make_int2(d, c0));   // FP64 on the CUDA cores
+        continue;
+      }
+      const int kcut = T.scatter_kmax > 0 ? std::max(1, T.scatter_kmax / 32) : nk;
+      for (int i0 = c0; i0 < md; i0 += 128)
+        for (int j0 = c0; j0 <= i0; j0 += 128) {
+          for (int kb = 0; kb < nk; kb += kcut)
+            by_wave[level[d] + 1].push_back(
+                ScTile{d, i0, j0, std::min(kcut, nk - kb), md, kb * 32, 128, 0, P.sc_coff[d], 0});
+          P.sc_flops += 2.0 * 128 * 128 * wd;
+        }
+      P.sc_used[d] |= 1;
+    }
+    // dense tiles of its own factorization: A operands through the 128-row maps, B through
+    // the 64-row maps
+    for (int s : P.big_list) P.sc_used[s] |= 3;
+    // every tile's supernode has the maps its loads use
+    for (const ScTile &t : P.sc_tiles)
+      if (!(P.sc_used[t.d] & 1)) { err = "internal: scatter tile without its tensor maps"; return false; }
+    for (const ScTile &t : P.sc_dense)
+      if ((P.sc_used[t.d] & 3) != 3) { err = "internal: dense tile without its tensor maps"; return false; }
+    // per level: larger K first (a shorter tail); one descendant's tiles stay together
+    int sc_launches = 0;
+    for (int lv = 0; lv < nlev; ++lv) {
+      std::vector<ScTile> &v = by_wave[lv];
+      std::stable_sort(v.begin(), v.end(),
+                       [](const ScTile &a, const ScTile &b) { return a.nk > b.nk; });
+      P.waves[lv].sc_off = (int)P.sc_tiles.size();
+      P.waves[lv].sc_cnt = (int)v.size();
+      P.sc_tiles.insert(P.sc_tiles.end(), v.begin(), v.end());
+      P.waves[lv].scs_off = (int)P.sc_small.size();
+      P.waves[lv].scs_cnt = (int)small_by_wave[lv].size();
+      P.sc_small.insert(P.sc_small.end(), small_by_wave[lv].begin(), small_by_wave[lv].end());
+      sc_launches += !v.empty() + !small_by_wave[lv].empty();
+    }
+    // one assemble launch up front instead of one per level; scatter instead of tile-owner
+    int asm_l = 0;
+    for (const Wave &W : P.waves) {
+      asm_l += W.asm_cnt > 0;
+      if (P.left) P.launches_scatter -= W.upd_cnt > 0;
+    }
+    P.launches_scatter += (asm_l > 0) - asm_l + sc_launches;
   return true;
 }
 
@@ -1226,6 +1367,10 @@ bool Engine::analyze(int n, const int *c, const int *r, const int64_t *lC, const
 
   std::shared_ptr<FrontPlan> FP = std::make_shared<FrontPlan>();
   build_front_plan(n, c, r, Ls, prunePtr, pruneSet, H, P, tuning_, *FP);
+  // without a multifrontal plan the left-looking tiles are needed (and, where the tree does not
+  // hold, the right-looking tables are checked) now
+  if (!FP->ok && !build_left_plan(Ls, prunePtr, pruneSet, H, P, err)) return false;
+  if (!FP->closed && !build_scatter_plan(n, Ls, H, FP.get(), P, tuning_, err)) return false;
   if (FP->ok) P.launches = FP->launches;
 
   // ---- solve plan: levels of the supernodal etree, per-level task lists ----
@@ -1257,77 +1402,67 @@ bool Engine::analyze(int n, const int *c, const int *r, const int64_t *lC, const
   }
 
   // ---- upload ----
+  mem_.age();
   release();
   cudaStream_t st = stream_;
-  std::vector<int64_t> rp(rowptr);
-  bool ok = upload(d_super_, super.data(), super.size(), st, err) &&
-            upload(d_rowptr_, rp.data(), rp.size(), st, err) &&
-            upload(d_Ls_, Ls, (size_t)nls, st, err) &&
-            upload(d_xptr_, xptr.data(), xptr.size(), st, err) &&
-            upload(d_Ap_, c, (size_t)n + 1, st, err) &&
-            upload(d_Ai_, r, (size_t)nnz, st, err) &&
-            upload(d_upd_ptr_, prunePtr, (size_t)supNo + 1, st, err) &&
-            upload(d_upd_, pruneSet, (size_t)nprune, st, err) &&
-            upload(d_upd_lbub_, H.upd_lbub.data(), H.upd_lbub.size(), st, err) &&
-            upload(d_small_, P.small_list.data(), P.small_list.size(), st, err) &&
-            upload(d_persist_, P.persist_list.data(), P.persist_list.size(), st, err) &&
-            upload(d_tiny_, P.tiny_list.data(), P.tiny_list.size(), st, err) &&
-            upload(d_big_, P.big_list.data(), P.big_list.size(), st, err) &&
-            upload(d_diag_, P.diag_list.data(), P.diag_list.size(), st, err) &&
-            upload(d_asm_, P.asm_tasks.data(), P.asm_tasks.size(), st, err) &&
-            upload(d_upd_tasks_, P.upd_tasks.data(), P.upd_tasks.size(), st, err) &&
-            upload(d_upd_end_, P.upd_end.data(), P.upd_end.size(), st, err) &&
-            upload(d_pairs_, P.upd_pairs.data(), P.upd_pairs.size(), st, err) &&
-            upload(d_panel_, P.panel_tasks.data(), P.panel_tasks.size(), st, err) &&
-            upload(d_syrk_, P.syrk_tasks.data(), P.syrk_tasks.size(), st, err) &&
-            upload(d_syrk_pairs_, P.syrk_pairs.data(), P.syrk_pairs.size(), st, err) &&
-            upload(d_syrk_end_, P.syrk_end.data(), P.syrk_end.size(), st, err) &&
-            upload(d_tc_pairs_, P.tc_pairs.data(), P.tc_pairs.size(), st, err) &&
-            upload(d_sc_tiles_, P.sc_tiles.data(), P.sc_tiles.size(), st, err) &&
-            upload(d_sc_small_, P.sc_small.data(), P.sc_small.size(), st, err) &&
-            upload(d_sc_dense_, P.sc_dense.data(), P.sc_dense.size(), st, err) &&
-            upload(d_sc_base_, P.sc_base.data(), P.sc_base.size(), st, err) &&
-            upload(d_sc_coff_, P.sc_coff.data(), P.sc_coff.size(), st, err) &&
-            upload(d_sc_rel_, P.sc_rel.data(), P.sc_rel.size(), st, err) &&
-            upload(d_sc_relidx_, P.sc_relidx.data(), P.sc_relidx.size(), st, err) &&
-            upload(d_dense_tasks_, P.dense_tasks.data(), P.dense_tasks.size(), st, err) &&
-            upload(d_dense_toff_, P.dense_toff.data(), P.dense_toff.size(), st, err) &&
-            upload(d_dinv_off_, H.dinv_off.data(), H.dinv_off.size(), st, err) &&
-            upload(d_slist_, SP.list.data(), SP.list.size(), st, err) &&
-            upload(d_swarp_, SP.warp_list.data(), SP.warp_list.size(), st, err) &&
-            upload(d_cptr_, SP.cptr.data(), SP.cptr.size(), st, err) &&
-            upload(d_cidx_, SP.cidx.data(), SP.cidx.size(), st, err) &&
-            upload(d_fchain_, SP.fchain.data(), SP.fchain.size(), st, err) &&
-            upload(d_bchain_, SP.bchain.data(), SP.bchain.size(), st, err) &&
-            upload(d_scontrib_, SP.contrib_tasks.data(), SP.contrib_tasks.size(), st, err) &&
-            upload(d_c8_tasks_, SP.c8_tasks.data(), SP.c8_tasks.size(), st, err) &&
-            upload(d_g8_tasks_, SP.g8_tasks.data(), SP.g8_tasks.size(), st, err) &&
-            upload(d_sgather_, SP.gather_tasks.data(), SP.gather_tasks.size(), st, err) &&
-            upload(d_csr_rp_, csr_rp.data(), csr_rp.size(), st, err) &&
-            upload(d_csr_ci_, csr_ci.data(), csr_ci.size(), st, err) &&
-            upload(d_csr_map_, csr_map.data(), csr_map.size(), st, err);
-  if (!ok) return false;
-  cudaError_t e = cudaMalloc(&d_Ax_, sizeof(double) * std::max<int64_t>(nnz, 1));
-  if (e == cudaSuccess) e = cudaMalloc(&dL_, sizeof(double) * std::max<int64_t>(xsize, 1));
-  if (e == cudaSuccess) e = cudaMalloc(&d_status_, kStatusWords * sizeof(int));
+  TableUpload up;
+  up.add(d_super_, super.data(), super.size());
+  up.add(d_rowptr_, rowptr.data(), rowptr.size());
+  up.add(d_Ls_, Ls, (size_t)nls);
+  up.add(d_xptr_, xptr.data(), xptr.size());
+  up.add(d_Ap_, c, (size_t)n + 1);
+  up.add(d_Ai_, r, (size_t)nnz);
+  up.add(d_upd_ptr_, prunePtr, (size_t)supNo + 1);
+  up.add(d_upd_, pruneSet, (size_t)nprune);
+  up.add(d_upd_lbub_, H.upd_lbub.data(), H.upd_lbub.size());
+  up.add(d_small_, P.small_list.data(), P.small_list.size());
+  up.add(d_persist_, P.persist_list.data(), P.persist_list.size());
+  up.add(d_tiny_, P.tiny_list.data(), P.tiny_list.size());
+  up.add(d_big_, P.big_list.data(), P.big_list.size());
+  up.add(d_diag_, P.diag_list.data(), P.diag_list.size());
+  up.add(d_asm_, P.asm_tasks.data(), P.asm_tasks.size());
+  up.add(d_panel_, P.panel_tasks.data(), P.panel_tasks.size());
+  up.add(d_syrk_, P.syrk_tasks.data(), P.syrk_tasks.size());
+  up.add(d_syrk_pairs_, P.syrk_pairs.data(), P.syrk_pairs.size());
+  up.add(d_syrk_end_, P.syrk_end.data(), P.syrk_end.size());
+  up.add(d_dense_tasks_, P.dense_tasks.data(), P.dense_tasks.size());
+  up.add(d_dense_toff_, P.dense_toff.data(), P.dense_toff.size());
+  up.add(d_dinv_off_, H.dinv_off.data(), H.dinv_off.size());
+  up.add(d_slist_, SP.list.data(), SP.list.size());
+  up.add(d_swarp_, SP.warp_list.data(), SP.warp_list.size());
+  up.add(d_cptr_, SP.cptr.data(), SP.cptr.size());
+  up.add(d_cidx_, SP.cidx.data(), SP.cidx.size());
+  up.add(d_fchain_, SP.fchain.data(), SP.fchain.size());
+  up.add(d_bchain_, SP.bchain.data(), SP.bchain.size());
+  up.add(d_scontrib_, SP.contrib_tasks.data(), SP.contrib_tasks.size());
+  up.add(d_c8_tasks_, SP.c8_tasks.data(), SP.c8_tasks.size());
+  up.add(d_g8_tasks_, SP.g8_tasks.data(), SP.g8_tasks.size());
+  up.add(d_sgather_, SP.gather_tasks.data(), SP.gather_tasks.size());
+  up.add(d_csr_rp_, csr_rp.data(), csr_rp.size());
+  up.add(d_csr_ci_, csr_ci.data(), csr_ci.size());
+  up.add(d_csr_map_, csr_map.data(), csr_map.size());
+  if (!up.commit(mem_, tables_, st, err)) return false;
+  cudaError_t e = mem_.get(d_Ax_, sizeof(double) * std::max<int64_t>(nnz, 1));
+  if (e == cudaSuccess) e = mem_.get(dL_, sizeof(double) * std::max<int64_t>(xsize, 1));
+  if (e == cudaSuccess) e = mem_.get(d_status_, kStatusWords * sizeof(int));
   if (e == cudaSuccess) e = cudaMemsetAsync(d_status_, 0, kStatusWords * sizeof(int), st);
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(d_status_ + 4, &wait_budget_, sizeof(int), cudaMemcpyHostToDevice, st);
-  if (e == cudaSuccess) e = cudaMalloc(&d_flags_, sizeof(int) * std::max<int64_t>(H.ndinv, 1));
+  if (e == cudaSuccess) e = mem_.get(d_flags_, sizeof(int) * std::max<int64_t>(H.ndinv, 1));
   if (e == cudaSuccess) e = cudaMemsetAsync(d_flags_, 0, sizeof(int) * std::max<int64_t>(H.ndinv, 1), st);
   if (e == cudaSuccess)
-    e = cudaMalloc(&d_dinv_, sizeof(double) * TB * TB * std::max<int64_t>(H.ndinv, 1));
+    e = mem_.get(d_dinv_, sizeof(double) * TB * TB * std::max<int64_t>(H.ndinv, 1));
   if (e == cudaSuccess)
-    e = cudaMalloc(&d_csr_val_, sizeof(double) * std::max<size_t>(csr_ci.size(), 1));
+    e = mem_.get(d_csr_val_, sizeof(double) * std::max<size_t>(csr_ci.size(), 1));
   // queue head of the CTA walk, done flags, queue head of the warp walk
-  if (e == cudaSuccess) e = cudaMalloc(&d_qctr_, sizeof(int) * ((size_t)supNo + 2));
+  if (e == cudaSuccess) e = mem_.get(d_qctr_, sizeof(int) * ((size_t)supNo + 2));
   if (e == cudaSuccess && !P.tiny_list.empty()) tiny_ctas_ = tiny_ctas((int)P.tiny_list.size());
   if (e == cudaSuccess && !P.persist_list.empty())
     persist_ctas_ = persist_ctas(P.persist_smem, (int)P.persist_list.size());
   // dense dataflow: one queue head per wave, then the tile version counters
   dense_ver_len_ = (int64_t)P.waves.size() + P.dense_tiles;
   if (e == cudaSuccess && !P.dense_tasks.empty())
-    e = cudaMalloc(&d_dense_ver_, sizeof(int) * dense_ver_len_);
+    e = mem_.get(d_dense_ver_, sizeof(int) * dense_ver_len_);
   for (Wave &W : P.waves)
     if (W.dense_cnt > 0) W.dense_ctas = dense_ctas(W.dense_cnt);
 
@@ -1362,19 +1497,29 @@ bool Engine::analyze(int n, const int *c, const int *r, const int64_t *lC, const
   sym_.xk = nullptr;
   sym_.dinv_off = d_dinv_off_;
   kmirror_len_ = kmirror_layout(H.super, H.rowptr, h_xk_);
-  hsym_ = H;
+  hsym_ = std::move(H);
   h_Ls_.assign(Ls, Ls + nls);
+  h_prune_ptr_.assign(prunePtr, prunePtr + supNo + 1);
+  h_prune_.assign(pruneSet, pruneSet + nprune);
   front_ = FP;
-
+  // the contribution blocks, also the mixed modes' mirror when it fits (a factorization uses
+  // one or the other); without the memory the left-looking kernels stay
+  if (FP->ok) {
+    cb_bytes_ = sizeof(double) * (size_t)std::max<int64_t>(FP->cb_len, 1);
+    const size_t lk = sizeof(float) * (size_t)kmirror_len_;
+    if (lk <= cb_bytes_ + cb_bytes_ / 4) cb_bytes_ = std::max(cb_bytes_, lk);
+    if (mem_.get(d_cb_, cb_bytes_) != cudaSuccess) {
+      cudaGetLastError();
+      cb_bytes_ = 0;
+    }
+  }
+  mem_.sweep();
   return true;
 }
 
 void Engine::release_front() {
-  void *ptrs[] = {d_frel_, d_fapos_, d_fppos_, d_fkids_, d_fwarp_, d_fcta_, d_fsmall_,
-                  d_fext_end_, d_fsch_end_, d_fext_, d_fsch_, d_fext_pairs_, d_fsch_pairs_,
-                  d_fcb_off_, d_cb_};
-  for (void *p : ptrs)
-    if (p) cudaFree(p);
+  mem_.put(d_cb_);
+  cb_bytes_ = 0;
   d_frel_ = d_fapos_ = d_fppos_ = nullptr;
   d_fkids_ = nullptr;
   d_fwarp_ = d_fcta_ = d_fsmall_ = nullptr;
@@ -1389,41 +1534,60 @@ void Engine::release_front() {
 
 bool Engine::prepare_tree(std::string &err) {
   if (d_frel_) return true;
-  const FrontPlan &F = *front_;
-  cudaStream_t st = stream_;
-  if (!(upload(d_fapos_, F.apos.data(), F.apos.size(), st, err) &&
-        upload(d_frel_, F.rel.data(), F.rel.size(), st, err)))
-    return false;
-  if (cudaStreamSynchronize(st) != cudaSuccess) { err = "device upload: elimination tree"; return false; }
-  return true;
+  TableUpload up;
+  up.add(d_fapos_, front_->apos);
+  up.add(d_frel_, front_->rel);
+  return up.commit(mem_, tables_, stream_, err);
 }
 
-// The multifrontal plan's tables and the contribution blocks on the device, on the first FP64
-// factorization of a structure; without the memory for them the left-looking kernels stay.
+bool Engine::prepare_left(std::string &err) {
+  if (d_pairs_) return true;
+  if (!plan_.left && !build_left_plan(h_Ls_.data(), h_prune_ptr_.data(), h_prune_.data(), hsym_, plan_, err))
+    return false;
+  TableUpload up;
+  up.add(d_upd_tasks_, plan_.upd_tasks);
+  up.add(d_upd_end_, plan_.upd_end);
+  up.add(d_pairs_, plan_.upd_pairs);
+  up.add(d_tc_pairs_, plan_.tc_pairs);
+  return up.commit(mem_, tables_, stream_, err);
+}
+
+bool Engine::prepare_scatter(std::string &err) {
+  if (d_sc_tiles_) return true;
+  if (plan_.sc_coff.empty() && !build_scatter_plan(n_, h_Ls_.data(), hsym_, front_.get(), plan_, tuning_, err)) return false;
+  TableUpload up;
+  up.add(d_sc_tiles_, plan_.sc_tiles);
+  up.add(d_sc_small_, plan_.sc_small);
+  up.add(d_sc_dense_, plan_.sc_dense);
+  up.add(d_sc_base_, plan_.sc_base);
+  up.add(d_sc_coff_, plan_.sc_coff);
+  up.add(d_sc_rel_, plan_.sc_rel);
+  up.add(d_sc_relidx_, plan_.sc_relidx);
+  return up.commit(mem_, tables_, stream_, err);
+}
+
+// The multifrontal plan's tables on the device, on the first FP64 factorization of a structure.
 bool Engine::prepare_front(std::string &err) {
-  if (front_tried_ || !front_ || !front_->ok) return true;
+  if (front_tried_) return front_ready_ || prepare_left(err);
+  if (!front_ || !front_->ok) return prepare_left(err);
   front_tried_ = true;
   const FrontPlan &F = *front_;
-  cudaStream_t st = stream_;
-  if (cudaMalloc(&d_cb_, sizeof(double) * std::max<int64_t>(F.cb_len, 1)) != cudaSuccess) {
-    cudaGetLastError();
-    d_cb_ = nullptr;
-    return true;
-  }
-  if (!(prepare_tree(err) && upload(d_fwarp_, F.warp_desc.data(), F.warp_desc.size(), st, err) &&
-        upload(d_fcta_, F.cta_desc.data(), F.cta_desc.size(), st, err) &&
-        upload(d_fsmall_, F.small_desc.data(), F.small_desc.size(), st, err) &&
-        upload(d_fkids_, F.kids.data(), F.kids.size(), st, err) &&
-        upload(d_fppos_, F.ppos.data(), F.ppos.size(), st, err) &&
-        upload(d_fext_, F.ext_tasks.data(), F.ext_tasks.size(), st, err) &&
-        upload(d_fext_end_, F.ext_end.data(), F.ext_end.size(), st, err) &&
-        upload(d_fext_pairs_, F.ext_pairs.data(), F.ext_pairs.size(), st, err) &&
-        upload(d_fsch_, F.sch_tasks.data(), F.sch_tasks.size(), st, err) &&
-        upload(d_fsch_end_, F.sch_end.data(), F.sch_end.size(), st, err) &&
-        upload(d_fsch_pairs_, F.sch_pairs.data(), F.sch_pairs.size(), st, err) &&
-        upload(d_fcb_off_, F.cb_off.data(), F.cb_off.size(), st, err)))
-    return false;
-  if (cudaStreamSynchronize(st) != cudaSuccess) { err = "device upload: front plan"; return false; }
+  if (!d_cb_) return prepare_left(err);
+  if (!prepare_tree(err)) return false;
+  TableUpload up;
+  up.add(d_fwarp_, F.warp_desc);
+  up.add(d_fcta_, F.cta_desc);
+  up.add(d_fsmall_, F.small_desc);
+  up.add(d_fkids_, F.kids);
+  up.add(d_fppos_, F.ppos);
+  up.add(d_fext_, F.ext_tasks);
+  up.add(d_fext_end_, F.ext_end);
+  up.add(d_fext_pairs_, F.ext_pairs);
+  up.add(d_fsch_, F.sch_tasks);
+  up.add(d_fsch_end_, F.sch_end);
+  up.add(d_fsch_pairs_, F.sch_pairs);
+  up.add(d_fcb_off_, F.cb_off);
+  if (!up.commit(mem_, tables_, stream_, err)) return false;
   front_dev_ = std::make_shared<FrontDev>(
       FrontDev{d_fkids_, d_frel_, d_fppos_, d_fcb_off_, d_cb_});
   if (!F.warp_list.empty()) fwarp_ctas_ = front_warp_walk_ctas((int)F.warp_list.size());
@@ -1624,42 +1788,36 @@ void Engine::launch_all(std::vector<std::pair<int, cudaEvent_t>> *prof, int prec
 }
 
 bool Engine::set_mode(int prec, std::string &err) {
-  if (prec != 0 && !d_Lk_) {   // the K-major split mirror, its format arrays, tensor maps
-    const size_t mb = tensor_map_bytes() * (size_t)nsuper_;
-    const size_t nx = h_xk_.size();   // nsuper + 1: offsets, then the format entry
-    std::vector<unsigned char> maps(mb);
-    std::vector<int64_t> xk16(h_xk_);
-    xk16[nx - 1] = 1;
-    cudaError_t e = cudaMalloc(&d_Lk_, sizeof(float) * std::max<int64_t>(kmirror_len_, 8));
-    if (e == cudaSuccess) e = cudaMalloc(&d_xk_, sizeof(int64_t) * nx);
-    if (e == cudaSuccess) e = cudaMalloc(&d_xk16_, sizeof(int64_t) * nx);
-    if (e == cudaSuccess) e = cudaMalloc(&d_tmaps_, std::max<size_t>(mb, 128));
+  if (prec != 0 && (!prepare_scatter(err) || (plan_.sc_coff.empty() && !prepare_left(err)))) return false;
+  if (prec != 0 && !d_Lk_) {   // the K-major split mirror and its format arrays
+    const size_t lk_bytes = sizeof(float) * (size_t)std::max<int64_t>(kmirror_len_, 8);
+    cudaError_t e = cudaSuccess;
+    if (lk_bytes <= cb_bytes_) d_Lk_ = reinterpret_cast<float *>(d_cb_);
+    else e = mem_.get(d_Lk_, lk_bytes);
     if (e != cudaSuccess) {
       err = std::string("mirror allocation: ") + cudaGetErrorString(e);
       return false;
     }
-    if (!build_tensor_maps(hsym_.super, hsym_.rowptr, h_xk_, d_Lk_, maps.data(), err)) return false;
-    for (int f = 0; f < 2 && !plan_.sc_coff.empty(); ++f) {
-      // plane maps of the right-looking update tiles, split-TF32 (f = 0) and BF16x3 layouts
-      std::vector<unsigned char> sm(tensor_map_bytes() * scatter_maps_count(nsuper_, f == 1), 0);
-      if (!build_scatter_maps(hsym_.super, hsym_.rowptr, h_xk_, plan_.sc_used, d_Lk_, f == 1,
-                              sm.data(), err))
-        return false;
-      void *&dst = f ? d_sc_maps16_ : d_sc_maps_;
-      e = cudaMalloc(&dst, sm.size());
-      if (e == cudaSuccess) e = cudaMemcpy(dst, sm.data(), sm.size(), cudaMemcpyHostToDevice);
-      if (e != cudaSuccess) {
-        err = std::string("scatter tensor maps: ") + cudaGetErrorString(e);
-        return false;
-      }
-    }
-    e = cudaMemcpy(d_xk_, h_xk_.data(), sizeof(int64_t) * nx, cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemcpy(d_xk16_, xk16.data(), sizeof(int64_t) * nx, cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemcpy(d_tmaps_, maps.data(), mb, cudaMemcpyHostToDevice);
-    if (e != cudaSuccess) {
-      err = std::string("mirror set-up: ") + cudaGetErrorString(e);
+    std::vector<int64_t> xk16(h_xk_);   // nsuper + 1: offsets, then the format entry
+    xk16.back() = 1;
+    TableUpload up;
+    up.add(d_xk_, h_xk_);
+    up.add(d_xk16_, xk16);
+    if (!up.commit(mem_, tables_, stream_, err)) return false;
+  }
+  // tensor maps over the mirror, of the launches the mode uses
+  const bool right = !plan_.sc_coff.empty(), bf16 = prec == 2;
+  void *&maps = !right ? d_tmaps_ : bf16 ? d_sc_maps16_ : d_sc_maps_;
+  if (prec != 0 && !maps && (right || (!bf16 && tuning_.tc_tma))) {
+    std::vector<unsigned char> h(tensor_map_bytes() * (right ? scatter_maps_count(nsuper_, bf16) : (size_t)nsuper_), 0);
+    if (right ? !build_scatter_maps(hsym_.super, hsym_.rowptr, h_xk_, plan_.sc_used, d_Lk_, bf16, h.data(), err)
+              : !build_tensor_maps(hsym_.super, hsym_.rowptr, h_xk_, d_Lk_, h.data(), err))
       return false;
-    }
+    TableUpload up;
+    unsigned char *dst = nullptr;
+    up.add(dst, h);
+    if (!up.commit(mem_, tables_, stream_, err)) return false;
+    maps = dst;
   }
   sym_.Lf = prec != 0 ? reinterpret_cast<float2 *>(d_Lk_) : nullptr;
   sym_.xk = prec == 2 ? d_xk16_ : prec == 1 ? d_xk_ : nullptr;
@@ -1679,7 +1837,9 @@ int Engine::factor(const double *values, bool values_on_device, int *info, std::
                                                    : cudaMemcpyHostToDevice, st);
   if (e != cudaSuccess) { err = std::string("values upload: ") + cudaGetErrorString(e); return -1; }
   h2d_bytes_ = values_on_device ? 0 : (int64_t)sizeof(double) * nnz_;
-  if (use_graph_) {
+  if (use_graph_ && ran_[prec]) {
+    // The first factorization of a structure is launched directly: instantiating a graph takes
+    // longer than the launches (100 kernels: 1.9 ms against 0.3), so it pays from the second on.
     // The whole launch sequence is fixed by the structure (and the mode): capture it once
     // per mode, replay it.
     cudaGraph_t &g = graph_[prec];
@@ -1697,6 +1857,7 @@ int Engine::factor(const double *values, bool values_on_device, int *info, std::
     if (e != cudaSuccess) { err = std::string("graph launch: ") + cudaGetErrorString(e); return -1; }
   } else {
     launch_all(nullptr, prec);
+    ran_[prec] = true;
   }
   return finish(info, err);
 }
@@ -1715,6 +1876,16 @@ int Engine::factor_profiled(const double *values, bool values_on_device, int *in
   std::vector<std::pair<int, cudaEvent_t>> prof;
   launch_all(&prof, prec);
   int rc = finish(info, err);
+  std::string werr;
+  if (!plan_.left) {   // the update class's algorithmic work comes with its tiles
+    Plan w;
+    w.waves = plan_.waves;
+    w.big_list = plan_.big_list;
+    if (build_left_plan(h_Ls_.data(), h_prune_ptr_.data(), h_prune_.data(), hsym_, w, werr)) {
+      plan_.work.flops[K_UPDATE] = w.work.flops[K_UPDATE];
+      plan_.work.bytes[K_UPDATE] = w.work.bytes[K_UPDATE];
+    }
+  }
   out = plan_.work;
   for (int k = 0; k < K_NKINDS; ++k) { out.launches[k] = 0; out.ms[k] = 0; }
   for (size_t i = 0; i + 1 < prof.size(); i += 2) {
@@ -1730,8 +1901,7 @@ int Engine::factor_profiled(const double *values, bool values_on_device, int *in
 
 int Engine::finish(int *info, std::string &err) {
   cudaStream_t st = stream_;
-  // full-CSR values of this matrix for residuals, and ||A||_inf
-  launch_gather_vals((int)csr_nnz_, d_csr_map_, d_Ax_, d_csr_val_, st);
+  csr_stale_ = true;
   cudaError_t e = cudaMemcpyAsync(h_status_, d_status_, 4 * sizeof(int), cudaMemcpyDeviceToHost, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   if (e == cudaSuccess) e = cudaGetLastError();
@@ -1749,6 +1919,12 @@ int Engine::finish(int *info, std::string &err) {
   }
   if (info) *info = 0;
   return 0;
+}
+
+// Full-CSR values of the last factor's matrix, for residuals and norms.
+void Engine::refresh_csr() {
+  if (csr_stale_) launch_gather_vals((int)csr_nnz_, d_csr_map_, d_Ax_, d_csr_val_, stream_);
+  csr_stale_ = false;
 }
 
 bool Engine::download(double *lValues, bool to_device, std::string &err) {
@@ -1794,23 +1970,20 @@ double *Engine::staging(size_t doubles, std::string &err) {
 bool Engine::ensure_work(int nrhs, std::string &err) {
   if (nrhs <= work_nrhs_) return true;
   release_solve_graphs();   // they hold the old buffers
-  for (double **p : {&d_sx_, &d_x8_, &d_c8_, &d_contrib_, &d_work_, &d_norms_, &d_npart_}) {
-    if (*p) cudaFree(*p);
-    *p = nullptr;
-  }
+  for (double **p : {&d_sx_, &d_x8_, &d_c8_, &d_contrib_, &d_work_, &d_norms_, &d_npart_}) mem_.put(*p);
   if (h_norms_) cudaFreeHost(h_norms_);
   h_norms_ = nullptr;
   // one vector, and (several right-hand sides) eight interleaved ones with their contributions
   const size_t clen = (size_t)std::max<int64_t>(splan_.contrib_len, 1);
-  cudaError_t e = cudaMalloc(&d_contrib_, sizeof(double) * clen);
-  if (e == cudaSuccess) e = cudaMalloc(&d_sx_, sizeof(double) * (size_t)n_);
-  if (e == cudaSuccess && nrhs > 1) e = cudaMalloc(&d_x8_, sizeof(double) * 8 * (size_t)n_);
-  if (e == cudaSuccess && nrhs > 1) e = cudaMalloc(&d_c8_, sizeof(double) * 8 * clen);
+  cudaError_t e = mem_.get(d_contrib_, sizeof(double) * clen);
+  if (e == cudaSuccess) e = mem_.get(d_sx_, sizeof(double) * (size_t)n_);
+  if (e == cudaSuccess && nrhs > 1) e = mem_.get(d_x8_, sizeof(double) * 8 * (size_t)n_);
+  if (e == cudaSuccess && nrhs > 1) e = mem_.get(d_c8_, sizeof(double) * 8 * clen);
   // work: r, d, p, q vectors (4 * n * nrhs) + row sums
-  if (e == cudaSuccess) e = cudaMalloc(&d_work_, sizeof(double) * ((size_t)4 * n_ * nrhs + n_));
-  if (e == cudaSuccess) e = cudaMalloc(&d_norms_, sizeof(double) * 8 * (nrhs + 1));
+  if (e == cudaSuccess) e = mem_.get(d_work_, sizeof(double) * ((size_t)4 * n_ * nrhs + n_));
+  if (e == cudaSuccess) e = mem_.get(d_norms_, sizeof(double) * 8 * (nrhs + 1));
   if (e == cudaSuccess) e = cudaMallocHost(&h_norms_, sizeof(double) * 8 * (nrhs + 1));
-  if (e == cudaSuccess) e = cudaMalloc(&d_npart_, sizeof(double) * norm_scratch_doubles(nrhs));
+  if (e == cudaSuccess) e = mem_.get(d_npart_, sizeof(double) * norm_scratch_doubles(nrhs));
   if (e != cudaSuccess) {
     err = std::string("solve workspace: ") + cudaGetErrorString(e);
     work_nrhs_ = 0;
@@ -1864,7 +2037,8 @@ void Engine::run_solve(double *x, int nrhs) {
     const int nr = std::min(8, nrhs - r0);
     double *xr = x + (size_t)r0 * n_;
     if (nr == 1) {
-      cudaGraphExec_t g = use_graph_ ? solve_graph(false) : nullptr;
+      cudaGraphExec_t g = use_graph_ && solved_[0] ? solve_graph(false) : nullptr;
+      solved_[0] = true;
       if (!g) {
         run_solve_with(xr, 1, d_contrib_);
       } else {
@@ -1875,7 +2049,8 @@ void Engine::run_solve(double *x, int nrhs) {
       }
     } else {
       launch_pack8(n_, nr, xr, d_x8_, stream_);
-      cudaGraphExec_t g = use_graph_ ? solve_graph(true) : nullptr;
+      cudaGraphExec_t g = use_graph_ && solved_[1] ? solve_graph(true) : nullptr;
+      solved_[1] = true;
       if (g) cudaGraphLaunch(g, stream_);
       else run_solve8(d_x8_);
       launch_unpack8(n_, nr, d_x8_, xr, stream_);
@@ -1965,6 +2140,7 @@ bool Engine::refine(const double *b, double *x, int nrhs, double tol, int maxit,
     return true;
   };
   cudaMemsetAsync(d_status_ + 2, 0, sizeof(int), st);
+  refresh_csr();
   // ||A||_inf
   launch_rowabs(n_, d_csr_rp_, d_csr_val_, rows, st);
   launch_norms(n_, 1, rows, nullptr, d_norms_, d_npart_, st);

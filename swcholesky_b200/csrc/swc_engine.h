@@ -12,6 +12,54 @@
 
 namespace swc {
 
+// Device memory of one engine.  Blocks given back by an analysis are taken again by the next
+// one (a repeated drop-in call otherwise spends about 3 ms in cudaMalloc and cudaFree); what a
+// whole analysis did not take again is freed at its end, so at most the last structure's
+// memory is held.  Not for use by several threads at once (an engine is not either).
+class DeviceMemory {
+ public:
+  ~DeviceMemory();
+  template <typename T>
+  cudaError_t get(T *&p, size_t bytes) {
+    void *q = nullptr;
+    const cudaError_t e = take(&q, bytes);
+    p = static_cast<T *>(q);
+    return e;
+  }
+  template <typename T>
+  void put(T *&p) {
+    if (p) give(p);
+    p = nullptr;
+  }
+  void age();        // marks the blocks that are free now; sweep() frees those still free
+  void sweep();
+
+ private:
+  struct Block { void *p; size_t bytes; bool used, old; };
+  std::vector<Block> blocks_;
+  cudaError_t take(void **p, size_t bytes);
+  void give(void *p);
+};
+
+// Host tables in one device block (the sources stay alive until commit).
+class TableUpload {
+ public:
+  template <typename T>
+  void add(T *&dst, const T *src, size_t count) {
+    slots_.push_back({reinterpret_cast<void **>(&dst), src, sizeof(T) * count, bytes_});
+    bytes_ += (sizeof(T) * count / 256 + 1) * 256;
+  }
+  template <typename T>
+  void add(T *&dst, const std::vector<T> &v) { add(dst, v.data(), v.size()); }
+  // The block is appended to `owned`.
+  bool commit(DeviceMemory &mem, std::vector<void *> &owned, cudaStream_t st, std::string &err);
+
+ private:
+  struct Slot { void **dst; const void *src; size_t len, at; };
+  std::vector<Slot> slots_;
+  size_t bytes_ = 256;
+};
+
 // Device view of one analysed matrix, passed by value to every kernel.
 struct DevSym {
   int n, nsuper;
@@ -111,6 +159,8 @@ struct KernelStats {
   double bytes[K_NKINDS] = {0};   // algorithmic DRAM bytes of one factorization
 };
 
+struct FrontPlan;     // multifrontal FP64 factorization (swc_front.h)
+
 struct Plan {
   std::vector<Wave> waves;
   std::vector<int> small_list;
@@ -138,8 +188,10 @@ struct Plan {
   std::vector<int64_t> sc_base, sc_coff;
   std::vector<int> sc_rel, sc_relidx;
   std::vector<char> sc_used;
+  int64_t sc_index_count = 0;        // relative indices the tables take
   double sc_flops = 0;               // executed flops of the tiles (128x128 blocks)
   int persist_smem = 0;
+  bool left = false;               // the left-looking tiles are built (build_left_plan)
   int launches = 0;  // kernel launches per factorization
   int launches_scatter = 0;  // the same in the mixed modes with right-looking updates
   KernelStats work;  // algorithmic flops/bytes per kernel class
@@ -241,6 +293,13 @@ bool build_plan(int n, const int *c, const int *r, const int64_t *lC, const int 
                 const int *pruneSet, HostSym &H, Plan &P, std::string &err,
                 const Tuning &T = Tuning());
 
+// The parts of a plan that not every handle needs, built on first use: left-looking update
+// tiles; the mixed modes' right-looking tables and dense tiles (a no-op when the plan has none).
+bool build_left_plan(const int *Ls, const int *prunePtr, const int *pruneSet, const HostSym &H, Plan &P,
+                     std::string &err);
+bool build_scatter_plan(int n, const int *Ls, const HostSym &H, const FrontPlan *tree, Plan &P,
+                        const Tuning &T, std::string &err);
+
 // Host check of a plan's right-looking update tables (a no-op without them): every scattered
 // entry's address against a direct lookup in the target's row list, every descendant's
 // lower triangle covered once per column of K, every tile in the level after its
@@ -263,7 +322,6 @@ void build_solve_plan(int n, const int *Ls, const HostSym &H, SolvePlan &SP);
 bool check_solve_plan(int n, const int *Ls, const HostSym &H, const SolvePlan &SP,
                       std::string &err);
 
-struct FrontPlan;     // multifrontal FP64 factorization (swc_front.h)
 struct FrontDev;
 struct FrontDesc;
 struct FrontChild;
@@ -349,8 +407,8 @@ class Engine {
   void release();
   void launch_all(std::vector<std::pair<int, cudaEvent_t>> *prof = nullptr, int prec = 0);
   bool set_mode(int prec, std::string &err);
-  // multifrontal FP64 factorization: the contribution blocks are allocated on first use; when
-  // the structure or the memory does not allow it, the left-looking kernels are used
+  // multifrontal FP64 factorization; when the structure or the memory does not allow it, the
+  // left-looking kernels are used
   std::shared_ptr<FrontPlan> front_;
   std::shared_ptr<FrontDev> front_dev_;
   bool front_ready_ = false, front_tried_ = false;
@@ -361,7 +419,18 @@ class Engine {
   int4 *d_fext_ = nullptr, *d_fsch_ = nullptr, *d_fext_pairs_ = nullptr, *d_fsch_pairs_ = nullptr;
   int64_t *d_fcb_off_ = nullptr;
   double *d_cb_ = nullptr;
+  size_t cb_bytes_ = 0;
   int fwarp_ctas_ = 0, fcta_ctas_ = 0;
+  DeviceMemory mem_;
+  std::vector<void *> tables_;                 // blocks of uploaded tables
+  std::vector<int> h_prune_ptr_, h_prune_;
+  bool prepare_left(std::string &err);         // left-looking update tiles
+  bool prepare_scatter(std::string &err);      // the mixed modes' right-looking tables
+  bool csr_stale_ = false;                     // d_csr_val_ does not hold the last factor's values
+  void refresh_csr();
+  bool ran_[3] = {false, false, false};        // a mode's first factorization is launched directly
+  bool solved_[2] = {false, false};            // likewise the solves (one vector, eight)
+  bool swept_ = false;                         // and the adjoint's sweep
   bool prepare_tree(std::string &err);   // the tree's tables (also the adjoint's)
   bool prepare_front(std::string &err);
   void release_front();
