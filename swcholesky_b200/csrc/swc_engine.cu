@@ -188,6 +188,7 @@ Engine::Engine(int device) : device_(device) {
   cudaStreamCreateWithFlags(&small_stream_, cudaStreamNonBlocking);
   cudaStreamCreateWithFlags(&grp_stream_, cudaStreamNonBlocking);
   for (int k = 0; k < 2; ++k) cudaEventCreateWithFlags(&ev_grp_[k], cudaEventDisableTiming);
+  cudaEventCreateWithFlags(&ev_next_, cudaEventDisableTiming);
   cudaEventCreateWithFlags(&ev_sfork_, cudaEventDisableTiming);
   cudaEventCreateWithFlags(&ev_sjoin_, cudaEventDisableTiming);
   cudaMallocHost(&h_status_, kStatusWords * sizeof(int));
@@ -206,6 +207,7 @@ Engine::~Engine() {
   if (grp_stream_) cudaStreamDestroy(grp_stream_);
   for (int k = 0; k < 2; ++k)
     if (ev_grp_[k]) cudaEventDestroy(ev_grp_[k]);
+  if (ev_next_) cudaEventDestroy(ev_next_);
   if (ev_sfork_) cudaEventDestroy(ev_sfork_);
   if (ev_sjoin_) cudaEventDestroy(ev_sjoin_);
 }
@@ -542,6 +544,16 @@ bool build_plan(int n, const int *c, const int *r, const int64_t *lC, const int 
       W.panel_off.push_back((int)P.panel_tasks.size());
       W.syrk_off.push_back((int)P.syrk_tasks.size());
       W.diag_off.push_back((int)P.diag_list.size());
+      std::vector<int4> late;   // (s, r0, cc, first block) of the grouped updates
+      auto add_syrk = [&](int s, int r0, int cc, int first) {
+        const int w = super[s + 1] - super[s], m = (int)(rowptr[s + 1] - rowptr[s]);
+        const int kc = j * TB + std::min(TB, w - j * TB) - first * TB;
+        // .w: the task's own index: its product (column blocks first..j) in syrk_pairs
+        P.syrk_pairs.push_back(TcPair{s, r0, cc, (first * TB) | (kc << 16), low_bits(std::min(TB, m - r0)),
+                                      low_bits(std::min(TB, w - cc))});
+        P.syrk_tasks.push_back(make_int4(s, r0, cc, (int)P.syrk_tasks.size()));
+        P.syrk_end.push_back((int)P.syrk_tasks.size());
+      };
       for (int s : big) {
         int w = super[s + 1] - super[s];
         int m = (int)(rowptr[s + 1] - rowptr[s]);
@@ -560,18 +572,15 @@ bool build_plan(int n, const int *c, const int *r, const int64_t *lC, const int 
           if (C == j + 1) first = j;
           else if ((C - 2 - j) % G == 0) first = std::max(0, j - G + 1);
           else continue;
-          for (int r0 = cc; r0 < m; r0 += TB)
-            if (!(cc == c0 + TB && r0 == cc)) {   // next diagonal tile: the TRSM task's update
-              // .w: the task's own index: its product (column blocks first..j) in syrk_pairs
-              P.syrk_pairs.push_back(TcPair{s, r0, cc, (first * TB) | ((c0 + bw - first * TB) << 16),
-                                            low_bits(std::min(TB, m - r0)),
-                                            low_bits(std::min(TB, w - cc))});
-              P.syrk_tasks.push_back(make_int4(s, r0, cc, (int)P.syrk_tasks.size()));
-              P.syrk_end.push_back((int)P.syrk_tasks.size());
-            }
+          for (int r0 = cc; r0 < m; r0 += TB) {
+            if (cc > c0 + TB) late.push_back(make_int4(s, r0, cc, first));
+            else if (r0 > cc) add_syrk(s, r0, cc, first);   // the next diagonal tile: k_diag_step
+          }
         }
         if (c0 + TB < w) P.diag_list.push_back(s);
       }
+      W.syrk_nc.push_back((int)P.syrk_tasks.size() - W.syrk_off.back());
+      for (const int4 &t : late) add_syrk(t.x, t.y, t.z, t.w);
       W.panel_cnt.push_back((int)P.panel_tasks.size() - W.panel_off.back());
       W.syrk_cnt.push_back((int)P.syrk_tasks.size() - W.syrk_off.back());
       W.diag_cnt.push_back((int)P.diag_list.size() - W.diag_off.back());
@@ -1763,6 +1772,33 @@ void Engine::launch_all(std::vector<std::pair<int, cudaEvent_t>> *prof, int prec
         launch_scatter_tc(sym_, sc_maps, d_sc_dense_ + W.scd_off[j], nc, scatter_cols(), 2, bf16, st);
         if (W.diag_cnt[j] > 0) cudaStreamWaitEvent(st, ev_join_, 0);
         if (j + 1 == W.panel_off.size()) cudaStreamWaitEvent(st, ev_grp_[j & 1], 0);
+      } else if (!prof && prec == 0) {
+        // FP64: two chains.  The diagonal blocks (auxiliary stream): block j+1 solves its own
+        // rows of column j (fold), so it waits for diagonal block j and for the updates by
+        // the columns before j, not for this step's TRSM.  The panel (this stream): TRSM of
+        // column j, then the update of column j+1; the grouped updates of the later columns
+        // run beside both.  Column j+1's tiles take the group that ends at step j-1 before
+        // block j's update.
+        const int nc = W.syrk_nc[j], ng = W.syrk_cnt[j] - nc;
+        cudaEventRecord(ev_fork_, st);   // column j solved
+        if (W.diag_cnt[j] > 0) {
+          cudaStreamWaitEvent(aux_stream_, j > 0 ? ev_next_ : ev_fork_, 0);
+          if (j > 0 && W.syrk_cnt[j - 1] > W.syrk_nc[j - 1])
+            cudaStreamWaitEvent(aux_stream_, ev_grp_[(j - 1) & 1], 0);
+          launch_diag_step(sym_, d_diag_ + W.diag_off[j], W.diag_cnt[j], (int)j + 1, aux_stream_, j > 0);
+          cudaEventRecord(ev_join_, aux_stream_);
+        }
+        if (ng > 0) {
+          cudaStreamWaitEvent(grp_stream_, ev_fork_, 0);
+          launch_syrk_step(sym_, d_syrk_ + W.syrk_off[j] + nc, d_syrk_pairs_, ng, grp_stream_);
+          cudaEventRecord(ev_grp_[j & 1], grp_stream_);
+        }
+        if (j > 0 && W.syrk_cnt[j - 1] > W.syrk_nc[j - 1])
+          cudaStreamWaitEvent(st, ev_grp_[(j - 1) & 1], 0);
+        launch_syrk_step(sym_, d_syrk_ + W.syrk_off[j], d_syrk_pairs_, nc, st);
+        cudaEventRecord(ev_next_, st);
+        if (W.diag_cnt[j] > 0) cudaStreamWaitEvent(st, ev_join_, 0);
+        if (j + 1 == W.panel_off.size() && ng > 0) cudaStreamWaitEvent(st, ev_grp_[j & 1], 0);
       } else if (prof) {
         // profiled runs keep one stream so every launch is bracketed by its own events
         mark(K_PANEL, W.diag_cnt[j]);

@@ -137,7 +137,7 @@ struct Wave {
   int upd_off = 0, upd_cnt = 0;    // (supernode, row tile, column tile) update tasks
   int big_off = 0, big_cnt = 0;    // tiled-class supernodes (block 0 POTRF)
   std::vector<int> panel_off, panel_cnt;  // per column block step: TRSM tiles
-  std::vector<int> syrk_off, syrk_cnt;
+  std::vector<int> syrk_off, syrk_cnt, syrk_nc;  // the first syrk_nc: column block j+1
   std::vector<int> diag_off, diag_cnt;    // per step j: supernodes whose block j+1 exists
   std::vector<int> scd_off, scd_cnt;      // per step j: the trailing updates as dense tiles,
   std::vector<int> scd_nc;                //   the first scd_nc of them for column block j+1
@@ -460,6 +460,7 @@ class Engine {
   cudaEvent_t ev_sfork_ = nullptr, ev_sjoin_ = nullptr;
   cudaStream_t grp_stream_ = nullptr;          // grouped trailing updates of the dense steps
   cudaEvent_t ev_grp_[2] = {nullptr, nullptr};
+  cudaEvent_t ev_next_ = nullptr;              // next-column update of the FP64 steps
   int2 *d_asm_ = nullptr, *d_panel_ = nullptr;
   int4 *d_upd_tasks_ = nullptr, *d_syrk_ = nullptr, *d_pairs_ = nullptr;
   int *d_upd_end_ = nullptr;
@@ -530,7 +531,10 @@ void launch_factor_small_persist(const DevSym &S, const int2 *lbub, const int *o
 void launch_assemble(const DevSym &S, const int2 *tasks, int count, cudaStream_t st);
 void launch_update_tiles(const DevSym &S, const int4 *tasks, const int *task_end,
                          const int4 *pairs, int count, cudaStream_t st);
-void launch_diag_step(const DevSym &S, const int *list, int count, int step, cudaStream_t st);
+// fold: the rows of this block in the previous column block are solved here, from the copy the
+// trailing update left in the block's place of dinv (launch_syrk_step), not read from L
+void launch_diag_step(const DevSym &S, const int *list, int count, int step, cudaStream_t st,
+                      bool fold = false);
 void launch_trsm_step(const DevSym &S, const int2 *tasks, int count, int step, cudaStream_t st);
 // tasks (s, r0, c0, product index): prod[index].kk names the column blocks applied
 void launch_syrk_step(const DevSym &S, const int4 *tasks, const TcPair *prod, int count,

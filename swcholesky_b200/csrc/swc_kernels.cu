@@ -584,14 +584,17 @@ __device__ __forceinline__ void mma8_abt(double (&c)[2], const double *Am, int a
 // dynamic shared memory: E, the inverse's inner products, the warps' scratch, then D.
 constexpr int E_ELEMS = TB * DLD, W_ELEMS = 16 * 64;
 constexpr int diag_smem(int nw) { return (E_ELEMS + W_ELEMS + TB + nw * 64 + TB * DLD) * 8; }
-constexpr int diag_prev_smem(int nw) { return diag_smem(nw) + TB * DLD * 8; }   // + X
+constexpr int diag_prev_smem(int nw) { return diag_smem(nw) + 2 * TB * DLD * 8; }   // + X, T
 constexpr int DIAG_SMEM = diag_smem(4);
 constexpr int DIAG_NW = 8;   // warps of the per-step diagonal-block kernel
 
-// PREV: the block still misses its update by column block c0/64 - 1 (the rows just above it
-// solved by the previous TRSM launch): it is applied here, on the tile in shared memory,
-// before the factorization (and to the panel rows below a narrower last block, in L).
-template <int NW, bool PREV = false>
+// PREV: the block still misses its update by column block c0/64 - 1 (X, the block's rows of that
+// column): it is applied here, on the tile in shared memory, before the factorization (and to
+// the panel rows below a narrower last block, in L).  X is read from L (solved by the previous
+// TRSM launch) or, FOLD, solved here: X = B T^T with T the previous block's inverse and B the
+// unsolved tile the trailing update left in this block's place of dinv.  The chain of diagonal
+// blocks then does not pass through the TRSM launch (6.7 us and a launch gap per 64 columns).
+template <int NW, bool PREV = false, bool FOLD = false>
 __device__ void factor_diag_block(const DevSym &S, int s, int c0, double *smem,
                                   const TileAcc *upd) {
   constexpr int NTH = 32 * NW;
@@ -606,21 +609,50 @@ __device__ void factor_diag_block(const DevSym &S, int s, int c0, double *smem,
   // the tile and, with PREV, X = rows c0.. of column block c0/64 - 1 (64 wide, [column][row]
   // after D): eight loads of each in flight per thread before the shared stores
   double *Xs = D + TB * DLD;
+  double *Bs = E, *Ts = Xs + TB * DLD;   // FOLD: B [k][row] (in E's place), T(c, k) as [k][c]
+  const double *Bg = nullptr;
+  if (FOLD) Bg = S.dinv + ((size_t)S.dinv_off[s] + c0 / TB) * (TB * TB);
   const int nr = min(TB, m - c0);
   for (int e0 = tid; e0 < TB * TB; e0 += 8 * NTH) {
-    double v[8], xv[8];
+    double v[8], xv[8], tv[8];
 #pragma unroll
     for (int q = 0; q < 8; ++q) {
       const int e = e0 + q * NTH, c = e >> 6, r = e & (TB - 1);
       if (c < bw && r < bw) v[q] = (!upd && r >= c) ? P[(size_t)(c0 + c) * m + c0 + r] : 0.0;
       else v[q] = (r == c) ? 1.0 : 0.0;
-      if (PREV) xv[q] = r < nr ? P[(size_t)(c0 - TB + c) * m + c0 + r] : 0.0;
+      if (FOLD) {
+        xv[q] = r < nr ? Bg[e] : 0.0;
+        tv[q] = Bg[e - TB * TB];
+      } else if (PREV) {
+        xv[q] = r < nr ? P[(size_t)(c0 - TB + c) * m + c0 + r] : 0.0;
+      }
     }
 #pragma unroll
     for (int q = 0; q < 8; ++q) {
       const int e = e0 + q * NTH;
       D[(e >> 6) * DLD + (e & (TB - 1))] = v[q];
-      if (PREV) Xs[(e >> 6) * DLD + (e & (TB - 1))] = xv[q];
+      if (PREV) (FOLD ? Bs : Xs)[(e >> 6) * DLD + (e & (TB - 1))] = xv[q];
+      if (FOLD) Ts[(e >> 6) * DLD + (e & (TB - 1))] = tv[q];
+    }
+  }
+  if (FOLD) {   // X = B T^T: warp w the rows 8w .. 8w + 7 (T is lower triangular)
+    static_assert(!FOLD || NW == TB / 8, "a row block per warp");
+    __syncthreads();
+    const int w8 = 8 * (tid >> 5), lane = tid & 31, g = lane >> 2, kq = lane & 3;
+    double acc[8][2];
+#pragma unroll
+    for (int n = 0; n < 8; ++n) acc[n][0] = acc[n][1] = 0.0;
+#pragma unroll
+    for (int k4 = 0; k4 < 16; ++k4) {
+      const int col = (4 * k4 + kq) * DLD + g;
+      const double a = Bs[col + w8];
+#pragma unroll
+      for (int n = k4 / 2; n < 8; ++n) dmma(acc[n], a, Ts[col + 8 * n]);
+    }
+#pragma unroll
+    for (int n = 0; n < 8; ++n) {
+      Xs[(8 * n + 2 * kq) * DLD + w8 + g] = acc[n][0];
+      Xs[(8 * n + 2 * kq + 1) * DLD + w8 + g] = acc[n][1];
     }
   }
   if (PREV) {
@@ -723,9 +755,9 @@ __device__ void syrk_tile_acc(const DevSym &S, int s, int r0, int c0, int kblk, 
                     stages, acc);
 }
 
-// ... stored back negated.
+// ... stored back negated (and to copy, [column][row] of 64, where it is given).
 __device__ void syrk_tile(const DevSym &S, int s, int r0, int c0, int kblk, double *stages,
-                          int nblk = 1) {
+                          int nblk = 1, double *copy = nullptr) {
   const int f = S.super[s];
   const int w = S.super[s + 1] - f;
   const int m = (int)(S.rowptr[s + 1] - S.rowptr[s]);
@@ -742,7 +774,10 @@ __device__ void syrk_tile(const DevSym &S, int s, int r0, int c0, int kblk, doub
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
         const int c = acc_col(j, e);
-        if (c < ncol && r0 + r >= c0 + c) P[(size_t)(c0 + c) * m + r0 + r] = neg(acc.v[i][j][e]);
+        if (c < ncol && r0 + r >= c0 + c) {
+          P[(size_t)(c0 + c) * m + r0 + r] = neg(acc.v[i][j][e]);
+          if (copy) copy[c * TB + r] = neg(acc.v[i][j][e]);
+        }
       }
   }
 }
@@ -762,10 +797,13 @@ __device__ void diag_task(const DevSym &S, int s, int step, double *smem) {
 
 // Per-step launches: one CTA per supernode of the list factors diagonal block `step`, after
 // applying its update by column block step-1 (the last one it misses).
+template <bool FOLD>
 __global__ void __launch_bounds__(DIAG_NW * 32) k_diag_step(DevSym S, const int *list, int count,
                                                            int step) {
   extern __shared__ double dyn[];
-  if (step > 0)
+  if (FOLD)
+    factor_diag_block<DIAG_NW, true, true>(S, list[blockIdx.x], step * TB, dyn, nullptr);
+  else if (step > 0)
     factor_diag_block<DIAG_NW, true>(S, list[blockIdx.x], step * TB, dyn, nullptr);
   else
     factor_diag_block<DIAG_NW, false>(S, list[blockIdx.x], 0, dyn, nullptr);
@@ -818,7 +856,9 @@ __global__ void __launch_bounds__(MT, 4) k_trsm_step(DevSym S, const int2 *tasks
 // Trailing update of a step: task = (s, r0, c0, product index) with c0 >= (step+1)*64,
 // r0 >= c0; the product names the column blocks applied (the step's block, or a group of
 // blocks ending with it).  The diagonal tile of the next block is updated by the TRSM
-// launch of the step and factored by k_diag_step, which runs concurrently.
+// launch of the step and factored by k_diag_step, which runs concurrently.  The tile just below
+// that one also goes to the place of its diagonal block's inverse in dinv (free until then),
+// unsolved, for the block's own solve of it.
 constexpr int SYRK_SMEM = 2 * STAGE * 8;
 
 __global__ void __launch_bounds__(MT) k_syrk_step(DevSym S, const int4 *tasks, const TcPair *prod,
@@ -826,7 +866,10 @@ __global__ void __launch_bounds__(MT) k_syrk_step(DevSym S, const int4 *tasks, c
   extern __shared__ double dyn[];
   const int4 t = tasks[blockIdx.x];
   const int kk = prod[t.w].kk;   // the task's column blocks: first = k0 / 64, then kcnt columns
-  syrk_tile(S, t.x, t.y, t.z, (kk & 0xffff) / TB, dyn, ((kk >> 16) + TB - 1) / TB);
+  const bool next = t.z == (kk & 0xffff) + (kk >> 16) && t.y == t.z + TB &&
+                    t.y < S.super[t.x + 1] - S.super[t.x];
+  double *copy = next ? S.dinv + ((size_t)S.dinv_off[t.x] + t.y / TB) * (TB * TB) : nullptr;
+  syrk_tile(S, t.x, t.y, t.z, (kk & 0xffff) / TB, dyn, ((kk >> 16) + TB - 1) / TB, copy);
 }
 
 // ---------------------------------------------------------------------------------------
@@ -1035,7 +1078,10 @@ bool kernels_configure(std::string &err) {
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(k_trsm_step, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * STAGE * 8);
   if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_diag_step, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    e = cudaFuncSetAttribute(k_diag_step<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             diag_prev_smem(DIAG_NW));
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(k_diag_step<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              diag_prev_smem(DIAG_NW));
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(k_syrk_step, cudaFuncAttributeMaxDynamicSharedMemorySize, SYRK_SMEM);
@@ -1087,9 +1133,10 @@ void launch_update_tiles(const DevSym &S, const int4 *tasks, const int *task_end
                          const int4 *pairs, int count, cudaStream_t st) {
   if (count > 0) k_update_tiles<<<count, MT, UPD_SMEM, st>>>(S, tasks, task_end, pairs, count);
 }
-void launch_diag_step(const DevSym &S, const int *list, int count, int step, cudaStream_t st) {
-  if (count > 0)
-    k_diag_step<<<count, DIAG_NW * 32, diag_prev_smem(DIAG_NW), st>>>(S, list, count, step);
+void launch_diag_step(const DevSym &S, const int *list, int count, int step, cudaStream_t st, bool fold) {
+  if (count <= 0) return;
+  if (fold) k_diag_step<true><<<count, DIAG_NW * 32, diag_prev_smem(DIAG_NW), st>>>(S, list, count, step);
+  else k_diag_step<false><<<count, DIAG_NW * 32, diag_prev_smem(DIAG_NW), st>>>(S, list, count, step);
 }
 void launch_trsm_step(const DevSym &S, const int2 *tasks, int count, int step, cudaStream_t st) {
   if (count > 0) k_trsm_step<<<count, MT, 2 * STAGE * 8, st>>>(S, tasks, count, step);
