@@ -189,6 +189,9 @@ Engine::Engine(int device) : device_(device) {
   cudaStreamCreateWithFlags(&grp_stream_, cudaStreamNonBlocking);
   for (int k = 0; k < 2; ++k) cudaEventCreateWithFlags(&ev_grp_[k], cudaEventDisableTiming);
   cudaEventCreateWithFlags(&ev_next_, cudaEventDisableTiming);
+  cudaStreamCreateWithFlags(&sch_stream_, cudaStreamNonBlocking);
+  cudaEventCreateWithFlags(&ev_sch_, cudaEventDisableTiming);
+  cudaDeviceGetAttribute(&num_sms_, cudaDevAttrMultiProcessorCount, device_);
   cudaEventCreateWithFlags(&ev_sfork_, cudaEventDisableTiming);
   cudaEventCreateWithFlags(&ev_sjoin_, cudaEventDisableTiming);
   cudaMallocHost(&h_status_, kStatusWords * sizeof(int));
@@ -208,6 +211,8 @@ Engine::~Engine() {
   for (int k = 0; k < 2; ++k)
     if (ev_grp_[k]) cudaEventDestroy(ev_grp_[k]);
   if (ev_next_) cudaEventDestroy(ev_next_);
+  if (ev_sch_) cudaEventDestroy(ev_sch_);
+  if (sch_stream_) cudaStreamDestroy(sch_stream_);
   if (ev_sfork_) cudaEventDestroy(ev_sfork_);
   if (ev_sjoin_) cudaEventDestroy(ev_sjoin_);
 }
@@ -1699,15 +1704,19 @@ void Engine::launch_all(std::vector<std::pair<int, cudaEvent_t>> *prof, int prec
       launch_small(st);
       mark(-1, small_cnt);
     }
-    // the end of the wave: its small supernodes joined, then (multifrontal) the tiles of its
-    // contribution blocks
+    // the end of the wave: its small supernodes joined, then (multifrontal) the rest of its
+    // contribution blocks (parts of them are formed beside the dense steps)
+    int parts = 0;
     auto finish_wave = [&]() {
       if (side) cudaStreamWaitEvent(st, ev_sjoin_, 0);
       if (!front) return;
-      mark(K_UPDATE, FWv->sch_cnt);
+      const int b0 = parts * FWv->sch_steps;
+      if (parts > 0) cudaStreamWaitEvent(st, ev_sch_, 0);
+      const int cnt = b0 > 0 ? FWv->sch_more[b0] : FWv->sch_cnt;
+      mark(K_UPDATE, cnt);
       launch_front_schur(sym_, *front_dev_, d_fsch_ + FWv->sch_off, d_fsch_end_ + FWv->sch_off,
-                         d_fsch_pairs_, FWv->sch_cnt, st);
-      mark(-1, FWv->sch_cnt);
+                         d_fsch_pairs_, cnt, b0 * TB, INT_MAX, 0, st);
+      mark(-1, cnt);
     };
     if (front) {
       mark(K_ASSEMBLE, FWv->ext_cnt);
@@ -1787,6 +1796,16 @@ void Engine::launch_all(std::vector<std::pair<int, cudaEvent_t>> *prof, int prec
             cudaStreamWaitEvent(aux_stream_, ev_grp_[(j - 1) & 1], 0);
           launch_diag_step(sym_, d_diag_ + W.diag_off[j], W.diag_cnt[j], (int)j + 1, aux_stream_, j > 0);
           cudaEventRecord(ev_join_, aux_stream_);
+        }
+        if (front && FWv->sch_steps > 0 && (j + 1) % FWv->sch_steps == 0 && j + 1 < W.panel_off.size()) {
+          const int b0 = (int)j + 1 - FWv->sch_steps;
+          cudaStreamWaitEvent(sch_stream_, ev_fork_, 0);
+          if (side && parts == 0) cudaStreamWaitEvent(sch_stream_, ev_sjoin_, 0);
+          launch_front_schur(sym_, *front_dev_, d_fsch_ + FWv->sch_off, d_fsch_end_ + FWv->sch_off, d_fsch_pairs_,
+                             FWv->sch_more[b0], b0 * TB, ((int)j + 1) * TB, num_sms_ - FRONT_BG_RESERVE,
+                             sch_stream_);
+          cudaEventRecord(ev_sch_, sch_stream_);
+          ++parts;
         }
         if (ng > 0) {
           cudaStreamWaitEvent(grp_stream_, ev_fork_, 0);

@@ -461,6 +461,9 @@ class Engine {
   cudaStream_t grp_stream_ = nullptr;          // grouped trailing updates of the dense steps
   cudaEvent_t ev_grp_[2] = {nullptr, nullptr};
   cudaEvent_t ev_next_ = nullptr;              // next-column update of the FP64 steps
+  cudaStream_t sch_stream_ = nullptr;          // contribution blocks formed beside the dense steps
+  cudaEvent_t ev_sch_ = nullptr;
+  int num_sms_ = 0;
   int2 *d_asm_ = nullptr, *d_panel_ = nullptr;
   int4 *d_upd_tasks_ = nullptr, *d_syrk_ = nullptr, *d_pairs_ = nullptr;
   int *d_upd_end_ = nullptr;

@@ -310,10 +310,10 @@ struct PairMaps {
 
 __device__ __forceinline__ void load_pair_maps(const DevSym &S, const FrontDev &F, const int4 *pairs,
                                                int q, int kids, int rbase, int cbase, PairMaps &M,
-                                               int nth) {
-  for (int i = threadIdx.x; i < kids * TB; i += nth) M.ia[i >> 6][i & 63] = M.ib[i >> 6][i & 63] = -1;
-  __syncthreads();
-  for (int i = threadIdx.x; i < kids * 2 * TB; i += nth) {
+                                               int nth, int tid = threadIdx.x, int bar = 0) {
+  for (int i = tid; i < kids * TB; i += nth) M.ia[i >> 6][i & 63] = M.ib[i >> 6][i & 63] = -1;
+  tile_sync(bar);
+  for (int i = tid; i < kids * 2 * TB; i += nth) {
     const int k = i >> 7, u = i & 63;
     const int4 pr = pairs[q + k];
     const int c = pr.x;
@@ -329,7 +329,7 @@ __device__ __forceinline__ void load_pair_maps(const DevSym &S, const FrontDev &
       }
     }
   }
-  __syncthreads();
+  tile_sync(bar);
 }
 
 // Extend-add into the panels of tiled supernodes: task = (s, r0, c0, first pair), a 64x64 tile
@@ -376,39 +376,48 @@ __global__ void __launch_bounds__(ET) k_front_extend(DevSym S, FrontDev F, const
   }
 }
 
-// One 64x64 tile of the contribution block of s: minus L_rs L_rs^T (DMMA, K = w) plus the
-// children's blocks.  task = (s, i0, j0, first pair), offsets in the block.  The accumulator
-// collects minus the children's entries and the product, and is stored back negated.
-constexpr int SCHUR_SMEM = 2 * STAGE * 8;
-__global__ void __launch_bounds__(MT, 4) k_front_schur(DevSym S, FrontDev F, const int4 *tasks,
-                                                       const int *end, const int4 *pairs) {
-  extern __shared__ double fsm[];
-  __shared__ PairMaps M;
-  const int4 tk = tasks[blockIdx.x];
-  const int p_end = end[blockIdx.x];
+// One 64x64 tile of the contribution block of s: minus L_rs L_rs^T over the columns k0 .. k1 - 1
+// (DMMA) plus, at k0 = 0, the children's blocks, else what the block holds.  task = (s, i0, j0,
+// first pair), offsets in the block.  The accumulator collects minus the tile's value and the
+// product, and is stored back negated.
+__device__ __forceinline__ void schur_tile(const DevSym &S, const FrontDev &F, int4 tk, int p_end,
+                                           const int4 *pairs, int k0, int k1, double *stages, PairMaps &M,
+                                           int tid, int bar) {
   const int s = tk.x, i0 = tk.y, j0 = tk.z;
   const int w = S.super[s + 1] - S.super[s], m = (int)(S.rowptr[s + 1] - S.rowptr[s]);
   const int r = m - w;
+  double *cbs = F.cb + F.cb_off[s];
+  k1 = min(k1, w);
   TileAcc acc;
-  acc.zero();
-  for (int q = tk.w; q < p_end; q += FRONT_KIDS) {
+  if (k0 == 0) acc.zero();
+  else
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const int ri = i0 + acc_row(i, tid), cj = j0 + acc_col(j, e, tid);
+          acc.v[i][j][e] = neg(ld_if(cbs + (int64_t)cj * r + ri, ri < r && cj <= ri));
+        }
+  for (int q = tk.w; q < p_end && k0 == 0; q += FRONT_KIDS) {
     const int kids = min(FRONT_KIDS, p_end - q);
-    if (q > tk.w) __syncthreads();
-    load_pair_maps(S, F, pairs, q, kids, w + i0, w + j0, M, MT);
+    if (q > tk.w) tile_sync(bar);
+    load_pair_maps(S, F, pairs, q, kids, w + i0, w + j0, M, MT, tid, bar);
     for (int k = 0; k < kids; ++k) {
       const double *cb = M.cb[k];
       const int ldc = M.ld[k];
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        const int pi = M.ia[k][acc_row(i)];
+        const int pi = M.ia[k][acc_row(i, tid)];
         double t[4][2];
 #pragma unroll
         for (int j = 0; j < 4; ++j)
 #pragma unroll
           for (int e = 0; e < 2; ++e) {
-            const int pj = M.ib[k][acc_col(j, e)];
+            const int pj = M.ib[k][acc_col(j, e, tid)];
             t[j][e] = ld_if(cb + (int64_t)pj * ldc + pi,
-                            pi >= 0 && pj >= 0 && i0 + acc_row(i) >= j0 + acc_col(j, e));
+                            pi >= 0 && pj >= 0 && i0 + acc_row(i, tid) >= j0 + acc_col(j, e, tid));
           }
 #pragma unroll
         for (int j = 0; j < 4; ++j)
@@ -417,19 +426,39 @@ __global__ void __launch_bounds__(MT, 4) k_front_schur(DevSym S, FrontDev F, con
       }
     }
   }
-  const double *Lr = S.L + S.xptr[s] + w;
-  dmma_tile_product(Lr + i0, m, min(TB, r - i0), Lr + j0, m, min(TB, r - j0), w, fsm, acc);
-  double *cbs = F.cb + F.cb_off[s];
+  const double *Lr = S.L + S.xptr[s] + (size_t)k0 * m + w;
+  dmma_tile_product(Lr + i0, m, min(TB, r - i0), Lr + j0, m, min(TB, r - j0), k1 - k0, stages, acc, tid, bar);
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    const int ri = i0 + acc_row(i);
+    const int ri = i0 + acc_row(i, tid);
 #pragma unroll
     for (int j = 0; j < 4; ++j)
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
-        const int cj = j0 + acc_col(j, e);
+        const int cj = j0 + acc_col(j, e, tid);
         if (ri < r && cj <= ri) cbs[(size_t)cj * r + ri] = neg(acc.v[i][j][e]);
       }
+  }
+}
+
+constexpr int SCHUR_SMEM = 2 * STAGE * 8;
+__global__ void __launch_bounds__(MT, 4) k_front_schur(DevSym S, FrontDev F, const int4 *tasks,
+                                                       const int *end, const int4 *pairs, int k0, int k1) {
+  extern __shared__ double fsm[];
+  __shared__ PairMaps M;
+  schur_tile(S, F, tasks[blockIdx.x], end[blockIdx.x], pairs, k0, k1, fsm, M, threadIdx.x, 0);
+}
+
+// The same beside the chain of diagonal blocks (see BG), as the panel's columns get done.
+__global__ void __launch_bounds__(BG * MT, 1) k_front_schur_bg(DevSym S, FrontDev F, const int4 *tasks,
+                                                               const int *end, const int4 *pairs, int count,
+                                                               int k0, int k1) {
+  extern __shared__ double fsm[];
+  __shared__ PairMaps M[BG];
+  const int grp = threadIdx.x / MT, tid = threadIdx.x - grp * MT;
+  for (int q = blockIdx.x * BG + grp; q < count; q += BG * gridDim.x) {
+    schur_tile(S, F, tasks[q], end[q], pairs, k0, k1, fsm + grp * 2 * STAGE, M[grp], tid, 1 + grp);
+    tile_sync(1 + grp);
   }
 }
 
@@ -455,6 +484,8 @@ bool front_configure(std::string &err) {
     e = cudaFuncSetAttribute(k_front_warp_walk, cudaFuncAttributeMaxDynamicSharedMemorySize, WARP_SMEM);
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(k_front_schur, cudaFuncAttributeMaxDynamicSharedMemorySize, SCHUR_SMEM);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(k_front_schur_bg, cudaFuncAttributeMaxDynamicSharedMemorySize, BG_SMEM);
   if (e != cudaSuccess) {
     err = std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(e);
     return false;
@@ -490,8 +521,13 @@ void launch_front_extend(const DevSym &S, const FrontDev &F, const int4 *tasks, 
   if (count > 0) k_front_extend<<<count, ET, 0, st>>>(S, F, tasks, end, pairs);
 }
 void launch_front_schur(const DevSym &S, const FrontDev &F, const int4 *tasks, const int *end,
-                        const int4 *pairs, int count, cudaStream_t st) {
-  if (count > 0) k_front_schur<<<count, MT, SCHUR_SMEM, st>>>(S, F, tasks, end, pairs);
+                        const int4 *pairs, int count, int k0, int k1, int bg_ctas, cudaStream_t st) {
+  if (count <= 0) return;
+  if (bg_ctas > 0)
+    k_front_schur_bg<<<std::min(bg_ctas, (count + BG - 1) / BG), BG * MT, BG_SMEM, st>>>(S, F, tasks, end, pairs,
+                                                                                        count, k0, k1);
+  else
+    k_front_schur<<<count, MT, SCHUR_SMEM, st>>>(S, F, tasks, end, pairs, k0, k1);
 }
 
 }  // namespace swc

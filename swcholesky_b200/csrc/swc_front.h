@@ -92,8 +92,20 @@ struct FrontDev {
 struct FrontWave {
   int small_off = 0, small_cnt = 0, small_smem = 0;
   int ext_off = 0, ext_cnt = 0;    // tiles of tiled panels that receive children's blocks
-  int sch_off = 0, sch_cnt = 0;    // tiles of contribution blocks
+  int sch_off = 0, sch_cnt = 0;    // tiles of contribution blocks, wide fronts first
+  std::vector<int> sch_more;       // [b]: the tiles of fronts with more than b column blocks
+  int sch_steps = 0;               // column blocks per part when formed beside the dense steps (0:
+                                   // in one launch after them)
 };
+
+// The contribution blocks of a wave are formed in parts of a quarter of its steps (at least
+// FRONT_BG_STEPS), on all but FRONT_BG_RESERVE SMs, beside the chain of diagonal blocks (about
+// FRONT_STEP_US per 64 columns), where that chain is what the wave waits for: its dense products
+// at FRONT_FLOPS_US flops per us take at most 1.5 times as long.  Waves of few small fronts
+// gain (24 x 23 x 22 3-unknown grid 3249 -> 3138 us, 41 x 37 x 43 7-point grid 3072 -> 3027);
+// with more work the launches only disturb each other (60^3: 14.6 -> 16.2 ms).
+constexpr int FRONT_BG_STEPS = 3, FRONT_BG_RESERVE = 40;
+constexpr double FRONT_STEP_US = 22.0, FRONT_FLOPS_US = 28e6;
 
 struct FrontPlan {
   bool closed = false;             // the tree below holds: children's rows among the parent's
@@ -142,7 +154,9 @@ void launch_front_small(const DevSym &S, const FrontDev &F, const FrontDesc *lis
                         cudaStream_t st);   // cb < 0: the block is formed by tiles
 void launch_front_extend(const DevSym &S, const FrontDev &F, const int4 *tasks, const int *end,
                          const int4 *pairs, int count, cudaStream_t st);
+// tiles of contribution blocks over the columns k0 .. k1 - 1 of each front (k1 beyond a front's
+// width: to its end); bg_ctas > 0: at most that many CTAs of one per SM, beside other kernels
 void launch_front_schur(const DevSym &S, const FrontDev &F, const int4 *tasks, const int *end,
-                        const int4 *pairs, int count, cudaStream_t st);
+                        const int4 *pairs, int count, int k0, int k1, int bg_ctas, cudaStream_t st);
 
 }  // namespace swc

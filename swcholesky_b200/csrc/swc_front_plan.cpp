@@ -243,18 +243,32 @@ void build_front_plan(int n, const int *c, const int *r, const int *Ls, const in
       }
     }
     std::stable_sort(by_width.begin(), by_width.end(), [&](int a, int b) { return width(a) > width(b); });
-    for (int s : by_width) add_tiles(s, width(s), rows(s), true, F.sch_tasks, F.sch_end, F.sch_pairs);
+    const Wave &B = P.waves[lv];
+    const int nsteps = (int)B.panel_off.size();
+    W.sch_more.assign(nsteps + 1, 0);
+    for (int s : by_width) {
+      add_tiles(s, width(s), rows(s), true, F.sch_tasks, F.sch_end, F.sch_pairs);
+      for (int b = 0; b < (width(s) + TB - 1) / TB && b <= nsteps; ++b)
+        W.sch_more[b] = (int)F.sch_tasks.size() - W.sch_off;
+    }
+    const int part = std::max(FRONT_BG_STEPS, (nsteps + 3) / 4);
+    double flops = 0.0;
+    for (int s : by_width) {
+      const double w = width(s), rr = rows(s) - width(s);
+      flops += rr * rr * w + rows(s) * w * w;
+    }
+    if (B.dense_cnt == 0 && nsteps > part && flops <= 1.5 * FRONT_FLOPS_US * FRONT_STEP_US * nsteps) W.sch_steps = part;
     W.small_cnt = (int)F.small_list.size() - W.small_off;
     W.ext_cnt = (int)F.ext_tasks.size() - W.ext_off;
     W.sch_cnt = (int)F.sch_tasks.size() - W.sch_off;
     launches += (W.small_cnt > 0) + (W.ext_cnt > 0) + (W.sch_cnt > 0);
-    const Wave &B = P.waves[lv];
+    for (int b = W.sch_steps; W.sch_steps && b < nsteps; b += W.sch_steps) launches += W.sch_more[b] > 0;
     if (B.dense_cnt > 0) {
       launches += 1;
     } else {
       launches += B.big_cnt > 0;
       for (size_t j = 0; j < B.panel_cnt.size(); ++j)
-        launches += (B.panel_cnt[j] > 0) + (B.syrk_cnt[j] > 0) + (B.diag_cnt[j] > 0);
+        launches += (B.panel_cnt[j] > 0) + (B.syrk_nc[j] > 0) + (B.syrk_cnt[j] > B.syrk_nc[j]) + (B.diag_cnt[j] > 0);
     }
   }
   F.launches = launches + !F.warp_list.empty() + !F.cta_list.empty();
@@ -388,6 +402,8 @@ bool check_front_plan(int n, const int *Ls, const HostSym &H, const Plan &P, con
             o + tk[t].z >= lim || seen[{s, {tk[t].y, tk[t].z}}]++)
           return bad("tile misplaced or twice", s);
         block_tiles[s] += part;
+        for (size_t b = 0; part && b < W.sch_more.size(); ++b)
+          if ((t - t0 < W.sch_more[b]) != ((int)b * TB < w)) return bad("tiles of the wider fronts not first", s);
         for (int q = tk[t].w; q < end[t]; ++q) {
           const int d = pr[q].x, na = pr[q].w & 0xffff, nb = pr[q].w >> 16;
           if (d < 0 || d >= ns || parent[d] != s || na <= 0 || nb <= 0 || na > TB || nb > TB ||

@@ -53,6 +53,9 @@ constexpr int KC = 16;
 constexpr int MT = 128;               // threads of the tensor-core tile kernels
 constexpr int LDS = TB + 4;           // padded row of a staged k-slice: 64-bit fragment loads conflict-free
 constexpr int STAGE = 2 * KC * LDS;   // doubles per pipeline stage (A and B slices)
+// Tile launches that run beside the chain of diagonal blocks: one CTA per SM of three groups (its
+// shared memory keeps a second one out), so the SMs the launch leaves free stay free.
+constexpr int BG = 3, BG_SMEM = BG * 2 * STAGE * 8;
 static_assert(MT == 2 * TB, "staging pattern: two threads per tile row");
 
 __device__ __forceinline__ void cp_async8(double *smem, const double *gmem, bool pred) {
@@ -80,12 +83,19 @@ struct TileAcc {
   }
 };
 
+// The tile functions run on 128 threads: a whole block (bar 0), or one of several groups of a
+// block, with the thread's index in its group and a named barrier of its own.
+__device__ __forceinline__ void tile_sync(int bar) {
+  if (bar == 0) __syncthreads();
+  else asm volatile("bar.sync %0, 128;\n" ::"r"(bar) : "memory");
+}
+
 // Thread t copies tile row t % 64 at chunk offsets t / 64, t / 64 + 2, ... (one pointer
 // step per copy).
 __device__ __forceinline__ void load_chunk(const double *__restrict__ Pa, int lda, int na,
                                            const double *__restrict__ Pb, int ldb, int nb,
-                                           int K, int k0, double *st) {
-  const int i = threadIdx.x & (TB - 1), kq = threadIdx.x >> 6;
+                                           int K, int k0, double *st, int tid) {
+  const int i = tid & (TB - 1), kq = tid >> 6;
   double *As = st + kq * LDS + i, *Bs = st + KC * LDS + kq * LDS + i;
   const double *pa = Pa + (size_t)(k0 + kq) * lda + i, *pb = Pb + (size_t)(k0 + kq) * ldb + i;
   const bool ina = i < na, inb = i < nb;
@@ -102,21 +112,22 @@ __device__ __forceinline__ void load_chunk(const double *__restrict__ Pa, int ld
 
 __device__ __forceinline__ void dmma_tile_product(const double *__restrict__ Pa, int lda, int na,
                                                   const double *__restrict__ Pb, int ldb, int nb,
-                                                  int K, double *stages, TileAcc &acc) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+                                                  int K, double *stages, TileAcc &acc,
+                                                  int tid = threadIdx.x, int bar = 0) {
+  const int lane = tid & 31, warp = tid >> 5;
   const int wr = (warp >> 1) * 32, wc = (warp & 1) * 32;
   const int kq = lane & 3, g = lane >> 2;
   const int nchunks = (K + KC - 1) / KC;
-  __syncthreads();   // stages free (previous users done)
-  load_chunk(Pa, lda, na, Pb, ldb, nb, K, 0, stages);
+  tile_sync(bar);   // stages free (previous users done)
+  load_chunk(Pa, lda, na, Pb, ldb, nb, K, 0, stages, tid);
   for (int c = 0; c < nchunks; ++c) {
     if (c + 1 < nchunks) {
-      load_chunk(Pa, lda, na, Pb, ldb, nb, K, (c + 1) * KC, stages + ((c + 1) & 1) * STAGE);
+      load_chunk(Pa, lda, na, Pb, ldb, nb, K, (c + 1) * KC, stages + ((c + 1) & 1) * STAGE, tid);
       cp_async_wait<1>();
     } else {
       cp_async_wait<0>();
     }
-    __syncthreads();
+    tile_sync(bar);
     const double *As = stages + (c & 1) * STAGE, *Bs = As + KC * LDS;
 #pragma unroll
     for (int k4 = 0; k4 < KC; k4 += 4) {
@@ -130,7 +141,7 @@ __device__ __forceinline__ void dmma_tile_product(const double *__restrict__ Pa,
 #pragma unroll
         for (int j = 0; j < 4; ++j) dmma(acc.v[i][j], a[i], b[j]);
     }
-    __syncthreads();
+    tile_sync(bar);
   }
 }
 
@@ -159,11 +170,11 @@ __device__ __forceinline__ double neg(double x) {
 }
 
 // Position of accumulator element (i, j, e) of this thread inside the 64x64 tile.
-__device__ __forceinline__ int acc_row(int i) {
-  return ((threadIdx.x >> 5) >> 1) * 32 + 8 * i + ((threadIdx.x & 31) >> 2);
+__device__ __forceinline__ int acc_row(int i, int tid = threadIdx.x) {
+  return ((tid >> 5) >> 1) * 32 + 8 * i + ((tid & 31) >> 2);
 }
-__device__ __forceinline__ int acc_col(int j, int e) {
-  return ((threadIdx.x >> 5) & 1) * 32 + 8 * j + 2 * (threadIdx.x & 3) + e;
+__device__ __forceinline__ int acc_col(int j, int e, int tid = threadIdx.x) {
+  return ((tid >> 5) & 1) * 32 + 8 * j + 2 * (tid & 3) + e;
 }
 
 // Cholesky of a panel in shared memory by NW = 1, 4 or 8 warps: P is [column][row] with
