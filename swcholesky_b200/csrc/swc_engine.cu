@@ -545,6 +545,16 @@ bool build_plan(int n, const int *c, const int *r, const int64_t *lC, const int 
       maxnb = std::max(maxnb, (w + TB - 1) / TB);
     }
     W.asm_cnt = (int)P.asm_tasks.size() - W.asm_off;
+    // column blocks per grouped FP64 update: 4, or 2 where the wave's trailing tiles fit the GPU
+    // (three CTAs per SM) even so: there a group's latency, not its arithmetic, holds the chain of
+    // diagonal blocks (41 x 37 x 43 7-point grid 3.04 -> 2.94 ms; 60^3 with 2 everywhere 14.8 ->
+    // 15.0)
+    int64_t trailing = 0;
+    for (int s : big) {
+      const int64_t nb = (super[s + 1] - super[s] + TB - 1) / TB, mb = (rowptr[s + 1] - rowptr[s] + TB - 1) / TB;
+      trailing += nb * (mb - nb / 2);
+    }
+    const int G = std::max(1, trailing <= 2 * GROUP_FULL_TILES ? std::min(2, T.dense_group) : T.dense_group);
     for (int j = 0; j < maxnb; ++j) {
       W.panel_off.push_back((int)P.panel_tasks.size());
       W.syrk_off.push_back((int)P.syrk_tasks.size());
@@ -570,7 +580,6 @@ bool build_plan(int n, const int *c, const int *r, const int64_t *lC, const int 
         // a column C >= j+2 by the group of blocks that closes at step j (blocks j-G+1..j,
         // at the steps j = C-2, C-2-G, ...), so it receives blocks 0..C-2 in groups and
         // block C-1 at step C-1, and every tile is read and written once per group
-        const int G = std::max(1, T.dense_group);
         for (int cc = c0 + TB; cc < w; cc += TB) {
           const int C = cc / TB;
           int first;

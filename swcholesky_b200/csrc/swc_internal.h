@@ -91,6 +91,9 @@ constexpr int TINY_M = 256;
 constexpr int TINY_SLAB = 512;     // >= TINY_M
 static_assert(SMALL_SLAB >= SMALL_MAX_M && TINY_SLAB >= TINY_M, "a slab holds one full column");
 
+// Trailing-update tiles that run at the same time (148 SMs, three CTAs each).
+constexpr int GROUP_FULL_TILES = 444;
+
 // Execution-plan parameters (defaults above; the batched path's autotuner varies them).
 struct Tuning {
   // size-class limits, at most the constants above.  Supernodes above 1,024 rows or 4,096
