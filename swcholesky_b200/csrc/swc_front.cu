@@ -264,7 +264,7 @@ __global__ void __launch_bounds__(T, T == 128 ? 3 : 1) k_front_cta_walk(DevSym S
 }
 
 // The same at warp granularity, for the crowded levels of tiny fronts.
-__global__ void __launch_bounds__(WW * 32) k_front_warp_walk(DevSym S, FrontDev F, const FrontDesc *order,
+__global__ void __launch_bounds__(WW * 32, 3) k_front_warp_walk(DevSym S, FrontDev F, const FrontDesc *order,
                                                              int count, int *qctr, int *qhead) {
   extern __shared__ double fsm[];
   const int lane = threadIdx.x & 31;
