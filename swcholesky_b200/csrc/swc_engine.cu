@@ -1776,10 +1776,12 @@ void Engine::launch_all(std::vector<std::pair<int, cudaEvent_t>> *prof, int prec
         // stream, where they may run on beside the next TRSM: only the diagonal block two
         // steps on (the next iteration's diagonal-block launch) waits for them
         cudaEventRecord(ev_fork_, st);
+        // as in FP64 (below), diagonal block j+1 solves its own rows of column j, from a copy of
+        // that tile made when its updates are complete, and does not wait for the TRSM
         if (W.diag_cnt[j] > 0) {
-          cudaStreamWaitEvent(aux_stream_, ev_fork_, 0);
+          cudaStreamWaitEvent(aux_stream_, j > 0 ? ev_next_ : ev_fork_, 0);
           if (j > 0) cudaStreamWaitEvent(aux_stream_, ev_grp_[(j - 1) & 1], 0);
-          launch_diag_step(sym_, d_diag_ + W.diag_off[j], W.diag_cnt[j], (int)j + 1, aux_stream_);
+          launch_diag_step(sym_, d_diag_ + W.diag_off[j], W.diag_cnt[j], (int)j + 1, aux_stream_, j > 0);
           cudaEventRecord(ev_join_, aux_stream_);
         }
         const int nc = W.scd_nc[j];
@@ -1788,6 +1790,11 @@ void Engine::launch_all(std::vector<std::pair<int, cudaEvent_t>> *prof, int prec
                           scatter_cols(), tuning_.grouped_reserve, bf16, grp_stream_);
         cudaEventRecord(ev_grp_[j & 1], grp_stream_);
         launch_scatter_tc(sym_, sc_maps, d_sc_dense_ + W.scd_off[j], nc, scatter_cols(), 2, bf16, st);
+        if (j + 1 < W.panel_off.size()) {
+          if (j > 0) cudaStreamWaitEvent(st, ev_grp_[(j - 1) & 1], 0);   // column j+1 complete
+          launch_copy_tile(sym_, d_diag_ + W.diag_off[j + 1], W.diag_cnt[j + 1], (int)j + 1, st);
+          cudaEventRecord(ev_next_, st);
+        }
         if (W.diag_cnt[j] > 0) cudaStreamWaitEvent(st, ev_join_, 0);
         if (j + 1 == W.panel_off.size()) cudaStreamWaitEvent(st, ev_grp_[j & 1], 0);
       } else if (!prof && prec == 0) {

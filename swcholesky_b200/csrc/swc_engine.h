@@ -538,6 +538,8 @@ void launch_update_tiles(const DevSym &S, const int4 *tasks, const int *task_end
 // trailing update left in the block's place of dinv (launch_syrk_step), not read from L
 void launch_diag_step(const DevSym &S, const int *list, int count, int step, cudaStream_t st,
                       bool fold = false);
+// the same copy by itself: rows 64 (step + 1) .. of column block `step` of the list's supernodes
+void launch_copy_tile(const DevSym &S, const int *list, int count, int step, cudaStream_t st);
 void launch_trsm_step(const DevSym &S, const int2 *tasks, int count, int step, cudaStream_t st);
 // tasks (s, r0, c0, product index): prod[index].kk names the column blocks applied
 void launch_syrk_step(const DevSym &S, const int4 *tasks, const TcPair *prod, int count,

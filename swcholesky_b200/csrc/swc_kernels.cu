@@ -809,6 +809,24 @@ __global__ void __launch_bounds__(DIAG_NW * 32) k_diag_step(DevSym S, const int 
     factor_diag_block<DIAG_NW, false>(S, list[blockIdx.x], 0, dyn, nullptr);
 }
 
+// Mixed modes: the tile below the next diagonal one to its place in dinv, when the atomic
+// updates of its column are complete (the FP64 update copies it itself, see k_syrk_step).
+__global__ void __launch_bounds__(256) k_copy_tile(DevSym S, const int *list, int step) {
+  const int s = list[blockIdx.x], c0 = step * TB, r0 = c0 + TB;
+  const int m = (int)(S.rowptr[s + 1] - S.rowptr[s]);
+  const double *P = S.L + S.xptr[s] + (size_t)c0 * m + r0;
+  double *dst = S.dinv + ((size_t)S.dinv_off[s] + step + 1) * (TB * TB);
+  constexpr int N = TB * TB / 256;
+  double v[N];
+#pragma unroll
+  for (int q = 0; q < N; ++q) {
+    const int e = threadIdx.x + q * 256, c = e >> 6, r = e & (TB - 1);
+    v[q] = ld_if(P + (size_t)c * m + r, r0 + r < m);
+  }
+#pragma unroll
+  for (int q = 0; q < N; ++q) dst[threadIdx.x + q * 256] = v[q];
+}
+
 // task = (s, r0): B = L[r0:r0+64, blk] := B * L_blk^{-T} = B * T^T with T = L_blk^{-1},
 // stored by the CTA that factored the block (T(r, c) at T[c * 64 + r]), as one DMMA tile
 // product.
@@ -1137,6 +1155,9 @@ void launch_diag_step(const DevSym &S, const int *list, int count, int step, cud
   if (count <= 0) return;
   if (fold) k_diag_step<true><<<count, DIAG_NW * 32, diag_prev_smem(DIAG_NW), st>>>(S, list, count, step);
   else k_diag_step<false><<<count, DIAG_NW * 32, diag_prev_smem(DIAG_NW), st>>>(S, list, count, step);
+}
+void launch_copy_tile(const DevSym &S, const int *list, int count, int step, cudaStream_t st) {
+  if (count > 0) k_copy_tile<<<count, 256, 0, st>>>(S, list, step);
 }
 void launch_trsm_step(const DevSym &S, const int2 *tasks, int count, int step, cudaStream_t st) {
   if (count > 0) k_trsm_step<<<count, MT, 2 * STAGE * 8, st>>>(S, tasks, count, step);
