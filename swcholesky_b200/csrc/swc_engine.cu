@@ -1121,6 +1121,7 @@ void build_solve_plan(int n, const int *Ls, const HostSym &H, SolvePlan &SP) {
   }
   for (int l = 0; l < nl; ++l) {
     SP.level_off.push_back((int)SP.list.size());
+    SP.level_smem.push_back(0);
     SP.warp_off.push_back((int)SP.warp_list.size());
     SP.chain_off.push_back((int)SP.fchain.size());
     SP.contrib_off.push_back((int)SP.contrib_tasks.size());
@@ -1147,7 +1148,7 @@ void build_solve_plan(int n, const int *Ls, const HostSym &H, SolvePlan &SP) {
     for (int s : bylev[l]) {
       const int w = super[s + 1] - super[s];
       const int64_t m = rowptr[s + 1] - rowptr[s];
-      if (w > SOLVE_NARROW_W && (H.dinv_off[s] >= 0 || !(warp_level[l] && warp_size_ok(s))))
+      if (w > SOLVE_NARROW_W && H.dinv_off[s] >= 0)
         n128 += (m - w + SOLVE_CONTRIB_WIDE_ROWS - 1) / SOLVE_CONTRIB_WIDE_ROWS;
     }
     const bool wide_level = n128 >= SOLVE_CONTRIB_WIDE_MIN;
@@ -1161,8 +1162,10 @@ void build_solve_plan(int n, const int *Ls, const HostSym &H, SolvePlan &SP) {
       } else if (warp_level[l] && warp_size_ok(s)) {
         SP.warp_list.push_back(s);   // its contributions and gathers are done by the warp
         continue;
-      } else {
+      } else {   // its contributions and gathers are done by its CTA
         SP.list.push_back(s);
+        SP.level_smem[l] = std::max(SP.level_smem[l], 8 * (m * w + m));
+        continue;
       }
       if (w > SOLVE_CONTRIB_BIG_W || (w > SOLVE_NARROW_W && !wide_level))
         for (int r0 = w; r0 < m; r0 += SOLVE_CONTRIB_ROWS) SP.contrib_tasks.push_back(make_int2(s, r0));
@@ -1203,12 +1206,12 @@ void build_solve_plan(int n, const int *Ls, const HostSym &H, SolvePlan &SP) {
   }
 }
 
-// The streaming tasks of a solve plan whose supernodes sit in `level` (by_warp: solved by
-// one warp, which does its own contributions and gathers): forward contribution tasks cover
+// The streaming tasks of a solve plan whose supernodes sit in `level` (alone: solved by one
+// warp or CTA, which does its own contributions and gathers): forward contribution tasks cover
 // each off-diagonal row once, backward gather tasks each 16-column group once, and the
 // per-column contribution lists name each contribution once, under the row it belongs to.
 static bool check_solve_tasks(int n, const int *Ls, const HostSym &H, const SolvePlan &SP,
-                              const std::vector<int> &level, const std::vector<char> &by_warp,
+                              const std::vector<int> &level, const std::vector<char> &alone,
                               std::string &err) {
   const int supNo = (int)H.super.size() - 1;
   const std::vector<int> &super = H.super;
@@ -1227,8 +1230,8 @@ static bool check_solve_tasks(int n, const int *Ls, const HostSym &H, const Solv
     if (nbig < 0 || nwide < 0 || nbig + nwide > t1 - t0) return bad("contribution classes");
     for (int k = t0; k < t1; ++k) {
       const int s = SP.contrib_tasks[k].x, r0 = SP.contrib_tasks[k].y;
-      if (s < 0 || s >= supNo || level[s] != l || by_warp[s])
-        return bad("contribution task of a supernode not solved by a CTA in its level");
+      if (s < 0 || s >= supNo || level[s] != l || alone[s])
+        return bad("contribution task of a supernode not chained in its level");
       const int w = super[s + 1] - super[s];
       const int m = (int)(rowptr[s + 1] - rowptr[s]);
       const int span = (k - t0 >= nbig && k - t0 < nbig + nwide) ? SOLVE_CONTRIB_WIDE_ROWS
@@ -1242,8 +1245,8 @@ static bool check_solve_tasks(int n, const int *Ls, const HostSym &H, const Solv
     }
     for (int k = SP.gather_off[l]; k < SP.gather_off[l + 1]; ++k) {
       const int s = SP.gather_tasks[k].x, j0 = SP.gather_tasks[k].y;
-      if (s < 0 || s >= supNo || level[s] != l || by_warp[s])
-        return bad("gather task of a supernode not solved by a CTA in its level");
+      if (s < 0 || s >= supNo || level[s] != l || alone[s])
+        return bad("gather task of a supernode not chained in its level");
       const int w = super[s + 1] - super[s];
       if (rowptr[s + 1] - rowptr[s] == w || j0 < 0 || j0 >= w || j0 % SOLVE_GATHER_COLS != 0)
         return bad("gather columns misaligned");
@@ -1259,9 +1262,9 @@ static bool check_solve_tasks(int n, const int *Ls, const HostSym &H, const Solv
     for (int a = w; a < m; ++a) {
       const int64_t idx = (rowptr[s] - super[s]) + (a - w);
       row_of[idx] = Ls[rowptr[s] + a];
-      if (!by_warp[s] && !row_done[idx]) return bad("an off-diagonal row in no contribution task");
+      if (!alone[s] && !row_done[idx]) return bad("an off-diagonal row in no contribution task");
     }
-    if (by_warp[s] || m == w) continue;
+    if (alone[s] || m == w) continue;
     for (int j0 = 0; j0 < w; j0 += SOLVE_GATHER_COLS)
       if (!col_done[super[s] + j0]) return bad("a column group in no gather task");
   }
@@ -1299,7 +1302,7 @@ bool check_solve_plan(int n, const int *Ls, const HostSym &H, const SolvePlan &S
   if (SP.contrib_len != H.nls - n) return bad("contribution length");
   // every supernode in exactly one level, by exactly one kind of task
   std::vector<int> level(supNo, -1);
-  std::vector<char> by_warp(supNo, 0);
+  std::vector<char> alone(supNo, 0);
   auto place = [&](int s, int l) {
     if (s < 0 || s >= supNo) return false;
     if (level[s] >= 0 && level[s] != l) return false;
@@ -1310,6 +1313,11 @@ bool check_solve_plan(int n, const int *Ls, const HostSym &H, const SolvePlan &S
     for (int k = SP.level_off[l]; k < SP.level_off[l + 1]; ++k) {
       const int s = SP.list[k];
       if (!place(s, l) || H.dinv_off[s] >= 0) return bad("small supernode misplaced");
+      const int w = super[s + 1] - super[s];
+      if (w > SMALL_MAX_W || 8 * (rowptr[s + 1] - rowptr[s]) * (w + 1) > SP.level_smem[l] ||
+          SP.level_smem[l] > SOLVE_SMALL_SMEM)
+        return bad("supernode larger than its launch's shared memory");
+      alone[s] = 1;
     }
     for (int k = SP.warp_off[l]; k < SP.warp_off[l + 1]; ++k) {
       const int s = SP.warp_list[k];
@@ -1317,7 +1325,7 @@ bool check_solve_plan(int n, const int *Ls, const HostSym &H, const SolvePlan &S
       const int w = super[s + 1] - super[s];
       if (w > SOLVE_WARP_W || rowptr[s + 1] - rowptr[s] - w > SOLVE_WARP_ROWS)
         return bad("supernode too large for one warp");
-      by_warp[s] = 1;
+      alone[s] = 1;
     }
     // chained blocks: one per 64 columns, forward increasing, backward decreasing
     const int c0 = SP.chain_off[l], c1 = SP.chain_off[l + 1];
@@ -1368,7 +1376,7 @@ bool check_solve_plan(int n, const int *Ls, const HostSym &H, const SolvePlan &S
     }
     if (c != SP.c8_off[l + 1] || g != SP.g8_off[l + 1]) return bad("tasks of eight right-hand sides left over");
   }
-  return check_solve_tasks(n, Ls, H, SP, level, by_warp, err);
+  return check_solve_tasks(n, Ls, H, SP, level, alone, err);
 }
 
 bool Engine::analyze(int n, const int *c, const int *r, const int64_t *lC, const int *Ls,
@@ -2139,15 +2147,14 @@ void Engine::run_solve_with(double *x, int nrhs, double *contrib) {
   cudaStream_t st = stream_;
   const SolvePlan &SP = splan_;
   const int nl = (int)SP.level_off.size() - 1;
-  const int smem = (int)sizeof(double) * std::max(SP.max_w, 1);
   const int64_t cs = std::max<int64_t>(SP.contrib_len, 1);
   const int base = 0;
   cudaMemsetAsync(d_flags_, 0, sizeof(int) * std::max<int64_t>(nflags_, 1), st);
   for (int l = 0; l < nl; ++l) {
     launch_fwd_warp(sym_, d_swarp_ + SP.warp_off[l], SP.warp_off[l + 1] - SP.warp_off[l], x,
                     contrib, d_cptr_, d_cidx_, n_, nrhs, cs, st);
-    launch_fwd_diag(sym_, d_slist_ + SP.level_off[l], SP.level_off[l + 1] - SP.level_off[l], smem,
-                    x, contrib, d_cptr_, d_cidx_, n_, nrhs, cs, st);
+    launch_fwd_small(sym_, d_slist_ + SP.level_off[l], SP.level_off[l + 1] - SP.level_off[l],
+                     SP.level_smem[l], x, contrib, d_cptr_, d_cidx_, n_, nrhs, cs, st);
     for (int r = 0; r < nrhs; ++r)
       launch_fwd_chain(sym_, d_fchain_ + SP.chain_off[l], SP.chain_off[l + 1] - SP.chain_off[l],
                        x + (size_t)r * n_, contrib + (size_t)r * cs, d_cptr_, d_cidx_, d_flags_,
@@ -2158,8 +2165,8 @@ void Engine::run_solve_with(double *x, int nrhs, double *contrib) {
   for (int l = nl - 1; l >= 0; --l) {
     launch_bwd_gather(sym_, d_sgather_ + SP.gather_off[l], SP.gather_off[l + 1] - SP.gather_off[l],
                       x, n_, nrhs, st);
-    launch_bwd_diag(sym_, d_slist_ + SP.level_off[l], SP.level_off[l + 1] - SP.level_off[l], smem,
-                    x, n_, nrhs, st);
+    launch_bwd_small(sym_, d_slist_ + SP.level_off[l], SP.level_off[l + 1] - SP.level_off[l],
+                     SP.level_smem[l], x, n_, nrhs, st);
     launch_bwd_warp(sym_, d_swarp_ + SP.warp_off[l], SP.warp_off[l + 1] - SP.warp_off[l], x, n_,
                     nrhs, st);
     for (int r = 0; r < nrhs; ++r)

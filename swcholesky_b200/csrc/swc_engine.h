@@ -200,15 +200,15 @@ struct Plan {
 
 // Triangular solves and refinement (swc_solve.cu)
 bool solve_configure(int max_w, std::string &err);
-void launch_fwd_diag(const DevSym &S, const int *list, int count, int smem, double *y,
-                     const double *contrib, const int *cptr, const int *cidx, int n, int nrhs,
+void launch_fwd_small(const DevSym &S, const int *list, int count, int smem, double *y,
+                      double *contrib, const int *cptr, const int *cidx, int n, int nrhs,
                      int64_t cstride, cudaStream_t st);
 void launch_fwd_contrib(const DevSym &S, const int2 *tasks, int count, int nbig, int nwide,
                         const double *y, double *contrib, int n, int nrhs, int64_t cstride,
                         cudaStream_t st);
 void launch_bwd_gather(const DevSym &S, const int2 *tasks, int count, double *x, int n, int nrhs,
                        cudaStream_t st);
-void launch_bwd_diag(const DevSym &S, const int *list, int count, int smem, double *x, int n,
+void launch_bwd_small(const DevSym &S, const int *list, int count, int smem, double *x, int n,
                      int nrhs, cudaStream_t st);
 // small supernodes, one warp each: forward (contributions in, diagonal solve, contributions
 // of the rows below out) and backward (gather from ancestors, transposed diagonal solve)
@@ -235,8 +235,9 @@ void launch_rowabs(int n, const int *rp, const double *val, double *out, cudaStr
 
 // Per-level task lists of the solves.
 struct SolvePlan {
-  std::vector<int> level_off;       // small-class supernodes of level l:
+  std::vector<int> level_off;       // small-class supernodes of level l, one CTA each:
   std::vector<int> list;            //   list[level_off[l] .. level_off[l+1])
+  std::vector<int> level_smem;      //   shared memory of the level's launches
   std::vector<int> warp_off;        // small supernodes solved by one warp each (level l):
   std::vector<int> warp_list;       //   warp_list[warp_off[l] .. warp_off[l+1])
   std::vector<int> chain_off;       // (s, block) tasks of the tiled class in level l:

@@ -91,6 +91,9 @@ constexpr int TINY_M = 256;
 constexpr int TINY_SLAB = 512;     // >= TINY_M
 static_assert(SMALL_SLAB >= SMALL_MAX_M && TINY_SLAB >= TINY_M, "a slab holds one full column");
 
+// Shared memory of the solves' small supernodes at most (panel, right-hand side, rows below).
+constexpr int SOLVE_SMALL_SMEM = 8 * (SMALL_MAX_ELEMS + SMALL_MAX_M);
+
 // Trailing-update tiles that run at the same time (148 SMs, three CTAs each).
 constexpr int GROUP_FULL_TILES = 444;
 

@@ -15,68 +15,95 @@ namespace swc {
 namespace {
 
 constexpr int ST = 256;   // threads of the solve kernels
-constexpr int SB = 32;    // column block of the dense triangular solves (one warp)
 
-// Forward solve, level by level (leaves first), in two kernels per level:
-//   k_fwd_diag    y[cols of s] := L_ss^{-1} (y[cols of s] - sum of the contributions the
-//                 descendants stored for those columns), one CTA per supernode; column j's
+// Forward solve, level by level (leaves first):
+//   k_fwd_small   small supernodes, one CTA each: y[cols of s] := L_ss^{-1} (y[cols of s] - sum
+//                 of the contributions the descendants stored for those columns), then the
+//                 contributions of its rows below, c_s = L_rs y[cols of s].  Column j's
 //                 contributions are listed in cidx[cptr[j] .. cptr[j+1]) (one entry per
-//                 off-diagonal row of L equal to j, in increasing supernode order), so
-//                 every column sums its own list with no barrier.
-//   k_fwd_contrib c_s = L_s[rows below the diagonal block, :] y[cols of s], one CTA per
-//                 32-row slab: the off-diagonal GEMV of every supernode runs in parallel.
+//                 off-diagonal row of L equal to j, in increasing supernode order).
+//   k_fwd_chain, k_fwd_contrib   tiled supernodes: the chained diagonal blocks, then one CTA
+//                 per slab of rows.
 // c_s lives at contrib + rowptr[s] - super[s] (one entry per off-diagonal row).
-__global__ void __launch_bounds__(ST) k_fwd_diag(DevSym S, const int *list, double *y,
-                                                 const double *contrib, const int *cptr,
-                                                 const int *cidx, int n, int nrhs,
-                                                 int64_t cstride) {
-  extern __shared__ double v[];
-  __shared__ double blk[SB * (SB + 1)];
+// The small kernels are bound by latency: the whole panel is loaded into shared memory while the
+// contributions (or the rows below) are gathered, so nothing after that waits for L, and one
+// launch per level does what the diagonal solve and the contributions (backward: the gather and
+// the solve) did in two: a solve of the 60^3 7-point grid 1413 -> 1301 us (B200).
+__device__ __forceinline__ void stage_panel(double *P, const double *Ls, int count) {
+  int e = threadIdx.x;
+  for (; e + 7 * ST < count; e += 8 * ST) {
+    double t[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) t[u] = Ls[e + u * ST];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) P[e + u * ST] = t[u];
+  }
+  for (; e < count; e += ST) P[e] = Ls[e];
+}
+
+// shared memory: the panel (column-major, ld m), then the right-hand side (w) and, backward, the
+// gathered rows below (m - w)
+static_assert(SMALL_MAX_W == 64, "two rows per lane of the solving warp");
+__global__ void __launch_bounds__(ST) k_fwd_small(DevSym S, const int *list, double *y, double *contrib,
+                                                  const int *cptr, const int *cidx, int n, int nrhs,
+                                                  int64_t cstride) {
+  extern __shared__ double P[];
   const int s = list[blockIdx.x];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int f = S.super[s], w = S.super[s + 1] - f;
-  const int m = (int)(S.rowptr[s + 1] - S.rowptr[s]);
-  const double *Ls_s = S.L + S.xptr[s];
+  const int64_t rb = S.rowptr[s];
+  const int m = (int)(S.rowptr[s + 1] - rb);
+  double *v = P + m * w;
+  stage_panel(P, S.L + S.xptr[s], m * w);
   for (int rhs = 0; rhs < nrhs; ++rhs) {
-    double *yr = y + (size_t)rhs * n;
-    const double *cr = contrib + (size_t)rhs * cstride;
-    __syncthreads();
-    // column j of s receives the contributions listed for it (descendant order)
-    for (int i = tid; i < w; i += ST) {
-      double acc = yr[f + i];
-      for (int q = cptr[f + i]; q < cptr[f + i + 1]; ++q) acc -= cr[cidx[q]];
-      v[i] = acc;
+    double *yr = y + (size_t)rhs * n + f;
+    double *cr = contrib + (size_t)rhs * cstride;
+    // column i of s receives the contributions listed for it (descendant order)
+    if (tid < w) {
+      double acc = yr[tid];
+      int q = cptr[f + tid];
+      const int q1 = cptr[f + tid + 1];
+      for (; q + 3 < q1; q += 4) {
+        const double a = cr[cidx[q]], b = cr[cidx[q + 1]], c = cr[cidx[q + 2]], d = cr[cidx[q + 3]];
+        acc -= (a + b) + (c + d);
+      }
+      for (; q < q1; ++q) acc -= cr[cidx[q]];
+      v[tid] = acc;
     }
     __syncthreads();
-    // dense lower solve with the diagonal block, blocked by SB columns; each SB x SB block
-    // and the reciprocals of its diagonal are staged first, so the serial chain of warp 0
-    // reads only shared memory
-    for (int j0 = 0; j0 < w; j0 += SB) {
-      const int jb = min(SB, w - j0);
-      for (int e = tid; e < jb * jb; e += ST) {
-        const int j = e / jb, i = e - j * jb;
-        blk[j * (SB + 1) + i] = Ls_s[(size_t)(j0 + j) * m + j0 + i];
+    if (warp == 0) {   // rows lane and lane + 32
+      const int i0 = lane, i1 = lane + 32;
+      double x0 = i0 < w ? v[i0] : 0.0, x1 = i1 < w ? v[i1] : 0.0;
+      const double d0 = i0 < w ? 1.0 / P[i0 * m + i0] : 0.0, d1 = i1 < w ? 1.0 / P[i1 * m + i1] : 0.0;
+      const int wa = min(w, 32);
+      for (int j = 0; j < wa; ++j) {
+        if (lane == j) x0 *= d0;
+        const double xj = __shfl_sync(0xffffffffu, x0, j);
+        if (i0 > j && i0 < w) x0 = fma(-P[j * m + i0], xj, x0);
+        if (i1 < w) x1 = fma(-P[j * m + i1], xj, x1);
       }
-      __syncthreads();
-      if (warp == 0) {
-        const double rdl = (lane < jb) ? 1.0 / blk[lane * (SB + 1) + lane] : 0.0;
-        double x = (lane < jb) ? v[j0 + lane] : 0.0;
-        for (int j = 0; j < jb; ++j) {
-          if (lane == j) x *= rdl;
-          const double xj = __shfl_sync(0xffffffffu, x, j);
-          if (lane > j && lane < jb) x = fma(-blk[j * (SB + 1) + lane], xj, x);
-        }
-        if (lane < jb) v[j0 + lane] = x;
+      for (int j = 32; j < w; ++j) {
+        if (i1 == j) x1 *= d1;
+        const double xj = __shfl_sync(0xffffffffu, x1, j - 32);
+        if (i1 > j && i1 < w) x1 = fma(-P[j * m + i1], xj, x1);
       }
-      __syncthreads();
-      for (int i = j0 + jb + tid; i < w; i += ST) {
-        double acc = v[i];
-        for (int j = 0; j < jb; ++j) acc = fma(-Ls_s[(size_t)(j0 + j) * m + i], v[j0 + j], acc);
-        v[i] = acc;
-      }
-      __syncthreads();
+      if (i0 < w) yr[i0] = v[i0] = x0;
+      if (i1 < w) yr[i1] = v[i1] = x1;
     }
-    for (int i = tid; i < w; i += ST) yr[f + i] = v[i];
+    __syncthreads();
+    for (int a = w + tid; a < m; a += ST) {
+      double a0 = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0;
+      int k = 0;
+      for (; k + 3 < w; k += 4) {
+        a0 = fma(P[k * m + a], v[k], a0);
+        a1 = fma(P[(k + 1) * m + a], v[k + 1], a1);
+        a2 = fma(P[(k + 2) * m + a], v[k + 2], a2);
+        a3 = fma(P[(k + 3) * m + a], v[k + 3], a3);
+      }
+      for (; k < w; ++k) a0 = fma(P[k * m + a], v[k], a0);
+      cr[(rb - f) + (a - w)] = (a0 + a1) + (a2 + a3);
+    }
+    __syncthreads();
   }
 }
 
@@ -219,10 +246,11 @@ __global__ void __launch_bounds__(CT) k_fwd_contrib(DevSym S, const int2 *tasks,
 }
 
 // Backward solve, level by level (root first):
-//   k_bwd_gather  x[f + j] := x[f + j] - sum_{a >= w} L(a, j) x[rows[a]] for the columns
-//                 j0..j0+15 of s (one warp per column, eight loads in flight per lane);
-//                 the rows below are columns of ancestors, already solved.
-//   k_bwd_diag    x[cols of s] := L_ss^{-T} x[cols of s], one CTA per supernode.
+//   k_bwd_gather  tiled supernodes: x[f + j] := x[f + j] - sum_{a >= w} L(a, j) x[rows[a]] for
+//                 the columns j0..j0+15 of s (one warp per column, eight loads in flight per
+//                 lane); the rows below are columns of ancestors, already solved.  Then
+//                 k_bwd_chain.
+//   k_bwd_small   small supernodes, one CTA each: the gather and L_ss^{-T}.
 constexpr int GCH = 2048;       // gathered rows staged per chunk
 constexpr int GT = 32 * SOLVE_GATHER_COLS;   // one warp per column of the task
 __global__ void __launch_bounds__(GT) k_bwd_gather(DevSym S, const int2 *tasks, double *x,
@@ -358,48 +386,54 @@ __global__ void __launch_bounds__(ST) k_bwd_warp(DevSym S, const int *list, int 
   }
 }
 
-__global__ void __launch_bounds__(ST) k_bwd_diag(DevSym S, const int *list, double *x, int n,
-                                                 int nrhs) {
-  extern __shared__ double v[];
-  __shared__ double blk[SB * (SB + 1)];
+__global__ void __launch_bounds__(ST) k_bwd_small(DevSym S, const int *list, double *x, int n, int nrhs) {
+  extern __shared__ double P[];
   const int s = list[blockIdx.x];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int f = S.super[s], w = S.super[s + 1] - f;
-  const int m = (int)(S.rowptr[s + 1] - S.rowptr[s]);
-  const double *Ls_s = S.L + S.xptr[s];
+  const int64_t rb = S.rowptr[s];
+  const int m = (int)(S.rowptr[s + 1] - rb);
+  const int *rows = S.Ls + rb;
+  double *v = P + m * w, *xg = v + w;
+  stage_panel(P, S.L + S.xptr[s], m * w);
   for (int rhs = 0; rhs < nrhs; ++rhs) {
     double *xr = x + (size_t)rhs * n;
+    for (int a = w + tid; a < m; a += ST) xg[a - w] = xr[rows[a]];
     __syncthreads();
-    for (int i = tid; i < w; i += ST) v[i] = xr[f + i];
-    __syncthreads();
-    for (int j1 = w; j1 > 0; j1 -= SB) {
-      const int j0 = max(0, j1 - SB), jb = j1 - j0;
-      // v[j0..j1) -= sum_{i >= j1} L(i, j) v[i]
-      for (int j = j0 + warp; j < j1; j += ST / 32) {
-        double acc = 0.0;
-        for (int i = j1 + lane; i < w; i += 32) acc = fma(Ls_s[(size_t)j * m + i], v[i], acc);
+    for (int j = warp; j < w; j += ST / 32) {   // a warp per column
+      const double *col = P + j * m + w;
+      double a0 = 0.0, a1 = 0.0;
+      int i = lane;
+      for (; i + 32 < m - w; i += 64) {
+        a0 = fma(col[i], xg[i], a0);
+        a1 = fma(col[i + 32], xg[i + 32], a1);
+      }
+      if (i < m - w) a0 = fma(col[i], xg[i], a0);
+      a0 += a1;
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-        if (lane == 0) v[j] -= acc;
-      }
-      for (int e = tid; e < jb * jb; e += ST) {
-        const int j = e / jb, i = e - j * jb;
-        blk[j * (SB + 1) + i] = Ls_s[(size_t)(j0 + j) * m + j0 + i];
-      }
-      __syncthreads();
-      if (warp == 0) {
-        const double rdl = (lane < jb) ? 1.0 / blk[lane * (SB + 1) + lane] : 0.0;
-        double xv = (lane < jb) ? v[j0 + lane] : 0.0;
-        for (int jj = jb - 1; jj >= 0; --jj) {
-          if (lane == jj) xv *= rdl;
-          const double xj = __shfl_sync(0xffffffffu, xv, jj);
-          if (lane < jj) xv = fma(-blk[lane * (SB + 1) + jj], xj, xv);
-        }
-        if (lane < jb) v[j0 + lane] = xv;
-      }
-      __syncthreads();
+      for (int o = 16; o > 0; o >>= 1) a0 += __shfl_xor_sync(0xffffffffu, a0, o);
+      if (lane == 0) v[j] = xr[f + j] - a0;
     }
-    for (int i = tid; i < w; i += ST) xr[f + i] = v[i];
+    __syncthreads();
+    if (warp == 0) {
+      const int i0 = lane, i1 = lane + 32;
+      double x0 = i0 < w ? v[i0] : 0.0, x1 = i1 < w ? v[i1] : 0.0;
+      const double d0 = i0 < w ? 1.0 / P[i0 * m + i0] : 0.0, d1 = i1 < w ? 1.0 / P[i1 * m + i1] : 0.0;
+      for (int j = w - 1; j >= 32; --j) {
+        if (i1 == j) x1 *= d1;
+        const double xj = __shfl_sync(0xffffffffu, x1, j - 32);
+        if (i1 < j) x1 = fma(-P[i1 * m + j], xj, x1);
+        x0 = fma(-P[i0 * m + j], xj, x0);
+      }
+      for (int j = min(w, 32) - 1; j >= 0; --j) {
+        if (i0 == j) x0 *= d0;
+        const double xj = __shfl_sync(0xffffffffu, x0, j);
+        if (i0 < j) x0 = fma(-P[i0 * m + j], xj, x0);
+      }
+      if (i0 < w) xr[f + i0] = x0;
+      if (i1 < w) xr[f + i1] = x1;
+    }
+    __syncthreads();
   }
 }
 
@@ -870,7 +904,7 @@ bool solve_configure(int max_w, std::string &err) {
     err = "supernode too wide for the shared-memory triangular solve";
     return false;
   }
-  cudaError_t e = cudaFuncSetAttribute(k_fwd_diag, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = cudaFuncSetAttribute(k_fwd_small, cudaFuncAttributeMaxDynamicSharedMemorySize, SOLVE_SMALL_SMEM);
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(k_fwd_chain<CHAIN_NS_BIG>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              chain_smem(CHAIN_NS_BIG, CHAIN_XW_FWD));
@@ -889,7 +923,7 @@ bool solve_configure(int max_w, std::string &err) {
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&g_num_sms, cudaDevAttrMultiProcessorCount, dev);
   }
   if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_bwd_diag, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    e = cudaFuncSetAttribute(k_bwd_small, cudaFuncAttributeMaxDynamicSharedMemorySize, SOLVE_SMALL_SMEM);
   if (e != cudaSuccess) {
     err = std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(e);
     return false;
@@ -897,11 +931,11 @@ bool solve_configure(int max_w, std::string &err) {
   return true;
 }
 
-void launch_fwd_diag(const DevSym &S, const int *list, int count, int smem, double *y,
-                     const double *contrib, const int *cptr, const int *cidx, int n, int nrhs,
+void launch_fwd_small(const DevSym &S, const int *list, int count, int smem, double *y,
+                      double *contrib, const int *cptr, const int *cidx, int n, int nrhs,
                      int64_t cstride, cudaStream_t st) {
   if (count > 0)
-    k_fwd_diag<<<count, ST, smem, st>>>(S, list, y, contrib, cptr, cidx, n, nrhs, cstride);
+    k_fwd_small<<<count, ST, smem, st>>>(S, list, y, contrib, cptr, cidx, n, nrhs, cstride);
 }
 void launch_fwd_contrib(const DevSym &S, const int2 *tasks, int count, int nbig, int nwide,
                         const double *y, double *contrib, int n, int nrhs, int64_t cstride,
@@ -928,9 +962,9 @@ void launch_bwd_gather(const DevSym &S, const int2 *tasks, int count, double *x,
                        cudaStream_t st) {
   if (count > 0) k_bwd_gather<<<count, GT, 0, st>>>(S, tasks, x, n, nrhs);
 }
-void launch_bwd_diag(const DevSym &S, const int *list, int count, int smem, double *x, int n,
+void launch_bwd_small(const DevSym &S, const int *list, int count, int smem, double *x, int n,
                      int nrhs, cudaStream_t st) {
-  if (count > 0) k_bwd_diag<<<count, ST, smem, st>>>(S, list, x, n, nrhs);
+  if (count > 0) k_bwd_small<<<count, ST, smem, st>>>(S, list, x, n, nrhs);
 }
 // the chains' launch configuration: a grid of whole clusters of CHAIN_CL CTAs
 static cudaLaunchConfig_t chain_config(int count, int smem, cudaStream_t st,
