@@ -1141,16 +1141,13 @@ void build_solve_plan(int n, const int *Ls, const HostSym &H, SolvePlan &SP) {
         for (int j0 = 0; j0 < w && m > w; j0 += SOLVE_GATHER_COLS) SP.g8_tasks.push_back(make_int2(s, j0));
       }
     }
-    std::vector<int2> narrow, wide;
-    // 128-row tasks of 8 warps for the wide supernodes only when the level has enough of
-    // them to fill the GPU; otherwise 32-row tasks of 32 warps (more, shorter CTAs)
+    std::vector<int2> wide;
+    // 128-row tasks only when the level has enough of them to fill the GPU
     int64_t n128 = 0;
-    for (int s : bylev[l]) {
-      const int w = super[s + 1] - super[s];
-      const int64_t m = rowptr[s + 1] - rowptr[s];
-      if (w > SOLVE_NARROW_W && H.dinv_off[s] >= 0)
-        n128 += (m - w + SOLVE_CONTRIB_WIDE_ROWS - 1) / SOLVE_CONTRIB_WIDE_ROWS;
-    }
+    for (int s : bylev[l])
+      if (H.dinv_off[s] >= 0)
+        n128 += (rowptr[s + 1] - rowptr[s] - (super[s + 1] - super[s]) + SOLVE_CONTRIB_WIDE_ROWS - 1) /
+                SOLVE_CONTRIB_WIDE_ROWS;
     const bool wide_level = n128 >= SOLVE_CONTRIB_WIDE_MIN;
     for (int s : bylev[l]) {
       const int w = super[s + 1] - super[s];
@@ -1167,19 +1164,15 @@ void build_solve_plan(int n, const int *Ls, const HostSym &H, SolvePlan &SP) {
         SP.level_smem[l] = std::max(SP.level_smem[l], 8 * (m * w + m));
         continue;
       }
-      if (w > SOLVE_CONTRIB_BIG_W || (w > SOLVE_NARROW_W && !wide_level))
+      if (!wide_level)
         for (int r0 = w; r0 < m; r0 += SOLVE_CONTRIB_ROWS) SP.contrib_tasks.push_back(make_int2(s, r0));
-      else if (w > SOLVE_NARROW_W)
-        for (int r0 = w; r0 < m; r0 += SOLVE_CONTRIB_WIDE_ROWS) wide.push_back(make_int2(s, r0));
       else
-        for (int r0 = w; r0 < m; r0 += SOLVE_CONTRIB_ROWS) narrow.push_back(make_int2(s, r0));
+        for (int r0 = w; r0 < m; r0 += SOLVE_CONTRIB_WIDE_ROWS) wide.push_back(make_int2(s, r0));
       if (m > w)
         for (int j0 = 0; j0 < w; j0 += SOLVE_GATHER_COLS) SP.gather_tasks.push_back(make_int2(s, j0));
     }
     SP.contrib_big.push_back((int)SP.contrib_tasks.size() - SP.contrib_off.back());
-    SP.contrib_wide.push_back((int)wide.size());
     SP.contrib_tasks.insert(SP.contrib_tasks.end(), wide.begin(), wide.end());
-    SP.contrib_tasks.insert(SP.contrib_tasks.end(), narrow.begin(), narrow.end());
   }
   SP.level_off.push_back((int)SP.list.size());
   SP.warp_off.push_back((int)SP.warp_list.size());
@@ -1226,16 +1219,15 @@ static bool check_solve_tasks(int n, const int *Ls, const HostSym &H, const Solv
   std::vector<char> col_done(n, 0);
   for (int l = 0; l < nl; ++l) {
     const int t0 = SP.contrib_off[l], t1 = SP.contrib_off[l + 1];
-    const int nbig = SP.contrib_big[l], nwide = SP.contrib_wide[l];
-    if (nbig < 0 || nwide < 0 || nbig + nwide > t1 - t0) return bad("contribution classes");
+    const int nbig = SP.contrib_big[l];
+    if (nbig < 0 || nbig > t1 - t0) return bad("contribution classes");
     for (int k = t0; k < t1; ++k) {
       const int s = SP.contrib_tasks[k].x, r0 = SP.contrib_tasks[k].y;
       if (s < 0 || s >= supNo || level[s] != l || alone[s])
         return bad("contribution task of a supernode not chained in its level");
       const int w = super[s + 1] - super[s];
       const int m = (int)(rowptr[s + 1] - rowptr[s]);
-      const int span = (k - t0 >= nbig && k - t0 < nbig + nwide) ? SOLVE_CONTRIB_WIDE_ROWS
-                                                                 : SOLVE_CONTRIB_ROWS;
+      const int span = k - t0 < nbig ? SOLVE_CONTRIB_ROWS : SOLVE_CONTRIB_WIDE_ROWS;
       if (r0 < w || r0 >= m || (r0 - w) % span != 0) return bad("contribution rows misaligned");
       for (int a = r0; a < std::min(m, r0 + span); ++a) {
         const int64_t idx = (rowptr[s] - super[s]) + (a - w);
@@ -1296,7 +1288,7 @@ bool check_solve_plan(int n, const int *Ls, const HostSym &H, const SolvePlan &S
   };
   if (nl < 0 || (int)SP.warp_off.size() != nl + 1 || (int)SP.chain_off.size() != nl + 1 ||
       (int)SP.contrib_off.size() != nl + 1 || (int)SP.gather_off.size() != nl + 1 ||
-      (int)SP.contrib_big.size() != nl || (int)SP.contrib_wide.size() != nl ||
+      (int)SP.contrib_big.size() != nl ||
       SP.fchain.size() != SP.bchain.size())
     return bad("per-level offsets of unequal length");
   if (SP.contrib_len != H.nls - n) return bad("contribution length");
@@ -2160,7 +2152,7 @@ void Engine::run_solve_with(double *x, int nrhs, double *contrib) {
                        x + (size_t)r * n_, contrib + (size_t)r * cs, d_cptr_, d_cidx_, d_flags_,
                        base + r + 1, n_, cs, st);
     launch_fwd_contrib(sym_, d_scontrib_ + SP.contrib_off[l], SP.contrib_off[l + 1] - SP.contrib_off[l],
-                       SP.contrib_big[l], SP.contrib_wide[l], x, contrib, n_, nrhs, cs, st);
+                       SP.contrib_big[l], x, contrib, n_, nrhs, cs, st);
   }
   for (int l = nl - 1; l >= 0; --l) {
     launch_bwd_gather(sym_, d_sgather_ + SP.gather_off[l], SP.gather_off[l + 1] - SP.gather_off[l],

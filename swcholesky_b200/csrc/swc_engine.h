@@ -203,9 +203,8 @@ bool solve_configure(int max_w, std::string &err);
 void launch_fwd_small(const DevSym &S, const int *list, int count, int smem, double *y,
                       double *contrib, const int *cptr, const int *cidx, int n, int nrhs,
                      int64_t cstride, cudaStream_t st);
-void launch_fwd_contrib(const DevSym &S, const int2 *tasks, int count, int nbig, int nwide,
-                        const double *y, double *contrib, int n, int nrhs, int64_t cstride,
-                        cudaStream_t st);
+void launch_fwd_contrib(const DevSym &S, const int2 *tasks, int count, int nbig, const double *y,
+                        double *contrib, int n, int nrhs, int64_t cstride, cudaStream_t st);
 void launch_bwd_gather(const DevSym &S, const int2 *tasks, int count, double *x, int n, int nrhs,
                        cudaStream_t st);
 void launch_bwd_small(const DevSym &S, const int *list, int count, int smem, double *x, int n,
@@ -242,9 +241,8 @@ struct SolvePlan {
   std::vector<int> warp_list;       //   warp_list[warp_off[l] .. warp_off[l+1])
   std::vector<int> chain_off;       // (s, block) tasks of the tiled class in level l:
   std::vector<int2> fchain, bchain; //   forward (increasing block) / backward (decreasing)
-  std::vector<int> contrib_off;     // (s, r0) tasks of level l: contrib_big[l] tasks of very
-  std::vector<int> contrib_big;     //   wide supernodes, contrib_wide[l] of wide ones (a CTA
-  std::vector<int> contrib_wide;    //   each), then narrow ones (a warp)
+  std::vector<int> contrib_off;     // (s, r0) tasks of level l: contrib_big[l] of 32 rows, then
+  std::vector<int> contrib_big;     //   those of 128
   std::vector<int2> contrib_tasks;
   std::vector<int> gather_off;      // (s, j0) tasks of level l
   std::vector<int2> gather_tasks;

@@ -58,11 +58,9 @@ constexpr int TB = 64;
 // Task shapes of the solve's streaming kernels: rows of an off-diagonal block per forward
 // contribution task, columns per backward gather task.
 constexpr int SOLVE_CONTRIB_ROWS = 32;
-constexpr int SOLVE_CONTRIB_WIDE_ROWS = 128;   // rows of a wide supernode's contribution task
-constexpr int SOLVE_CONTRIB_BIG_W = 512;       // wider: 32-row tasks of 32 warps each
-constexpr int SOLVE_CONTRIB_WIDE_MIN = 300;    // 128-row tasks only on levels with this many
+constexpr int SOLVE_CONTRIB_WIDE_ROWS = 128;   // rows on levels with at least WIDE_MIN such tasks
+constexpr int SOLVE_CONTRIB_WIDE_MIN = 300;    // (two CTAs per SM; with 148 a batch of 48 grids is 1% slower)
 constexpr int SOLVE_GATHER_COLS = 16;
-constexpr int SOLVE_NARROW_W = 64;   // contribution tasks of supernodes this narrow: a warp each
 // Supernodes of the small class at most this wide, with at most SOLVE_WARP_ROWS rows below
 // the diagonal block, are solved by one warp each (both directions, fused) on levels that
 // hold at least SOLVE_WARP_LEVEL_MIN of them (enough warps to fill the GPU; a CTA per

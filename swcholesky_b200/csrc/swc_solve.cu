@@ -9,6 +9,7 @@
 
 #include "swc_engine.h"
 #include "swc_chain.h"
+#include "swc_tile.h"
 
 namespace swc {
 
@@ -29,6 +30,28 @@ constexpr int ST = 256;   // threads of the solve kernels
 // contributions (or the rows below) are gathered, so nothing after that waits for L, and one
 // launch per level does what the diagonal solve and the contributions (backward: the gather and
 // the solve) did in two: a solve of the 60^3 7-point grid 1413 -> 1301 us (B200).
+// The contributions q0, q0 + step, .. < q1 of a column's list, four at a time: an index and the
+// value behind it are two trips to memory, which a plain loop makes one entry after the other.
+__device__ __forceinline__ double sum_contribs(const double *cr, const int *cidx, int q0, int q1, int step) {
+  double acc = 0.0;
+  for (int q = q0; q < q1; q += 4 * step) {
+    int at[4];
+    double v[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) at[u] = cidx[min(q + u * step, q1 - 1)];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) v[u] = ld_if(cr + at[u], q + u * step < q1);
+    acc += (v[0] + v[1]) + (v[2] + v[3]);
+  }
+  return acc;
+}
+// Four threads of one warp per column (sub = 0 .. 3): the sum in all four.
+__device__ __forceinline__ double sum_contribs4(const double *cr, const int *cidx, int q0, int q1, int sub) {
+  double acc = sum_contribs(cr, cidx, q0 + sub, q1, 4);
+  acc += __shfl_xor_sync(0xffffffffu, acc, 1);
+  return acc + __shfl_xor_sync(0xffffffffu, acc, 2);
+}
+
 __device__ __forceinline__ void stage_panel(double *P, const double *Ls, int count) {
   int e = threadIdx.x;
   for (; e + 7 * ST < count; e += 8 * ST) {
@@ -59,16 +82,11 @@ __global__ void __launch_bounds__(ST) k_fwd_small(DevSym S, const int *list, dou
     double *yr = y + (size_t)rhs * n + f;
     double *cr = contrib + (size_t)rhs * cstride;
     // column i of s receives the contributions listed for it (descendant order)
-    if (tid < w) {
-      double acc = yr[tid];
-      int q = cptr[f + tid];
-      const int q1 = cptr[f + tid + 1];
-      for (; q + 3 < q1; q += 4) {
-        const double a = cr[cidx[q]], b = cr[cidx[q + 1]], c = cr[cidx[q + 2]], d = cr[cidx[q + 3]];
-        acc -= (a + b) + (c + d);
-      }
-      for (; q < q1; ++q) acc -= cr[cidx[q]];
-      v[tid] = acc;
+    {
+      const int i = tid >> 2;
+      const int q0 = i < w ? cptr[f + i] : 0, q1 = i < w ? cptr[f + i + 1] : 0;
+      const double yi = i < w ? yr[i] : 0.0, acc = sum_contribs4(cr, cidx, q0, q1, tid & 3);
+      if ((tid & 3) == 0 && i < w) v[i] = yi - acc;
     }
     __syncthreads();
     if (warp == 0) {   // rows lane and lane + 32
@@ -107,142 +125,71 @@ __global__ void __launch_bounds__(ST) k_fwd_small(DevSym S, const int *list, dou
   }
 }
 
-// Contribution tasks.  Very wide supernodes (w > SOLVE_CONTRIB_BIG_W; few of them, each a
-// long row of work): task = (s, r0), 32 rows, one CTA of 32 warps, warp q summing the
-// columns k = q (mod 32) with four loads in flight, so a level of one or two such
-// supernodes still spreads over the GPU.  Wide supernodes (w > SOLVE_NARROW_W): task = (s, r0), rows
-// r0 .. r0 + SOLVE_CONTRIB_WIDE_ROWS - 1 of the off-diagonal block (r0 >= w), one CTA of CW
-// warps: warp q sums the columns k = q (mod CW), lane l the rows r0 + l + 32 t (t < 4), with
-// four columns unrolled (sixteen loads in flight per lane, each warp load 32 consecutive
-// rows of a column), and the CW partial sums meet in shared memory in a fixed order.
-// Narrow supernodes: task = (s, r0), 32 rows, one warp (lane = row, all w columns), CW per
-// CTA after the nwide wide tasks.
-constexpr int CR = SOLVE_CONTRIB_ROWS, CRW = SOLVE_CONTRIB_WIDE_ROWS, CW = 8, CT = 32 * CW;
-constexpr int CTB = 1024, CQB = CTB / CR;
-__global__ void __launch_bounds__(CTB) k_fwd_contrib_big(DevSym S, const int2 *tasks,
-                                                        const double *y, double *contrib, int n,
-                                                        int nrhs, int64_t cstride) {
-  __shared__ double part[CQB][CR];
-  const int s = tasks[blockIdx.x].x, r0 = tasks[blockIdx.x].y;
+// Contribution tasks (s, r0): rows r0 .. r0 + 31 (levels with few tasks) or r0 .. r0 + 127 of the
+// off-diagonal block (r0 >= w), one CTA of CW warps: warp q sums the columns
+// k = q (mod CW), lane l the rows r0 + l + 32 t, and the CW partial sums meet in shared memory in
+// a fixed order.
+// Bound by the bytes in flight (about 50 KB per SM keep the memory busy, and the top levels have
+// one CTA per SM): sixteen predicated loads per lane are issued together, 64 KB per CTA.  With
+// four at a time the ten levels of the 60^3 grid took 255 us, now 192; the gathers 224, now 197.
+constexpr int CR = SOLVE_CONTRIB_ROWS, CRW = SOLVE_CONTRIB_WIDE_ROWS, CW = 16, CT = 32 * CW;
+constexpr int CU = 16;   // loads of L in flight per lane
+// rows r0 .. r0 + R - 1, R / 32 of them per lane, CU columns' worth of loads at a time
+template <int R>
+__device__ __forceinline__ void fwd_contrib_rows(const DevSym &S, int2 task, const double *y, double *contrib,
+                                                 int n, int nrhs, int64_t cstride, double *part) {
+  constexpr int RL = R / 32, C = CU / RL;
+  const int s = task.x, r0 = task.y;
   const int f = S.super[s], w = S.super[s + 1] - f;
   const int64_t rb = S.rowptr[s];
   const int m = (int)(S.rowptr[s + 1] - rb);
-  const double *Ls_s = S.L + S.xptr[s];
-  const int r = threadIdx.x & (CR - 1), q = threadIdx.x / CR;
-  const int a = r0 + r;
-  for (int rhs = 0; rhs < nrhs; ++rhs) {
-    const double *yr = y + (size_t)rhs * n + f;
-    double acc0 = 0.0, acc1 = 0.0, acc2 = 0.0, acc3 = 0.0;
-    if (a < m) {
-      const double *col = Ls_s + a;
-      int k = q;
-      for (; k + 3 * CQB < w; k += 4 * CQB) {
-        acc0 = fma(col[(size_t)k * m], yr[k], acc0);
-        acc1 = fma(col[(size_t)(k + CQB) * m], yr[k + CQB], acc1);
-        acc2 = fma(col[(size_t)(k + 2 * CQB) * m], yr[k + 2 * CQB], acc2);
-        acc3 = fma(col[(size_t)(k + 3 * CQB) * m], yr[k + 3 * CQB], acc3);
-      }
-      for (; k < w; k += CQB) acc0 = fma(col[(size_t)k * m], yr[k], acc0);
-    }
-    part[q][r] = (acc0 + acc1) + (acc2 + acc3);
-    __syncthreads();
-    if (q == 0 && a < m) {
-      double t = 0.0;
-#pragma unroll
-      for (int g = 0; g < CQB; ++g) t += part[g][r];
-      contrib[(size_t)rhs * cstride + (rb - f) + (a - w)] = t;
-    }
-    __syncthreads();
-  }
-}
-
-static_assert(CR == 32 && CRW == 4 * CR, "a lane covers four rows of a wide task");
-__device__ void fwd_contrib_narrow(const DevSym &S, int2 task, const double *y, double *contrib,
-                                   int n, int nrhs, int64_t cstride) {
-  const int s = task.x, r0 = task.y, lane = threadIdx.x & 31;
-  const int f = S.super[s], w = S.super[s + 1] - f;
-  const int64_t rb = S.rowptr[s];
-  const int m = (int)(S.rowptr[s + 1] - rb);
-  const int a = r0 + lane;
-  if (a >= m) return;
-  const double *col = S.L + S.xptr[s] + a;
-  for (int rhs = 0; rhs < nrhs; ++rhs) {
-    const double *yr = y + (size_t)rhs * n + f;
-    double acc0 = 0.0, acc1 = 0.0, acc2 = 0.0, acc3 = 0.0;
-    int k = 0;
-    for (; k + 3 < w; k += 4) {
-      acc0 = fma(col[(size_t)k * m], yr[k], acc0);
-      acc1 = fma(col[(size_t)(k + 1) * m], yr[k + 1], acc1);
-      acc2 = fma(col[(size_t)(k + 2) * m], yr[k + 2], acc2);
-      acc3 = fma(col[(size_t)(k + 3) * m], yr[k + 3], acc3);
-    }
-    for (; k < w; ++k) acc0 = fma(col[(size_t)k * m], yr[k], acc0);
-    contrib[(size_t)rhs * cstride + (rb - f) + (a - w)] = (acc0 + acc1) + (acc2 + acc3);
-  }
-}
-
-__global__ void __launch_bounds__(CT) k_fwd_contrib(DevSym S, const int2 *tasks, int count,
-                                                    int nwide, const double *y, double *contrib,
-                                                    int n, int nrhs, int64_t cstride) {
-  __shared__ double part[CW][CRW];
-  if ((int)blockIdx.x >= nwide) {
-    const int t = nwide + ((int)blockIdx.x - nwide) * CW + (int)(threadIdx.x >> 5);
-    if (t < count) fwd_contrib_narrow(S, tasks[t], y, contrib, n, nrhs, cstride);
-    return;
-  }
-  const int s = tasks[blockIdx.x].x, r0 = tasks[blockIdx.x].y;
-  const int f = S.super[s], w = S.super[s + 1] - f;
-  const int64_t rb = S.rowptr[s];
-  const int m = (int)(S.rowptr[s + 1] - rb);
-  const double *Ls_s = S.L + S.xptr[s];
   const int lane = threadIdx.x & 31, q = threadIdx.x >> 5;
-  // rows of this lane (rows past the panel read row r0 and are dropped)
-  int ra[4];
-  bool in[4];
-#pragma unroll
-  for (int t = 0; t < 4; ++t) {
-    ra[t] = r0 + lane + 32 * t;
-    in[t] = ra[t] < m;
-    if (!in[t]) ra[t] = r0;
-  }
+  const double *row = S.L + S.xptr[s] + r0 + lane;
   for (int rhs = 0; rhs < nrhs; ++rhs) {
     const double *yr = y + (size_t)rhs * n + f;
-    double acc[4][2];
+    double acc[RL][2];
 #pragma unroll
-    for (int t = 0; t < 4; ++t) acc[t][0] = acc[t][1] = 0.0;
-    int k = q;
-    for (; k + 3 * CW < w; k += 4 * CW) {
-      const double y0 = yr[k], y1 = yr[k + CW], y2 = yr[k + 2 * CW], y3 = yr[k + 3 * CW];
-      const double *c0 = Ls_s + (size_t)k * m, *c1 = c0 + (size_t)CW * m;
-      const double *c2 = c1 + (size_t)CW * m, *c3 = c2 + (size_t)CW * m;
+    for (int t = 0; t < RL; ++t) acc[t][0] = acc[t][1] = 0.0;
+    for (int k0 = q; k0 < w; k0 += C * CW) {
+      double l[C][RL];
 #pragma unroll
-      for (int t = 0; t < 4; ++t) {
-        acc[t][0] = fma(c0[ra[t]], y0, acc[t][0]);
-        acc[t][1] = fma(c1[ra[t]], y1, acc[t][1]);
-        acc[t][0] = fma(c2[ra[t]], y2, acc[t][0]);
-        acc[t][1] = fma(c3[ra[t]], y3, acc[t][1]);
+      for (int c = 0; c < C; ++c) {
+        const int k = k0 + c * CW;
+#pragma unroll
+        for (int t = 0; t < RL; ++t)
+          l[c][t] = ld_if(row + (size_t)k * m + 32 * t, k < w && r0 + lane + 32 * t < m);
+      }
+#pragma unroll
+      for (int c = 0; c < C; ++c) {
+        const int k = k0 + c * CW;
+        const double yk = yr[min(k, w - 1)], yc = k < w ? yk : 0.0;
+#pragma unroll
+        for (int t = 0; t < RL; ++t) acc[t][c & 1] = fma(l[c][t], yc, acc[t][c & 1]);
       }
     }
-    for (; k < w; k += CW) {
-      const double yk = yr[k];
-      const double *ck = Ls_s + (size_t)k * m;
 #pragma unroll
-      for (int t = 0; t < 4; ++t) acc[t][0] = fma(ck[ra[t]], yk, acc[t][0]);
-    }
-#pragma unroll
-    for (int t = 0; t < 4; ++t) part[q][lane + 32 * t] = acc[t][0] + acc[t][1];
+    for (int t = 0; t < RL; ++t) part[q * R + lane + 32 * t] = acc[t][0] + acc[t][1];
     __syncthreads();
-    if (threadIdx.x < CRW) {
+    if ((int)threadIdx.x < R) {
       const int a = r0 + (int)threadIdx.x;
       if (a < m) {
         double t = 0.0;
 #pragma unroll
-        for (int g = 0; g < CW; ++g) t += part[g][threadIdx.x];
+        for (int g = 0; g < CW; ++g) t += part[g * R + threadIdx.x];
         contrib[(size_t)rhs * cstride + (rb - f) + (a - w)] = t;
       }
     }
     __syncthreads();
   }
+}
+
+__global__ void __launch_bounds__(CT, 2) k_fwd_contrib(DevSym S, const int2 *tasks, int nbig, const double *y,
+                                                       double *contrib, int n, int nrhs, int64_t cstride) {
+  __shared__ double part[CW * CRW];
+  if ((int)blockIdx.x < nbig)
+    fwd_contrib_rows<CR>(S, tasks[blockIdx.x], y, contrib, n, nrhs, cstride, part);
+  else
+    fwd_contrib_rows<CRW>(S, tasks[blockIdx.x], y, contrib, n, nrhs, cstride, part);
 }
 
 // Backward solve, level by level (root first):
@@ -251,10 +198,11 @@ __global__ void __launch_bounds__(CT) k_fwd_contrib(DevSym S, const int2 *tasks,
 //                 lane); the rows below are columns of ancestors, already solved.  Then
 //                 k_bwd_chain.
 //   k_bwd_small   small supernodes, one CTA each: the gather and L_ss^{-T}.
-constexpr int GCH = 2048;       // gathered rows staged per chunk
+constexpr int GCH = 4096;       // gathered rows staged per chunk
+constexpr int GU = 16;          // loads in flight per lane
 constexpr int GT = 32 * SOLVE_GATHER_COLS;   // one warp per column of the task
-__global__ void __launch_bounds__(GT) k_bwd_gather(DevSym S, const int2 *tasks, double *x,
-                                                   int n, int nrhs) {
+__global__ void __launch_bounds__(GT, 2) k_bwd_gather(DevSym S, const int2 *tasks, double *x,
+                                                      int n, int nrhs) {
   __shared__ double xg[GCH];
   const int s = tasks[blockIdx.x].x, j0 = tasks[blockIdx.x].y;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -265,27 +213,34 @@ __global__ void __launch_bounds__(GT) k_bwd_gather(DevSym S, const int2 *tasks, 
   const double *Ls_s = S.L + S.xptr[s];
   const int j = j0 + warp;
   const bool own = j < w;
-  // every column of this CTA reads the same x[rows[a]]: gather them once per chunk
+  const double *col = Ls_s + (size_t)(own ? j : j0) * m + lane;
+  // every column of this CTA reads the same x[rows[a]]: gather them once per chunk, while the
+  // column's first loads are under way
   for (int rhs = 0; rhs < nrhs; ++rhs) {
     double *xr = x + (size_t)rhs * n;
-    double acc[8];
-#pragma unroll
-    for (int u = 0; u < 8; ++u) acc[u] = 0.0;
+    double acc[4] = {0.0, 0.0, 0.0, 0.0};
     for (int a0 = w; a0 < m; a0 += GCH) {
       const int len = min(GCH, m - a0);
+      double c[GU];
+#pragma unroll
+      for (int u = 0; u < GU; ++u) c[u] = ld_if(col + a0 + 32 * u, own && 32 * u + lane < len);
       __syncthreads();
+#pragma unroll 4
       for (int i = threadIdx.x; i < len; i += GT) xg[i] = xr[rows[a0 + i]];
       __syncthreads();
-      if (own) {
-        const double *col = Ls_s + (size_t)j * m + a0;
-        int i = lane;
-        for (; i + 7 * 32 < len; i += 8 * 32)
+      for (int i = 0;;) {
 #pragma unroll
-          for (int u = 0; u < 8; ++u) acc[u] = fma(col[i + 32 * u], xg[i + 32 * u], acc[u]);
-        for (; i < len; i += 32) acc[0] = fma(col[i], xg[i], acc[0]);
+        for (int u = 0; u < GU; ++u) {
+          const int r = i + 32 * u + lane;
+          acc[u & 3] = fma(c[u], r < len ? xg[r] : 0.0, acc[u & 3]);
+        }
+        i += 32 * GU;
+        if (i >= len) break;
+#pragma unroll
+        for (int u = 0; u < GU; ++u) c[u] = ld_if(col + a0 + i + 32 * u, own && i + 32 * u + lane < len);
       }
     }
-    double t = ((acc[0] + acc[1]) + (acc[2] + acc[3])) + ((acc[4] + acc[5]) + (acc[6] + acc[7]));
+    double t = (acc[0] + acc[1]) + (acc[2] + acc[3]);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
     if (lane == 0 && own) xr[f + j] -= t;
@@ -319,8 +274,7 @@ __global__ void __launch_bounds__(ST) k_fwd_warp(DevSym S, const int *list, int 
     double *cr = contrib + (size_t)rhs * cstride;
     double v = 0.0;
     if (lane < w) {
-      v = yr[f + lane];
-      for (int q = cptr[f + lane]; q < cptr[f + lane + 1]; ++q) v -= cr[cidx[q]];
+      v = yr[f + lane] - sum_contribs(cr, cidx, cptr[f + lane], cptr[f + lane + 1], 1);
     }
     // L_ss y = v
 #pragma unroll 4
@@ -579,14 +533,12 @@ __global__ void __launch_bounds__(ST, NS == CHAIN_NS_SMALL ? 2 : 1) k_fwd_chain(
       tr[i][1] = T[(size_t)(lane + 32) * TB + w8 + i];
     }
     // right-hand side minus the descendants' contributions (read after the last barrier)
-    if (threadIdx.x < TB) {
-      double v = 0.0;
-      if ((int)threadIdx.x < bw) {
-        const int j = f + r0 + threadIdx.x;
-        v = y[j];
-        for (int qq = cptr[j]; qq < cptr[j + 1]; ++qq) v -= contrib[cidx[qq]];
-      }
-      vs[threadIdx.x] = v;
+    {
+      static_assert(ST == 4 * TB, "four threads per column");
+      const int i = (int)threadIdx.x >> 2, j = f + r0 + i;
+      const int q0 = i < bw ? cptr[j] : 0, q1 = i < bw ? cptr[j + 1] : 0;
+      const double yj = i < bw ? y[j] : 0.0, v = sum_contribs4(contrib, cidx, q0, q1, threadIdx.x & 3);
+      if ((threadIdx.x & 3) == 0) vs[i] = yj - v;
     }
     double acc0 = 0.0, acc1 = 0.0;   // rows lane, lane + 32 over this warp's columns
     bool ok = true;
@@ -937,15 +889,9 @@ void launch_fwd_small(const DevSym &S, const int *list, int count, int smem, dou
   if (count > 0)
     k_fwd_small<<<count, ST, smem, st>>>(S, list, y, contrib, cptr, cidx, n, nrhs, cstride);
 }
-void launch_fwd_contrib(const DevSym &S, const int2 *tasks, int count, int nbig, int nwide,
-                        const double *y, double *contrib, int n, int nrhs, int64_t cstride,
-                        cudaStream_t st) {
-  if (nbig > 0) k_fwd_contrib_big<<<nbig, CTB, 0, st>>>(S, tasks, y, contrib, n, nrhs, cstride);
-  tasks += nbig;
-  count -= nbig;
-  const int blocks = nwide + (count - nwide + CW - 1) / CW;
-  if (count > 0)
-    k_fwd_contrib<<<blocks, CT, 0, st>>>(S, tasks, count, nwide, y, contrib, n, nrhs, cstride);
+void launch_fwd_contrib(const DevSym &S, const int2 *tasks, int count, int nbig, const double *y,
+                        double *contrib, int n, int nrhs, int64_t cstride, cudaStream_t st) {
+  if (count > 0) k_fwd_contrib<<<count, CT, 0, st>>>(S, tasks, nbig, y, contrib, n, nrhs, cstride);
 }
 void launch_fwd_warp(const DevSym &S, const int *list, int count, double *y, double *contrib,
                      const int *cptr, const int *cidx, int n, int nrhs, int64_t cstride,
