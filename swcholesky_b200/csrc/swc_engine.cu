@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <queue>
 #include <climits>
 #include <cstdlib>
 #include <cstring>
@@ -1084,6 +1085,46 @@ bool check_scatter_plan(int n, const int *Ls, const HostSym &H, const Plan &P, c
   return true;
 }
 
+// Two halves of the tree for the solves: starting from the roots, the heaviest subtree is replaced
+// by its children until the rest divide into two parts of similar weight (panel elements); half[s]
+// is 0 or 1, or 2 for the supernodes above.  False when that does not happen within SOLVE_TOP
+// replacements or the lighter half is smaller than SOLVE_HALF_MIN elements.
+static bool solve_halves(int supNo, const std::vector<int> &parent, const std::vector<int> &super,
+                         const std::vector<int64_t> &rowptr, std::vector<char> &half) {
+  std::vector<int64_t> weight(supNo);
+  std::vector<std::vector<int>> child(supNo);
+  std::priority_queue<std::pair<int64_t, int>> open;
+  for (int s = 0; s < supNo; ++s) weight[s] = (rowptr[s + 1] - rowptr[s]) * (super[s + 1] - super[s]);
+  for (int s = 0; s < supNo; ++s)   // parents have larger numbers
+    if (parent[s] >= 0) {
+      weight[parent[s]] += weight[s];
+      child[parent[s]].push_back(s);
+    }
+  for (int s = 0; s < supNo; ++s)
+    if (parent[s] < 0) open.push({weight[s], s});
+  for (int k = 0; k <= SOLVE_TOP && !open.empty(); ++k) {
+    // the heaviest first, to the lighter half
+    int64_t sum[2] = {0, 0};
+    half.assign(supNo, 2);
+    for (auto rest = open; !rest.empty(); rest.pop()) {
+      const int h = sum[1] < sum[0];
+      sum[h] += rest.top().first;
+      half[rest.top().second] = (char)h;
+    }
+    const int64_t light = std::min(sum[0], sum[1]), all = sum[0] + sum[1];
+    if (all < 2 * SOLVE_HALF_MIN) return false;
+    if (light >= SOLVE_HALF_MIN && 5 * light >= 2 * all) {
+      for (int s = supNo - 1; s >= 0; --s)
+        if (half[s] == 2 && parent[s] >= 0) half[s] = half[parent[s]];
+      return true;
+    }
+    const int top = open.top().second;
+    open.pop();
+    for (int c : child[top]) open.push({weight[c], c});
+  }
+  return false;
+}
+
 // Per-level task lists of the supernodal solves (no device work).
 void build_solve_plan(int n, const int *Ls, const HostSym &H, SolvePlan &SP) {
   const int supNo = (int)H.super.size() - 1;
@@ -1093,7 +1134,7 @@ void build_solve_plan(int n, const int *Ls, const HostSym &H, SolvePlan &SP) {
   SP = SolvePlan();
   std::vector<int> lev(supNo, 0);
   int nl = 0;
-  std::vector<int> col2sup(n);
+  std::vector<int> col2sup(n), parent(supNo, -1);
   for (int s = 0; s < supNo; ++s)
     for (int j = super[s]; j < super[s + 1]; ++j) col2sup[j] = s;
   for (int s = 0; s < supNo; ++s) {
@@ -1101,13 +1142,32 @@ void build_solve_plan(int n, const int *Ls, const HostSym &H, SolvePlan &SP) {
     const int64_t m = rowptr[s + 1] - rowptr[s];
     nl = std::max(nl, lev[s] + 1);
     if (m > w) {
-      const int p = col2sup[Ls[rowptr[s] + w]];
+      const int p = parent[s] = col2sup[Ls[rowptr[s] + w]];
       lev[p] = std::max(lev[p], lev[s] + 1);
     }
     SP.max_w = std::max(SP.max_w, w);
   }
-  std::vector<std::vector<int>> bylev(nl);
-  for (int s = 0; s < supNo; ++s) bylev[lev[s]].push_back(s);
+  std::vector<std::vector<int>> full(nl), bylev;
+  for (int s = 0; s < supNo; ++s) full[lev[s]].push_back(s);
+  // the levels of the two halves, then those above; each as its level of the whole tree (height:
+  // the classes below count that one, whose halves run together)
+  std::vector<int> height;
+  {
+    std::vector<char> half;
+    const bool two = solve_halves(supNo, parent, super, rowptr, half);
+    for (int h = 0; h <= (two ? 2 : 0); ++h) {
+      for (int l = 0; l < nl; ++l) {
+        std::vector<int> part;
+        for (int s : full[l])
+          if (!two || half[s] == h) part.push_back(s);
+        if (part.empty()) continue;
+        bylev.push_back(std::move(part));
+        height.push_back(l);
+      }
+      if (two && h == 0) SP.half0 = (int)bylev.size();
+      if (two && h == 1) SP.half1 = (int)bylev.size();
+    }
+  }
   auto warp_size_ok = [&](int s) {
     const int w = super[s + 1] - super[s];
     const int64_t m = rowptr[s + 1] - rowptr[s];
@@ -1116,10 +1176,11 @@ void build_solve_plan(int n, const int *Ls, const HostSym &H, SolvePlan &SP) {
   std::vector<int> warp_level(nl, 0);
   for (int l = 0; l < nl; ++l) {
     int cnt = 0;
-    for (int s : bylev[l]) cnt += warp_size_ok(s);
+    for (int s : full[l]) cnt += warp_size_ok(s);
     warp_level[l] = cnt >= SOLVE_WARP_LEVEL_MIN;
   }
-  for (int l = 0; l < nl; ++l) {
+  for (int l = 0; l < (int)bylev.size(); ++l) {
+    const std::vector<int> &whole = full[height[l]];
     SP.level_off.push_back((int)SP.list.size());
     SP.level_smem.push_back(0);
     SP.warp_off.push_back((int)SP.warp_list.size());
@@ -1130,7 +1191,7 @@ void build_solve_plan(int n, const int *Ls, const HostSym &H, SolvePlan &SP) {
     SP.g8_off.push_back((int)SP.g8_tasks.size());
     {
       int64_t nt = 0;
-      for (int s : bylev[l])
+      for (int s : whole)
         if (H.dinv_off[s] >= 0) nt += (rowptr[s + 1] - rowptr[s] - (super[s + 1] - super[s]) + 127) / 128;
       const bool split = nt < SOLVE8_FULL_TASKS;
       SP.c8_split.push_back(split);
@@ -1144,7 +1205,7 @@ void build_solve_plan(int n, const int *Ls, const HostSym &H, SolvePlan &SP) {
     std::vector<int2> wide;
     // 128-row tasks only when the level has enough of them to fill the GPU
     int64_t n128 = 0;
-    for (int s : bylev[l])
+    for (int s : whole)
       if (H.dinv_off[s] >= 0)
         n128 += (rowptr[s + 1] - rowptr[s] - (super[s + 1] - super[s]) + SOLVE_CONTRIB_WIDE_ROWS - 1) /
                 SOLVE_CONTRIB_WIDE_ROWS;
@@ -1156,7 +1217,7 @@ void build_solve_plan(int n, const int *Ls, const HostSym &H, SolvePlan &SP) {
         const int nb = (w + TB - 1) / TB;
         for (int k = 0; k < nb; ++k) SP.fchain.push_back(make_int2(s, k));
         for (int k = nb - 1; k >= 0; --k) SP.bchain.push_back(make_int2(s, k));
-      } else if (warp_level[l] && warp_size_ok(s)) {
+      } else if (warp_level[height[l]] && warp_size_ok(s)) {
         SP.warp_list.push_back(s);   // its contributions and gathers are done by the warp
         continue;
       } else {   // its contributions and gathers are done by its CTA
@@ -1289,7 +1350,7 @@ bool check_solve_plan(int n, const int *Ls, const HostSym &H, const SolvePlan &S
   if (nl < 0 || (int)SP.warp_off.size() != nl + 1 || (int)SP.chain_off.size() != nl + 1 ||
       (int)SP.contrib_off.size() != nl + 1 || (int)SP.gather_off.size() != nl + 1 ||
       (int)SP.contrib_big.size() != nl ||
-      SP.fchain.size() != SP.bchain.size())
+      SP.fchain.size() != SP.bchain.size() || SP.half0 < 0 || SP.half1 < SP.half0 || SP.half1 > nl)
     return bad("per-level offsets of unequal length");
   if (SP.contrib_len != H.nls - n) return bad("contribution length");
   // every supernode in exactly one level, by exactly one kind of task
@@ -1350,6 +1411,8 @@ bool check_solve_plan(int n, const int *Ls, const HostSym &H, const SolvePlan &S
     if (rowptr[s + 1] - rowptr[s] > w) {
       const int p = col2sup[Ls[rowptr[s] + w]];   // the parent: first off-diagonal row's
       if (level[p] <= level[s]) return bad("a parent not in a later level");
+      if (level[p] < SP.half1 && (level[p] < SP.half0) != (level[s] < SP.half0))
+        return bad("a parent in the other half");
     }
   }
   // eight right-hand sides: the tiled supernodes' rows and column groups, each once, in order
@@ -2096,7 +2159,34 @@ void Engine::run_solve8(double *x8) {
   cudaMemsetAsync(d_flags_, 0, sizeof(int) * std::max<int64_t>(nflags_, 1), stream_);
   const Solve8Dev D{d_slist_, d_swarp_, d_cptr_, d_cidx_, d_fchain_, d_bchain_, d_c8_tasks_,
                     d_g8_tasks_, d_flags_};
-  launch_solve8(sym_, splan_, D, x8, d_c8_, stream_);
+  run_halves([&](int l0, int l1, bool fwd, SolveQueue &st) {
+    launch_solve8(sym_, splan_, D, x8, d_c8_, l0, l1, fwd, st);
+  });
+}
+
+// The levels of a solve, forward and backward: the second half of the tree on the auxiliary
+// stream, beside the first.  The halves share no column and no contribution.  A level is a
+// latency-bound chain and then a stream through the panels bound by bandwidth, so that one
+// half's chains hide behind the other's streams.
+template <class F>
+void Engine::run_halves(F levels) {
+  const int h0 = splan_.half0, h1 = splan_.half1, nl = (int)splan_.level_off.size() - 1;
+  SolveQueue main{stream_, false}, aux{aux_stream_, false};
+  for (int pass = 0; pass < 2; ++pass) {
+    const bool fwd = pass == 0;
+    if (!fwd) levels(h1, nl, false, main);
+    if (h1 > 0) {
+      cudaEventRecord(ev_fork_, stream_);
+      cudaStreamWaitEvent(aux_stream_, ev_fork_, 0);
+      main.chained = aux.chained = false;
+      levels(h0, h1, fwd, aux);
+      cudaEventRecord(ev_join_, aux_stream_);
+      levels(0, h0, fwd, main);
+      cudaStreamWaitEvent(stream_, ev_join_, 0);
+      main.chained = false;
+    }
+    if (fwd) levels(h1, nl, true, main);
+  }
 }
 
 // x := (L L^T)^{-1} x for device x (n x nrhs), eight right-hand sides at a time (a single one
@@ -2136,13 +2226,16 @@ void Engine::run_solve(double *x, int nrhs) {
 // r + 1 forward, nrhs + r + 1 backward) are the same in every solve and a graph of this
 // sequence can be replayed.
 void Engine::run_solve_with(double *x, int nrhs, double *contrib) {
-  cudaStream_t st = stream_;
+  cudaMemsetAsync(d_flags_, 0, sizeof(int) * std::max<int64_t>(nflags_, 1), stream_);
+  run_halves([&](int l0, int l1, bool fwd, SolveQueue &st) {
+    solve_levels(x, nrhs, contrib, l0, l1, fwd, st);
+  });
+}
+
+void Engine::solve_levels(double *x, int nrhs, double *contrib, int l0, int l1, bool fwd, SolveQueue &st) {
   const SolvePlan &SP = splan_;
-  const int nl = (int)SP.level_off.size() - 1;
   const int64_t cs = std::max<int64_t>(SP.contrib_len, 1);
-  const int base = 0;
-  cudaMemsetAsync(d_flags_, 0, sizeof(int) * std::max<int64_t>(nflags_, 1), st);
-  for (int l = 0; l < nl; ++l) {
+  for (int l = l0; fwd && l < l1; ++l) {
     launch_fwd_warp(sym_, d_swarp_ + SP.warp_off[l], SP.warp_off[l + 1] - SP.warp_off[l], x,
                     contrib, d_cptr_, d_cidx_, n_, nrhs, cs, st);
     launch_fwd_small(sym_, d_slist_ + SP.level_off[l], SP.level_off[l + 1] - SP.level_off[l],
@@ -2150,11 +2243,11 @@ void Engine::run_solve_with(double *x, int nrhs, double *contrib) {
     for (int r = 0; r < nrhs; ++r)
       launch_fwd_chain(sym_, d_fchain_ + SP.chain_off[l], SP.chain_off[l + 1] - SP.chain_off[l],
                        x + (size_t)r * n_, contrib + (size_t)r * cs, d_cptr_, d_cidx_, d_flags_,
-                       base + r + 1, n_, cs, st);
+                       r + 1, n_, cs, st);
     launch_fwd_contrib(sym_, d_scontrib_ + SP.contrib_off[l], SP.contrib_off[l + 1] - SP.contrib_off[l],
                        SP.contrib_big[l], x, contrib, n_, nrhs, cs, st);
   }
-  for (int l = nl - 1; l >= 0; --l) {
+  for (int l = l1 - 1; !fwd && l >= l0; --l) {
     launch_bwd_gather(sym_, d_sgather_ + SP.gather_off[l], SP.gather_off[l + 1] - SP.gather_off[l],
                       x, n_, nrhs, st);
     launch_bwd_small(sym_, d_slist_ + SP.level_off[l], SP.level_off[l + 1] - SP.level_off[l],
@@ -2163,7 +2256,7 @@ void Engine::run_solve_with(double *x, int nrhs, double *contrib) {
                     nrhs, st);
     for (int r = 0; r < nrhs; ++r)
       launch_bwd_chain(sym_, d_bchain_ + SP.chain_off[l], SP.chain_off[l + 1] - SP.chain_off[l],
-                       x + (size_t)r * n_, d_flags_, base + nrhs + r + 1, st);
+                       x + (size_t)r * n_, d_flags_, nrhs + r + 1, st);
   }
 }
 

@@ -199,28 +199,58 @@ struct Plan {
 
 
 // Triangular solves and refinement (swc_solve.cu)
+// Where a solve's kernels go.  chained: the last operation of the stream is one of them, so that
+// the next may start before it ends (programmatic dependent launch).
+struct SolveQueue {
+  cudaStream_t st;
+  bool chained;
+};
+template <class... P, class... A>
+void launch_solve(SolveQueue &q, int cluster, void (*kernel)(P...), int grid, int block, int smem, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute at[2];
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3((unsigned)block);
+  cfg.dynamicSmemBytes = (size_t)smem;
+  cfg.stream = q.st;
+  cfg.attrs = at;
+  if (cluster > 1) {
+    at[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+    at[cfg.numAttrs].val.clusterDim.x = (unsigned)cluster;
+    at[cfg.numAttrs].val.clusterDim.y = at[cfg.numAttrs].val.clusterDim.z = 1;
+    ++cfg.numAttrs;
+  }
+  if (q.chained) {
+    at[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[cfg.numAttrs].val.programmaticStreamSerializationAllowed = 1;
+    ++cfg.numAttrs;
+  }
+  cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+  q.chained = true;
+}
+
 bool solve_configure(int max_w, std::string &err);
 void launch_fwd_small(const DevSym &S, const int *list, int count, int smem, double *y,
                       double *contrib, const int *cptr, const int *cidx, int n, int nrhs,
-                     int64_t cstride, cudaStream_t st);
+                     int64_t cstride, SolveQueue &st);
 void launch_fwd_contrib(const DevSym &S, const int2 *tasks, int count, int nbig, const double *y,
-                        double *contrib, int n, int nrhs, int64_t cstride, cudaStream_t st);
+                        double *contrib, int n, int nrhs, int64_t cstride, SolveQueue &st);
 void launch_bwd_gather(const DevSym &S, const int2 *tasks, int count, double *x, int n, int nrhs,
-                       cudaStream_t st);
+                       SolveQueue &st);
 void launch_bwd_small(const DevSym &S, const int *list, int count, int smem, double *x, int n,
-                     int nrhs, cudaStream_t st);
+                     int nrhs, SolveQueue &st);
 // small supernodes, one warp each: forward (contributions in, diagonal solve, contributions
 // of the rows below out) and backward (gather from ancestors, transposed diagonal solve)
 void launch_fwd_warp(const DevSym &S, const int *list, int count, double *y, double *contrib,
                      const int *cptr, const int *cidx, int n, int nrhs, int64_t cstride,
-                     cudaStream_t st);
+                     SolveQueue &st);
 void launch_bwd_warp(const DevSym &S, const int *list, int count, double *x, int n, int nrhs,
-                     cudaStream_t st);
+                     SolveQueue &st);
 void launch_fwd_chain(const DevSym &S, const int2 *tasks, int count, double *y,
                       const double *contrib, const int *cptr, const int *cidx, int *flags,
-                      int epoch, int n, int64_t cstride, cudaStream_t st);
+                      int epoch, int n, int64_t cstride, SolveQueue &st);
 void launch_bwd_chain(const DevSym &S, const int2 *tasks, int count, double *x, int *flags,
-                      int epoch, cudaStream_t st);
+                      int epoch, SolveQueue &st);
 void launch_spmv(int n, const int *rp, const int *ci, const double *val, const double *x,
                  double *y, int nrhs, cudaStream_t st);
 void launch_gather_vals(int nnz, const int *map, const double *ax, double *val, cudaStream_t st);
@@ -232,8 +262,11 @@ void launch_norms(int n, int nrhs, const double *x, const double *y, double *out
 int norm_scratch_doubles(int nrhs);
 void launch_rowabs(int n, const int *rp, const double *val, double *out, cudaStream_t st);
 
-// Per-level task lists of the solves.
+// Per-level task lists of the solves.  "Levels" [0, half0) hold one half of the tree (unions of
+// whole subtrees), [half0, half1) the other, which may run beside it, and the rest the supernodes
+// above both; half0 = half1 = 0 when the tree is not divided.
 struct SolvePlan {
+  int half0 = 0, half1 = 0;
   std::vector<int> level_off;       // small-class supernodes of level l, one CTA each:
   std::vector<int> list;            //   list[level_off[l] .. level_off[l+1])
   std::vector<int> level_smem;      //   shared memory of the level's launches
@@ -265,8 +298,9 @@ struct Solve8Dev {
 bool solve8_configure(std::string &err);
 void launch_pack8(int n, int nr, const double *x, double *x8, cudaStream_t st);
 void launch_unpack8(int n, int nr, const double *x8, double *x, cudaStream_t st);
+// the levels l0 .. l1 - 1, forward or backward
 void launch_solve8(const DevSym &S, const SolvePlan &SP, const Solve8Dev &D, double *x8, double *c8,
-                   cudaStream_t st);
+                   int l0, int l1, bool fwd, SolveQueue &st);
 
 // Result of a refined solve, per right-hand side.
 struct RefineInfo {
@@ -515,6 +549,8 @@ class Engine {
   bool ensure_work(int nrhs, std::string &err);
   void run_solve(double *x, int nrhs);
   void run_solve_with(double *x, int nrhs, double *contrib);
+  void solve_levels(double *x, int nrhs, double *contrib, int l0, int l1, bool fwd, SolveQueue &st);
+  template <class F> void run_halves(F levels);
   bool solve_status_ok(std::string &err);
 };
 

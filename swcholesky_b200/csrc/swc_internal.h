@@ -68,6 +68,13 @@ constexpr int SOLVE_GATHER_COLS = 16;
 constexpr int SOLVE_WARP_W = 32;
 constexpr int SOLVE_WARP_ROWS = 256;
 constexpr int SOLVE_WARP_LEVEL_MIN = 4096;
+// The solves divide the tree into two halves that run beside each other when the lighter one holds
+// at least this many panel elements (found within SOLVE_TOP steps from the roots).  B200, one /
+// eight right-hand sides, undivided -> divided: 60^3 grid 1124 -> 1045 us, 301 x 287 grid eight
+// 370 -> 359, 230 x 220 grid 198 / 288 -> 198 / 282; below, the fork and the join cost more than
+// they hide: 24 x 23 x 25 grid 197 / 277 -> 201 / 280, 60 x 61 grid 122 / 139 -> 130 / 143.
+constexpr int SOLVE_TOP = 64;
+constexpr int64_t SOLVE_HALF_MIN = (int64_t)1 << 20;
 // Several right-hand sides: contribution tasks of 128 rows on levels with at least one per SM,
 // else 32-row tasks whose warps split the columns.
 constexpr int SOLVE8_FULL_TASKS = 148;

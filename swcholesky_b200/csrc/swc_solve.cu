@@ -71,6 +71,7 @@ __global__ void __launch_bounds__(ST) k_fwd_small(DevSym S, const int *list, dou
                                                   const int *cptr, const int *cidx, int n, int nrhs,
                                                   int64_t cstride) {
   extern __shared__ double P[];
+  pdl_trigger();
   const int s = list[blockIdx.x];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int f = S.super[s], w = S.super[s + 1] - f;
@@ -78,6 +79,7 @@ __global__ void __launch_bounds__(ST) k_fwd_small(DevSym S, const int *list, dou
   const int m = (int)(S.rowptr[s + 1] - rb);
   double *v = P + m * w;
   stage_panel(P, S.L + S.xptr[s], m * w);
+  pdl_wait();
   for (int rhs = 0; rhs < nrhs; ++rhs) {
     double *yr = y + (size_t)rhs * n + f;
     double *cr = contrib + (size_t)rhs * cstride;
@@ -145,6 +147,7 @@ __device__ __forceinline__ void fwd_contrib_rows(const DevSym &S, int2 task, con
   const int m = (int)(S.rowptr[s + 1] - rb);
   const int lane = threadIdx.x & 31, q = threadIdx.x >> 5;
   const double *row = S.L + S.xptr[s] + r0 + lane;
+  bool first = true;
   for (int rhs = 0; rhs < nrhs; ++rhs) {
     const double *yr = y + (size_t)rhs * n + f;
     double acc[RL][2];
@@ -159,6 +162,8 @@ __device__ __forceinline__ void fwd_contrib_rows(const DevSym &S, int2 task, con
         for (int t = 0; t < RL; ++t)
           l[c][t] = ld_if(row + (size_t)k * m + 32 * t, k < w && r0 + lane + 32 * t < m);
       }
+      if (first) pdl_wait();
+      first = false;
 #pragma unroll
       for (int c = 0; c < C; ++c) {
         const int k = k0 + c * CW;
@@ -186,6 +191,7 @@ __device__ __forceinline__ void fwd_contrib_rows(const DevSym &S, int2 task, con
 __global__ void __launch_bounds__(CT, 2) k_fwd_contrib(DevSym S, const int2 *tasks, int nbig, const double *y,
                                                        double *contrib, int n, int nrhs, int64_t cstride) {
   __shared__ double part[CW * CRW];
+  pdl_trigger();
   if ((int)blockIdx.x < nbig)
     fwd_contrib_rows<CR>(S, tasks[blockIdx.x], y, contrib, n, nrhs, cstride, part);
   else
@@ -213,6 +219,8 @@ __global__ void __launch_bounds__(GT, 2) k_bwd_gather(DevSym S, const int2 *task
   const double *Ls_s = S.L + S.xptr[s];
   const int j = j0 + warp;
   const bool own = j < w;
+  pdl_trigger();
+  bool first = true;
   const double *col = Ls_s + (size_t)(own ? j : j0) * m + lane;
   // every column of this CTA reads the same x[rows[a]]: gather them once per chunk, while the
   // column's first loads are under way
@@ -224,6 +232,8 @@ __global__ void __launch_bounds__(GT, 2) k_bwd_gather(DevSym S, const int2 *task
       double c[GU];
 #pragma unroll
       for (int u = 0; u < GU; ++u) c[u] = ld_if(col + a0 + 32 * u, own && 32 * u + lane < len);
+      if (first) pdl_wait();
+      first = false;
       __syncthreads();
 #pragma unroll 4
       for (int i = threadIdx.x; i < len; i += GT) xg[i] = xr[rows[a0 + i]];
@@ -261,6 +271,8 @@ __global__ void __launch_bounds__(ST) k_fwd_warp(DevSym S, const int *list, int 
                                                  const int *cidx, int n, int nrhs,
                                                  int64_t cstride) {
   const int t = blockIdx.x * WPC + (threadIdx.x >> 5);
+  pdl_trigger();
+  pdl_wait();
   if (t >= count) return;
   const unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31;
@@ -303,6 +315,8 @@ __global__ void __launch_bounds__(ST) k_fwd_warp(DevSym S, const int *list, int 
 __global__ void __launch_bounds__(ST) k_bwd_warp(DevSym S, const int *list, int count, double *x,
                                                  int n, int nrhs) {
   const int t = blockIdx.x * WPC + (threadIdx.x >> 5);
+  pdl_trigger();
+  pdl_wait();
   if (t >= count) return;
   const unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31;
@@ -342,6 +356,7 @@ __global__ void __launch_bounds__(ST) k_bwd_warp(DevSym S, const int *list, int 
 
 __global__ void __launch_bounds__(ST) k_bwd_small(DevSym S, const int *list, double *x, int n, int nrhs) {
   extern __shared__ double P[];
+  pdl_trigger();
   const int s = list[blockIdx.x];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int f = S.super[s], w = S.super[s + 1] - f;
@@ -350,6 +365,7 @@ __global__ void __launch_bounds__(ST) k_bwd_small(DevSym S, const int *list, dou
   const int *rows = S.Ls + rb;
   double *v = P + m * w, *xg = v + w;
   stage_panel(P, S.L + S.xptr[s], m * w);
+  pdl_wait();
   for (int rhs = 0; rhs < nrhs; ++rhs) {
     double *xr = x + (size_t)rhs * n;
     for (int a = w + tid; a < m; a += ST) xg[a - w] = xr[rows[a]];
@@ -492,6 +508,7 @@ __global__ void __launch_bounds__(ST, NS == CHAIN_NS_SMALL ? 2 : 1) k_fwd_chain(
   extern __shared__ double csm[];
   __shared__ double vs[TB], part[CHAIN_WARPS][TB];
   __shared__ ChainCluster cc;
+  pdl_trigger();
   cluster_bars_init(cc.bar, CHAIN_CL, TB * 8);
   const int me = (int)chain_rank();
   if ((int)blockIdx.x < count) {
@@ -532,6 +549,7 @@ __global__ void __launch_bounds__(ST, NS == CHAIN_NS_SMALL ? 2 : 1) k_fwd_chain(
       tr[i][0] = T[(size_t)lane * TB + w8 + i];
       tr[i][1] = T[(size_t)(lane + 32) * TB + w8 + i];
     }
+    pdl_wait();
     // right-hand side minus the descendants' contributions (read after the last barrier)
     {
       static_assert(ST == 4 * TB, "four threads per column");
@@ -618,6 +636,7 @@ __global__ void __launch_bounds__(ST, NS == CHAIN_NS_SMALL ? 2 : 1) k_bwd_chain(
   extern __shared__ double csm[];
   __shared__ double vs[TB];
   __shared__ ChainCluster cc;
+  pdl_trigger();
   cluster_bars_init(cc.bar, CHAIN_CL, TB * 8);
   const int me = (int)chain_rank();
   if ((int)blockIdx.x < count) {
@@ -660,6 +679,7 @@ __global__ void __launch_bounds__(ST, NS == CHAIN_NS_SMALL ? 2 : 1) k_bwd_chain(
       tr[i][0] = T[(size_t)(w8 + i) * TB + lane];
       tr[i][1] = T[(size_t)(w8 + i) * TB + lane + 32];
     }
+    pdl_wait();
     double v = (row < bw) ? x[f + r0 + row] : 0.0;
     bool ok = true;
     int xb0 = nb, nbt = 0;               // the batch in xw: blocks xb0, .., xb0 - nbt + 1
@@ -885,75 +905,57 @@ bool solve_configure(int max_w, std::string &err) {
 
 void launch_fwd_small(const DevSym &S, const int *list, int count, int smem, double *y,
                       double *contrib, const int *cptr, const int *cidx, int n, int nrhs,
-                     int64_t cstride, cudaStream_t st) {
+                      int64_t cstride, SolveQueue &st) {
   if (count > 0)
-    k_fwd_small<<<count, ST, smem, st>>>(S, list, y, contrib, cptr, cidx, n, nrhs, cstride);
+    launch_solve(st, 1, k_fwd_small, count, ST, smem, S, list, y, contrib, cptr, cidx, n, nrhs, cstride);
 }
 void launch_fwd_contrib(const DevSym &S, const int2 *tasks, int count, int nbig, const double *y,
-                        double *contrib, int n, int nrhs, int64_t cstride, cudaStream_t st) {
-  if (count > 0) k_fwd_contrib<<<count, CT, 0, st>>>(S, tasks, nbig, y, contrib, n, nrhs, cstride);
+                        double *contrib, int n, int nrhs, int64_t cstride, SolveQueue &st) {
+  if (count > 0)
+    launch_solve(st, 1, k_fwd_contrib, count, CT, 0, S, tasks, nbig, y, contrib, n, nrhs, cstride);
 }
 void launch_fwd_warp(const DevSym &S, const int *list, int count, double *y, double *contrib,
                      const int *cptr, const int *cidx, int n, int nrhs, int64_t cstride,
-                     cudaStream_t st) {
+                     SolveQueue &st) {
   if (count > 0)
-    k_fwd_warp<<<(count + WPC - 1) / WPC, ST, 0, st>>>(S, list, count, y, contrib, cptr, cidx, n,
-                                                       nrhs, cstride);
+    launch_solve(st, 1, k_fwd_warp, (count + WPC - 1) / WPC, ST, 0, S, list, count, y, contrib, cptr, cidx,
+                 n, nrhs, cstride);
 }
 void launch_bwd_warp(const DevSym &S, const int *list, int count, double *x, int n, int nrhs,
-                     cudaStream_t st) {
-  if (count > 0) k_bwd_warp<<<(count + WPC - 1) / WPC, ST, 0, st>>>(S, list, count, x, n, nrhs);
+                     SolveQueue &st) {
+  if (count > 0)
+    launch_solve(st, 1, k_bwd_warp, (count + WPC - 1) / WPC, ST, 0, S, list, count, x, n, nrhs);
 }
 void launch_bwd_gather(const DevSym &S, const int2 *tasks, int count, double *x, int n, int nrhs,
-                       cudaStream_t st) {
-  if (count > 0) k_bwd_gather<<<count, GT, 0, st>>>(S, tasks, x, n, nrhs);
+                       SolveQueue &st) {
+  if (count > 0) launch_solve(st, 1, k_bwd_gather, count, GT, 0, S, tasks, x, n, nrhs);
 }
 void launch_bwd_small(const DevSym &S, const int *list, int count, int smem, double *x, int n,
-                     int nrhs, cudaStream_t st) {
-  if (count > 0) k_bwd_small<<<count, ST, smem, st>>>(S, list, x, n, nrhs);
-}
-// the chains' launch configuration: a grid of whole clusters of CHAIN_CL CTAs
-static cudaLaunchConfig_t chain_config(int count, int smem, cudaStream_t st,
-                                       cudaLaunchAttribute *at) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)chain_grid(count));
-  cfg.blockDim = dim3(ST);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = CHAIN_CL;
-  at[0].val.clusterDim.y = 1;
-  at[0].val.clusterDim.z = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = 1;
-  return cfg;
+                      int nrhs, SolveQueue &st) {
+  if (count > 0) launch_solve(st, 1, k_bwd_small, count, ST, smem, S, list, x, n, nrhs);
 }
 void launch_fwd_chain(const DevSym &S, const int2 *tasks, int count, double *y,
                       const double *contrib, const int *cptr, const int *cidx, int *flags,
-                      int epoch, int n, int64_t cstride, cudaStream_t st) {
+                      int epoch, int n, int64_t cstride, SolveQueue &st) {
   if (count <= 0) return;
-  cudaLaunchAttribute at[1];
-  if (chain_grid(count) <= g_num_sms) {
-    const cudaLaunchConfig_t cfg = chain_config(count, chain_smem(CHAIN_NS_BIG, CHAIN_XW_FWD), st, at);
-    cudaLaunchKernelEx(&cfg, k_fwd_chain<CHAIN_NS_BIG>, S, tasks, count, y, contrib, cptr, cidx,
-                       flags, epoch, n, cstride);
-  } else {
-    const cudaLaunchConfig_t cfg = chain_config(count, chain_smem(CHAIN_NS_SMALL, CHAIN_XW_FWD), st, at);
-    cudaLaunchKernelEx(&cfg, k_fwd_chain<CHAIN_NS_SMALL>, S, tasks, count, y, contrib, cptr, cidx,
-                       flags, epoch, n, cstride);
-  }
+  const int grid = chain_grid(count);
+  if (grid <= g_num_sms)
+    launch_solve(st, CHAIN_CL, k_fwd_chain<CHAIN_NS_BIG>, grid, ST, chain_smem(CHAIN_NS_BIG, CHAIN_XW_FWD), S,
+                 tasks, count, y, contrib, cptr, cidx, flags, epoch, n, cstride);
+  else
+    launch_solve(st, CHAIN_CL, k_fwd_chain<CHAIN_NS_SMALL>, grid, ST, chain_smem(CHAIN_NS_SMALL, CHAIN_XW_FWD), S,
+                 tasks, count, y, contrib, cptr, cidx, flags, epoch, n, cstride);
 }
 void launch_bwd_chain(const DevSym &S, const int2 *tasks, int count, double *x, int *flags,
-                      int epoch, cudaStream_t st) {
+                      int epoch, SolveQueue &st) {
   if (count <= 0) return;
-  cudaLaunchAttribute at[1];
-  if (chain_grid(count) <= g_num_sms) {
-    const cudaLaunchConfig_t cfg = chain_config(count, chain_smem(CHAIN_NS_BIG, CHAIN_XW_BWD), st, at);
-    cudaLaunchKernelEx(&cfg, k_bwd_chain<CHAIN_NS_BIG>, S, tasks, count, x, flags, epoch);
-  } else {
-    const cudaLaunchConfig_t cfg = chain_config(count, chain_smem(CHAIN_NS_SMALL, CHAIN_XW_BWD), st, at);
-    cudaLaunchKernelEx(&cfg, k_bwd_chain<CHAIN_NS_SMALL>, S, tasks, count, x, flags, epoch);
-  }
+  const int grid = chain_grid(count);
+  if (grid <= g_num_sms)
+    launch_solve(st, CHAIN_CL, k_bwd_chain<CHAIN_NS_BIG>, grid, ST, chain_smem(CHAIN_NS_BIG, CHAIN_XW_BWD), S,
+                 tasks, count, x, flags, epoch);
+  else
+    launch_solve(st, CHAIN_CL, k_bwd_chain<CHAIN_NS_SMALL>, grid, ST, chain_smem(CHAIN_NS_SMALL, CHAIN_XW_BWD), S,
+                 tasks, count, x, flags, epoch);
 }
 void launch_spmv(int n, const int *rp, const int *ci, const double *val, const double *x,
                  double *y, int nrhs, cudaStream_t st) {

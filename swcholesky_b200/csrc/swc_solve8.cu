@@ -30,14 +30,16 @@ constexpr int NT8 = 256, W8 = NT8 / 32;
 // v - sum of the contributions listed for column j, right-hand side r.
 __device__ __forceinline__ double take_contribs(const double *c8, const int *cptr, const int *cidx,
                                                 int j, int r, double v) {
-  int q = cptr[j];
   const int q1 = cptr[j + 1];
-  for (; q + 3 < q1; q += 4) {
-    const double a = c8[(size_t)cidx[q] * R8 + r], b = c8[(size_t)cidx[q + 1] * R8 + r];
-    const double c = c8[(size_t)cidx[q + 2] * R8 + r], d = c8[(size_t)cidx[q + 3] * R8 + r];
-    v -= (a + b) + (c + d);
+  for (int q = cptr[j]; q < q1; q += 4) {
+    int at[4];
+    double t[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) at[u] = cidx[min(q + u, q1 - 1)];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) t[u] = ld_if(c8 + (size_t)at[u] * R8 + r, q + u < q1);
+    v -= (t[0] + t[1]) + (t[2] + t[3]);
   }
-  for (; q < q1; ++q) v -= c8[(size_t)cidx[q] * R8 + r];
   return v;
 }
 
@@ -50,17 +52,15 @@ __device__ __forceinline__ void contrib_rows8(const double *Ls, int m, int w, in
   const bool in = a < m;
   const double *col = Ls + (in ? a : 0);
   double c0[2] = {0.0, 0.0}, c1[2] = {0.0, 0.0};
-  int k = 0;
-  for (; k + 8 <= w; k += 8) {
-    const double l0 = in ? col[(size_t)(k + kq) * m] : 0.0;
-    const double l1 = in ? col[(size_t)(k + 4 + kq) * m] : 0.0;
-    dmma(c0, l0, v[(k + kq) * R8 + g]);
-    dmma(c1, l1, v[(k + 4 + kq) * R8 + g]);
-  }
-  for (; k < w; k += 4) {
-    const bool kin = k + kq < w;
-    const double l = in && kin ? col[(size_t)(k + kq) * m] : 0.0;
-    dmma(c0, l, kin ? v[(k + kq) * R8 + g] : 0.0);
+  for (int k = 0; k < w; k += 16) {
+    double l[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) l[u] = ld_if(col + (size_t)(k + 4 * u + kq) * m, in && k + 4 * u + kq < w);
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int c = k + 4 * u + kq;
+      if (k + 4 * u < w) dmma(u & 1 ? c1 : c0, l[u], c < w ? v[c * R8 + g] : 0.0);
+    }
   }
   if (in)
     *reinterpret_cast<double2 *>(out + (size_t)(a - w) * R8 + 2 * kq) =
@@ -84,6 +84,7 @@ __device__ __forceinline__ void stage_block(double *Ld, const double *Ls, int m,
 __global__ void __launch_bounds__(NT8) k_fwd_small8(DevSym S, const int *list, double *y8, double *c8,
                                                     const int *cptr, const int *cidx) {
   extern __shared__ double sm8[];
+  pdl_trigger();
   double *Ld = sm8, *v = sm8 + SMALL_MAX_W * LDW;   // v[column][rhs]
   const int s = list[blockIdx.x];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -92,6 +93,7 @@ __global__ void __launch_bounds__(NT8) k_fwd_small8(DevSym S, const int *list, d
   const int m = (int)(S.rowptr[s + 1] - rb);
   const double *Ls = S.L + S.xptr[s];
   stage_block(Ld, Ls, m, w);
+  pdl_wait();
   for (int e = tid; e < w * R8; e += NT8)
     v[e] = take_contribs(c8, cptr, cidx, f + (e >> 3), e & 7, y8[(size_t)f * R8 + e]);
   __syncthreads();
@@ -122,6 +124,7 @@ __global__ void __launch_bounds__(NT8) k_fwd_small8(DevSym S, const int *list, d
 
 __global__ void __launch_bounds__(NT8) k_bwd_small8(DevSym S, const int *list, double *x8) {
   extern __shared__ double sm8[];
+  pdl_trigger();
   double *Ld = sm8, *v = sm8 + SMALL_MAX_W * LDW;
   const int s = list[blockIdx.x];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, kq = lane & 3;
@@ -133,16 +136,20 @@ __global__ void __launch_bounds__(NT8) k_bwd_small8(DevSym S, const int *list, d
   // sum over the rows below of L(a, j) x[rows[a]]: warps take four rows at a time, eight
   // columns per product
   const int nt = (w + 7) >> 3;
+  pdl_wait();
   double c[SMALL_MAX_W / 8][2];
 #pragma unroll
   for (int i = 0; i < SMALL_MAX_W / 8; ++i) c[i][0] = c[i][1] = 0.0;
   for (int a0 = w + 4 * warp; a0 < m; a0 += 4 * W8) {
     const int a = a0 + kq;
     const bool in = a < m;
-    const double b = in ? x8[(size_t)rows[a] * R8 + g] : 0.0;
+    double l[SMALL_MAX_W / 8];
+#pragma unroll
+    for (int i = 0; i < SMALL_MAX_W / 8; ++i) l[i] = ld_if(Ls + (size_t)(8 * i + g) * m + a, in && 8 * i + g < w);
+    const double b = ld_if(x8 + (size_t)rows[in ? a : 0] * R8 + g, in);
 #pragma unroll
     for (int i = 0; i < SMALL_MAX_W / 8; ++i)
-      if (i < nt) dmma(c[i], in && 8 * i + g < w ? Ls[(size_t)(8 * i + g) * m + a] : 0.0, b);
+      if (i < nt) dmma(c[i], l[i], b);
   }
   double *part = sm8;   // [warp][column][rhs], before the diagonal block is staged
 #pragma unroll
@@ -199,6 +206,8 @@ __global__ void __launch_bounds__(WN * 32) k_fwd_warp8(DevSym S, const int *list
                                                        double *c8, const int *cptr, const int *cidx) {
   __shared__ Warp8 sm[WN];
   const int t = blockIdx.x * WN + (threadIdx.x >> 5);
+  pdl_trigger();
+  pdl_wait();
   if (t >= count) return;
   Warp8 &M = sm[threadIdx.x >> 5];
   const int lane = threadIdx.x & 31, r = lane & 7, q = lane >> 3;
@@ -248,6 +257,8 @@ __global__ void __launch_bounds__(WN * 32) k_fwd_warp8(DevSym S, const int *list
 __global__ void __launch_bounds__(WN * 32) k_bwd_warp8(DevSym S, const int *list, int count, double *x8) {
   __shared__ Warp8 sm[WN];
   const int t = blockIdx.x * WN + (threadIdx.x >> 5);
+  pdl_trigger();
+  pdl_wait();
   if (t >= count) return;
   Warp8 &M = sm[threadIdx.x >> 5];
   const int lane = threadIdx.x & 31, r = lane & 7, q = lane >> 3, g = lane >> 2, kq = lane & 3;
@@ -266,10 +277,13 @@ __global__ void __launch_bounds__(WN * 32) k_bwd_warp8(DevSym S, const int *list
   for (int a0 = w; a0 < m; a0 += 4) {
     const int a = a0 + kq;
     const bool in = a < m;
-    const double b = in ? x8[(size_t)rows[a] * R8 + g] : 0.0;
+    double l[SOLVE_WARP_W / 8];
+#pragma unroll
+    for (int i = 0; i < SOLVE_WARP_W / 8; ++i) l[i] = ld_if(Ls + (size_t)(8 * i + g) * m + a, in && 8 * i + g < w);
+    const double b = ld_if(x8 + (size_t)rows[in ? a : 0] * R8 + g, in);
 #pragma unroll
     for (int i = 0; i < SOLVE_WARP_W / 8; ++i)
-      if (i < nt) dmma(c[i], in && 8 * i + g < w ? Ls[(size_t)(8 * i + g) * m + a] : 0.0, b);
+      if (i < nt) dmma(c[i], l[i], b);
   }
 #pragma unroll
   for (int i = 0; i < SOLVE_WARP_W / 8; ++i)
@@ -316,6 +330,8 @@ __global__ void __launch_bounds__(NT8) k_contrib8(DevSym S, const int2 *tasks, c
   const int f = S.super[s], w = S.super[s + 1] - f;
   const int64_t rb = S.rowptr[s];
   const int m = (int)(S.rowptr[s + 1] - rb);
+  pdl_trigger();
+  pdl_wait();
   if (a0 >= m) return;
   const double *Ls = S.L + S.xptr[s];
   const double *yv = y8 + (size_t)f * R8 + g;
@@ -351,9 +367,10 @@ __global__ void __launch_bounds__(NT8) k_contrib8(DevSym S, const int2 *tasks, c
 }
 
 constexpr int CS_W = 16;   // warps of the column-split kernel
-__global__ void __launch_bounds__(CS_W * 32) k_contrib8_split(DevSym S, const int2 *tasks,
+__global__ void __launch_bounds__(CS_W * 32, 1) k_contrib8_split(DevSym S, const int2 *tasks,
                                                               const double *y8, double *c8) {
   __shared__ __align__(16) double part[CS_W][32 * R8];
+  pdl_trigger();
   const int s = tasks[blockIdx.x].x, a0 = tasks[blockIdx.x].y;
   const int lane = threadIdx.x & 31, wq = threadIdx.x >> 5, g = lane >> 2, kq = lane & 3;
   const int f = S.super[s], w = S.super[s + 1] - f;
@@ -367,18 +384,19 @@ __global__ void __launch_bounds__(CS_W * 32) k_contrib8_split(DevSym S, const in
   double c[4][2];
 #pragma unroll
   for (int i = 0; i < 4; ++i) c[i][0] = c[i][1] = 0.0;
-  for (int k = 8 * wq; k < w; k += 8 * CS_W) {
-    double l[2][4], b[2];
+  bool first = true;
+  for (int k = 16 * wq; k < w || first; k += 16 * CS_W) {
+    double l[4][4], b[4];
 #pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      const bool kin = k + 4 * u + kq < w;
-      const size_t col = (size_t)(kin ? k + 4 * u + kq : 0);
-      b[u] = kin ? yv[col * R8] : 0.0;
+    for (int u = 0; u < 4; ++u)
 #pragma unroll
-      for (int i = 0; i < 4; ++i) l[u][i] = kin ? p[i][col * m] : 0.0;
-    }
+      for (int i = 0; i < 4; ++i) l[u][i] = ld_if(p[i] + (size_t)(k + 4 * u + kq) * m, k + 4 * u + kq < w);
+    if (first) pdl_wait();
+    first = false;
 #pragma unroll
-    for (int u = 0; u < 2; ++u)
+    for (int u = 0; u < 4; ++u) b[u] = ld_if(yv + (size_t)(k + 4 * u + kq) * R8, k + 4 * u + kq < w);
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
 #pragma unroll
       for (int i = 0; i < 4; ++i) dmma(c[i], l[u][i], b[u]);
   }
@@ -396,9 +414,13 @@ __global__ void __launch_bounds__(CS_W * 32) k_contrib8_split(DevSym S, const in
 }
 
 // ---- gathers of tiled supernodes: x[cols j0 .. j0 + 15] -= L(rows below, cols)^T x[rows];
-// warps take sixteen rows at a time, partial sums in shared memory.
-__global__ void __launch_bounds__(NT8) k_gather8(DevSym S, const int2 *tasks, double *x8) {
-  __shared__ __align__(16) double part[W8][SOLVE_GATHER_COLS * R8];
+// warps take 32 rows at a time, partial sums in shared memory.  As with the column-split
+// contributions above, the top levels have one CTA per SM and the bytes in flight set the rate:
+// sixteen predicated loads of L per lane and sixteen warps, 64 KB.
+constexpr int G8_W = 16;
+__global__ void __launch_bounds__(G8_W * 32, 1) k_gather8(DevSym S, const int2 *tasks, double *x8) {
+  __shared__ __align__(16) double part[G8_W][SOLVE_GATHER_COLS * R8];
+  pdl_trigger();
   static_assert(SOLVE_GATHER_COLS == 16, "two products per four rows");
   const int s = tasks[blockIdx.x].x, j0 = tasks[blockIdx.x].y;
   const int lane = threadIdx.x & 31, wq = threadIdx.x >> 5, g = lane >> 2, kq = lane & 3;
@@ -413,18 +435,23 @@ __global__ void __launch_bounds__(NT8) k_gather8(DevSym S, const int2 *tasks, do
   for (int i = 0; i < 2; ++i)
 #pragma unroll
     for (int h = 0; h < 2; ++h) c[i][h][0] = c[i][h][1] = 0.0;
-  for (int a0 = w + 16 * wq; a0 < m; a0 += 16 * W8) {
-    double l0[4], l1[4], b[4];
+  bool first = true;
+  for (int a0 = w + 32 * wq; a0 < m || first; a0 += 32 * G8_W) {
+    double l0[8], l1[8], b[8];
+    int row[8];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
+    for (int u = 0; u < 8; ++u) {
       const int a = a0 + 4 * u + kq;
-      const bool in = a < m;
-      b[u] = in ? x8[(size_t)rows[a] * R8 + g] : 0.0;
-      l0[u] = in ? p0[a] : 0.0;
-      l1[u] = in ? p1[a] : 0.0;
+      row[u] = rows[min(a, m - 1)];
+      l0[u] = ld_if(p0 + a, a < m);
+      l1[u] = ld_if(p1 + a, a < m);
     }
+    if (first) pdl_wait();
+    first = false;
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
+    for (int u = 0; u < 8; ++u) b[u] = ld_if(x8 + (size_t)row[u] * R8 + g, a0 + 4 * u + kq < m);
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
       dmma(c[0][u & 1], l0[u], b[u]);
       dmma(c[1][u & 1], l1[u], b[u]);
     }
@@ -438,7 +465,7 @@ __global__ void __launch_bounds__(NT8) k_gather8(DevSym S, const int2 *tasks, do
   if (e < SOLVE_GATHER_COLS * R8 && j0 + (e >> 3) < w) {
     double t = 0.0;
 #pragma unroll
-    for (int q = 0; q < W8; ++q) t += part[q][e];
+    for (int q = 0; q < G8_W; ++q) t += part[q][e];
     x8[(size_t)(f + j0) * R8 + e] -= t;
   }
 }
@@ -495,6 +522,7 @@ __global__ void __launch_bounds__(NT8, 1) k_fwd_chain8(DevSym S, const int2 *tas
   extern __shared__ double sm8[];
   __shared__ unsigned long long bar[CL];
   double *yin = sm8 + NS8 * W8 * SLOT8 + W8 * XB8 * 8 * R8, *vs = yin + CL * BLK8;
+  pdl_trigger();
   cluster_bars_init(bar, CL, BLK8 * 8);
   const int me = (int)chain_rank();
   if ((int)blockIdx.x < count) {
@@ -526,6 +554,7 @@ __global__ void __launch_bounds__(NT8, 1) k_fwd_chain8(DevSym S, const int2 *tas
     double tr[16];
 #pragma unroll
     for (int t = 0; t < 16; ++t) tr[t] = T[(4 * t + kq) * TB + w8 + g];
+    pdl_wait();
     // right-hand sides minus the descendants' contributions
 #pragma unroll
     for (int h = 0; h < BLK8 / NT8; ++h) {
@@ -604,6 +633,7 @@ __global__ void __launch_bounds__(NT8, 1) k_bwd_chain8(DevSym S, const int2 *tas
   extern __shared__ double sm8[];
   __shared__ unsigned long long bar[CL];
   double *yin = sm8 + NS8 * W8 * SLOT8 + W8 * XB8 * 8 * R8, *vs = yin + CL * BLK8;
+  pdl_trigger();
   cluster_bars_init(bar, CL, BLK8 * 8);
   const int me = (int)chain_rank();
   if ((int)blockIdx.x < count) {
@@ -636,6 +666,7 @@ __global__ void __launch_bounds__(NT8, 1) k_bwd_chain8(DevSym S, const int2 *tas
     double tr[16];   // T^T(8 wp + g, 4 t + kq)
 #pragma unroll
     for (int t = 0; t < 16; ++t) tr[t] = T[(w8 + g) * TB + 4 * t + kq];
+    pdl_wait();
     double acc[4][2];
 #pragma unroll
     for (int i = 0; i < 4; ++i) acc[i][0] = acc[i][1] = 0.0;
@@ -725,49 +756,38 @@ void launch_unpack8(int n, int nr, const double *x8, double *x, cudaStream_t st)
 }
 
 void launch_solve8(const DevSym &S, const SolvePlan &SP, const Solve8Dev &D, double *x8, double *c8,
-                   cudaStream_t st) {
-  const int nl = (int)SP.level_off.size() - 1;
-  auto chain = [&](bool fwd, int off, int cnt) {
+                   int l0, int l1, bool fwd, SolveQueue &st) {
+  auto chain = [&](int off, int cnt) {
+    const int grid = (cnt + CL - 1) / CL * CL;
     if (cnt <= 0) return;
-    cudaLaunchConfig_t cfg = {};
-    cudaLaunchAttribute at[1];
-    cfg.gridDim = dim3((unsigned)((cnt + CL - 1) / CL * CL));
-    cfg.blockDim = dim3(NT8);
-    cfg.dynamicSmemBytes = CHAIN8_SMEM;
-    cfg.stream = st;
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = CL;
-    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
     if (fwd)
-      cudaLaunchKernelEx(&cfg, k_fwd_chain8, S, D.fchain + off, cnt, x8, (const double *)c8, D.cptr, D.cidx,
-                         D.flags);
+      launch_solve(st, CL, k_fwd_chain8, grid, NT8, CHAIN8_SMEM, S, D.fchain + off, cnt, x8, c8, D.cptr, D.cidx,
+                   D.flags);
     else
-      cudaLaunchKernelEx(&cfg, k_bwd_chain8, S, D.bchain + off, cnt, x8, D.flags);
+      launch_solve(st, CL, k_bwd_chain8, grid, NT8, CHAIN8_SMEM, S, D.bchain + off, cnt, x8, D.flags);
   };
-  for (int l = 0; l < nl; ++l) {
+  for (int l = l0; fwd && l < l1; ++l) {
     const int nw = SP.warp_off[l + 1] - SP.warp_off[l], ns = SP.level_off[l + 1] - SP.level_off[l];
     const int nc = SP.c8_off[l + 1] - SP.c8_off[l];
     if (nw > 0)
-      k_fwd_warp8<<<(nw + WN - 1) / WN, WN * 32, 0, st>>>(S, D.warp_list + SP.warp_off[l], nw, x8, c8,
-                                                          D.cptr, D.cidx);
+      launch_solve(st, 1, k_fwd_warp8, (nw + WN - 1) / WN, WN * 32, 0, S, D.warp_list + SP.warp_off[l], nw, x8,
+                   c8, D.cptr, D.cidx);
     if (ns > 0)
-      k_fwd_small8<<<ns, NT8, SMALL8_SMEM, st>>>(S, D.list + SP.level_off[l], x8, c8, D.cptr, D.cidx);
-    chain(true, SP.chain_off[l], SP.chain_off[l + 1] - SP.chain_off[l]);
+      launch_solve(st, 1, k_fwd_small8, ns, NT8, SMALL8_SMEM, S, D.list + SP.level_off[l], x8, c8, D.cptr, D.cidx);
+    chain(SP.chain_off[l], SP.chain_off[l + 1] - SP.chain_off[l]);
     if (nc > 0 && SP.c8_split[l])
-      k_contrib8_split<<<nc, CS_W * 32, 0, st>>>(S, D.c8_tasks + SP.c8_off[l], x8, c8);
+      launch_solve(st, 1, k_contrib8_split, nc, CS_W * 32, 0, S, D.c8_tasks + SP.c8_off[l], x8, c8);
     else if (nc > 0)
-      k_contrib8<<<nc, NT8, 0, st>>>(S, D.c8_tasks + SP.c8_off[l], x8, c8);
+      launch_solve(st, 1, k_contrib8, nc, NT8, 0, S, D.c8_tasks + SP.c8_off[l], x8, c8);
   }
-  for (int l = nl - 1; l >= 0; --l) {
+  for (int l = l1 - 1; !fwd && l >= l0; --l) {
     const int nw = SP.warp_off[l + 1] - SP.warp_off[l], ns = SP.level_off[l + 1] - SP.level_off[l];
     const int ng = SP.g8_off[l + 1] - SP.g8_off[l];
-    if (ng > 0) k_gather8<<<ng, NT8, 0, st>>>(S, D.g8_tasks + SP.g8_off[l], x8);
-    chain(false, SP.chain_off[l], SP.chain_off[l + 1] - SP.chain_off[l]);
-    if (ns > 0) k_bwd_small8<<<ns, NT8, SMALL8_SMEM, st>>>(S, D.list + SP.level_off[l], x8);
+    if (ng > 0) launch_solve(st, 1, k_gather8, ng, G8_W * 32, 0, S, D.g8_tasks + SP.g8_off[l], x8);
+    chain(SP.chain_off[l], SP.chain_off[l + 1] - SP.chain_off[l]);
+    if (ns > 0) launch_solve(st, 1, k_bwd_small8, ns, NT8, SMALL8_SMEM, S, D.list + SP.level_off[l], x8);
     if (nw > 0)
-      k_bwd_warp8<<<(nw + WN - 1) / WN, WN * 32, 0, st>>>(S, D.warp_list + SP.warp_off[l], nw, x8);
+      launch_solve(st, 1, k_bwd_warp8, (nw + WN - 1) / WN, WN * 32, 0, S, D.warp_list + SP.warp_off[l], nw, x8);
   }
 }
 
