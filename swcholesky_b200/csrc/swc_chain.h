@@ -55,16 +55,6 @@ __device__ __forceinline__ void cp8(double *dst, const double *src, bool in) {
                "l"(src), "r"(in ? 8 : 0));
 }
 
-// The solves' kernels follow each other by programmatic launches: a kernel's CTAs start while the
-// one before still runs and ask for their parts of L, which no solve changes; pdl_wait, before
-// anything else is read or written, waits until that one (and so all before it, every kernel
-// having waited itself) has finished.  The trigger stands first in every kernel: the waiting CTAs
-// take only what the running kernel's CTAs, all started by then, leave free.  With this and the
-// predicated loads a solve of the 301 x 287 grid with eight right-hand sides went from 435 to
-// 370 us, one of the 60^3 grid with one from 1158 to 1124 us (B200).
-__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;\n" ::); }
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
-
 __device__ __forceinline__ uint32_t chain_rank() {
   uint32_t r;
   asm volatile("mov.u32 %0, %%cluster_ctarank;\n" : "=r"(r));

@@ -2159,7 +2159,7 @@ void Engine::run_solve8(double *x8) {
   cudaMemsetAsync(d_flags_, 0, sizeof(int) * std::max<int64_t>(nflags_, 1), stream_);
   const Solve8Dev D{d_slist_, d_swarp_, d_cptr_, d_cidx_, d_fchain_, d_bchain_, d_c8_tasks_,
                     d_g8_tasks_, d_flags_};
-  run_halves([&](int l0, int l1, bool fwd, SolveQueue &st) {
+  run_halves([&](int l0, int l1, bool fwd, LaunchQueue &st) {
     launch_solve8(sym_, splan_, D, x8, d_c8_, l0, l1, fwd, st);
   });
 }
@@ -2171,7 +2171,7 @@ void Engine::run_solve8(double *x8) {
 template <class F>
 void Engine::run_halves(F levels) {
   const int h0 = splan_.half0, h1 = splan_.half1, nl = (int)splan_.level_off.size() - 1;
-  SolveQueue main{stream_, false}, aux{aux_stream_, false};
+  LaunchQueue main{stream_, false}, aux{aux_stream_, false};
   for (int pass = 0; pass < 2; ++pass) {
     const bool fwd = pass == 0;
     if (!fwd) levels(h1, nl, false, main);
@@ -2227,12 +2227,12 @@ void Engine::run_solve(double *x, int nrhs) {
 // sequence can be replayed.
 void Engine::run_solve_with(double *x, int nrhs, double *contrib) {
   cudaMemsetAsync(d_flags_, 0, sizeof(int) * std::max<int64_t>(nflags_, 1), stream_);
-  run_halves([&](int l0, int l1, bool fwd, SolveQueue &st) {
+  run_halves([&](int l0, int l1, bool fwd, LaunchQueue &st) {
     solve_levels(x, nrhs, contrib, l0, l1, fwd, st);
   });
 }
 
-void Engine::solve_levels(double *x, int nrhs, double *contrib, int l0, int l1, bool fwd, SolveQueue &st) {
+void Engine::solve_levels(double *x, int nrhs, double *contrib, int l0, int l1, bool fwd, LaunchQueue &st) {
   const SolvePlan &SP = splan_;
   const int64_t cs = std::max<int64_t>(SP.contrib_len, 1);
   for (int l = l0; fwd && l < l1; ++l) {

@@ -199,14 +199,15 @@ struct Plan {
 
 
 // Triangular solves and refinement (swc_solve.cu)
-// Where a solve's kernels go.  chained: the last operation of the stream is one of them, so that
-// the next may start before it ends (programmatic dependent launch).
-struct SolveQueue {
+// Where a sequence of kernels goes.  chained: the last operation of the stream is one of them, so
+// that the next may start before it ends (programmatic dependent launch); such a kernel calls
+// pdl_wait before it touches anything an earlier one writes.
+struct LaunchQueue {
   cudaStream_t st;
   bool chained;
 };
 template <class... P, class... A>
-void launch_solve(SolveQueue &q, int cluster, void (*kernel)(P...), int grid, int block, int smem, A... args) {
+void launch_early(LaunchQueue &q, int cluster, void (*kernel)(P...), int grid, int block, int smem, A... args) {
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute at[2];
   cfg.gridDim = dim3((unsigned)grid);
@@ -232,25 +233,25 @@ void launch_solve(SolveQueue &q, int cluster, void (*kernel)(P...), int grid, in
 bool solve_configure(int max_w, std::string &err);
 void launch_fwd_small(const DevSym &S, const int *list, int count, int smem, double *y,
                       double *contrib, const int *cptr, const int *cidx, int n, int nrhs,
-                     int64_t cstride, SolveQueue &st);
+                     int64_t cstride, LaunchQueue &st);
 void launch_fwd_contrib(const DevSym &S, const int2 *tasks, int count, int nbig, const double *y,
-                        double *contrib, int n, int nrhs, int64_t cstride, SolveQueue &st);
+                        double *contrib, int n, int nrhs, int64_t cstride, LaunchQueue &st);
 void launch_bwd_gather(const DevSym &S, const int2 *tasks, int count, double *x, int n, int nrhs,
-                       SolveQueue &st);
+                       LaunchQueue &st);
 void launch_bwd_small(const DevSym &S, const int *list, int count, int smem, double *x, int n,
-                     int nrhs, SolveQueue &st);
+                     int nrhs, LaunchQueue &st);
 // small supernodes, one warp each: forward (contributions in, diagonal solve, contributions
 // of the rows below out) and backward (gather from ancestors, transposed diagonal solve)
 void launch_fwd_warp(const DevSym &S, const int *list, int count, double *y, double *contrib,
                      const int *cptr, const int *cidx, int n, int nrhs, int64_t cstride,
-                     SolveQueue &st);
+                     LaunchQueue &st);
 void launch_bwd_warp(const DevSym &S, const int *list, int count, double *x, int n, int nrhs,
-                     SolveQueue &st);
+                     LaunchQueue &st);
 void launch_fwd_chain(const DevSym &S, const int2 *tasks, int count, double *y,
                       const double *contrib, const int *cptr, const int *cidx, int *flags,
-                      int epoch, int n, int64_t cstride, SolveQueue &st);
+                      int epoch, int n, int64_t cstride, LaunchQueue &st);
 void launch_bwd_chain(const DevSym &S, const int2 *tasks, int count, double *x, int *flags,
-                      int epoch, SolveQueue &st);
+                      int epoch, LaunchQueue &st);
 void launch_spmv(int n, const int *rp, const int *ci, const double *val, const double *x,
                  double *y, int nrhs, cudaStream_t st);
 void launch_gather_vals(int nnz, const int *map, const double *ax, double *val, cudaStream_t st);
@@ -300,7 +301,7 @@ void launch_pack8(int n, int nr, const double *x, double *x8, cudaStream_t st);
 void launch_unpack8(int n, int nr, const double *x8, double *x, cudaStream_t st);
 // the levels l0 .. l1 - 1, forward or backward
 void launch_solve8(const DevSym &S, const SolvePlan &SP, const Solve8Dev &D, double *x8, double *c8,
-                   int l0, int l1, bool fwd, SolveQueue &st);
+                   int l0, int l1, bool fwd, LaunchQueue &st);
 
 // Result of a refined solve, per right-hand side.
 struct RefineInfo {
@@ -549,7 +550,7 @@ class Engine {
   bool ensure_work(int nrhs, std::string &err);
   void run_solve(double *x, int nrhs);
   void run_solve_with(double *x, int nrhs, double *contrib);
-  void solve_levels(double *x, int nrhs, double *contrib, int l0, int l1, bool fwd, SolveQueue &st);
+  void solve_levels(double *x, int nrhs, double *contrib, int l0, int l1, bool fwd, LaunchQueue &st);
   template <class F> void run_halves(F levels);
   bool solve_status_ok(std::string &err);
 };

@@ -801,12 +801,15 @@ template <bool FOLD>
 __global__ void __launch_bounds__(DIAG_NW * 32) k_diag_step(DevSym S, const int *list, int count,
                                                            int step) {
   extern __shared__ double dyn[];
-  if (FOLD)
+  if (FOLD) {
+    pdl_trigger();
+    pdl_wait();
     factor_diag_block<DIAG_NW, true, true>(S, list[blockIdx.x], step * TB, dyn, nullptr);
-  else if (step > 0)
+  } else if (step > 0) {
     factor_diag_block<DIAG_NW, true>(S, list[blockIdx.x], step * TB, dyn, nullptr);
-  else
+  } else {
     factor_diag_block<DIAG_NW, false>(S, list[blockIdx.x], 0, dyn, nullptr);
+  }
 }
 
 // Mixed modes: the tile below the next diagonal one to its place in dinv, when the atomic
@@ -1153,7 +1156,11 @@ void launch_update_tiles(const DevSym &S, const int4 *tasks, const int *task_end
 }
 void launch_diag_step(const DevSym &S, const int *list, int count, int step, cudaStream_t st, bool fold) {
   if (count <= 0) return;
-  if (fold) k_diag_step<true><<<count, DIAG_NW * 32, diag_prev_smem(DIAG_NW), st>>>(S, list, count, step);
+  // started early: the chain of diagonal blocks sets the time of the smaller waves, and the launch
+  // was 2 us of 22 per block (41 x 37 x 43 grid 2957 -> 2885 us, 24 x 23 x 22 elastic 3063 -> 3008;
+  // with the TRSM and the updates started early too, 2928 and 3032)
+  LaunchQueue q{st, true};
+  if (fold) launch_early(q, 1, k_diag_step<true>, count, DIAG_NW * 32, diag_prev_smem(DIAG_NW), S, list, count, step);
   else k_diag_step<false><<<count, DIAG_NW * 32, diag_prev_smem(DIAG_NW), st>>>(S, list, count, step);
 }
 void launch_copy_tile(const DevSym &S, const int *list, int count, int step, cudaStream_t st) {

@@ -905,56 +905,56 @@ bool solve_configure(int max_w, std::string &err) {
 
 void launch_fwd_small(const DevSym &S, const int *list, int count, int smem, double *y,
                       double *contrib, const int *cptr, const int *cidx, int n, int nrhs,
-                      int64_t cstride, SolveQueue &st) {
+                      int64_t cstride, LaunchQueue &st) {
   if (count > 0)
-    launch_solve(st, 1, k_fwd_small, count, ST, smem, S, list, y, contrib, cptr, cidx, n, nrhs, cstride);
+    launch_early(st, 1, k_fwd_small, count, ST, smem, S, list, y, contrib, cptr, cidx, n, nrhs, cstride);
 }
 void launch_fwd_contrib(const DevSym &S, const int2 *tasks, int count, int nbig, const double *y,
-                        double *contrib, int n, int nrhs, int64_t cstride, SolveQueue &st) {
+                        double *contrib, int n, int nrhs, int64_t cstride, LaunchQueue &st) {
   if (count > 0)
-    launch_solve(st, 1, k_fwd_contrib, count, CT, 0, S, tasks, nbig, y, contrib, n, nrhs, cstride);
+    launch_early(st, 1, k_fwd_contrib, count, CT, 0, S, tasks, nbig, y, contrib, n, nrhs, cstride);
 }
 void launch_fwd_warp(const DevSym &S, const int *list, int count, double *y, double *contrib,
                      const int *cptr, const int *cidx, int n, int nrhs, int64_t cstride,
-                     SolveQueue &st) {
+                     LaunchQueue &st) {
   if (count > 0)
-    launch_solve(st, 1, k_fwd_warp, (count + WPC - 1) / WPC, ST, 0, S, list, count, y, contrib, cptr, cidx,
+    launch_early(st, 1, k_fwd_warp, (count + WPC - 1) / WPC, ST, 0, S, list, count, y, contrib, cptr, cidx,
                  n, nrhs, cstride);
 }
 void launch_bwd_warp(const DevSym &S, const int *list, int count, double *x, int n, int nrhs,
-                     SolveQueue &st) {
+                     LaunchQueue &st) {
   if (count > 0)
-    launch_solve(st, 1, k_bwd_warp, (count + WPC - 1) / WPC, ST, 0, S, list, count, x, n, nrhs);
+    launch_early(st, 1, k_bwd_warp, (count + WPC - 1) / WPC, ST, 0, S, list, count, x, n, nrhs);
 }
 void launch_bwd_gather(const DevSym &S, const int2 *tasks, int count, double *x, int n, int nrhs,
-                       SolveQueue &st) {
-  if (count > 0) launch_solve(st, 1, k_bwd_gather, count, GT, 0, S, tasks, x, n, nrhs);
+                       LaunchQueue &st) {
+  if (count > 0) launch_early(st, 1, k_bwd_gather, count, GT, 0, S, tasks, x, n, nrhs);
 }
 void launch_bwd_small(const DevSym &S, const int *list, int count, int smem, double *x, int n,
-                      int nrhs, SolveQueue &st) {
-  if (count > 0) launch_solve(st, 1, k_bwd_small, count, ST, smem, S, list, x, n, nrhs);
+                      int nrhs, LaunchQueue &st) {
+  if (count > 0) launch_early(st, 1, k_bwd_small, count, ST, smem, S, list, x, n, nrhs);
 }
 void launch_fwd_chain(const DevSym &S, const int2 *tasks, int count, double *y,
                       const double *contrib, const int *cptr, const int *cidx, int *flags,
-                      int epoch, int n, int64_t cstride, SolveQueue &st) {
+                      int epoch, int n, int64_t cstride, LaunchQueue &st) {
   if (count <= 0) return;
   const int grid = chain_grid(count);
   if (grid <= g_num_sms)
-    launch_solve(st, CHAIN_CL, k_fwd_chain<CHAIN_NS_BIG>, grid, ST, chain_smem(CHAIN_NS_BIG, CHAIN_XW_FWD), S,
+    launch_early(st, CHAIN_CL, k_fwd_chain<CHAIN_NS_BIG>, grid, ST, chain_smem(CHAIN_NS_BIG, CHAIN_XW_FWD), S,
                  tasks, count, y, contrib, cptr, cidx, flags, epoch, n, cstride);
   else
-    launch_solve(st, CHAIN_CL, k_fwd_chain<CHAIN_NS_SMALL>, grid, ST, chain_smem(CHAIN_NS_SMALL, CHAIN_XW_FWD), S,
+    launch_early(st, CHAIN_CL, k_fwd_chain<CHAIN_NS_SMALL>, grid, ST, chain_smem(CHAIN_NS_SMALL, CHAIN_XW_FWD), S,
                  tasks, count, y, contrib, cptr, cidx, flags, epoch, n, cstride);
 }
 void launch_bwd_chain(const DevSym &S, const int2 *tasks, int count, double *x, int *flags,
-                      int epoch, SolveQueue &st) {
+                      int epoch, LaunchQueue &st) {
   if (count <= 0) return;
   const int grid = chain_grid(count);
   if (grid <= g_num_sms)
-    launch_solve(st, CHAIN_CL, k_bwd_chain<CHAIN_NS_BIG>, grid, ST, chain_smem(CHAIN_NS_BIG, CHAIN_XW_BWD), S,
+    launch_early(st, CHAIN_CL, k_bwd_chain<CHAIN_NS_BIG>, grid, ST, chain_smem(CHAIN_NS_BIG, CHAIN_XW_BWD), S,
                  tasks, count, x, flags, epoch);
   else
-    launch_solve(st, CHAIN_CL, k_bwd_chain<CHAIN_NS_SMALL>, grid, ST, chain_smem(CHAIN_NS_SMALL, CHAIN_XW_BWD), S,
+    launch_early(st, CHAIN_CL, k_bwd_chain<CHAIN_NS_SMALL>, grid, ST, chain_smem(CHAIN_NS_SMALL, CHAIN_XW_BWD), S,
                  tasks, count, x, flags, epoch);
 }
 void launch_spmv(int n, const int *rp, const int *ci, const double *val, const double *x,

@@ -756,38 +756,38 @@ void launch_unpack8(int n, int nr, const double *x8, double *x, cudaStream_t st)
 }
 
 void launch_solve8(const DevSym &S, const SolvePlan &SP, const Solve8Dev &D, double *x8, double *c8,
-                   int l0, int l1, bool fwd, SolveQueue &st) {
+                   int l0, int l1, bool fwd, LaunchQueue &st) {
   auto chain = [&](int off, int cnt) {
     const int grid = (cnt + CL - 1) / CL * CL;
     if (cnt <= 0) return;
     if (fwd)
-      launch_solve(st, CL, k_fwd_chain8, grid, NT8, CHAIN8_SMEM, S, D.fchain + off, cnt, x8, c8, D.cptr, D.cidx,
+      launch_early(st, CL, k_fwd_chain8, grid, NT8, CHAIN8_SMEM, S, D.fchain + off, cnt, x8, c8, D.cptr, D.cidx,
                    D.flags);
     else
-      launch_solve(st, CL, k_bwd_chain8, grid, NT8, CHAIN8_SMEM, S, D.bchain + off, cnt, x8, D.flags);
+      launch_early(st, CL, k_bwd_chain8, grid, NT8, CHAIN8_SMEM, S, D.bchain + off, cnt, x8, D.flags);
   };
   for (int l = l0; fwd && l < l1; ++l) {
     const int nw = SP.warp_off[l + 1] - SP.warp_off[l], ns = SP.level_off[l + 1] - SP.level_off[l];
     const int nc = SP.c8_off[l + 1] - SP.c8_off[l];
     if (nw > 0)
-      launch_solve(st, 1, k_fwd_warp8, (nw + WN - 1) / WN, WN * 32, 0, S, D.warp_list + SP.warp_off[l], nw, x8,
+      launch_early(st, 1, k_fwd_warp8, (nw + WN - 1) / WN, WN * 32, 0, S, D.warp_list + SP.warp_off[l], nw, x8,
                    c8, D.cptr, D.cidx);
     if (ns > 0)
-      launch_solve(st, 1, k_fwd_small8, ns, NT8, SMALL8_SMEM, S, D.list + SP.level_off[l], x8, c8, D.cptr, D.cidx);
+      launch_early(st, 1, k_fwd_small8, ns, NT8, SMALL8_SMEM, S, D.list + SP.level_off[l], x8, c8, D.cptr, D.cidx);
     chain(SP.chain_off[l], SP.chain_off[l + 1] - SP.chain_off[l]);
     if (nc > 0 && SP.c8_split[l])
-      launch_solve(st, 1, k_contrib8_split, nc, CS_W * 32, 0, S, D.c8_tasks + SP.c8_off[l], x8, c8);
+      launch_early(st, 1, k_contrib8_split, nc, CS_W * 32, 0, S, D.c8_tasks + SP.c8_off[l], x8, c8);
     else if (nc > 0)
-      launch_solve(st, 1, k_contrib8, nc, NT8, 0, S, D.c8_tasks + SP.c8_off[l], x8, c8);
+      launch_early(st, 1, k_contrib8, nc, NT8, 0, S, D.c8_tasks + SP.c8_off[l], x8, c8);
   }
   for (int l = l1 - 1; !fwd && l >= l0; --l) {
     const int nw = SP.warp_off[l + 1] - SP.warp_off[l], ns = SP.level_off[l + 1] - SP.level_off[l];
     const int ng = SP.g8_off[l + 1] - SP.g8_off[l];
-    if (ng > 0) launch_solve(st, 1, k_gather8, ng, G8_W * 32, 0, S, D.g8_tasks + SP.g8_off[l], x8);
+    if (ng > 0) launch_early(st, 1, k_gather8, ng, G8_W * 32, 0, S, D.g8_tasks + SP.g8_off[l], x8);
     chain(SP.chain_off[l], SP.chain_off[l + 1] - SP.chain_off[l]);
-    if (ns > 0) launch_solve(st, 1, k_bwd_small8, ns, NT8, SMALL8_SMEM, S, D.list + SP.level_off[l], x8);
+    if (ns > 0) launch_early(st, 1, k_bwd_small8, ns, NT8, SMALL8_SMEM, S, D.list + SP.level_off[l], x8);
     if (nw > 0)
-      launch_solve(st, 1, k_bwd_warp8, (nw + WN - 1) / WN, WN * 32, 0, S, D.warp_list + SP.warp_off[l], nw, x8);
+      launch_early(st, 1, k_bwd_warp8, (nw + WN - 1) / WN, WN * 32, 0, S, D.warp_list + SP.warp_off[l], nw, x8);
   }
 }
 
