@@ -167,7 +167,7 @@ __device__ void adj_small_body(const DevSym &S, const AdjDev &A, int s, double *
 #pragma unroll
           for (int u = 0; u < 4; ++u) {
             const int k = k0 + 4 * u + kq;
-            a[u] = iin && k < r ? zrow[(size_t)rel[k] * mp] : 0.0;
+            a[u] = ld_if(zrow + (size_t)rel[k < r ? k : 0] * mp, iin && k < r);
           }
 #pragma unroll
           for (int u = 0; u < 4; ++u) {
@@ -279,7 +279,7 @@ __device__ __forceinline__ void load_tinv(double *Ts, const double *ti, int w) {
 #pragma unroll 8
   for (int e = threadIdx.x; e < TB * TB; e += MT) {
     const int c = e >> 6, k = e & (TB - 1);
-    Ts[k * LDS + c] = (k < w && c < w) ? ti[e] : 0.0;
+    Ts[k * LDS + c] = ld_if(ti + e, k < w && c < w);
   }
 }
 
@@ -297,7 +297,7 @@ __global__ void __launch_bounds__(MT) k_adj_u(DevSym S, AdjDev A, const int4 *ta
 #pragma unroll 8
   for (int e = threadIdx.x; e < TB * TB; e += MT) {
     const int k = e >> 6, q = e & (TB - 1);
-    Lx[k * LDS + q] = (q < nrow && k < w) ? Lb[(size_t)k * m + q] : 0.0;
+    Lx[k * LDS + q] = ld_if(Lb + (size_t)k * m + q, q < nrow && k < w);
   }
   __syncthreads();
   TileAcc acc;   // U^T: rows are columns of the block
@@ -339,7 +339,7 @@ __global__ void __launch_bounds__(MT, 3) k_adj_zrk(DevSym S, AdjDev A, const int
 #pragma unroll 8
   for (int e = threadIdx.x; e < TB * TB; e += MT) {
     const int r = e >> 6, c = e & (TB - 1);
-    ux[r * LDS + c] = (r < nrow && c < w) ? UT[(size_t)(x0 + r) * TB + c] : 0.0;
+    ux[r * LDS + c] = ld_if(UT + (size_t)(x0 + r) * TB + c, r < nrow && c < w);
   }
   __syncthreads();
   for (int e = threadIdx.x; e < TB * TB; e += MT) {

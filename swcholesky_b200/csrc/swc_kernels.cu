@@ -507,8 +507,7 @@ __global__ void __launch_bounds__(MT, 4) k_update_tiles(DevSym S, const int4 *ta
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
         const int c = acc_col(j, e);
-        acc.v[i][j][e] = (r < nrow && c < ncol && r0 + r >= c0 + c)
-                             ? neg(P[(size_t)(c0 + c) * m + r0 + r]) : 0.0;
+        acc.v[i][j][e] = neg(ld_if(P + (size_t)(c0 + c) * m + r0 + r, r < nrow && c < ncol && r0 + r >= c0 + c));
       }
   }
   for (int q = p_begin; q < p_end; ++q) {
@@ -618,19 +617,19 @@ __device__ void factor_diag_block(const DevSym &S, int s, int c0, double *smem,
 #pragma unroll
     for (int q = 0; q < 8; ++q) {
       const int e = e0 + q * NTH, c = e >> 6, r = e & (TB - 1);
-      if (c < bw && r < bw) v[q] = (!upd && r >= c) ? P[(size_t)(c0 + c) * m + c0 + r] : 0.0;
-      else v[q] = (r == c) ? 1.0 : 0.0;
+      v[q] = ld_if(P + (size_t)(c0 + c) * m + c0 + r, !upd && c < bw && r < bw && r >= c);
       if (FOLD) {
-        xv[q] = r < nr ? Bg[e] : 0.0;
-        tv[q] = Bg[e - TB * TB];
+        xv[q] = ld_if(Bg + e, r < nr);
+        tv[q] = ld_if(Bg + e - TB * TB, true);
       } else if (PREV) {
-        xv[q] = r < nr ? P[(size_t)(c0 - TB + c) * m + c0 + r] : 0.0;
+        xv[q] = ld_if(P + (size_t)(c0 - TB + c) * m + c0 + r, r < nr);
       }
     }
 #pragma unroll
     for (int q = 0; q < 8; ++q) {
       const int e = e0 + q * NTH;
-      D[(e >> 6) * DLD + (e & (TB - 1))] = v[q];
+      const int c = e >> 6, r = e & (TB - 1);
+      D[c * DLD + r] = r == c && r >= bw ? 1.0 : v[q];
       if (PREV) (FOLD ? Bs : Xs)[(e >> 6) * DLD + (e & (TB - 1))] = xv[q];
       if (FOLD) Ts[(e >> 6) * DLD + (e & (TB - 1))] = tv[q];
     }
@@ -739,6 +738,9 @@ __device__ void syrk_tile_acc(const DevSym &S, int s, int r0, int c0, int kblk, 
   const int k0 = kblk * TB;
   const int bk = min(nblk * TB, w - k0);
   const int nrow = min(TB, m - r0), ncol = min(TB, w - c0);
+  const double *Pa = P + (size_t)k0 * m + r0, *Pb = P + (size_t)k0 * m + c0;
+  tile_sync(0);
+  load_chunk(Pa, m, nrow, Pb, m, ncol, bk, 0, stages, threadIdx.x);
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     const int r = acc_row(i);
@@ -747,12 +749,10 @@ __device__ void syrk_tile_acc(const DevSym &S, int s, int r0, int c0, int kblk, 
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
         const int c = acc_col(j, e);
-        acc.v[i][j][e] = (r < nrow && c < ncol && r0 + r >= c0 + c)
-                             ? neg(P[(size_t)(c0 + c) * m + r0 + r]) : 0.0;
+        acc.v[i][j][e] = neg(ld_if(P + (size_t)(c0 + c) * m + r0 + r, r < nrow && c < ncol && r0 + r >= c0 + c));
       }
   }
-  dmma_tile_product(P + (size_t)k0 * m + r0, m, nrow, P + (size_t)k0 * m + c0, m, ncol, bk,
-                    stages, acc);
+  dmma_tile_product<true>(Pa, m, nrow, Pb, m, ncol, bk, stages, acc);
 }
 
 // ... stored back negated (and to copy, [column][row] of 64, where it is given).

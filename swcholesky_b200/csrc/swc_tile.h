@@ -121,6 +121,8 @@ __device__ __forceinline__ void load_chunk(const double *__restrict__ Pa, int ld
   cp_async_commit();
 }
 
+// BEGUN: the caller has synchronised and asked for chunk 0 itself, before loads of its own.
+template <bool BEGUN = false>
 __device__ __forceinline__ void dmma_tile_product(const double *__restrict__ Pa, int lda, int na,
                                                   const double *__restrict__ Pb, int ldb, int nb,
                                                   int K, double *stages, TileAcc &acc,
@@ -129,8 +131,10 @@ __device__ __forceinline__ void dmma_tile_product(const double *__restrict__ Pa,
   const int wr = (warp >> 1) * 32, wc = (warp & 1) * 32;
   const int kq = lane & 3, g = lane >> 2;
   const int nchunks = (K + KC - 1) / KC;
-  tile_sync(bar);   // stages free (previous users done)
-  load_chunk(Pa, lda, na, Pb, ldb, nb, K, 0, stages, tid);
+  if (!BEGUN) {
+    tile_sync(bar);   // stages free (previous users done)
+    load_chunk(Pa, lda, na, Pb, ldb, nb, K, 0, stages, tid);
+  }
   for (int c = 0; c < nchunks; ++c) {
     if (c + 1 < nchunks) {
       load_chunk(Pa, lda, na, Pb, ldb, nb, K, (c + 1) * KC, stages + ((c + 1) & 1) * STAGE, tid);
