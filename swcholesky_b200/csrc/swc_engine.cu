@@ -1191,9 +1191,13 @@ void build_solve_plan(int n, const int *Ls, const HostSym &H, SolvePlan &SP) {
     SP.g8_off.push_back((int)SP.g8_tasks.size());
     {
       int64_t nt = 0;
+      int widest = 0;
       for (int s : whole)
-        if (H.dinv_off[s] >= 0) nt += (rowptr[s + 1] - rowptr[s] - (super[s + 1] - super[s]) + 127) / 128;
-      const bool split = nt < SOLVE8_FULL_TASKS;
+        if (H.dinv_off[s] >= 0) {
+          nt += (rowptr[s + 1] - rowptr[s] - (super[s + 1] - super[s]) + 127) / 128;
+          widest = std::max(widest, super[s + 1] - super[s]);
+        }
+      const bool split = nt < (widest >= SOLVE8_WIDE ? 4 : 1) * SOLVE8_FULL_TASKS;
       SP.c8_split.push_back(split);
       for (int s : bylev[l]) {
         if (H.dinv_off[s] < 0) continue;

@@ -75,9 +75,12 @@ constexpr int SOLVE_WARP_LEVEL_MIN = 4096;
 // they hide: 24 x 23 x 25 grid 197 / 277 -> 201 / 280, 60 x 61 grid 122 / 139 -> 130 / 143.
 constexpr int SOLVE_TOP = 64;
 constexpr int64_t SOLVE_HALF_MIN = (int64_t)1 << 20;
-// Several right-hand sides: contribution tasks of 128 rows on levels with at least one per SM,
-// else 32-row tasks whose warps split the columns.
-constexpr int SOLVE8_FULL_TASKS = 148;
+// Several right-hand sides: contribution tasks of 128 rows on levels with at least one per SM (four
+// where a supernode is SOLVE8_WIDE wide or more: a 128-row task walks all its columns), else 32-row
+// tasks whose warps split the columns.  B200, eight right-hand sides, one for all widths -> four for
+// wide ones: 60^3 grid 1780 -> 1651 us, 36 x 35 x 33 elastic 1730 -> 1563; four for all widths loses
+// 2% on the 24 x 23 x 22 elastic operator.
+constexpr int SOLVE8_FULL_TASKS = 148, SOLVE8_WIDE = 256;
 
 // Size classes of the executor (the B200 counterpart of the reference's triple queue,
 // cholesky/tripleQueue.c:17-170): a supernode whose whole panel fits in shared memory is

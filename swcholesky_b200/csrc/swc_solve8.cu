@@ -322,44 +322,39 @@ __global__ void __launch_bounds__(WN * 32) k_bwd_warp8(DevSym S, const int *list
 // ---- contributions of tiled supernodes.  Levels with at least one 128-row task per SM: 128
 // rows per CTA, warp q forms rows 16 q .. 16 q + 15 over all columns; other levels: 32 rows
 // per CTA of 16 warps that split the columns, partial sums in shared memory.
+constexpr int C8_U = 8;   // four columns each: loads in flight per lane and row
 __global__ void __launch_bounds__(NT8) k_contrib8(DevSym S, const int2 *tasks, const double *y8,
                                                   double *c8) {
+  pdl_trigger();
   const int s = tasks[blockIdx.x].x;
   const int lane = threadIdx.x & 31, g = lane >> 2, kq = lane & 3;
   const int a0 = tasks[blockIdx.x].y + 16 * (int)(threadIdx.x >> 5);
   const int f = S.super[s], w = S.super[s + 1] - f;
   const int64_t rb = S.rowptr[s];
   const int m = (int)(S.rowptr[s + 1] - rb);
-  pdl_trigger();
-  pdl_wait();
-  if (a0 >= m) return;
   const double *Ls = S.L + S.xptr[s];
   const double *yv = y8 + (size_t)f * R8 + g;
   const bool in0 = a0 + g < m, in1 = a0 + 8 + g < m;
-  const double *p0 = Ls + (in0 ? a0 + g : 0), *p1 = Ls + (in1 ? a0 + 8 + g : 0);
+  const double *p0 = Ls + a0 + g;
   double c[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
-  int k = 0;
-  for (; k + 16 <= w; k += 16) {
-    double l0[4], l1[4], b[4];
+  bool first = true;
+  for (int k = 0; k < w; k += 4 * C8_U) {
+    double l0[C8_U], l1[C8_U], b[C8_U];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const size_t col = (size_t)(k + 4 * u + kq);
-      l0[u] = p0[col * m];
-      l1[u] = p1[col * m];
-      b[u] = yv[col * R8];
+    for (int u = 0; u < C8_U; ++u) {
+      const int col = k + 4 * u + kq;
+      l0[u] = ld_if(p0 + (size_t)col * m, in0 && col < w);
+      l1[u] = ld_if(p0 + 8 + (size_t)col * m, in1 && col < w);
     }
+    if (first) pdl_wait();
+    first = false;
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
+    for (int u = 0; u < C8_U; ++u) b[u] = ld_if(yv + (size_t)(k + 4 * u + kq) * R8, k + 4 * u + kq < w);
+#pragma unroll
+    for (int u = 0; u < C8_U; ++u) {
       dmma(c[0], l0[u], b[u]);
       dmma(c[1], l1[u], b[u]);
     }
-  }
-  for (; k < w; k += 4) {
-    const bool kin = k + kq < w;
-    const size_t col = (size_t)(kin ? k + kq : 0);
-    const double b = kin ? yv[col * R8] : 0.0;
-    dmma(c[0], kin ? p0[col * m] : 0.0, b);
-    dmma(c[1], kin ? p1[col * m] : 0.0, b);
   }
   double *out = c8 + (size_t)((rb - f) + (a0 + g - w)) * R8 + 2 * kq;
   if (in0) *reinterpret_cast<double2 *>(out) = make_double2(c[0][0], c[0][1]);
