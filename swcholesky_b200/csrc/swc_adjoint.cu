@@ -88,12 +88,12 @@ __device__ void adj_small_body(const DevSym &S, const AdjDev &A, int s, double *
   double *Z = A.Z + A.zoff[s];
   const bool front = A.kids[s] != 0;
   // the panel (upper triangle, padding: zeros; padded diagonal: ones) and the row map
+#pragma unroll 8
   for (int e = t; e < wp * ld; e += NTH) {
     const int j = e / ld, i = e - j * ld;
-    double v = i == j && j >= w ? 1.0 : 0.0;
     const int row = i < wp ? i : i - pad;
-    if (j < w && (i < wp ? i < w && i >= j : row < m)) v = Ls[(size_t)j * m + row];
-    Pm[e] = v;
+    const double v = ld_if(Ls + (size_t)j * m + row, j < w && (i < wp ? i < w && i >= j : row < m));
+    Pm[e] = i == j && j >= w ? 1.0 : v;
   }
   for (int e = t; e < wp * ldt; e += NTH) T[e] = 0.0;
   const int *grel = A.rel + (S.rowptr[s] - f);
@@ -149,6 +149,7 @@ __device__ void adj_small_body(const DevSym &S, const AdjDev &A, int s, double *
     }
   }
   zsync<NW>();
+  pdl_wait();   // so far from L alone
   // Y = Z_RR U, Z_RR read from the parent's front and, for a front of its own, written to it
   if (r > 0) {
     const int p = A.parent[s], mp = nrows_of(S, p);
@@ -236,6 +237,7 @@ __device__ void adj_small_body(const DevSym &S, const AdjDev &A, int s, double *
 
 __global__ void __launch_bounds__(ZC_T) k_adj_small(DevSym S, AdjDev A, const int *list) {
   extern __shared__ double zsm[];
+  pdl_trigger();
   const int e = list[blockIdx.x], s = e < 0 ? ~e : e;   // ~s: y_global
   const int w = S.super[s + 1] - S.super[s], m = nrows_of(S, s);
   const int pe = front_wp(w) * front_ld(w, m);
@@ -246,6 +248,7 @@ __global__ void __launch_bounds__(ZC_T) k_adj_small(DevSym S, AdjDev A, const in
 
 __global__ void __launch_bounds__(ZW_WARPS * 32) k_adj_warp(DevSym S, AdjDev A, const int *list, int count) {
   extern __shared__ double zsm[];
+  pdl_trigger();
   const int q = blockIdx.x * ZW_WARPS + (threadIdx.x >> 5);
   if (q >= count) return;
   double *P = reinterpret_cast<double *>(reinterpret_cast<unsigned char *>(zsm) +
@@ -263,6 +266,8 @@ __global__ void __launch_bounds__(256) k_adj_copy(DevSym S, AdjDev A, const int4
   const int p = A.parent[s], mp = nrows_of(S, p);
   const int *rel = A.rel + (S.rowptr[s] - S.super[s]);
   const int i = tk.y + (threadIdx.x & 63);
+  pdl_trigger();
+  pdl_wait();
   if (i >= r) return;
   const double *src = A.Z + A.zoff[p] + rel[i];
   double *dst = A.Z + A.zoff[s] + (size_t)w * m + w + i;
@@ -288,6 +293,7 @@ static_assert(2 * TB * LDS >= 2 * STAGE, "the product's stages fit");
 __global__ void __launch_bounds__(MT) k_adj_u(DevSym S, AdjDev A, const int4 *tasks) {
   extern __shared__ double zsm[];
   double *Ts = zsm, *Lx = zsm + TB * LDS;   // [k][column], [k][row]
+  pdl_trigger();
   const int4 tk = tasks[blockIdx.x];
   const int s = tk.x, c0 = tk.y * TB, x0 = tk.z;
   const int m = nrows_of(S, s), w = min(TB, S.super[s + 1] - S.super[s] - c0), off = c0 + w;
@@ -303,6 +309,7 @@ __global__ void __launch_bounds__(MT) k_adj_u(DevSym S, AdjDev A, const int4 *ta
   TileAcc acc;   // U^T: rows are columns of the block
   acc.zero();
   dmma_tile_smem(Ts, Lx, TB, acc);
+  pdl_wait();   // UT may be read until the kernel ahead ends
   double *UT = A.UT + (size_t)tk.w * (TB * TB) + (size_t)x0 * TB;
 #pragma unroll
   for (int i = 0; i < 4; ++i)
@@ -319,6 +326,8 @@ __global__ void __launch_bounds__(MT, 3) k_adj_zrk(DevSym S, AdjDev A, const int
   const int4 tk = tasks[blockIdx.x];
   const int s = tk.x, c0 = tk.y * TB, x0 = tk.z;
   const int m = nrows_of(S, s), w = min(TB, S.super[s + 1] - S.super[s] - c0), off = c0 + w;
+  pdl_trigger();
+  pdl_wait();
   const int mr = m - off, nrow = min(TB, mr - x0);
   double *Z = A.Z + A.zoff[s];
   const double *UT = A.UT + (size_t)tk.w * (TB * TB);
@@ -364,6 +373,7 @@ __global__ void __launch_bounds__(MT, 3) k_adj_zrk(DevSym S, AdjDev A, const int
 // Z_KK = T^T T + the row blocks' shares.  unit = (s, column block, first task, tasks).
 __global__ void __launch_bounds__(MT) k_adj_zkk(DevSym S, AdjDev A, const int4 *units) {
   extern __shared__ double zsm[];
+  pdl_trigger();
   const int4 un = units[blockIdx.x];
   const int s = un.x, c0 = un.y * TB;
   const int m = nrows_of(S, s), w = min(TB, S.super[s + 1] - S.super[s] - c0);
@@ -372,6 +382,7 @@ __global__ void __launch_bounds__(MT) k_adj_zkk(DevSym S, AdjDev A, const int4 *
   TileAcc acc;
   acc.zero();
   dmma_tile_smem(zsm, zsm, TB, acc);
+  pdl_wait();
   for (int t = un.z; t < un.z + un.w; ++t) {
     const double *P = A.P + (size_t)t * (TB * TB);
 #pragma unroll
@@ -401,6 +412,8 @@ __global__ void __launch_bounds__(MT) k_adj_zkk(DevSym S, AdjDev A, const int4 *
 // Gradient of the entries of A in a wide supernode's columns: one warp per (s, column).
 __global__ void k_adj_grad(DevSym S, AdjDev A, const int2 *cols, int count) {
   const int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  pdl_trigger();
+  pdl_wait();
   if (t >= count) return;
   const int s = cols[t].x, j = cols[t].y, c = j - S.super[s];
   const double *col = A.Z + A.zoff[s] + (size_t)c * nrows_of(S, s);
@@ -624,29 +637,33 @@ bool Engine::logdet(double *out, std::string &err) {
   return true;
 }
 
-// The reverse sweep's launches (fixed by the structure), gradient into d_adj_grad_.
+// The reverse sweep's launches (fixed by the structure), gradient into d_adj_grad_.  A chain of
+// short kernels: each is started early and does what L alone allows (the small fronts' inverses and
+// U, the wide ones' U and T^T T) before it waits for the one ahead.
 void Engine::run_adjoint() {
   const AdjointPlan &AP = *adj_;
-  cudaStream_t st = stream_;
+  LaunchQueue q{stream_, false};
   const AdjDev A{d_adj_parent_, d_frel_, d_fapos_, d_adj_zoff_, d_adj_kids_,
                  d_adj_Z_,      d_adj_UT_, d_adj_P_, d_adj_grad_};
   for (size_t v = 0; v < AP.waves.size(); ++v) {
     const AdjointPlan::AdjWave &W = AP.waves[v];
-    if (W.copy_cnt > 0) k_adj_copy<<<W.copy_cnt, 256, 0, st>>>(sym_, A, d_adj_copies_ + W.copy_off);
-    if (W.cta_cnt > 0) k_adj_small<<<W.cta_cnt, ZC_T, W.cta_smem, st>>>(sym_, A, d_adj_cta_ + W.cta_off);
+    if (W.copy_cnt > 0) launch_early(q, 1, k_adj_copy, W.copy_cnt, 256, 0, sym_, A, d_adj_copies_ + W.copy_off);
+    if (W.cta_cnt > 0)
+      launch_early(q, 1, k_adj_small, W.cta_cnt, ZC_T, W.cta_smem, sym_, A, d_adj_cta_ + W.cta_off);
     if (W.warp_cnt > 0)
-      k_adj_warp<<<(W.warp_cnt + ZW_WARPS - 1) / ZW_WARPS, ZW_WARPS * 32, ZW_WARPS * ZW_SLICE, st>>>(
-          sym_, A, d_adj_warp_ + W.warp_off, W.warp_cnt);
+      launch_early(q, 1, k_adj_warp, (W.warp_cnt + ZW_WARPS - 1) / ZW_WARPS, ZW_WARPS * 32, ZW_WARPS * ZW_SLICE,
+                   sym_, A, d_adj_warp_ + W.warp_off, W.warp_cnt);
     for (const AdjointPlan::Step &t : W.steps) {
       if (t.task_cnt > 0) {
-        k_adj_u<<<t.task_cnt, MT, TT_SMEM, st>>>(sym_, A, d_adj_tasks_ + t.task_off);
-        k_adj_zrk<<<t.task_cnt, MT, TT_SMEM, st>>>(sym_, A, d_adj_tasks_ + t.task_off);
+        launch_early(q, 1, k_adj_u, t.task_cnt, MT, TT_SMEM, sym_, A, d_adj_tasks_ + t.task_off);
+        launch_early(q, 1, k_adj_zrk, t.task_cnt, MT, TT_SMEM, sym_, A, d_adj_tasks_ + t.task_off);
       }
-      if (t.unit_cnt > 0) k_adj_zkk<<<t.unit_cnt, MT, TB * LDS * 8, st>>>(sym_, A, d_adj_units_ + t.unit_off);
+      if (t.unit_cnt > 0)
+        launch_early(q, 1, k_adj_zkk, t.unit_cnt, MT, TB * LDS * 8, sym_, A, d_adj_units_ + t.unit_off);
     }
     const Wave &B = plan_.waves[AP.waves.size() - 1 - v];
     if (B.asm_cnt > 0)
-      k_adj_grad<<<(B.asm_cnt * 32 + 255) / 256, 256, 0, st>>>(sym_, A, d_asm_ + B.asm_off, B.asm_cnt);
+      launch_early(q, 1, k_adj_grad, (B.asm_cnt * 32 + 255) / 256, 256, 0, sym_, A, d_asm_ + B.asm_off, B.asm_cnt);
   }
 }
 
