@@ -1757,6 +1757,9 @@ void Engine::launch_all(std::vector<std::pair<int, cudaEvent_t>> *prof, int prec
                                 plan_.persist_smem, persist_ctas_, d_qctr_, st);
     mark(-1, 1);
   }
+  // multifrontal: a kernel of the walks or of a wave stands before the next on this stream (not one
+  // of the memsets above), which may start early then
+  bool behind = front && !prof && (!FP->warp_list.empty() || !FP->cta_list.empty());
   for (const Wave &W : plan_.waves) {
     // the wave's small supernodes read only earlier waves' panels and write only their own,
     // so they run beside the wave's tiled work (updates and dense steps) on a second
@@ -1791,13 +1794,13 @@ void Engine::launch_all(std::vector<std::pair<int, cudaEvent_t>> *prof, int prec
       const int cnt = b0 > 0 ? FWv->sch_more[b0] : FWv->sch_cnt;
       mark(K_UPDATE, cnt);
       launch_front_schur(sym_, *front_dev_, d_fsch_ + FWv->sch_off, d_fsch_end_ + FWv->sch_off,
-                         d_fsch_pairs_, cnt, b0 * TB, INT_MAX, 0, st);
+                         d_fsch_pairs_, cnt, b0 * TB, INT_MAX, 0, LaunchQueue{st, behind});
       mark(-1, cnt);
     };
     if (front) {
       mark(K_ASSEMBLE, FWv->ext_cnt);
       launch_front_extend(sym_, *front_dev_, d_fext_ + FWv->ext_off, d_fext_end_ + FWv->ext_off,
-                          d_fext_pairs_, FWv->ext_cnt, st);
+                          d_fext_pairs_, FWv->ext_cnt, LaunchQueue{st, behind});
       mark(-1, FWv->ext_cnt);
     } else if (scatter) {
       mark(K_UPDATE, W.scs_cnt);
@@ -1831,11 +1834,14 @@ void Engine::launch_all(std::vector<std::pair<int, cudaEvent_t>> *prof, int prec
       continue;
     }
     mark(K_PANEL, W.big_cnt);
-    launch_diag_step(sym_, d_big_ + W.big_off, W.big_cnt, 0, st);
+    launch_diag_step(sym_, d_big_ + W.big_off, W.big_cnt, 0, LaunchQueue{st, behind});
+    behind = behind || (front && !prof && W.big_cnt > 0);
     mark(-1, W.big_cnt);
     for (size_t j = 0; j < W.panel_off.size(); ++j) {
       mark(K_PANEL, W.panel_cnt[j]);
-      launch_trsm_step(sym_, d_panel_ + W.panel_off[j], W.panel_cnt[j], (int)j, st);
+      // (the later steps' TRSMs, and the updates, started early cost more than they gain: their CTAs
+      // wait where the grouped updates could run; 60^3 grid 14.78 -> 14.99 ms)
+      launch_trsm_step(sym_, d_panel_ + W.panel_off[j], W.panel_cnt[j], (int)j, LaunchQueue{st, behind && j == 0});
       mark(-1, W.panel_cnt[j]);
       if (syrk_tc && !prof) {
         // look-ahead: the step's trailing update split in two.  Column block j+1 (the next
@@ -1848,7 +1854,7 @@ void Engine::launch_all(std::vector<std::pair<int, cudaEvent_t>> *prof, int prec
         if (W.diag_cnt[j] > 0) {
           cudaStreamWaitEvent(aux_stream_, j > 0 ? ev_next_ : ev_fork_, 0);
           if (j > 0) cudaStreamWaitEvent(aux_stream_, ev_grp_[(j - 1) & 1], 0);
-          launch_diag_step(sym_, d_diag_ + W.diag_off[j], W.diag_cnt[j], (int)j + 1, aux_stream_, j > 0);
+          launch_diag_step(sym_, d_diag_ + W.diag_off[j], W.diag_cnt[j], (int)j + 1, LaunchQueue{aux_stream_, j > 0}, j > 0);
           cudaEventRecord(ev_join_, aux_stream_);
         }
         const int nc = W.scd_nc[j];
@@ -1871,13 +1877,16 @@ void Engine::launch_all(std::vector<std::pair<int, cudaEvent_t>> *prof, int prec
         // column j, then the update of column j+1; the grouped updates of the later columns
         // run beside both.  Column j+1's tiles take the group that ends at step j-1 before
         // block j's update.
+        // The diagonal blocks' kernels start early: their chain sets the time of the smaller waves,
+        // and the launch was 2 us of 22 per block (41 x 37 x 43 grid 2957 -> 2885 us, 24 x 23 x 22
+        // elastic 3063 -> 3008).
         const int nc = W.syrk_nc[j], ng = W.syrk_cnt[j] - nc;
         cudaEventRecord(ev_fork_, st);   // column j solved
         if (W.diag_cnt[j] > 0) {
           cudaStreamWaitEvent(aux_stream_, j > 0 ? ev_next_ : ev_fork_, 0);
           if (j > 0 && W.syrk_cnt[j - 1] > W.syrk_nc[j - 1])
             cudaStreamWaitEvent(aux_stream_, ev_grp_[(j - 1) & 1], 0);
-          launch_diag_step(sym_, d_diag_ + W.diag_off[j], W.diag_cnt[j], (int)j + 1, aux_stream_, j > 0);
+          launch_diag_step(sym_, d_diag_ + W.diag_off[j], W.diag_cnt[j], (int)j + 1, LaunchQueue{aux_stream_, j > 0}, j > 0);
           cudaEventRecord(ev_join_, aux_stream_);
         }
         if (front && FWv->sch_steps > 0 && (j + 1) % FWv->sch_steps == 0 && j + 1 < W.panel_off.size()) {
@@ -1886,7 +1895,7 @@ void Engine::launch_all(std::vector<std::pair<int, cudaEvent_t>> *prof, int prec
           if (side && parts == 0) cudaStreamWaitEvent(sch_stream_, ev_sjoin_, 0);
           launch_front_schur(sym_, *front_dev_, d_fsch_ + FWv->sch_off, d_fsch_end_ + FWv->sch_off, d_fsch_pairs_,
                              FWv->sch_more[b0], b0 * TB, ((int)j + 1) * TB, num_sms_ - FRONT_BG_RESERVE,
-                             sch_stream_);
+                             LaunchQueue{sch_stream_, false});
           cudaEventRecord(ev_sch_, sch_stream_);
           ++parts;
         }
@@ -1904,7 +1913,7 @@ void Engine::launch_all(std::vector<std::pair<int, cudaEvent_t>> *prof, int prec
       } else if (prof) {
         // profiled runs keep one stream so every launch is bracketed by its own events
         mark(K_PANEL, W.diag_cnt[j]);
-        launch_diag_step(sym_, d_diag_ + W.diag_off[j], W.diag_cnt[j], (int)j + 1, st);
+        launch_diag_step(sym_, d_diag_ + W.diag_off[j], W.diag_cnt[j], (int)j + 1, LaunchQueue{st, false});
         mark(-1, W.diag_cnt[j]);
         mark(K_SYRK, W.syrk_cnt[j]);
         syrk(W, (int)j);
@@ -1913,7 +1922,7 @@ void Engine::launch_all(std::vector<std::pair<int, cudaEvent_t>> *prof, int prec
         // fork: next diagonal block on the auxiliary stream, trailing update here; join
         cudaEventRecord(ev_fork_, st);
         cudaStreamWaitEvent(aux_stream_, ev_fork_, 0);
-        launch_diag_step(sym_, d_diag_ + W.diag_off[j], W.diag_cnt[j], (int)j + 1, aux_stream_);
+        launch_diag_step(sym_, d_diag_ + W.diag_off[j], W.diag_cnt[j], (int)j + 1, LaunchQueue{aux_stream_, false});
         cudaEventRecord(ev_join_, aux_stream_);
         syrk(W, (int)j);
         cudaStreamWaitEvent(st, ev_join_, 0);

@@ -572,11 +572,11 @@ void launch_update_tiles(const DevSym &S, const int4 *tasks, const int *task_end
                          const int4 *pairs, int count, cudaStream_t st);
 // fold: the rows of this block in the previous column block are solved here, from the copy the
 // trailing update left in the block's place of dinv (launch_syrk_step), not read from L
-void launch_diag_step(const DevSym &S, const int *list, int count, int step, cudaStream_t st,
+void launch_diag_step(const DevSym &S, const int *list, int count, int step, LaunchQueue q,
                       bool fold = false);
 // the same copy by itself: rows 64 (step + 1) .. of column block `step` of the list's supernodes
 void launch_copy_tile(const DevSym &S, const int *list, int count, int step, cudaStream_t st);
-void launch_trsm_step(const DevSym &S, const int2 *tasks, int count, int step, cudaStream_t st);
+void launch_trsm_step(const DevSym &S, const int2 *tasks, int count, int step, LaunchQueue q);
 // tasks (s, r0, c0, product index): prod[index].kk names the column blocks applied
 void launch_syrk_step(const DevSym &S, const int4 *tasks, const TcPair *prod, int count,
                       cudaStream_t st);

@@ -345,6 +345,10 @@ __global__ void __launch_bounds__(ET) k_front_extend(DevSym S, FrontDev F, const
   double *Lt = S.L + S.xptr[s] + (size_t)c0 * m + r0;
   const int row = threadIdx.x & 63, cq = threadIdx.x >> 6;   // columns cq, cq + 4, ..
   constexpr int NE = TB * TB / ET;
+  pdl_trigger();
+  int kids = min(FRONT_KIDS, p_end - tk.w);
+  load_pair_maps(S, F, pairs, tk.w, kids, r0, c0, M, ET);   // symbolic data
+  pdl_wait();
   double v[NE];
 #pragma unroll
   for (int e = 0; e < NE; ++e) {
@@ -352,9 +356,11 @@ __global__ void __launch_bounds__(ET) k_front_extend(DevSym S, FrontDev F, const
     v[e] = ld_if(Lt + (size_t)col * m + row, r0 + row < m && c0 + col < w && r0 + row >= c0 + col);
   }
   for (int q = tk.w; q < p_end; q += FRONT_KIDS) {
-    const int kids = min(FRONT_KIDS, p_end - q);
-    if (q > tk.w) __syncthreads();
-    load_pair_maps(S, F, pairs, q, kids, r0, c0, M, ET);
+    if (q > tk.w) {
+      kids = min(FRONT_KIDS, p_end - q);
+      __syncthreads();
+      load_pair_maps(S, F, pairs, q, kids, r0, c0, M, ET);
+    }
     for (int k = 0; k < kids; ++k) {
       const int pi = M.ia[k][row];
       const double *cb = M.cb[k] + pi;
@@ -380,6 +386,7 @@ __global__ void __launch_bounds__(ET) k_front_extend(DevSym S, FrontDev F, const
 // (DMMA) plus, at k0 = 0, the children's blocks, else what the block holds.  task = (s, i0, j0,
 // first pair), offsets in the block.  The accumulator collects minus the tile's value and the
 // product, and is stored back negated.
+template <bool EARLY>
 __device__ __forceinline__ void schur_tile(const DevSym &S, const FrontDev &F, int4 tk, int p_end,
                                            const int4 *pairs, int k0, int k1, double *stages, PairMaps &M,
                                            int tid, int bar) {
@@ -388,6 +395,9 @@ __device__ __forceinline__ void schur_tile(const DevSym &S, const FrontDev &F, i
   const int r = m - w;
   double *cbs = F.cb + F.cb_off[s];
   k1 = min(k1, w);
+  int kids = min(FRONT_KIDS, p_end - tk.w);
+  if (k0 == 0 && kids > 0) load_pair_maps(S, F, pairs, tk.w, kids, w + i0, w + j0, M, MT, tid, bar);
+  if (EARLY) pdl_wait();   // so far symbolic data
   TileAcc acc;
   if (k0 == 0) acc.zero();
   else
@@ -401,9 +411,11 @@ __device__ __forceinline__ void schur_tile(const DevSym &S, const FrontDev &F, i
           acc.v[i][j][e] = neg(ld_if(cbs + (int64_t)cj * r + ri, ri < r && cj <= ri));
         }
   for (int q = tk.w; q < p_end && k0 == 0; q += FRONT_KIDS) {
-    const int kids = min(FRONT_KIDS, p_end - q);
-    if (q > tk.w) tile_sync(bar);
-    load_pair_maps(S, F, pairs, q, kids, w + i0, w + j0, M, MT, tid, bar);
+    if (q > tk.w) {
+      kids = min(FRONT_KIDS, p_end - q);
+      tile_sync(bar);
+      load_pair_maps(S, F, pairs, q, kids, w + i0, w + j0, M, MT, tid, bar);
+    }
     for (int k = 0; k < kids; ++k) {
       const double *cb = M.cb[k];
       const int ldc = M.ld[k];
@@ -446,7 +458,8 @@ __global__ void __launch_bounds__(MT, 4) k_front_schur(DevSym S, FrontDev F, con
                                                        const int *end, const int4 *pairs, int k0, int k1) {
   extern __shared__ double fsm[];
   __shared__ PairMaps M;
-  schur_tile(S, F, tasks[blockIdx.x], end[blockIdx.x], pairs, k0, k1, fsm, M, threadIdx.x, 0);
+  pdl_trigger();
+  schur_tile<true>(S, F, tasks[blockIdx.x], end[blockIdx.x], pairs, k0, k1, fsm, M, threadIdx.x, 0);
 }
 
 // The same beside the chain of diagonal blocks (see BG), as the panel's columns get done.
@@ -457,7 +470,7 @@ __global__ void __launch_bounds__(BG * MT, 1) k_front_schur_bg(DevSym S, FrontDe
   __shared__ PairMaps M[BG];
   const int grp = threadIdx.x / MT, tid = threadIdx.x - grp * MT;
   for (int q = blockIdx.x * BG + grp; q < count; q += BG * gridDim.x) {
-    schur_tile(S, F, tasks[q], end[q], pairs, k0, k1, fsm + grp * 2 * STAGE, M[grp], tid, 1 + grp);
+    schur_tile<false>(S, F, tasks[q], end[q], pairs, k0, k1, fsm + grp * 2 * STAGE, M[grp], tid, 1 + grp);
     tile_sync(1 + grp);
   }
 }
@@ -517,17 +530,17 @@ void launch_front_small(const DevSym &S, const FrontDev &F, const FrontDesc *lis
   if (count > 0) k_front_small<<<count, FT, smem, st>>>(S, F, list);
 }
 void launch_front_extend(const DevSym &S, const FrontDev &F, const int4 *tasks, const int *end,
-                         const int4 *pairs, int count, cudaStream_t st) {
-  if (count > 0) k_front_extend<<<count, ET, 0, st>>>(S, F, tasks, end, pairs);
+                         const int4 *pairs, int count, LaunchQueue q) {
+  if (count > 0) launch_early(q, 1, k_front_extend, count, ET, 0, S, F, tasks, end, pairs);
 }
 void launch_front_schur(const DevSym &S, const FrontDev &F, const int4 *tasks, const int *end,
-                        const int4 *pairs, int count, int k0, int k1, int bg_ctas, cudaStream_t st) {
+                        const int4 *pairs, int count, int k0, int k1, int bg_ctas, LaunchQueue q) {
   if (count <= 0) return;
   if (bg_ctas > 0)
-    k_front_schur_bg<<<std::min(bg_ctas, (count + BG - 1) / BG), BG * MT, BG_SMEM, st>>>(S, F, tasks, end, pairs,
+    k_front_schur_bg<<<std::min(bg_ctas, (count + BG - 1) / BG), BG * MT, BG_SMEM, q.st>>>(S, F, tasks, end, pairs,
                                                                                         count, k0, k1);
   else
-    k_front_schur<<<count, MT, SCHUR_SMEM, st>>>(S, F, tasks, end, pairs, k0, k1);
+    launch_early(q, 1, k_front_schur, count, MT, SCHUR_SMEM, S, F, tasks, end, pairs, k0, k1);
 }
 
 }  // namespace swc

@@ -153,10 +153,10 @@ void launch_front_cta_walk(const DevSym &S, const FrontDev &F, const FrontDesc *
 void launch_front_small(const DevSym &S, const FrontDev &F, const FrontDesc *list, int count, int smem,
                         cudaStream_t st);   // cb < 0: the block is formed by tiles
 void launch_front_extend(const DevSym &S, const FrontDev &F, const int4 *tasks, const int *end,
-                         const int4 *pairs, int count, cudaStream_t st);
+                         const int4 *pairs, int count, LaunchQueue q);
 // tiles of contribution blocks over the columns k0 .. k1 - 1 of each front (k1 beyond a front's
 // width: to its end); bg_ctas > 0: at most that many CTAs of one per SM, beside other kernels
 void launch_front_schur(const DevSym &S, const FrontDev &F, const int4 *tasks, const int *end,
-                        const int4 *pairs, int count, int k0, int k1, int bg_ctas, cudaStream_t st);
+                        const int4 *pairs, int count, int k0, int k1, int bg_ctas, LaunchQueue q);
 
 }  // namespace swc

@@ -801,9 +801,9 @@ template <bool FOLD>
 __global__ void __launch_bounds__(DIAG_NW * 32) k_diag_step(DevSym S, const int *list, int count,
                                                            int step) {
   extern __shared__ double dyn[];
+  pdl_trigger();
+  pdl_wait();
   if (FOLD) {
-    pdl_trigger();
-    pdl_wait();
     factor_diag_block<DIAG_NW, true, true>(S, list[blockIdx.x], step * TB, dyn, nullptr);
   } else if (step > 0) {
     factor_diag_block<DIAG_NW, true>(S, list[blockIdx.x], step * TB, dyn, nullptr);
@@ -871,7 +871,10 @@ __device__ void trsm_task(const DevSym &S, int s, int r0, int step, double *dyn)
 __global__ void __launch_bounds__(MT, 4) k_trsm_step(DevSym S, const int2 *tasks, int count,
                                                   int step) {
   extern __shared__ double dyn[];
-  trsm_task(S, tasks[blockIdx.x].x, tasks[blockIdx.x].y, step, dyn);
+  const int2 t = tasks[blockIdx.x];
+  pdl_trigger();
+  pdl_wait();
+  trsm_task(S, t.x, t.y, step, dyn);
 }
 
 // Trailing update of a step: task = (s, r0, c0, product index) with c0 >= (step+1)*64,
@@ -1154,20 +1157,17 @@ void launch_update_tiles(const DevSym &S, const int4 *tasks, const int *task_end
                          const int4 *pairs, int count, cudaStream_t st) {
   if (count > 0) k_update_tiles<<<count, MT, UPD_SMEM, st>>>(S, tasks, task_end, pairs, count);
 }
-void launch_diag_step(const DevSym &S, const int *list, int count, int step, cudaStream_t st, bool fold) {
+void launch_diag_step(const DevSym &S, const int *list, int count, int step, LaunchQueue q, bool fold) {
   if (count <= 0) return;
-  // started early: the chain of diagonal blocks sets the time of the smaller waves, and the launch
-  // was 2 us of 22 per block (41 x 37 x 43 grid 2957 -> 2885 us, 24 x 23 x 22 elastic 3063 -> 3008;
-  // with the TRSM and the updates started early too, 2928 and 3032)
-  LaunchQueue q{st, true};
-  if (fold) launch_early(q, 1, k_diag_step<true>, count, DIAG_NW * 32, diag_prev_smem(DIAG_NW), S, list, count, step);
-  else k_diag_step<false><<<count, DIAG_NW * 32, diag_prev_smem(DIAG_NW), st>>>(S, list, count, step);
+  const int smem = diag_prev_smem(DIAG_NW);
+  if (fold) launch_early(q, 1, k_diag_step<true>, count, DIAG_NW * 32, smem, S, list, count, step);
+  else launch_early(q, 1, k_diag_step<false>, count, DIAG_NW * 32, smem, S, list, count, step);
 }
 void launch_copy_tile(const DevSym &S, const int *list, int count, int step, cudaStream_t st) {
   if (count > 0) k_copy_tile<<<count, 256, 0, st>>>(S, list, step);
 }
-void launch_trsm_step(const DevSym &S, const int2 *tasks, int count, int step, cudaStream_t st) {
-  if (count > 0) k_trsm_step<<<count, MT, 2 * STAGE * 8, st>>>(S, tasks, count, step);
+void launch_trsm_step(const DevSym &S, const int2 *tasks, int count, int step, LaunchQueue q) {
+  if (count > 0) launch_early(q, 1, k_trsm_step, count, MT, 2 * STAGE * 8, S, tasks, count, step);
 }
 void launch_syrk_step(const DevSym &S, const int4 *tasks, const TcPair *prod, int count,
                       cudaStream_t st) {
