@@ -2319,16 +2319,20 @@ bool Engine::refine(const double *b, double *x, int nrhs, double tol, int maxit,
   refresh_csr();
   // ||A||_inf
   launch_rowabs(n_, d_csr_rp_, d_csr_val_, rows, st);
-  launch_norms(n_, 1, rows, nullptr, d_norms_, d_npart_, st);
+  launch_norms(n_, 1, rows, nullptr, nullptr, d_norms_, d_npart_, st);
   if (!sync_norms(1)) return false;
   anorm_ = h_norms_[0];
   // residual r = b - A x and backward errors; returns the max over right-hand sides
   std::vector<double> berr(nrhs, 0.0);
   auto residual = [&](const double *xx) -> bool {
-    launch_spmv(n_, d_csr_rp_, d_csr_ci_, d_csr_val_, xx, r, nrhs, st);
-    launch_residual(len, b, r, st);
-    launch_norms(n_, nrhs, r, nullptr, d_norms_, d_npart_, st);
-    launch_norms(n_, nrhs, xx, nullptr, d_norms_ + 2 * nrhs, d_npart_, st);
+    for (int k = 0; nrhs > 1 && k < nrhs; k += 8) {
+      const int nr = std::min(8, nrhs - k);
+      const size_t at = (size_t)k * n_;
+      launch_pack8(n_, nr, xx + at, d_x8_, st);
+      launch_spmv8(n_, d_csr_rp_, d_csr_ci_, d_csr_val_, d_x8_, b + at, r + at, nr, st);
+    }
+    if (nrhs == 1) launch_spmv(n_, d_csr_rp_, d_csr_ci_, d_csr_val_, xx, b, r, st);
+    launch_norms(n_, nrhs, r, nullptr, xx, d_norms_, d_npart_, st);
     if (!sync_norms(2 * nrhs)) return false;
     for (int k = 0; k < nrhs; ++k) {
       const double rn = h_norms_[2 * k], xn = h_norms_[2 * (nrhs + k)];
@@ -2365,18 +2369,17 @@ bool Engine::refine(const double *b, double *x, int nrhs, double tol, int maxit,
       double *zk = dv + (size_t)k * n_, *pk = pv + (size_t)k * n_, *qk = qv + (size_t)k * n_;
       const double *bk = b + (size_t)k * n_;
       auto norms1 = [&](const double *a, const double *bb) -> bool {
-        launch_norms(n_, 1, a, bb, d_norms_, d_npart_, st);
+        launch_norms(n_, 1, a, bb, nullptr, d_norms_, d_npart_, st);
         return sync_norms(1);
       };
-      launch_spmv(n_, d_csr_rp_, d_csr_ci_, d_csr_val_, xk, rk, 1, st);
-      launch_residual((size_t)n_, bk, rk, st);
+      launch_spmv(n_, d_csr_rp_, d_csr_ci_, d_csr_val_, xk, bk, rk, st);
       cudaMemcpyAsync(zk, rk, sizeof(double) * n_, cudaMemcpyDeviceToDevice, st);
       run_solve(zk, 1);
       cudaMemcpyAsync(pk, zk, sizeof(double) * n_, cudaMemcpyDeviceToDevice, st);
       if (!norms1(rk, zk)) return false;
       double rz = h_norms_[1];
       for (int it = 0; it < maxit * 10; ++it) {
-        launch_spmv(n_, d_csr_rp_, d_csr_ci_, d_csr_val_, pk, qk, 1, st);
+        launch_spmv(n_, d_csr_rp_, d_csr_ci_, d_csr_val_, pk, nullptr, qk, st);
         if (!norms1(pk, qk)) return false;
         const double pq = h_norms_[1];
         if (!(pq > 0)) break;

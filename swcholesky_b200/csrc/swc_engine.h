@@ -252,13 +252,15 @@ void launch_fwd_chain(const DevSym &S, const int2 *tasks, int count, double *y,
                       int epoch, int n, int64_t cstride, LaunchQueue &st);
 void launch_bwd_chain(const DevSym &S, const int2 *tasks, int count, double *x, int *flags,
                       int epoch, LaunchQueue &st);
-void launch_spmv(int n, const int *rp, const int *ci, const double *val, const double *x,
-                 double *y, int nrhs, cudaStream_t st);
+// y = A x, or b - A x where b is given; the second for nr <= 8 vectors, x interleaved by eight
+void launch_spmv(int n, const int *rp, const int *ci, const double *val, const double *x, const double *b,
+                 double *y, cudaStream_t st);
+void launch_spmv8(int n, const int *rp, const int *ci, const double *val, const double *x8, const double *b,
+                  double *y, int nr, cudaStream_t st);
 void launch_gather_vals(int nnz, const int *map, const double *ax, double *val, cudaStream_t st);
-void launch_residual(size_t len, const double *b, double *r, cudaStream_t st);
 void launch_axpy(size_t len, double a, const double *x, double *y, cudaStream_t st);
 void launch_xpby(size_t len, const double *z, double beta, double *p, cudaStream_t st);
-void launch_norms(int n, int nrhs, const double *x, const double *y, double *out, double *part,
+void launch_norms(int n, int nrhs, const double *x, const double *y, const double *x2, double *out, double *part,
                   cudaStream_t st);
 int norm_scratch_doubles(int nrhs);
 void launch_rowabs(int n, const int *rp, const double *val, double *out, cudaStream_t st);

@@ -750,35 +750,76 @@ __global__ void __launch_bounds__(ST, NS == CHAIN_NS_SMALL ? 2 : 1) k_bwd_chain(
   cluster_sync_all();
 }
 
-// y = A x for the symmetric matrix held as full CSR (both triangles), nrhs vectors.
-__global__ void __launch_bounds__(256) k_spmv(int n, const int *rp, const int *ci,
-                                              const double *val, const double *x, double *y,
-                                              int nrhs) {
-  // eight lanes per row (rows of a stencil matrix hold 7 to 81 entries: a warp per row
-  // left most lanes idle), 32 rows per CTA; the eight partial sums meet by shuffles
-  const int row = blockIdx.x * 32 + (int)(threadIdx.x >> 3);
+// y = A x, or b - A x where b is given, for the symmetric matrix held as full CSR (both triangles).
+// Eight lanes per row (rows of a stencil matrix hold 7 to 81 entries) and four rows per group of
+// eight lanes at the same time: bound by the trips to memory (row pointers, entries, x), and most
+// rows are over after one or two steps.
+__global__ void __launch_bounds__(256) k_spmv(int n, const int *rp, const int *ci, const double *val,
+                                              const double *x, const double *b, double *y) {
+  constexpr int RW = 4;
+  const int row0 = (blockIdx.x * 32 + (int)(threadIdx.x >> 3)) * RW;
   const int sub = threadIdx.x & 7;
-  const bool ok = row < n;
-  const int p0 = ok ? rp[row] : 0, p1 = ok ? rp[row + 1] : 0;
-  // four vectors per pass over the matrix
-  for (int r0 = 0; r0 < nrhs; r0 += 4) {
-    const int nr = min(4, nrhs - r0);
-    const double *xr = x + (size_t)r0 * n;
-    double acc[4] = {0.0, 0.0, 0.0, 0.0};
-    for (int p = p0 + sub; p < p1; p += 8) {
-      const double v = val[p];
-      const int c = ci[p];
+  int p0[RW], p1[RW], longest = 0;
 #pragma unroll
-      for (int u = 0; u < 4; ++u)
-        if (u < nr) acc[u] = fma(v, xr[(size_t)u * n + c], acc[u]);
+  for (int i = 0; i < RW; ++i) {
+    p0[i] = rp[min(row0 + i, n)];
+    p1[i] = rp[min(row0 + i + 1, n)];
+    longest = max(longest, p1[i] - p0[i]);
+  }
+  double acc[RW] = {0.0, 0.0, 0.0, 0.0};
+  for (int q = sub; q < longest; q += 8) {
+    double v[RW];
+    int c[RW];
+#pragma unroll
+    for (int i = 0; i < RW; ++i) {
+      v[i] = ld_if(val + p0[i] + q, p0[i] + q < p1[i]);
+      c[i] = p0[i] + q < p1[i] ? ci[p0[i] + q] : -1;
     }
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      acc[u] += __shfl_xor_sync(0xffffffffu, acc[u], 4);
-      acc[u] += __shfl_xor_sync(0xffffffffu, acc[u], 2);
-      acc[u] += __shfl_xor_sync(0xffffffffu, acc[u], 1);
-      if (ok && sub == 0 && u < nr) y[(size_t)(r0 + u) * n + row] = acc[u];
+    for (int i = 0; i < RW; ++i) acc[i] = fma(v[i], ld_if(x + c[i], c[i] >= 0), acc[i]);
+  }
+#pragma unroll
+  for (int i = 0; i < RW; ++i) {
+    double t = acc[i];
+    t += __shfl_xor_sync(0xffffffffu, t, 4);
+    t += __shfl_xor_sync(0xffffffffu, t, 2);
+    t += __shfl_xor_sync(0xffffffffu, t, 1);
+    if (row0 + i < n && sub == 0) y[row0 + i] = b ? b[row0 + i] - t : t;
+  }
+}
+
+// The same for nr <= 8 vectors, x interleaved by eight: lane u of a group takes vector u, so an
+// entry costs one 64-byte piece of x instead of eight pieces of as many vectors; the group's lanes
+// load eight entries and pass them around (the next eight on the way).  36 x 35 x 33 elastic operator,
+// eight vectors: 85 + 5 us (product by vectors, then the difference) -> 72 + 4 (interleaving).
+__global__ void __launch_bounds__(256) k_spmv8(int n, const int *rp, const int *ci, const double *val,
+                                               const double *x8, const double *b, double *y, int nr) {
+  const int row = blockIdx.x * 32 + (int)(threadIdx.x >> 3), u = threadIdx.x & 7;
+  const int p0 = rp[min(row, n)], p1 = rp[min(row + 1, n)];
+  const int steps = __reduce_max_sync(0xffffffffu, (p1 - p0 + 7) >> 3);
+  double a0 = 0.0, a1 = 0.0;
+  double vn = ld_if(val + p0 + u, p0 + u < p1);   // the next step's entries
+  int cn = p0 + u < p1 ? ci[p0 + u] : -1;
+  for (int t = 0; t < steps; ++t) {
+    const int p = p0 + 8 * (t + 1) + u, c = cn;
+    const double v = vn;
+    vn = ld_if(val + p, p < p1);
+    cn = p < p1 ? ci[p] : -1;
+    double xv[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const int ck = __shfl_sync(0xffffffffu, c, k, 8);
+      xv[k] = ld_if(x8 + (int64_t)ck * 8 + u, ck >= 0);
     }
+#pragma unroll
+    for (int k = 0; k < 8; k += 2) {
+      a0 = fma(__shfl_sync(0xffffffffu, v, k, 8), xv[k], a0);
+      a1 = fma(__shfl_sync(0xffffffffu, v, k + 1, 8), xv[k + 1], a1);
+    }
+  }
+  if (row < n && u < nr) {
+    const size_t at = (size_t)u * n + row;
+    y[at] = b ? b[at] - (a0 + a1) : a0 + a1;
   }
 }
 
@@ -797,12 +838,6 @@ __global__ void k_gather_vals(int nnz, const int *map, const double *ax, double 
   if (i < nnz) val[i] = ax[map[i]];
 }
 
-// r = b - r (r holds A x on entry)
-__global__ void k_residual(size_t len, const double *b, double *r) {
-  size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < len) r[i] = b[i] - r[i];
-}
-
 // p = z + beta p
 __global__ void k_xpby(size_t len, const double *z, double beta, double *p) {
   size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -814,14 +849,16 @@ __global__ void k_axpy(size_t len, double a, const double *x, double *y) {
   if (i < len) y[i] = fma(a, x[i], y[i]);
 }
 
-// per-vector max |x| and sum x*y for nrhs vectors of length n (out[2*r], out[2*r+1]),
+// per-vector max |x| and sum x*y for nrhs vectors of length n (out[2*r], out[2*r+1]), then (x2 given)
+// max |x2| of as many more,
 // deterministic: NORM_BLOCKS fixed slices per vector, then one CTA per vector sums the
 // slices in order.
 constexpr int NORM_BLOCKS = 128;
-__global__ void k_norms_part(int n, const double *x, const double *y, double *part) {
+__global__ void k_norms_part(int n, int nrhs, const double *x, const double *y, const double *x2, double *part) {
   __shared__ double smax[ST], sdot[ST];
   const int r = blockIdx.y, b = blockIdx.x;
-  const double *xr = x + (size_t)r * n, *yr = y ? y + (size_t)r * n : nullptr;
+  const double *xr = r < nrhs ? x + (size_t)r * n : x2 + (size_t)(r - nrhs) * n;
+  const double *yr = y && r < nrhs ? y + (size_t)r * n : nullptr;
   const int per = (n + NORM_BLOCKS - 1) / NORM_BLOCKS;
   const int lo = b * per, hi = min(n, lo + per);
   double mx = 0.0, dt = 0.0;
@@ -957,9 +994,13 @@ void launch_bwd_chain(const DevSym &S, const int2 *tasks, int count, double *x, 
     launch_early(st, CHAIN_CL, k_bwd_chain<CHAIN_NS_SMALL>, grid, ST, chain_smem(CHAIN_NS_SMALL, CHAIN_XW_BWD), S,
                  tasks, count, x, flags, epoch);
 }
-void launch_spmv(int n, const int *rp, const int *ci, const double *val, const double *x,
-                 double *y, int nrhs, cudaStream_t st) {
-  k_spmv<<<(n + 31) / 32, 256, 0, st>>>(n, rp, ci, val, x, y, nrhs);
+void launch_spmv(int n, const int *rp, const int *ci, const double *val, const double *x, const double *b,
+                 double *y, cudaStream_t st) {
+  k_spmv<<<(n + 127) / 128, 256, 0, st>>>(n, rp, ci, val, x, b, y);
+}
+void launch_spmv8(int n, const int *rp, const int *ci, const double *val, const double *x8, const double *b,
+                  double *y, int nr, cudaStream_t st) {
+  k_spmv8<<<(n + 31) / 32, 256, 0, st>>>(n, rp, ci, val, x8, b, y, nr);
 }
 void launch_gather_vals(int nnz, const int *map, const double *ax, double *val, cudaStream_t st) {
   if (nnz > 0) k_gather_vals<<<(nnz + 255) / 256, 256, 0, st>>>(nnz, map, ax, val);
@@ -967,20 +1008,18 @@ void launch_gather_vals(int nnz, const int *map, const double *ax, double *val, 
 void launch_rowabs(int n, const int *rp, const double *val, double *out, cudaStream_t st) {
   k_rowabs<<<(n + 255) / 256, 256, 0, st>>>(n, rp, val, out);
 }
-void launch_residual(size_t len, const double *b, double *r, cudaStream_t st) {
-  if (len) k_residual<<<(unsigned)((len + 255) / 256), 256, 0, st>>>(len, b, r);
-}
 void launch_xpby(size_t len, const double *z, double beta, double *p, cudaStream_t st) {
   if (len) k_xpby<<<(unsigned)((len + 255) / 256), 256, 0, st>>>(len, z, beta, p);
 }
 void launch_axpy(size_t len, double a, const double *x, double *y, cudaStream_t st) {
   if (len) k_axpy<<<(unsigned)((len + 255) / 256), 256, 0, st>>>(len, a, x, y);
 }
-void launch_norms(int n, int nrhs, const double *x, const double *y, double *out, double *part,
+void launch_norms(int n, int nrhs, const double *x, const double *y, const double *x2, double *out, double *part,
                   cudaStream_t st) {
-  k_norms_part<<<dim3(NORM_BLOCKS, nrhs), ST, 0, st>>>(n, x, y, part);
-  k_norms_final<<<nrhs, NORM_BLOCKS, 0, st>>>(part, out);
+  const int sets = x2 ? 2 * nrhs : nrhs;
+  k_norms_part<<<dim3(NORM_BLOCKS, sets), ST, 0, st>>>(n, nrhs, x, y, x2, part);
+  k_norms_final<<<sets, NORM_BLOCKS, 0, st>>>(part, out);
 }
-int norm_scratch_doubles(int nrhs) { return 2 * NORM_BLOCKS * nrhs; }
+int norm_scratch_doubles(int nrhs) { return 4 * NORM_BLOCKS * nrhs; }
 
 }  // namespace swc

@@ -49,3 +49,26 @@ def test_widths(cuda_ok, max_width):
 @pytest.mark.parametrize("n,max_width", [(1, 1), (33, 33), (64, 64), (65, 64), (190, 64), (2053, 5)])
 def test_dense(cuda_ok, n, max_width):
     solve_both(dense_spd(n, n), np.arange(n), max_width)
+
+
+@pytest.mark.parametrize("nrhs", [1, 2, 4, 5, 8, 9])
+@pytest.mark.parametrize("dense", [False, True])
+def test_residuals(cuda_ok, dense, nrhs):
+    """The backward errors that a refinement reports (its residuals take one, four or eight vectors
+    per pass, rows of 4 to 190 entries, a row count that no block divides) against the same norms in
+    numpy: each residual entry is a sum of at most n + 1 terms, so both are within (n + 2) 2^-53 of
+    the exact value, relative to max |A| row sum times max |x|."""
+    A, perm = (dense_spd(190, 3), np.arange(190)) if dense else (M.laplacian_2d(29), M.nested_dissection((29, 29)))
+    P = W.assemble_own(A, perm)
+    h = swc.Handle(0)
+    h.analyze(P.n, P.A2p, P.A2i, P.lC, P.Ls, P.Li_ptr, P.super, P.prunePtr, P.pruneSet)
+    assert h.factor(P.A2x) == 0
+    D = np.zeros((P.n, P.n))
+    cols = np.repeat(np.arange(P.n), np.diff(P.A2p))
+    D[P.A2i, cols] = P.A2x
+    D[cols, P.A2i] = P.A2x
+    B = np.random.default_rng(7).standard_normal((P.n, nrhs))
+    X, berr, _, _ = h.refine(B if nrhs > 1 else B[:, 0], tol=1e-14)
+    X = np.asarray(X).reshape(P.n, -1)
+    want = np.abs(B - D @ X).max(0) / (np.abs(D).sum(1).max() * np.abs(X).max(0))
+    assert np.abs(np.asarray(berr) - want).max() <= 2 * (P.n + 2) * 2.0 ** -53
