@@ -415,10 +415,10 @@ def run_ours(args, rank, world, local_rank):
         cls_kernel = {"update": ("k_update_tc", peak32 / 8.0, src_bf16),
                       "syrk": ("k_syrk_step", peak64, src64)}
     else:
-        cls_kernel = {"update": ("k_update_tiles", peak64, src64),
+        cls_kernel = {"update": ("k_front_extend + k_front_schur", peak64, src64),
                       "syrk": ("k_syrk_step", peak64, src64)}
     cls_kernel["panel"] = ("k_diag_step + k_trsm_step", peak64, src64)
-    cls_kernel["small"] = ("k_factor_small*", peak64, src64)
+    cls_kernel["small"] = ("k_factor_small*" if mixed else "k_front_*", peak64, src64)
     # the dominant kernel: classes grouped by the kernel that runs them (the split-TF32 scatter
     # kernel runs both the descendant updates and the trailing SYRK steps); the panel class is
     # two kernels (TRSM, diagonal block) of about equal share

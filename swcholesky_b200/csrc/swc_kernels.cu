@@ -1,4 +1,5 @@
-// FP64 kernels of the supernodal numeric factorization.
+// FP64 kernels of the supernodal numeric factorization (the multifrontal fronts and contribution
+// blocks of the FP64 mode are in swc_front.cu).
 //
 // The work of the reference executor (cholesky/sw_parallel_PB_Cholesky_05.c:209-484) is
 // split by supernode size class:
@@ -6,21 +7,22 @@
 //   k_factor_small   one CTA factors one supernode whose panel fits in shared memory:
 //                    assembly of A (.c:211-224), every update from its prune set with the
 //                    relative-index scatter fused in (.c:254-378), then POTRF and TRSM on
-//                    the panel (.c:419-484).  Many such CTAs run per level.
+//                    the panel (.c:419-484).  Many such CTAs run per level.  Mixed modes, and
+//                    FP64 where the multifrontal plan does not apply.
 //   k_assemble       copies A's columns into the panels of the tiled class.
-//   k_update_tiles   tile-owner left-looking update: each CTA owns a 64x64 tile of a
-//                    target panel and accumulates, in shared memory, the contribution of
-//                    every descendant in the prune set (the SYRK/GEMM of .c:299-359 limited
-//                    to the tile, scattered through relative indices, .c:364-378); the tile
-//                    is written once.  Deterministic: no atomics, fixed update order.
+//   k_update_tiles   tile-owner left-looking update, for FP64 where the multifrontal plan does
+//                    not apply: each CTA owns a 64x64 tile of a target panel and accumulates
+//                    the contribution of every descendant in the prune set (the SYRK/GEMM of
+//                    .c:299-359 limited to the tile, scattered through relative indices,
+//                    .c:364-378); the tile is written once.  Deterministic: no atomics, fixed
+//                    update order.
 //   k_diag_step,     blocked right-looking dense factorization of a wide supernode by
 //   k_trsm_step,     64-column blocks: per block, POTRF of the diagonal block (and its
 //   k_syrk_step      inverse), the TRSM of the tiles below it as a DMMA product with that
-//                    inverse, and the trailing SYRK/GEMM update; the next diagonal block's
-//                    update and POTRF run concurrently with that trailing update.
+//                    inverse, and the trailing SYRK/GEMM update; the next diagonal block
+//                    solves its own rows and is updated and factored beside both.
 //
-// All arithmetic is FP64; tiles are 64x64 with 256 threads, each thread holding a 4x4
-// register micro-tile.
+// All arithmetic is FP64; tiles are 64x64 on 128 threads (DMMA, see swc_tile.h).
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -61,26 +63,9 @@ __device__ __forceinline__ Bf16x3 split_bf16x3(double x) {
   return Bf16x3{__bfloat16_as_ushort(hi), __bfloat16_as_ushort(mid), __bfloat16_as_ushort(lo)};
 }
 
-// The mirror entries of value x of row r, column c of supernode s (m rows, w columns), in
-// the K-major split mirror at (float *)Lf + xk[s], format xk[nsuper]: 0, hi / lo TF32
-// planes; 1, hi / mid / lo bfloat16 planes (row pitch kmirror_pitch_tf32 / _bf16 (w)).
-__device__ __forceinline__ void store_mirror(const DevSym &S, int s, int m, int w, int r, int c,
-                                             double x) {
-  float *base = reinterpret_cast<float *>(S.Lf) + S.xk[s];
-  if (S.xk[S.nsuper] == 0) {
-    const int wp = kmirror_pitch_tf32(w);
-    const float2 v = split_tf32(x);
-    base[(size_t)r * wp + c] = v.x;
-    base[((size_t)m + r) * wp + c] = v.y;
-  } else {
-    const int wq = kmirror_pitch_bf16(w);
-    unsigned short *b = reinterpret_cast<unsigned short *>(base);
-    const Bf16x3 v = split_bf16x3(x);
-    b[(size_t)r * wq + c] = v.hi;
-    b[((size_t)m + r) * wq + c] = v.mid;
-    b[((size_t)2 * m + r) * wq + c] = v.lo;
-  }
-}
+// The K-major split mirror of supernode s (m rows, w columns) is at (float *)Lf + xk[s], format
+// xk[nsuper]: 0, hi / lo TF32 planes; 1, hi / mid / lo bfloat16 planes (row pitch
+// kmirror_pitch_tf32 / _bf16 (w)).
 
 // The whole m x w panel P (column-major, ld m) of supernode s into the mirror; threads
 // t, t + nt, ... (consecutive threads write consecutive mirror entries of a row).
