@@ -3,7 +3,6 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <queue>
 #include <climits>
 #include <cstdlib>
 #include <cstring>
@@ -1093,23 +1092,25 @@ static bool solve_halves(int supNo, const std::vector<int> &parent, const std::v
                          const std::vector<int64_t> &rowptr, std::vector<char> &half) {
   std::vector<int64_t> weight(supNo);
   std::vector<std::vector<int>> child(supNo);
-  std::priority_queue<std::pair<int64_t, int>> open;
+  std::vector<std::pair<int64_t, int>> open;   // the subtrees' roots, by weight
   for (int s = 0; s < supNo; ++s) weight[s] = (rowptr[s + 1] - rowptr[s]) * (super[s + 1] - super[s]);
-  for (int s = 0; s < supNo; ++s)   // parents have larger numbers
+  for (int s = 0; s < supNo; ++s) {   // parents have larger numbers
     if (parent[s] >= 0) {
       weight[parent[s]] += weight[s];
       child[parent[s]].push_back(s);
+    } else {
+      open.emplace_back(weight[s], s);
     }
-  for (int s = 0; s < supNo; ++s)
-    if (parent[s] < 0) open.push({weight[s], s});
+  }
   for (int k = 0; k <= SOLVE_TOP && !open.empty(); ++k) {
+    std::sort(open.begin(), open.end());
     // the heaviest first, to the lighter half
     int64_t sum[2] = {0, 0};
     half.assign(supNo, 2);
-    for (auto rest = open; !rest.empty(); rest.pop()) {
+    for (size_t q = open.size(); q-- > 0;) {
       const int h = sum[1] < sum[0];
-      sum[h] += rest.top().first;
-      half[rest.top().second] = (char)h;
+      sum[h] += open[q].first;
+      half[open[q].second] = (char)h;
     }
     const int64_t light = std::min(sum[0], sum[1]), all = sum[0] + sum[1];
     if (all < 2 * SOLVE_HALF_MIN) return false;
@@ -1118,9 +1119,9 @@ static bool solve_halves(int supNo, const std::vector<int> &parent, const std::v
         if (half[s] == 2 && parent[s] >= 0) half[s] = half[parent[s]];
       return true;
     }
-    const int top = open.top().second;
-    open.pop();
-    for (int c : child[top]) open.push({weight[c], c});
+    const int top = open.back().second;
+    open.pop_back();
+    for (int c : child[top]) open.emplace_back(weight[c], c);
   }
   return false;
 }
