@@ -2257,7 +2257,7 @@ void Engine::solve_levels(double *x, int nrhs, double *contrib, int l0, int l1, 
     for (int r = 0; r < nrhs; ++r)
       launch_fwd_chain(sym_, d_fchain_ + SP.chain_off[l], SP.chain_off[l + 1] - SP.chain_off[l],
                        x + (size_t)r * n_, contrib + (size_t)r * cs, d_cptr_, d_cidx_, d_flags_,
-                       r + 1, n_, cs, st);
+                       r + 1, n_, cs, l < SP.half1, st);
     launch_fwd_contrib(sym_, d_scontrib_ + SP.contrib_off[l], SP.contrib_off[l + 1] - SP.contrib_off[l],
                        SP.contrib_big[l], x, contrib, n_, nrhs, cs, st);
   }
@@ -2270,7 +2270,7 @@ void Engine::solve_levels(double *x, int nrhs, double *contrib, int l0, int l1, 
                     nrhs, st);
     for (int r = 0; r < nrhs; ++r)
       launch_bwd_chain(sym_, d_bchain_ + SP.chain_off[l], SP.chain_off[l + 1] - SP.chain_off[l],
-                       x + (size_t)r * n_, d_flags_, nrhs + r + 1, st);
+                       x + (size_t)r * n_, d_flags_, nrhs + r + 1, l < SP.half1, st);
   }
 }
 

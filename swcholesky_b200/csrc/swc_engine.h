@@ -249,9 +249,9 @@ void launch_bwd_warp(const DevSym &S, const int *list, int count, double *x, int
                      LaunchQueue &st);
 void launch_fwd_chain(const DevSym &S, const int2 *tasks, int count, double *y,
                       const double *contrib, const int *cptr, const int *cidx, int *flags,
-                      int epoch, int n, int64_t cstride, LaunchQueue &st);
+                      int epoch, int n, int64_t cstride, bool beside, LaunchQueue &st);
 void launch_bwd_chain(const DevSym &S, const int2 *tasks, int count, double *x, int *flags,
-                      int epoch, LaunchQueue &st);
+                      int epoch, bool beside, LaunchQueue &st);
 // y = A x, or b - A x where b is given; the second for nr <= 8 vectors, x interleaved by eight
 void launch_spmv(int n, const int *rp, const int *ci, const double *val, const double *x, const double *b,
                  double *y, cudaStream_t st);

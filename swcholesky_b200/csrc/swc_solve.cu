@@ -902,8 +902,9 @@ __global__ void k_norms_final(const double *part, double *out) {
 
 }  // namespace
 
-// the chains' grids: whole clusters of CHAIN_CL CTAs; launches that fit the SMs at one CTA
-// each take the deep ring
+// the chains' grids: whole clusters of CHAIN_CL CTAs; launches that fit the SMs at one CTA each take
+// the deep ring, which fills an SM's shared memory; beside the other half of the tree, those that
+// leave it half of the SMs (solve of the 60^3 grid: all SMs 1049 us, half 1027, none 1072)
 static int g_num_sms = 148;
 static int chain_grid(int count) { return (count + CHAIN_CL - 1) / CHAIN_CL * CHAIN_CL; }
 
@@ -973,10 +974,10 @@ void launch_bwd_small(const DevSym &S, const int *list, int count, int smem, dou
 }
 void launch_fwd_chain(const DevSym &S, const int2 *tasks, int count, double *y,
                       const double *contrib, const int *cptr, const int *cidx, int *flags,
-                      int epoch, int n, int64_t cstride, LaunchQueue &st) {
+                      int epoch, int n, int64_t cstride, bool beside, LaunchQueue &st) {
   if (count <= 0) return;
   const int grid = chain_grid(count);
-  if (grid <= g_num_sms)
+  if (grid <= (beside ? g_num_sms / 2 : g_num_sms))
     launch_early(st, CHAIN_CL, k_fwd_chain<CHAIN_NS_BIG>, grid, ST, chain_smem(CHAIN_NS_BIG, CHAIN_XW_FWD), S,
                  tasks, count, y, contrib, cptr, cidx, flags, epoch, n, cstride);
   else
@@ -984,10 +985,10 @@ void launch_fwd_chain(const DevSym &S, const int2 *tasks, int count, double *y,
                  tasks, count, y, contrib, cptr, cidx, flags, epoch, n, cstride);
 }
 void launch_bwd_chain(const DevSym &S, const int2 *tasks, int count, double *x, int *flags,
-                      int epoch, LaunchQueue &st) {
+                      int epoch, bool beside, LaunchQueue &st) {
   if (count <= 0) return;
   const int grid = chain_grid(count);
-  if (grid <= g_num_sms)
+  if (grid <= (beside ? g_num_sms / 2 : g_num_sms))
     launch_early(st, CHAIN_CL, k_bwd_chain<CHAIN_NS_BIG>, grid, ST, chain_smem(CHAIN_NS_BIG, CHAIN_XW_BWD), S,
                  tasks, count, x, flags, epoch);
   else
