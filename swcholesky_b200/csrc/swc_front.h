@@ -10,9 +10,11 @@
 // factor is reproducible bit for bit.  Against the left-looking kernels (B200, ms per
 // factorization): 5-point grids 20 x 20 0.50 -> 0.13, 100 x 100 1.81 -> 0.42; 7-point grids
 // 41 x 37 x 43 5.43 -> 3.41, 60^3 24.7 -> 16.3 (the descendants' updates 16.3 -> 6.4);
-// 3-unknown 27-point grid 24 x 23 x 22 5.56 -> 3.60.  The blocks alive at once take about as
-// much memory as L; the left-looking kernels remain for handles that cannot have it, for prune
-// sets that are not the complete descendant lists, and for the mixed modes.
+// 3-unknown 27-point grid 24 x 23 x 22 5.56 -> 3.60.  The blocks alive at once take once to twice
+// the memory of L on grids and geometric graphs, but r x r doubles per front whatever its width:
+// many narrow supernodes under a wide border would take hundreds of times L, and stay left-looking
+// (front_memory_limit).  So do handles that cannot have the memory, prune sets that are not the
+// complete descendant lists, and the mixed modes.
 #pragma once
 #include <cuda_runtime.h>
 
@@ -52,6 +54,15 @@ __host__ __device__ inline int adj_ldt(int w) { return front_wp(w) + ((4 - front
 inline int64_t adj_small_smem(int w, int64_t m, bool y_global) {
   const int64_t pe = (int64_t)front_wp(w) * front_ld(w, (int)m);
   return 8 * (pe + (pe > 512 && !y_global ? pe : 512) + (int64_t)front_wp(w) * adj_ldt(w)) + 4 * (m + 1);
+}
+
+// Doubles that blocks alive together may take: four times L (measured: 5-point grids up to 2.2
+// times, 7-point 1.0 to 2.0, 3-unknown 27-point 1.2 to 3.3, random geometric graphs 0.8 to 1.3), or
+// 256 MB where L is small.  Beyond are bordered structures: 4,000 columns under a border of 1,000 take
+// 800 times L.
+inline int64_t front_memory_limit(int64_t xsize) {
+  const int64_t floor = (int64_t)1 << 25;
+  return 4 * xsize > floor ? 4 * xsize : floor;
 }
 
 // First-fit placement of blocks that live over a range of waves.
@@ -130,7 +141,8 @@ struct FrontPlan {
 
 // Derives the multifrontal plan of an analysed structure.  P.ok stays false, and the
 // left-looking kernels are used, when the prune sets are not exactly the descendants that
-// touch each supernode or a child's rows are not among its parent's.
+// touch each supernode, a child's rows are not among its parent's, or the blocks would take more
+// than front_memory_limit.
 void build_front_plan(int n, const int *c, const int *r, const int *Ls, const int *prunePtr,
                       const int *pruneSet, const HostSym &H, const Plan &P, const Tuning &T,
                       FrontPlan &F);

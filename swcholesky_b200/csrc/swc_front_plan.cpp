@@ -157,6 +157,30 @@ void build_front_plan(int n, const int *c, const int *r, const int *Ls, const in
   std::vector<std::vector<int>> by_level(nlev);
   for (int s = 0; s < ns; ++s) by_level[level[s]].push_back(s);
 
+  // contribution blocks: a block lives from its supernode's wave (the walks': from the start)
+  // to the end of its parent's wave (the walks': the end of the walks)
+  F.cb_off.assign(ns, 0);
+  FrontArena A;
+  auto len = [&](int s) {
+    const int64_t rr = rows(s) - width(s);
+    return (rr * rr + 15) & ~(int64_t)15;
+  };
+  auto walk = [&](int s) { return in_warp[s] || in_cta[s]; };
+  for (int s = 0; s < ns; ++s)
+    if (walk(s) && len(s)) F.cb_off[s] = A.take(len(s));
+  for (int s = 0; s < ns; ++s)
+    if (walk(s) && len(s) && walk(parent[s])) A.give(F.cb_off[s], len(s));
+  for (int lv = 0; lv < nlev; ++lv) {
+    for (int s : by_level[lv])
+      if (!walk(s) && len(s)) F.cb_off[s] = A.take(len(s));
+    for (int s : by_level[lv])
+      if (!walk(s))
+        for (int q = F.child_ptr[s]; q < F.child_ptr[s + 1]; ++q)
+          A.give(F.cb_off[F.child[q]], len(F.child[q]));
+  }
+  F.cb_len = A.end();
+  if (F.cb_len > front_memory_limit(H.xsize)) return;
+
   // tasks: the tiles of s's list with origin o (positions o + 64 t of its rows; columns up to
   // clim) and the pairs of children's rows that fall in each; tiles without pairs only if `all`
   struct Run { int tile, start, count; };
@@ -273,29 +297,6 @@ void build_front_plan(int n, const int *c, const int *r, const int *Ls, const in
   }
   F.launches = launches + !F.warp_list.empty() + !F.cta_list.empty();
 
-  // contribution blocks: a block lives from its supernode's wave (the walks': from the start)
-  // to the end of its parent's wave (the walks': the end of the walks)
-  F.cb_off.assign(ns, 0);
-  FrontArena A;
-  auto len = [&](int s) {
-    const int64_t rr = rows(s) - width(s);
-    return (rr * rr + 15) & ~(int64_t)15;
-  };
-  auto walk = [&](int s) { return in_warp[s] || in_cta[s]; };
-  for (int s = 0; s < ns; ++s)
-    if (walk(s) && len(s)) F.cb_off[s] = A.take(len(s));
-  for (int s = 0; s < ns; ++s)
-    if (walk(s) && len(s) && walk(parent[s])) A.give(F.cb_off[s], len(s));
-  for (int lv = 0; lv < nlev; ++lv) {
-    for (int s : by_level[lv])
-      if (!walk(s) && len(s)) F.cb_off[s] = A.take(len(s));
-    for (int s : by_level[lv])
-      if (!walk(s))
-        for (int q = F.child_ptr[s]; q < F.child_ptr[s + 1]; ++q)
-          A.give(F.cb_off[F.child[q]], len(F.child[q]));
-  }
-  F.cb_len = A.end();
-
   // descriptors, and the entries of A of the small fronts in their padded panels
   for (int d : F.child)
     F.kids.push_back(FrontChild{d, rows(d) - width(d), F.child_n1[d], 0, rowptr[d] - super[d], F.cb_off[d]});
@@ -329,6 +330,7 @@ bool check_front_plan(int n, const int *Ls, const HostSym &H, const Plan &P, con
   if ((int)F.child_ptr.size() != ns + 1 || F.waves.size() != P.waves.size() ||
       (int64_t)F.rel.size() < H.nls - n)
     return bad("array sizes", -1);
+  if (F.cb_len > front_memory_limit(H.xsize)) return bad("contribution blocks larger than their bound", -1);
   // the children's maps
   std::vector<int> parent(ns, -1), level(ns, 0);
   for (int s = 0; s < ns; ++s)
