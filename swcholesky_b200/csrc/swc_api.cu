@@ -46,6 +46,14 @@ void set_last_error(const std::string &msg) { g_err = msg; }
 }  // namespace swc
 
 namespace {
+// Device memory for one call; what the handle can do without is given back if need be.
+cudaError_t device_alloc(swc_handle_t h, double **p, size_t bytes) {
+  cudaError_t e = cudaMalloc(p, std::max<size_t>(bytes, 8));
+  if (e != cudaSuccess && h->eng->make_room()) e = cudaMalloc(p, std::max<size_t>(bytes, 8));
+  if (e != cudaSuccess) *p = nullptr;
+  return e;
+}
+
 // Runs fn on device copies of host right-hand sides (and copies x back) when needed; the
 // copies go through the handle's staging buffer (allocated once, grown on demand).
 template <typename F>
@@ -217,7 +225,7 @@ int swc_logdet_grad(swc_handle_t h, double *grad, int on_device) {
   std::string err;
   const size_t bytes = sizeof(double) * (size_t)h->eng->nnz();
   double *dg = grad;
-  if (!on_device && cudaMalloc(&dg, std::max<size_t>(bytes, 8)) != cudaSuccess)
+  if (!on_device && device_alloc(h, &dg, bytes) != cudaSuccess)
     return fail(SWC_CUDA_ERROR, "gradient buffer");
   int rc = SWC_OK;
   if (!h->eng->logdet_grad(dg, err)) rc = fail(SWC_CUDA_ERROR, err);
@@ -239,9 +247,9 @@ int swc_solve_grad(swc_handle_t h, const double *x, const double *lam, double *g
     return SWC_OK;
   }
   double *dx = nullptr, *dl = nullptr, *dg = nullptr;
-  cudaError_t e = cudaMalloc(&dx, vbytes);
-  if (e == cudaSuccess) e = cudaMalloc(&dl, vbytes);
-  if (e == cudaSuccess) e = cudaMalloc(&dg, std::max<size_t>(gbytes, 8));
+  cudaError_t e = device_alloc(h, &dx, vbytes);
+  if (e == cudaSuccess) e = device_alloc(h, &dl, vbytes);
+  if (e == cudaSuccess) e = device_alloc(h, &dg, gbytes);
   if (e == cudaSuccess) e = cudaMemcpy(dx, x, vbytes, cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemcpy(dl, lam, vbytes, cudaMemcpyHostToDevice);
   int rc = SWC_OK;
@@ -280,7 +288,7 @@ int swc_batch_autotune(swc_handle_t h, const double *values, int values_on_devic
   const double *dv = values;
   double *tmp = nullptr;
   if (!values_on_device) {
-    if (cudaMalloc(&tmp, std::max<size_t>(bytes, 8)) != cudaSuccess ||
+    if (device_alloc(h, &tmp, bytes) != cudaSuccess ||
         cudaMemcpy(tmp, values, bytes, cudaMemcpyHostToDevice) != cudaSuccess) {
       if (tmp) cudaFree(tmp);
       return fail(SWC_CUDA_ERROR, "autotune: values upload failed");
@@ -309,8 +317,8 @@ int swc_batch_berr(swc_handle_t h, const double *b, const double *x, int on_devi
   const double *db = b, *dx = x;
   double *tb = nullptr, *tx = nullptr;
   if (!on_device) {
-    cudaError_t e = cudaMalloc(&tb, bytes);
-    if (e == cudaSuccess) e = cudaMalloc(&tx, bytes);
+    cudaError_t e = device_alloc(h, &tb, bytes);
+    if (e == cudaSuccess) e = device_alloc(h, &tx, bytes);
     if (e == cudaSuccess) e = cudaMemcpy(tb, b, bytes, cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemcpy(tx, x, bytes, cudaMemcpyHostToDevice);
     if (e != cudaSuccess) {

@@ -129,12 +129,8 @@ cudaError_t DeviceMemory::take(void **p, size_t bytes) {
     return cudaSuccess;
   }
   cudaError_t e = cudaMalloc(p, bytes);
-  if (e != cudaSuccess) {   // the free blocks may be what is missing
-    cudaGetLastError();
-    for (Block &b : blocks_) b.old = true;
-    sweep();
-    e = cudaMalloc(p, bytes);
-  }
+  if (e != cudaSuccess && make_room()) e = cudaMalloc(p, bytes);
+  if (e != cudaSuccess) cudaGetLastError();
   if (e == cudaSuccess) blocks_.push_back({*p, bytes, true, false});
   else *p = nullptr;
   return e;
@@ -146,6 +142,15 @@ void DeviceMemory::give(void *p) {
       b.used = b.old = false;
       return;
     }
+}
+
+bool DeviceMemory::make_room() {
+  cudaGetLastError();   // of the allocation that failed
+  if (spare_) spare_();
+  const size_t held = blocks_.size();
+  for (Block &b : blocks_) b.old = true;
+  sweep();
+  return blocks_.size() < held;
 }
 
 void DeviceMemory::age() {
@@ -194,6 +199,7 @@ Engine::Engine(int device) : device_(device) {
   cudaDeviceGetAttribute(&num_sms_, cudaDevAttrMultiProcessorCount, device_);
   cudaEventCreateWithFlags(&ev_sfork_, cudaEventDisableTiming);
   cudaEventCreateWithFlags(&ev_sjoin_, cudaEventDisableTiming);
+  mem_.on_shortage([this] { drop_blocks(); });
   cudaMallocHost(&h_status_, kStatusWords * sizeof(int));
 }
 
@@ -1593,19 +1599,24 @@ bool Engine::analyze(int n, const int *c, const int *r, const int64_t *lC, const
   h_prune_ptr_.assign(prunePtr, prunePtr + supNo + 1);
   h_prune_.assign(pruneSet, pruneSet + nprune);
   front_ = FP;
-  // the contribution blocks, also the mixed modes' mirror when it fits (a factorization uses
-  // one or the other); without the memory the left-looking kernels stay
-  if (FP->ok) {
-    cb_bytes_ = sizeof(double) * (size_t)std::max<int64_t>(FP->cb_len, 1);
-    const size_t lk = sizeof(float) * (size_t)kmirror_len_;
-    if (lk <= cb_bytes_ + cb_bytes_ / 4) cb_bytes_ = std::max(cb_bytes_, lk);
-    if (mem_.get(d_cb_, cb_bytes_) != cudaSuccess) {
-      cudaGetLastError();
-      cb_bytes_ = 0;
-    }
-  }
   mem_.sweep();
   return true;
+}
+
+// Gives the contribution blocks' memory back for another allocation of the handle: from then on
+// its FP64 factorizations are left-looking.
+void Engine::drop_blocks() {
+  if (!d_cb_ || d_cb_ == reinterpret_cast<double *>(d_Lk_)) return;   // none, or also the mirror
+  cudaStreamSynchronize(stream_);
+  mem_.put(d_cb_);
+  cb_bytes_ = 0;
+  front_dev_.reset();
+  front_ready_ = false;   // front_tried_ stays
+  if (graph_exec_[0]) cudaGraphExecDestroy(graph_exec_[0]);
+  if (graph_[0]) cudaGraphDestroy(graph_[0]);
+  graph_exec_[0] = nullptr;
+  graph_[0] = nullptr;
+  ran_[0] = false;
 }
 
 void Engine::release_front() {
@@ -1657,14 +1668,17 @@ bool Engine::prepare_scatter(std::string &err) {
   return up.commit(mem_, tables_, stream_, err);
 }
 
-// The multifrontal plan's tables on the device, on the first FP64 factorization of a structure.
+// The multifrontal plan's tables and the contribution blocks' memory, on the first FP64
+// factorization of a structure; where they cannot be had the left-looking kernels stay.  The blocks
+// and the mixed modes' mirror take the same memory where one has room for the other (a
+// factorization uses one of them).
 bool Engine::prepare_front(std::string &err) {
   if (front_tried_) return front_ready_ || prepare_left(err);
   if (!front_ || !front_->ok) return prepare_left(err);
   front_tried_ = true;
   const FrontPlan &F = *front_;
-  if (!d_cb_) return prepare_left(err);
-  if (!prepare_tree(err)) return false;
+  std::string shortage;
+  if (!prepare_tree(shortage)) return prepare_left(err);
   TableUpload up;
   up.add(d_fwarp_, F.warp_desc);
   up.add(d_fcta_, F.cta_desc);
@@ -1678,7 +1692,17 @@ bool Engine::prepare_front(std::string &err) {
   up.add(d_fsch_end_, F.sch_end);
   up.add(d_fsch_pairs_, F.sch_pairs);
   up.add(d_fcb_off_, F.cb_off);
-  if (!up.commit(mem_, tables_, stream_, err)) return false;
+  if (!up.commit(mem_, tables_, stream_, shortage)) return prepare_left(err);
+  const size_t need = sizeof(double) * (size_t)std::max<int64_t>(F.cb_len, 1), lk = mirror_bytes();
+  if (d_Lk_ && need <= lk) {
+    d_cb_ = reinterpret_cast<double *>(d_Lk_);
+  } else {
+    cb_bytes_ = !d_Lk_ && lk <= need + need / 4 ? std::max(need, lk) : need;
+    if (mem_.get(d_cb_, cb_bytes_) != cudaSuccess) {
+      cb_bytes_ = 0;
+      return prepare_left(err);
+    }
+  }
   front_dev_ = std::make_shared<FrontDev>(
       FrontDev{d_fkids_, d_frel_, d_fppos_, d_fcb_off_, d_cb_});
   if (!F.warp_list.empty()) fwarp_ctas_ = front_warp_walk_ctas((int)F.warp_list.size());
@@ -1937,11 +1961,10 @@ void Engine::launch_all(std::vector<std::pair<int, cudaEvent_t>> *prof, int prec
 
 bool Engine::set_mode(int prec, std::string &err) {
   if (prec != 0 && (!prepare_scatter(err) || (plan_.sc_coff.empty() && !prepare_left(err)))) return false;
-  if (prec != 0 && !d_Lk_) {   // the K-major split mirror and its format arrays
-    const size_t lk_bytes = sizeof(float) * (size_t)std::max<int64_t>(kmirror_len_, 8);
+  if (prec != 0 && !d_xk_) {   // the K-major split mirror and its format arrays
     cudaError_t e = cudaSuccess;
-    if (lk_bytes <= cb_bytes_) d_Lk_ = reinterpret_cast<float *>(d_cb_);
-    else e = mem_.get(d_Lk_, lk_bytes);
+    if (mirror_bytes() <= cb_bytes_) d_Lk_ = reinterpret_cast<float *>(d_cb_);
+    else if (!d_Lk_) e = mem_.get(d_Lk_, mirror_bytes());
     if (e != cudaSuccess) {
       err = std::string("mirror allocation: ") + cudaGetErrorString(e);
       return false;
@@ -2105,6 +2128,7 @@ double *Engine::staging(size_t doubles, std::string &err) {
     d_stage_ = nullptr;
     stage_len_ = 0;
     cudaError_t e = cudaMalloc(&d_stage_, sizeof(double) * doubles);
+    if (e != cudaSuccess && mem_.make_room()) e = cudaMalloc(&d_stage_, sizeof(double) * doubles);
     if (e != cudaSuccess) {
       d_stage_ = nullptr;
       err = std::string("staging buffer: ") + cudaGetErrorString(e);

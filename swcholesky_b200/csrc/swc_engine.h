@@ -3,7 +3,9 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
+#include <functional>
 #include <memory>
 #include <string>
 #include <vector>
@@ -33,10 +35,16 @@ class DeviceMemory {
   }
   void age();        // marks the blocks that are free now; sweep() frees those still free
   void sweep();
+  // Called first when an allocation fails: gives back what the engine can do without.
+  void on_shortage(std::function<void()> spare) { spare_ = std::move(spare); }
+  // After a failed allocation (any, also one elsewhere): frees every block not in use; false if there
+  // was none.
+  bool make_room();
 
  private:
   struct Block { void *p; size_t bytes; bool used, old; };
   std::vector<Block> blocks_;
+  std::function<void()> spare_;
   cudaError_t take(void **p, size_t bytes);
   void give(void *p);
 };
@@ -393,6 +401,9 @@ class Engine {
   // Device staging buffer of at least `doubles` entries (host-vector calls of the C ABI);
   // allocated on first use and grown when needed, freed with the engine.  nullptr on error.
   double *staging(size_t doubles, std::string &err);
+  // After a device allocation of the caller failed: frees what the handle can do without; false if
+  // there was nothing.
+  bool make_room() { return mem_.make_room(); }
   int64_t h2d_bytes() const { return h2d_bytes_; }
   int64_t d2h_bytes() const { return d2h_bytes_; }
   bool download(double *lValues, bool to_device, std::string &err);
@@ -469,7 +480,9 @@ class Engine {
   bool swept_ = false;                         // and the adjoint's sweep
   bool prepare_tree(std::string &err);   // the tree's tables (also the adjoint's)
   bool prepare_front(std::string &err);
+  void drop_blocks();
   void release_front();
+  size_t mirror_bytes() const { return sizeof(float) * (size_t)std::max<int64_t>(kmirror_len_, 8); }
   int finish(int *info, std::string &err);
   int64_t h2d_bytes_ = 0, d2h_bytes_ = 0;
   int wait_budget_ = kDefaultWaitBudget;
