@@ -121,7 +121,8 @@ cudaError_t DeviceMemory::take(void **p, size_t bytes) {
   bytes = std::max<size_t>((bytes + 255) & ~(size_t)255, 256);
   Block *best = nullptr;
   for (Block &b : blocks_)
-    if (!b.used && b.bytes >= bytes && b.bytes <= 2 * bytes + (1 << 16) && (!best || b.bytes < best->bytes))
+    if (!b.used && b.bytes >= bytes && b.bytes <= bytes + bytes / 8 + (1 << 16) &&
+        (!best || b.bytes < best->bytes))
       best = &b;
   if (best) {
     best->used = true;
@@ -130,16 +131,23 @@ cudaError_t DeviceMemory::take(void **p, size_t bytes) {
   }
   cudaError_t e = cudaMalloc(p, bytes);
   if (e != cudaSuccess && make_room()) e = cudaMalloc(p, bytes);
-  if (e != cudaSuccess) cudaGetLastError();
-  if (e == cudaSuccess) blocks_.push_back({*p, bytes, true, false});
-  else *p = nullptr;
+  if (e == cudaSuccess) {
+    blocks_.push_back({*p, bytes, true});
+  } else {
+    cudaGetLastError();
+    *p = nullptr;
+  }
   return e;
 }
 
-void DeviceMemory::give(void *p) {
+void DeviceMemory::give(void *p, bool keep) {
   for (Block &b : blocks_)
     if (b.p == p) {
-      b.used = b.old = false;
+      b.used = false;
+      if (!keep) {
+        cudaFree(b.p);
+        blocks_.erase(blocks_.begin() + (&b - blocks_.data()));
+      }
       return;
     }
 }
@@ -147,23 +155,29 @@ void DeviceMemory::give(void *p) {
 bool DeviceMemory::make_room() {
   cudaGetLastError();   // of the allocation that failed
   if (spare_) spare_();
-  const size_t held = blocks_.size();
-  for (Block &b : blocks_) b.old = true;
-  sweep();
-  return blocks_.size() < held;
+  return trim(0);
 }
 
-void DeviceMemory::age() {
-  for (Block &b : blocks_) b.old = !b.used;
-}
-
-void DeviceMemory::sweep() {
-  size_t k = 0;
-  for (Block &b : blocks_) {
-    if (!b.used && b.old) cudaFree(b.p);
-    else blocks_[k++] = b;
+bool DeviceMemory::trim(size_t limit) {
+  size_t idle = 0;
+  for (const Block &b : blocks_) idle += b.used ? 0 : b.bytes;
+  bool any = false;
+  while (idle > limit) {
+    size_t k = blocks_.size();
+    for (size_t q = 0; q < blocks_.size(); ++q)
+      if (!blocks_[q].used && (k == blocks_.size() || blocks_[q].bytes > blocks_[k].bytes)) k = q;
+    cudaFree(blocks_[k].p);
+    idle -= blocks_[k].bytes;
+    blocks_.erase(blocks_.begin() + k);
+    any = true;
   }
-  blocks_.resize(k);
+  return any;
+}
+
+size_t DeviceMemory::in_use() const {
+  size_t n = 0;
+  for (const Block &b : blocks_) n += b.used ? b.bytes : 0;
+  return n;
 }
 
 bool TableUpload::commit(DeviceMemory &mem, std::vector<void *> &owned, cudaStream_t st, std::string &err) {
@@ -1499,7 +1513,6 @@ bool Engine::analyze(int n, const int *c, const int *r, const int64_t *lC, const
   }
 
   // ---- upload ----
-  mem_.age();
   release();
   cudaStream_t st = stream_;
   TableUpload up;
@@ -1599,7 +1612,7 @@ bool Engine::analyze(int n, const int *c, const int *r, const int64_t *lC, const
   h_prune_ptr_.assign(prunePtr, prunePtr + supNo + 1);
   h_prune_.assign(pruneSet, pruneSet + nprune);
   front_ = FP;
-  mem_.sweep();
+  mem_.trim(std::max(KEEP_BYTES, 2 * mem_.in_use()));
   return true;
 }
 
@@ -2013,6 +2026,7 @@ int Engine::factor(const double *values, bool values_on_device, int *info, std::
     // longer than the launches (100 kernels: 1.9 ms against 0.3), so it pays from the second on.
     // The whole launch sequence is fixed by the structure (and the mode): capture it once
     // per mode, replay it.
+    if (!graph_exec_[prec]) mem_.trim(0);   // a structure that stays: only what it uses
     cudaGraph_t &g = graph_[prec];
     cudaGraphExec_t &ge = graph_exec_[prec];
     if (!ge) {
@@ -2142,7 +2156,8 @@ double *Engine::staging(size_t doubles, std::string &err) {
 bool Engine::ensure_work(int nrhs, std::string &err) {
   if (nrhs <= work_nrhs_) return true;
   release_solve_graphs();   // they hold the old buffers
-  for (double **p : {&d_sx_, &d_x8_, &d_c8_, &d_contrib_, &d_work_, &d_norms_, &d_npart_}) mem_.put(*p);
+  for (double **p : {&d_sx_, &d_x8_, &d_c8_, &d_contrib_}) mem_.put(*p);
+  for (double **p : {&d_work_, &d_norms_, &d_npart_}) mem_.free(*p);   // outgrown
   if (h_norms_) cudaFreeHost(h_norms_);
   h_norms_ = nullptr;
   // one vector, and (several right-hand sides) eight interleaved ones with their contributions

@@ -15,9 +15,11 @@
 namespace swc {
 
 // Device memory of one engine.  Blocks given back by an analysis are taken again by the next
-// one (a repeated drop-in call otherwise spends about 3 ms in cudaMalloc and cudaFree); what a
-// whole analysis did not take again is freed at its end, so at most the last structure's
-// memory is held.  Not for use by several threads at once (an engine is not either).
+// one or by its first calls (a repeated drop-in call otherwise spends about 3 ms in cudaMalloc and
+// cudaFree): an analysis keeps free blocks of at most twice what it took itself (or KEEP_BYTES), and
+// the second factorization of a structure frees those left.  A block serves requests of 8/9 of its
+// size or more.  Not for use by several threads at once (an engine is not either).
+constexpr size_t KEEP_BYTES = (size_t)64 << 20;
 class DeviceMemory {
  public:
   ~DeviceMemory();
@@ -30,11 +32,16 @@ class DeviceMemory {
   }
   template <typename T>
   void put(T *&p) {
-    if (p) give(p);
+    if (p) give(p, true);
     p = nullptr;
   }
-  void age();        // marks the blocks that are free now; sweep() frees those still free
-  void sweep();
+  template <typename T>
+  void free(T *&p) {   // not for another request
+    if (p) give(p, false);
+    p = nullptr;
+  }
+  bool trim(size_t limit);   // frees the largest free blocks until at most `limit` bytes are; any freed?
+  size_t in_use() const;
   // Called first when an allocation fails: gives back what the engine can do without.
   void on_shortage(std::function<void()> spare) { spare_ = std::move(spare); }
   // After a failed allocation (any, also one elsewhere): frees every block not in use; false if there
@@ -42,11 +49,11 @@ class DeviceMemory {
   bool make_room();
 
  private:
-  struct Block { void *p; size_t bytes; bool used, old; };
+  struct Block { void *p; size_t bytes; bool used; };
   std::vector<Block> blocks_;
   std::function<void()> spare_;
   cudaError_t take(void **p, size_t bytes);
-  void give(void *p);
+  void give(void *p, bool keep);
 };
 
 // Host tables in one device block (the sources stay alive until commit).

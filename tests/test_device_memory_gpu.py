@@ -27,13 +27,13 @@ def analyzed(P):
 def free_bytes():
     import torch
     torch.cuda.synchronize()
+    torch.cuda.empty_cache()     # torch's own idle memory is not the library's
     return torch.cuda.mem_get_info()[0]
 
 
 def fill(leave):
     """Device memory taken until `leave` bytes are free."""
     import torch
-    torch.cuda.empty_cache()
     return torch.empty(free_bytes() - leave, dtype=torch.uint8, device="cuda")
 
 
@@ -100,3 +100,39 @@ def test_mixed_handles_take_no_blocks(cuda_ok, problem):
     assert before - after <= 8 * P.xsize + 100 * MB
     assert h.factor(P.A2x) == 0
     assert after - free_bytes() >= 150 * MB
+
+
+def test_a_large_structures_memory_is_given_back(cuda_ok, problem):
+    """A handle that goes on to a small structure holds no more than a small multiple of it."""
+    small = plate(20, 20)
+    values = (problem.A2x, small.A2x)
+    h = swc.Handle(0)
+    before = free_bytes()
+
+    def step(P, x):
+        h.analyze(P.n, P.A2p, P.A2i, P.lC, P.Ls, P.Li_ptr, P.super, P.prunePtr, P.pruneSet)
+        after = free_bytes()
+        assert h.factor(x) == 0
+        assert h.factor(x) == 0
+        return after
+
+    step(problem, values[0])
+    assert before - free_bytes() >= 8 * problem.xsize
+    assert before - step(small, values[1]) <= 100 * MB
+    assert before - free_bytes() <= 40 * MB      # a few tables, the two graphs
+
+
+def test_growing_numbers_of_right_hand_sides_keep_one_workspace(cuda_ok, problem):
+    import torch
+    P = problem
+    b = torch.randn(48, P.n, dtype=torch.float64, device="cuda")
+    used = []
+    for counts in ([48], [1, 2, 3, 5, 8, 13, 21, 34, 48]):
+        h = analyzed(P)
+        assert h.factor(P.A2x) == 0
+        before = free_bytes()
+        for k in counts:
+            h.solve(b[:k].contiguous() if k > 1 else b[0].contiguous())
+        used.append(before - free_bytes())
+        del h
+    assert used[1] <= used[0] + 32 * MB
