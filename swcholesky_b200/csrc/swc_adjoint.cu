@@ -35,8 +35,8 @@
 #include <climits>
 #include <cmath>
 #include <cstdint>
+#include <map>
 #include <string>
-#include <type_traits>
 #include <vector>
 
 #include "swc_engine.h"
@@ -469,21 +469,82 @@ __global__ void k_solve_grad(DevSym S, const double *x, const double *lam, doubl
 
 // ---------------------------------------------------------------------------------------
 
-// Reverse sweep: waves by decreasing level.
+// Reverse sweep: waves of supernodes, parents before children.
 struct AdjointPlan {
   struct Step { int task_off, task_cnt, unit_off, unit_cnt; };   // one 64-column step of a wave
   struct AdjWave {
-    int warp_off, warp_cnt, cta_off, cta_cnt, cta_smem, copy_off, copy_cnt;
+    int warp_off, warp_cnt, cta_off, cta_cnt, cta_smem, copy_off, copy_cnt, col_off, col_cnt;
     std::vector<Step> steps;
   };
   std::vector<AdjWave> waves;
   std::vector<int> warp_list, cta_list, parent;
   std::vector<int4> copies, tasks, units;
+  std::vector<int2> cols;          // (s, column) of the wide supernodes
   std::vector<char> kids;
   std::vector<int64_t> zoff;
   int64_t z_len = 0;
   int max_tasks = 0;
 };
+
+// Doubles of a supernode's place in Z: its whole front where it has children (they read it) or is
+// wide, else its panel.
+static int64_t adj_front_len(const HostSym &H, int s, bool whole) {
+  const int64_t m = H.rowptr[s + 1] - H.rowptr[s];
+  return (m * (whole ? m : H.super[s + 1] - H.super[s]) + 15) & ~(int64_t)15;
+}
+
+// Places of the fronts when the waves run in this order: a front is read by its children only, and
+// freed once the last one is done.
+static int64_t place_adjoint(const std::vector<std::vector<int>> &waves, const std::vector<int64_t> &len,
+                             const FrontPlan &F, const std::vector<int> &parent, std::vector<int64_t> &zoff) {
+  FrontArena A;
+  std::vector<int> left(len.size());   // children not done yet
+  for (size_t s = 0; s < len.size(); ++s) left[s] = F.child_ptr[s + 1] - F.child_ptr[s];
+  for (const std::vector<int> &here : waves) {
+    for (int s : here) zoff[s] = A.take(len[s]);
+    for (int s : here) {
+      if (F.child_ptr[s + 1] == F.child_ptr[s]) A.give(zoff[s], len[s]);
+      const int p = parent[s];
+      if (p >= 0 && --left[p] == 0) A.give(zoff[p], len[p]);
+    }
+  }
+  return A.end();
+}
+
+// The order when a level's fronts are too many to be held together (many narrow supernodes under a
+// wide border: a front is as large as the border squared): groups of at most `budget` doubles, one
+// after the other, each with everything below it before the next; small subtrees first, so that
+// little is held while the large ones run.
+static std::vector<std::vector<int>> adjoint_groups(const std::vector<int64_t> &len, const FrontPlan &F,
+                                                    const std::vector<int> &parent, int64_t budget) {
+  const int ns = (int)len.size();
+  std::vector<int64_t> weight(len);   // of the subtree
+  std::vector<std::vector<int>> open(1), waves;   // open: lists whose parents are done, last one first
+  for (int s = 0; s < ns; ++s) {   // parents have larger numbers
+    if (parent[s] >= 0) weight[parent[s]] += weight[s];
+    else open[0].push_back(s);
+  }
+  while (!open.empty()) {
+    std::vector<int> here = std::move(open.back());
+    open.pop_back();
+    int64_t sum = 0;
+    for (int s : here) sum += len[s];
+    if (sum > budget && here.size() > 1) {
+      std::stable_sort(here.begin(), here.end(), [&](int a, int b) { return weight[a] < weight[b]; });
+      size_t k = 1;
+      for (sum = len[here[0]]; k < here.size() && sum + len[here[k]] <= budget; ++k) sum += len[here[k]];
+      if (k < here.size()) {
+        open.emplace_back(here.begin() + k, here.end());
+        here.resize(k);
+      }
+    }
+    std::vector<int> next;
+    for (int s : here) next.insert(next.end(), F.child.begin() + F.child_ptr[s], F.child.begin() + F.child_ptr[s + 1]);
+    if (!next.empty()) open.push_back(std::move(next));
+    waves.push_back(std::move(here));
+  }
+  return waves;
+}
 
 static void build_adjoint_plan(const HostSym &H, const Plan &P, const FrontPlan &F, AdjointPlan &AP) {
   const std::vector<int> &super = H.super;
@@ -500,23 +561,34 @@ static void build_adjoint_plan(const HostSym &H, const Plan &P, const FrontPlan 
       AP.kids[s] = 1;
       level[s] = std::max(level[s], level[F.child[q]] + 1);
     }
-  std::vector<std::vector<int>> by_level(nlev);
   std::vector<char> tiled(ns, 0);
   for (int s : P.big_list) tiled[s] = 1;
-  for (int s = 0; s < ns; ++s) by_level[level[s]].push_back(s);
-  FrontArena A;
-  auto len = [&](int s) {
-    return ((int64_t)rows(s) * (AP.kids[s] || tiled[s] ? rows(s) : width(s)) + 15) & ~(int64_t)15;
-  };
-  std::vector<int> left(ns, 0);   // children not done yet
-  for (int s = 0; s < ns; ++s) left[s] = F.child_ptr[s + 1] - F.child_ptr[s];
-  AP.waves.resize(nlev);
-  for (int v = 0; v < nlev; ++v) {
-    const std::vector<int> &here = by_level[nlev - 1 - v];
+  std::vector<int64_t> len(ns);
+  for (int s = 0; s < ns; ++s) len[s] = adj_front_len(H, s, AP.kids[s] || tiled[s]);
+  // a wave per level, the root's first, where that needs no more memory than the factorization's
+  // blocks may take (grids: 0.3 to 0.9 times L); else groups of a quarter of it
+  std::vector<std::vector<int>> lists(nlev);
+  for (int s = 0; s < ns; ++s) lists[nlev - 1 - level[s]].push_back(s);
+  AP.z_len = place_adjoint(lists, len, F, AP.parent, AP.zoff);
+  const int64_t limit = front_memory_limit(H.xsize);
+  if (AP.z_len > limit) {
+    std::vector<int64_t> zoff(ns, 0);
+    std::vector<std::vector<int>> groups = adjoint_groups(len, F, AP.parent, limit / 4);
+    const int64_t z_len = place_adjoint(groups, len, F, AP.parent, zoff);
+    if (z_len < AP.z_len) {
+      AP.z_len = z_len;
+      AP.zoff = std::move(zoff);
+      lists = std::move(groups);
+    }
+  }
+  AP.waves.resize(lists.size());
+  for (size_t v = 0; v < lists.size(); ++v) {
+    const std::vector<int> &here = lists[v];
     AdjointPlan::AdjWave &W = AP.waves[v];
     W.warp_off = (int)AP.warp_list.size();
     W.cta_off = (int)AP.cta_list.size();
     W.copy_off = (int)AP.copies.size();
+    W.col_off = (int)AP.cols.size();
     W.cta_smem = 0;
     int fit = 0, maxnb = 0;
     auto warp_fits = [&](int s) {
@@ -526,10 +598,10 @@ static void build_adjoint_plan(const HostSym &H, const Plan &P, const FrontPlan 
     for (int s : here) fit += warp_fits(s);
     for (int s : here) {
       const int w = width(s), m = rows(s);
-      AP.zoff[s] = A.take(len(s));
       if (tiled[s]) {
         for (int j0 = 0; j0 < m - w; j0 += TB)
           for (int i0 = 0; i0 < m - w; i0 += TB) AP.copies.push_back(make_int4(s, i0, j0, 0));
+        for (int j = 0; j < w; ++j) AP.cols.push_back(make_int2(s, super[s] + j));
         maxnb = std::max(maxnb, (w + TB - 1) / TB);
       } else if (fit >= FRONT_WARP_LEVEL_MIN && warp_fits(s)) {
         AP.warp_list.push_back(s);
@@ -542,6 +614,7 @@ static void build_adjoint_plan(const HostSym &H, const Plan &P, const FrontPlan 
     W.warp_cnt = (int)AP.warp_list.size() - W.warp_off;
     W.cta_cnt = (int)AP.cta_list.size() - W.cta_off;
     W.copy_cnt = (int)AP.copies.size() - W.copy_off;
+    W.col_cnt = (int)AP.cols.size() - W.col_off;
     for (int t = 0; t < maxnb; ++t) {   // last column block first
       AdjointPlan::Step st{(int)AP.tasks.size(), 0, (int)AP.units.size(), 0};
       for (int s : here) {
@@ -557,14 +630,82 @@ static void build_adjoint_plan(const HostSym &H, const Plan &P, const FrontPlan 
       AP.max_tasks = std::max(AP.max_tasks, st.task_cnt);
       W.steps.push_back(st);
     }
-    // a front is read by its children only: free it once the last one is done
+  }
+}
+
+bool check_adjoint_plan(const HostSym &H, const Plan &P, const FrontPlan &F, std::string &err) {
+  if (!F.closed) return true;
+  AdjointPlan AP;
+  build_adjoint_plan(H, P, F, AP);
+  const int ns = (int)H.super.size() - 1;
+  auto width = [&](int s) { return H.super[s + 1] - H.super[s]; };
+  auto bad = [&](const char *what, int s) {
+    err = std::string("reverse sweep: ") + what + ", supernode " + std::to_string(s);
+    return false;
+  };
+  std::vector<char> tiled(ns, 0), done(ns, 0);
+  for (int s : P.big_list) tiled[s] = 1;
+  std::vector<int64_t> len(ns);
+  std::vector<int> left(ns), blocks(ns, 0), cols(ns, 0);
+  for (int s = 0; s < ns; ++s) {
+    left[s] = F.child_ptr[s + 1] - F.child_ptr[s];
+    len[s] = adj_front_len(H, s, left[s] > 0 || tiled[s]);
+  }
+  std::map<int64_t, int64_t> live;   // the fronts held, by place
+  for (const AdjointPlan::AdjWave &W : AP.waves) {
+    std::vector<int> here;
+    for (int k = W.warp_off; k < W.warp_off + W.warp_cnt; ++k) here.push_back(AP.warp_list[k]);
+    for (int k = W.cta_off; k < W.cta_off + W.cta_cnt; ++k)
+      here.push_back(AP.cta_list[k] < 0 ? ~AP.cta_list[k] : AP.cta_list[k]);
+    for (int s : here)
+      if (s < 0 || s >= ns || tiled[s]) return bad("a wide supernode among the small", s);
+    for (size_t t = 0; t < W.steps.size(); ++t) {
+      const AdjointPlan::Step &st = W.steps[t];
+      int next = 0;
+      for (int k = st.unit_off; k < st.unit_off + st.unit_cnt; ++k) {
+        const int4 un = AP.units[k];
+        const int s = un.x, nb = (width(s) + TB - 1) / TB;
+        if (t == 0) here.push_back(s);
+        if (!tiled[s] || un.y != nb - 1 - (int)t || un.z != next) return bad("column block out of order", s);
+        const int mr = (int)(H.rowptr[s + 1] - H.rowptr[s]) - std::min(width(s), (un.y + 1) * TB);
+        if (un.w != (mr + TB - 1) / TB || next + un.w > st.task_cnt) return bad("rows of a column block", s);
+        for (int q = 0; q < un.w; ++q) {
+          const int4 tk = AP.tasks[st.task_off + next + q];
+          if (tk.x != s || tk.y != un.y || tk.z != q * TB || tk.w != next) return bad("task of a column block", s);
+        }
+        next += un.w;
+        ++blocks[s];
+      }
+      if (next != st.task_cnt || next > AP.max_tasks) return bad("tasks of a step", -1);
+    }
+    for (int k = W.col_off; k < W.col_off + W.col_cnt; ++k) {
+      const int s = AP.cols[k].x;
+      if (!tiled[s] || AP.cols[k].y != H.super[s] + cols[s]++) return bad("gradient column", s);
+    }
     for (int s : here) {
-      if (!AP.kids[s]) A.give(AP.zoff[s], len(s));
+      if (done[s]) return bad("a supernode twice", s);
       const int p = AP.parent[s];
-      if (p >= 0 && --left[p] == 0) A.give(AP.zoff[p], len(p));
+      if (p >= 0 && done[p] != 2) return bad("a supernode before its parent", s);
+      done[s] = 1;
+      const int64_t at = AP.zoff[s];
+      auto nx = live.lower_bound(at);
+      if (at < 0 || at + len[s] > AP.z_len || (nx != live.end() && nx->first < at + len[s]) ||
+          (nx != live.begin() && std::prev(nx)->second > at))
+        return bad("fronts overlap", s);
+      live[at] = at + len[s];
+    }
+    for (int s : here) {
+      done[s] = 2;
+      if (tiled[s] && (blocks[s] != (width(s) + TB - 1) / TB || cols[s] != width(s)))
+        return bad("column blocks or gradient columns missing", s);
+      if (left[s] == 0) live.erase(AP.zoff[s]);
+      const int p = AP.parent[s];
+      if (p >= 0 && --left[p] == 0) live.erase(AP.zoff[p]);
     }
   }
-  AP.z_len = A.end();
+  for (int s = 0; s < ns; ++s)
+    if (!done[s]) return bad("a supernode in no wave", s);
+  return true;
 }
 
 bool Engine::prepare_adjoint(std::string &err) {
@@ -586,6 +727,7 @@ bool Engine::prepare_adjoint(std::string &err) {
   up.add(d_adj_copies_, AP.copies);
   up.add(d_adj_tasks_, AP.tasks);
   up.add(d_adj_units_, AP.units);
+  up.add(d_adj_cols_, AP.cols);
   if (!up.commit(mem_, tables_, stream_, err)) return false;
   cudaError_t e = cudaSuccess;
   const size_t scratch = sizeof(double) * TB * TB * std::max(AP.max_tasks, 1);
@@ -614,6 +756,7 @@ void Engine::release_adjoint() {
   d_adj_kids_ = nullptr;
   d_adj_zoff_ = nullptr;
   d_adj_copies_ = d_adj_tasks_ = d_adj_units_ = nullptr;
+  d_adj_cols_ = nullptr;
   adj_.reset();
 }
 
@@ -645,8 +788,7 @@ void Engine::run_adjoint() {
   LaunchQueue q{stream_, false};
   const AdjDev A{d_adj_parent_, d_frel_, d_fapos_, d_adj_zoff_, d_adj_kids_,
                  d_adj_Z_,      d_adj_UT_, d_adj_P_, d_adj_grad_};
-  for (size_t v = 0; v < AP.waves.size(); ++v) {
-    const AdjointPlan::AdjWave &W = AP.waves[v];
+  for (const AdjointPlan::AdjWave &W : AP.waves) {
     if (W.copy_cnt > 0) launch_early(q, 1, k_adj_copy, W.copy_cnt, 256, 0, sym_, A, d_adj_copies_ + W.copy_off);
     if (W.cta_cnt > 0)
       launch_early(q, 1, k_adj_small, W.cta_cnt, ZC_T, W.cta_smem, sym_, A, d_adj_cta_ + W.cta_off);
@@ -661,9 +803,8 @@ void Engine::run_adjoint() {
       if (t.unit_cnt > 0)
         launch_early(q, 1, k_adj_zkk, t.unit_cnt, MT, TB * LDS * 8, sym_, A, d_adj_units_ + t.unit_off);
     }
-    const Wave &B = plan_.waves[AP.waves.size() - 1 - v];
-    if (B.asm_cnt > 0)
-      launch_early(q, 1, k_adj_grad, (B.asm_cnt * 32 + 255) / 256, 256, 0, sym_, A, d_asm_ + B.asm_off, B.asm_cnt);
+    if (W.col_cnt > 0)
+      launch_early(q, 1, k_adj_grad, (W.col_cnt * 32 + 255) / 256, 256, 0, sym_, A, d_adj_cols_ + W.col_off, W.col_cnt);
   }
 }
 

@@ -432,7 +432,8 @@ int swc_plan_stats(int n, const int *c, const int *r, const size_t *lC, const in
     return fail(SWC_INVALID_INPUT, err);
   if (!swc::check_scatter_plan(n, Ls, H, P, swc::plan_candidate(plan), err))
     return fail(SWC_INVALID_INPUT, err);
-  if (!swc::check_front_plan(n, Ls, H, P, FP, err)) return fail(SWC_INVALID_INPUT, err);
+  if (!swc::check_front_plan(n, Ls, H, P, FP, err) || !swc::check_adjoint_plan(H, P, FP, err))
+    return fail(SWC_INVALID_INPUT, err);
   if (FP.ok) P.launches = FP.launches;
   swc::SolvePlan SP;
   swc::build_solve_plan(n, Ls, H, SP);

@@ -452,6 +452,7 @@ class Engine {
   int *d_adj_parent_ = nullptr, *d_adj_warp_ = nullptr, *d_adj_cta_ = nullptr;
   char *d_adj_kids_ = nullptr;
   int64_t *d_adj_zoff_ = nullptr;
+  int2 *d_adj_cols_ = nullptr;
   int4 *d_adj_copies_ = nullptr, *d_adj_tasks_ = nullptr, *d_adj_units_ = nullptr;
   double *d_adj_Z_ = nullptr, *d_adj_UT_ = nullptr, *d_adj_P_ = nullptr, *d_adj_grad_ = nullptr;
   cudaGraphExec_t adj_graph_ = nullptr;

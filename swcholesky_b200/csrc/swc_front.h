@@ -155,6 +155,11 @@ void build_front_plan(int n, const int *c, const int *r, const int *Ls, const in
 bool check_front_plan(int n, const int *Ls, const HostSym &H, const Plan &P, const FrontPlan &F,
                       std::string &err);
 
+// Host check of the adjoint's reverse sweep (a no-op where the tree does not hold): every
+// supernode once, after its parent; every wide one's column blocks, their rows and its gradient's
+// columns each once, the last block first; no two fronts held in one place.
+bool check_adjoint_plan(const HostSym &H, const Plan &P, const FrontPlan &F, std::string &err);
+
 bool front_configure(std::string &err);
 int front_cta_walk_ctas(int smem, int count);
 int front_warp_walk_ctas(int count);
