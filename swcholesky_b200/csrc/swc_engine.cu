@@ -2196,7 +2196,7 @@ cudaGraphExec_t Engine::solve_graph(bool eight) {
   cudaStream_t st = stream_;
   cudaGraph_t graph = nullptr;
   if (cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal) != cudaSuccess) return nullptr;
-  if (eight) run_solve8(d_x8_);
+  if (eight) run_solve8(d_x8_, d_c8_, 8);
   else run_solve_with(d_sx_, 1, d_contrib_);
   cudaError_t e = cudaStreamEndCapture(st, &graph);
   if (e == cudaSuccess) e = cudaGraphInstantiate(&exec, graph, 0);
@@ -2208,12 +2208,12 @@ cudaGraphExec_t Engine::solve_graph(bool eight) {
   return exec;
 }
 
-void Engine::run_solve8(double *x8) {
+void Engine::run_solve8(double *x8, double *c8, int stride) {
   cudaMemsetAsync(d_flags_, 0, sizeof(int) * std::max<int64_t>(nflags_, 1), stream_);
   const Solve8Dev D{d_slist_, d_swarp_, d_cptr_, d_cidx_, d_fchain_, d_bchain_, d_c8_tasks_,
                     d_g8_tasks_, d_flags_};
   run_halves([&](int l0, int l1, bool fwd, LaunchQueue &st) {
-    launch_solve8(sym_, splan_, D, x8, d_c8_, l0, l1, fwd, st);
+    launch_solve8(sym_, splan_, D, x8, c8, stride, l0, l1, fwd, st);
   });
 }
 
@@ -2266,7 +2266,7 @@ void Engine::run_solve(double *x, int nrhs) {
       cudaGraphExec_t g = use_graph_ && solved_[1] ? solve_graph(true) : nullptr;
       solved_[1] = true;
       if (g) cudaGraphLaunch(g, stream_);
-      else run_solve8(d_x8_);
+      else run_solve8(d_x8_, d_c8_, 8);
       launch_unpack8(n_, nr, d_x8_, xr, stream_);
     }
   }
@@ -2466,7 +2466,21 @@ bool Engine::solve_in_scratch(const double *b, double *x, int nrhs, double *scra
   if (x != b) e = cudaMemcpyAsync(x, b, sizeof(double) * n_ * nrhs, cudaMemcpyDeviceToDevice, st);
   if (e == cudaSuccess) e = cudaMemsetAsync(d_status_ + 2, 0, sizeof(int), st);
   if (e != cudaSuccess) { err = std::string("solve: ") + cudaGetErrorString(e); return false; }
-  run_solve_with(x, nrhs, scratch);
+  // the groups and the kernels of run_solve; a group that the scratch cannot hold interleaved, with
+  // its contributions, goes one vector at a time through the same products
+  for (int r0 = 0; r0 < nrhs; r0 += 8) {
+    const int nr = std::min(8, nrhs - r0);
+    double *xr = x + (size_t)r0 * n_, *x8 = scratch + 8 * cs;
+    if (nr == 1) {
+      run_solve_with(xr, 1, scratch);
+    } else if (8 * (cs + n_) <= capacity) {
+      launch_pack8(n_, nr, xr, x8, st);
+      run_solve8(x8, scratch, 8);
+      launch_unpack8(n_, nr, x8, xr, st);
+    } else {
+      for (int r = 0; r < nr; ++r) run_solve8(xr + (size_t)r * n_, scratch, 1);
+    }
+  }
   e = cudaStreamSynchronize(st);
   if (e == cudaSuccess) e = cudaGetLastError();
   if (e != cudaSuccess) { err = std::string("solve: ") + cudaGetErrorString(e); return false; }

@@ -316,8 +316,9 @@ struct Solve8Dev {
 bool solve8_configure(std::string &err);
 void launch_pack8(int n, int nr, const double *x, double *x8, cudaStream_t st);
 void launch_unpack8(int n, int nr, const double *x8, double *x, cudaStream_t st);
-// the levels l0 .. l1 - 1, forward or backward
-void launch_solve8(const DevSym &S, const SolvePlan &SP, const Solve8Dev &D, double *x8, double *c8,
+// the levels l0 .. l1 - 1, forward or backward; stride 8, or 1: one plain vector in x8, its
+// contributions in c8, the same arithmetic
+void launch_solve8(const DevSym &S, const SolvePlan &SP, const Solve8Dev &D, double *x8, double *c8, int stride,
                    int l0, int l1, bool fwd, LaunchQueue &st);
 
 // Result of a refined solve, per right-hand side.
@@ -558,7 +559,7 @@ class Engine {
   int2 *d_c8_tasks_ = nullptr, *d_g8_tasks_ = nullptr;
   cudaGraphExec_t solve_graph_[2] = {nullptr, nullptr};            // one vector; eight
   cudaGraphExec_t solve_graph(bool eight);
-  void run_solve8(double *x8);
+  void run_solve8(double *x8, double *c8, int stride);
   void release_solve_graphs();
   int2 *d_scontrib_ = nullptr, *d_sgather_ = nullptr;
   int *d_csr_rp_ = nullptr, *d_csr_ci_ = nullptr, *d_csr_map_ = nullptr;

@@ -11,6 +11,11 @@
 // descendants, solve with their diagonal block and form the contributions of their rows below
 // in one kernel (a warp or a CTA each); tiled ones are solved by the chained blocks and form
 // their contributions in a second kernel.  Backward: the mirror image.
+//
+// A right-hand side's result does not depend on the others of its group, nor on its place among
+// them (a tensor-core product's columns are independent).  The kernels come with vectors R = 8 apart
+// and with R = 1, one plain vector in place of the interleaved ones and seven zero columns: the
+// same result bit for bit, for callers whose scratch has no room for eight.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -27,7 +32,21 @@ namespace {
 constexpr int R8 = 8;
 constexpr int NT8 = 256, W8 = NT8 / 32;
 
+// Right-hand side r of row i in vectors R apart; zero where there is none.
+template <int R>
+__device__ __forceinline__ double rhs_of(const double *x, int64_t i, int r) {
+  return R == R8 || r < R ? x[i * R + r] : 0.0;
+}
+
+// Right-hand sides 2 kq, 2 kq + 1 of a row.
+template <int R>
+__device__ __forceinline__ void store_pair(double *row, int kq, double a, double b) {
+  if (R == R8) *reinterpret_cast<double2 *>(row + 2 * kq) = make_double2(a, b);
+  else if (kq == 0) row[0] = a;
+}
+
 // v - sum of the contributions listed for column j, right-hand side r.
+template <int R>
 __device__ __forceinline__ double take_contribs(const double *c8, const int *cptr, const int *cidx,
                                                 int j, int r, double v) {
   const int q1 = cptr[j + 1];
@@ -37,7 +56,7 @@ __device__ __forceinline__ double take_contribs(const double *c8, const int *cpt
 #pragma unroll
     for (int u = 0; u < 4; ++u) at[u] = cidx[min(q + u, q1 - 1)];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) t[u] = ld_if(c8 + (size_t)at[u] * R8 + r, q + u < q1);
+    for (int u = 0; u < 4; ++u) t[u] = ld_if(c8 + (size_t)at[u] * R + r, q + u < q1 && r < R);
     v -= (t[0] + t[1]) + (t[2] + t[3]);
   }
   return v;
@@ -45,6 +64,7 @@ __device__ __forceinline__ double take_contribs(const double *c8, const int *cpt
 
 // Contributions of rows a0 .. a0 + 7 of supernode s: L(a, 0 .. w - 1) y, y in shared memory
 // ([column][right-hand side]).
+template <int R>
 __device__ __forceinline__ void contrib_rows8(const double *Ls, int m, int w, int a0, const double *v,
                                               double *out) {
   const int lane = threadIdx.x & 31, g = lane >> 2, kq = lane & 3;
@@ -62,9 +82,7 @@ __device__ __forceinline__ void contrib_rows8(const double *Ls, int m, int w, in
       if (k + 4 * u < w) dmma(u & 1 ? c1 : c0, l[u], c < w ? v[c * R8 + g] : 0.0);
     }
   }
-  if (in)
-    *reinterpret_cast<double2 *>(out + (size_t)(a - w) * R8 + 2 * kq) =
-        make_double2(c0[0] + c1[0], c0[1] + c1[1]);
+  if (in) store_pair<R>(out + (size_t)(a - w) * R, kq, c0[0] + c1[0], c0[1] + c1[1]);
 }
 
 // ---- small supernodes (w <= SMALL_MAX_W), one CTA each; warp r solves right-hand side r with
@@ -81,6 +99,7 @@ __device__ __forceinline__ void stage_block(double *Ld, const double *Ls, int m,
   }
 }
 
+template <int R>
 __global__ void __launch_bounds__(NT8) k_fwd_small8(DevSym S, const int *list, double *y8, double *c8,
                                                     const int *cptr, const int *cidx) {
   extern __shared__ double sm8[];
@@ -95,7 +114,7 @@ __global__ void __launch_bounds__(NT8) k_fwd_small8(DevSym S, const int *list, d
   stage_block(Ld, Ls, m, w);
   pdl_wait();
   for (int e = tid; e < w * R8; e += NT8)
-    v[e] = take_contribs(c8, cptr, cidx, f + (e >> 3), e & 7, y8[(size_t)f * R8 + e]);
+    v[e] = take_contribs<R>(c8, cptr, cidx, f + (e >> 3), e & 7, rhs_of<R>(y8, f + (e >> 3), e & 7));
   __syncthreads();
   {
     const int i0 = lane, i1 = lane + 32;
@@ -117,11 +136,12 @@ __global__ void __launch_bounds__(NT8) k_fwd_small8(DevSym S, const int *list, d
     if (i1 < w) v[i1 * R8 + warp] = x1;
   }
   __syncthreads();
-  for (int e = tid; e < w * R8; e += NT8) y8[(size_t)f * R8 + e] = v[e];
-  double *out = c8 + (size_t)(rb - f) * R8;
-  for (int a0 = w + 8 * warp; a0 < m; a0 += 8 * W8) contrib_rows8(Ls, m, w, a0, v, out);
+  for (int e = tid; e < w * R; e += NT8) y8[(size_t)f * R + e] = v[e / R * R8 + e % R];
+  double *out = c8 + (size_t)(rb - f) * R;
+  for (int a0 = w + 8 * warp; a0 < m; a0 += 8 * W8) contrib_rows8<R>(Ls, m, w, a0, v, out);
 }
 
+template <int R>
 __global__ void __launch_bounds__(NT8) k_bwd_small8(DevSym S, const int *list, double *x8) {
   extern __shared__ double sm8[];
   pdl_trigger();
@@ -146,7 +166,7 @@ __global__ void __launch_bounds__(NT8) k_bwd_small8(DevSym S, const int *list, d
     double l[SMALL_MAX_W / 8];
 #pragma unroll
     for (int i = 0; i < SMALL_MAX_W / 8; ++i) l[i] = ld_if(Ls + (size_t)(8 * i + g) * m + a, in && 8 * i + g < w);
-    const double b = ld_if(x8 + (size_t)rows[in ? a : 0] * R8 + g, in);
+    const double b = ld_if(x8 + (size_t)rows[in ? a : 0] * R + g, in && g < R);
 #pragma unroll
     for (int i = 0; i < SMALL_MAX_W / 8; ++i)
       if (i < nt) dmma(c[i], l[i], b);
@@ -162,7 +182,7 @@ __global__ void __launch_bounds__(NT8) k_bwd_small8(DevSym S, const int *list, d
     double t = 0.0;
 #pragma unroll
     for (int q = 0; q < W8; ++q) t += part[q * SMALL_MAX_W * R8 + e];
-    v[e] = x8[(size_t)f * R8 + e] - t;
+    v[e] = rhs_of<R>(x8, f + (e >> 3), e & 7) - t;
   }
   __syncthreads();
   stage_block(Ld, Ls, m, w);
@@ -186,7 +206,7 @@ __global__ void __launch_bounds__(NT8) k_bwd_small8(DevSym S, const int *list, d
     if (i1 < w) v[i1 * R8 + warp] = x1;
   }
   __syncthreads();
-  for (int e = tid; e < w * R8; e += NT8) x8[(size_t)f * R8 + e] = v[e];
+  for (int e = tid; e < w * R; e += NT8) x8[(size_t)f * R + e] = v[e / R * R8 + e % R];
 }
 
 // ---- the small supernodes of crowded levels (w <= SOLVE_WARP_W), one warp each: lane (r, q)
@@ -202,6 +222,7 @@ __device__ __forceinline__ void stage_block_warp(Warp8 &M, const double *Ls, int
     if (lane >= j && lane < w) M.L[j * LDT + lane] = Ls[(size_t)j * m + lane];
 }
 
+template <int R>
 __global__ void __launch_bounds__(WN * 32) k_fwd_warp8(DevSym S, const int *list, int count, double *y8,
                                                        double *c8, const int *cptr, const int *cidx) {
   __shared__ Warp8 sm[WN];
@@ -221,7 +242,7 @@ __global__ void __launch_bounds__(WN * 32) k_fwd_warp8(DevSym S, const int *list
 #pragma unroll
   for (int u = 0; u < NX; ++u) {
     const int i = 4 * u + q;
-    x[u] = i < w ? take_contribs(c8, cptr, cidx, f + i, r, y8[(size_t)(f + i) * R8 + r]) : 0.0;
+    x[u] = i < w ? take_contribs<R>(c8, cptr, cidx, f + i, r, rhs_of<R>(y8, f + i, r)) : 0.0;
   }
   __syncwarp();
 #pragma unroll
@@ -246,14 +267,15 @@ __global__ void __launch_bounds__(WN * 32) k_fwd_warp8(DevSym S, const int *list
     const int i = 4 * u + q;
     if (i < w) {
       M.v[i * R8 + r] = x[u];
-      y8[(size_t)(f + i) * R8 + r] = x[u];
+      if (r < R) y8[(size_t)(f + i) * R + r] = x[u];
     }
   }
   __syncwarp();
-  double *out = c8 + (size_t)(rb - f) * R8;
-  for (int a0 = w; a0 < m; a0 += 8) contrib_rows8(Ls, m, w, a0, M.v, out);
+  double *out = c8 + (size_t)(rb - f) * R;
+  for (int a0 = w; a0 < m; a0 += 8) contrib_rows8<R>(Ls, m, w, a0, M.v, out);
 }
 
+template <int R>
 __global__ void __launch_bounds__(WN * 32) k_bwd_warp8(DevSym S, const int *list, int count, double *x8) {
   __shared__ Warp8 sm[WN];
   const int t = blockIdx.x * WN + (threadIdx.x >> 5);
@@ -280,7 +302,7 @@ __global__ void __launch_bounds__(WN * 32) k_bwd_warp8(DevSym S, const int *list
     double l[SOLVE_WARP_W / 8];
 #pragma unroll
     for (int i = 0; i < SOLVE_WARP_W / 8; ++i) l[i] = ld_if(Ls + (size_t)(8 * i + g) * m + a, in && 8 * i + g < w);
-    const double b = ld_if(x8 + (size_t)rows[in ? a : 0] * R8 + g, in);
+    const double b = ld_if(x8 + (size_t)rows[in ? a : 0] * R + g, in && g < R);
 #pragma unroll
     for (int i = 0; i < SOLVE_WARP_W / 8; ++i)
       if (i < nt) dmma(c[i], l[i], b);
@@ -294,7 +316,7 @@ __global__ void __launch_bounds__(WN * 32) k_bwd_warp8(DevSym S, const int *list
 #pragma unroll
   for (int u = 0; u < NX; ++u) {
     const int i = 4 * u + q;
-    x[u] = i < w ? x8[(size_t)(f + i) * R8 + r] - M.v[i * R8 + r] : 0.0;
+    x[u] = i < w ? rhs_of<R>(x8, f + i, r) - M.v[i * R8 + r] : 0.0;
     d[u] = i < w ? 1.0 / M.L[i * LDT + i] : 0.0;
   }
 #pragma unroll
@@ -315,7 +337,7 @@ __global__ void __launch_bounds__(WN * 32) k_bwd_warp8(DevSym S, const int *list
 #pragma unroll
   for (int u = 0; u < NX; ++u) {
     const int i = 4 * u + q;
-    if (i < w) x8[(size_t)(f + i) * R8 + r] = x[u];
+    if (i < w && r < R) x8[(size_t)(f + i) * R + r] = x[u];
   }
 }
 
@@ -323,6 +345,7 @@ __global__ void __launch_bounds__(WN * 32) k_bwd_warp8(DevSym S, const int *list
 // rows per CTA, warp q forms rows 16 q .. 16 q + 15 over all columns; other levels: 32 rows
 // per CTA of 16 warps that split the columns, partial sums in shared memory.
 constexpr int C8_U = 8;   // four columns each: loads in flight per lane and row
+template <int R>
 __global__ void __launch_bounds__(NT8) k_contrib8(DevSym S, const int2 *tasks, const double *y8,
                                                   double *c8) {
   pdl_trigger();
@@ -333,7 +356,7 @@ __global__ void __launch_bounds__(NT8) k_contrib8(DevSym S, const int2 *tasks, c
   const int64_t rb = S.rowptr[s];
   const int m = (int)(S.rowptr[s + 1] - rb);
   const double *Ls = S.L + S.xptr[s];
-  const double *yv = y8 + (size_t)f * R8 + g;
+  const double *yv = y8 + (size_t)f * R + g;
   const bool in0 = a0 + g < m, in1 = a0 + 8 + g < m;
   const double *p0 = Ls + a0 + g;
   double c[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
@@ -349,19 +372,20 @@ __global__ void __launch_bounds__(NT8) k_contrib8(DevSym S, const int2 *tasks, c
     if (first) pdl_wait();
     first = false;
 #pragma unroll
-    for (int u = 0; u < C8_U; ++u) b[u] = ld_if(yv + (size_t)(k + 4 * u + kq) * R8, k + 4 * u + kq < w);
+    for (int u = 0; u < C8_U; ++u) b[u] = ld_if(yv + (size_t)(k + 4 * u + kq) * R, k + 4 * u + kq < w && g < R);
 #pragma unroll
     for (int u = 0; u < C8_U; ++u) {
       dmma(c[0], l0[u], b[u]);
       dmma(c[1], l1[u], b[u]);
     }
   }
-  double *out = c8 + (size_t)((rb - f) + (a0 + g - w)) * R8 + 2 * kq;
-  if (in0) *reinterpret_cast<double2 *>(out) = make_double2(c[0][0], c[0][1]);
-  if (in1) *reinterpret_cast<double2 *>(out + 8 * R8) = make_double2(c[1][0], c[1][1]);
+  double *out = c8 + (size_t)((rb - f) + (a0 + g - w)) * R;
+  if (in0) store_pair<R>(out, kq, c[0][0], c[0][1]);
+  if (in1) store_pair<R>(out + 8 * R, kq, c[1][0], c[1][1]);
 }
 
 constexpr int CS_W = 16;   // warps of the column-split kernel
+template <int R>
 __global__ void __launch_bounds__(CS_W * 32, 1) k_contrib8_split(DevSym S, const int2 *tasks,
                                                               const double *y8, double *c8) {
   __shared__ __align__(16) double part[CS_W][32 * R8];
@@ -372,7 +396,7 @@ __global__ void __launch_bounds__(CS_W * 32, 1) k_contrib8_split(DevSym S, const
   const int64_t rb = S.rowptr[s];
   const int m = (int)(S.rowptr[s + 1] - rb);
   const double *Ls = S.L + S.xptr[s];
-  const double *yv = y8 + (size_t)f * R8 + g;
+  const double *yv = y8 + (size_t)f * R + g;
   const double *p[4];
 #pragma unroll
   for (int i = 0; i < 4; ++i) p[i] = Ls + (a0 + 8 * i + g < m ? a0 + 8 * i + g : 0);
@@ -389,7 +413,7 @@ __global__ void __launch_bounds__(CS_W * 32, 1) k_contrib8_split(DevSym S, const
     if (first) pdl_wait();
     first = false;
 #pragma unroll
-    for (int u = 0; u < 4; ++u) b[u] = ld_if(yv + (size_t)(k + 4 * u + kq) * R8, k + 4 * u + kq < w);
+    for (int u = 0; u < 4; ++u) b[u] = ld_if(yv + (size_t)(k + 4 * u + kq) * R, k + 4 * u + kq < w && g < R);
 #pragma unroll
     for (int u = 0; u < 4; ++u)
 #pragma unroll
@@ -400,11 +424,11 @@ __global__ void __launch_bounds__(CS_W * 32, 1) k_contrib8_split(DevSym S, const
     *reinterpret_cast<double2 *>(&part[wq][(8 * i + g) * R8 + 2 * kq]) = make_double2(c[i][0], c[i][1]);
   __syncthreads();
   const int e = threadIdx.x;
-  if (e < 32 * R8 && a0 + (e >> 3) < m) {
+  if (e < 32 * R8 && a0 + (e >> 3) < m && (e & 7) < R) {
     double t = 0.0;
 #pragma unroll
     for (int q = 0; q < CS_W; ++q) t += part[q][e];
-    c8[(size_t)((rb - f) + (a0 - w)) * R8 + e] = t;
+    c8[(size_t)((rb - f) + (a0 - w) + (e >> 3)) * R + (e & 7)] = t;
   }
 }
 
@@ -413,6 +437,7 @@ __global__ void __launch_bounds__(CS_W * 32, 1) k_contrib8_split(DevSym S, const
 // contributions above, the top levels have one CTA per SM and the bytes in flight set the rate:
 // sixteen predicated loads of L per lane and sixteen warps, 64 KB.
 constexpr int G8_W = 16;
+template <int R>
 __global__ void __launch_bounds__(G8_W * 32, 1) k_gather8(DevSym S, const int2 *tasks, double *x8) {
   __shared__ __align__(16) double part[G8_W][SOLVE_GATHER_COLS * R8];
   pdl_trigger();
@@ -444,7 +469,7 @@ __global__ void __launch_bounds__(G8_W * 32, 1) k_gather8(DevSym S, const int2 *
     if (first) pdl_wait();
     first = false;
 #pragma unroll
-    for (int u = 0; u < 8; ++u) b[u] = ld_if(x8 + (size_t)row[u] * R8 + g, a0 + 4 * u + kq < m);
+    for (int u = 0; u < 8; ++u) b[u] = ld_if(x8 + (size_t)row[u] * R + g, a0 + 4 * u + kq < m && g < R);
 #pragma unroll
     for (int u = 0; u < 8; ++u) {
       dmma(c[0][u & 1], l0[u], b[u]);
@@ -457,11 +482,11 @@ __global__ void __launch_bounds__(G8_W * 32, 1) k_gather8(DevSym S, const int2 *
         make_double2(c[i][0][0] + c[i][1][0], c[i][0][1] + c[i][1][1]);
   __syncthreads();
   const int e = threadIdx.x;
-  if (e < SOLVE_GATHER_COLS * R8 && j0 + (e >> 3) < w) {
+  if (e < SOLVE_GATHER_COLS * R8 && j0 + (e >> 3) < w && (e & 7) < R) {
     double t = 0.0;
 #pragma unroll
     for (int q = 0; q < G8_W; ++q) t += part[q][e];
-    x8[(size_t)(f + j0) * R8 + e] -= t;
+    x8[(size_t)(f + j0 + (e >> 3)) * R + (e & 7)] -= t;
   }
 }
 
@@ -492,6 +517,7 @@ __device__ __forceinline__ void chain8_send(double *yin, unsigned long long *bar
 }
 
 // The block's rows 8 warp .. 8 warp + 7 of T v (tr: this warp's rows of T as operands), sent on.
+template <int R>
 __device__ __forceinline__ void chain8_finish(const double (&tr)[16], const double *vs, double *yin,
                                               unsigned long long *bar, int me, int last, int bw,
                                               double *dst, int *flag) {
@@ -506,11 +532,12 @@ __device__ __forceinline__ void chain8_finish(const double (&tr)[16], const doub
   const int row = 8 * wp + g;
   const bool in = row < bw;
   chain8_send(yin, bar, me, last, row * R8 + 2 * kq, in ? a : 0.0, in ? b : 0.0);
-  if (in) *reinterpret_cast<double2 *>(dst + (size_t)row * R8 + 2 * kq) = make_double2(a, b);
+  if (in) store_pair<R>(dst + (size_t)row * R, kq, a, b);
   __syncwarp();
   if (lane == 0) red_release_add(flag, 1);
 }
 
+template <int R>
 __global__ void __launch_bounds__(NT8, 1) k_fwd_chain8(DevSym S, const int2 *tasks, int count, double *y8,
                                                        const double *c8, const int *cptr,
                                                        const int *cidx, int *flags) {
@@ -554,8 +581,8 @@ __global__ void __launch_bounds__(NT8, 1) k_fwd_chain8(DevSym S, const int2 *tas
 #pragma unroll
     for (int h = 0; h < BLK8 / NT8; ++h) {
       const int e = tid + h * NT8, row = e >> 3;
-      vs[e] = row < bw ? take_contribs(c8, cptr, cidx, f + r0 + row, e & 7,
-                                       y8[(size_t)(f + r0) * R8 + e]) : 0.0;
+      vs[e] = row < bw ? take_contribs<R>(c8, cptr, cidx, f + r0 + row, e & 7,
+                                          rhs_of<R>(y8, f + r0 + row, e & 7)) : 0.0;
     }
     double acc[8][2];
 #pragma unroll
@@ -589,7 +616,7 @@ __global__ void __launch_bounds__(NT8, 1) k_fwd_chain8(DevSym S, const int2 *tas
           for (int u = 0; u < XB8; ++u)
 #pragma unroll
             for (int h = 0; h < 2; ++h)
-              t[u][h] = u < nbt ? __ldcg(&y8[(size_t)(f + (c + u) * TB + w8 + 4 * h + kq) * R8 + g]) : 0.0;
+              t[u][h] = u < nbt && g < R ? __ldcg(&y8[(size_t)(f + (c + u) * TB + w8 + 4 * h + kq) * R + g]) : 0.0;
 #pragma unroll
           for (int u = 0; u < XB8; ++u)
 #pragma unroll
@@ -618,11 +645,12 @@ __global__ void __launch_bounds__(NT8, 1) k_fwd_chain8(DevSym S, const int2 *tas
       vs[e] -= t;
     }
     __syncthreads();
-    if (ok) chain8_finish(tr, vs, yin, bar, me, last, bw, y8 + (size_t)(f + r0) * R8, &flags[base + k]);
+    if (ok) chain8_finish<R>(tr, vs, yin, bar, me, last, bw, y8 + (size_t)(f + r0) * R, &flags[base + k]);
   }
   cluster_sync_all();
 }
 
+template <int R>
 __global__ void __launch_bounds__(NT8, 1) k_bwd_chain8(DevSym S, const int2 *tasks, int count, double *x8,
                                                        int *flags) {
   extern __shared__ double sm8[];
@@ -669,7 +697,7 @@ __global__ void __launch_bounds__(NT8, 1) k_bwd_chain8(DevSym S, const int2 *tas
       const int cw = min(TB, w - c * TB);
 #pragma unroll
       for (int t = 0; t < 16; ++t)
-        b[t] = 4 * t + kq < cw ? __ldcg(&x8[(size_t)(f + c * TB + 4 * t + kq) * R8 + g]) : 0.0;
+        b[t] = 4 * t + kq < cw && g < R ? __ldcg(&x8[(size_t)(f + c * TB + 4 * t + kq) * R + g]) : 0.0;
     };
     bool ok = true;
     int xb0 = nb, nbt = 0;
@@ -709,11 +737,12 @@ __global__ void __launch_bounds__(NT8, 1) k_bwd_chain8(DevSym S, const int2 *tas
       const double s0 = (acc[0][0] + acc[1][0]) + (acc[2][0] + acc[3][0]);
       const double s1 = (acc[0][1] + acc[1][1]) + (acc[2][1] + acc[3][1]);
       double2 v = make_double2(0.0, 0.0);
-      if (row < bw) v = *reinterpret_cast<const double2 *>(&x8[(size_t)(f + r0 + row) * R8 + 2 * kq]);
+      if (R == R8 && row < bw) v = *reinterpret_cast<const double2 *>(&x8[(size_t)(f + r0 + row) * R8 + 2 * kq]);
+      if (R == 1 && row < bw && kq == 0) v.x = x8[f + r0 + row];
       *reinterpret_cast<double2 *>(vs + row * R8 + 2 * kq) = make_double2(v.x - s0, v.y - s1);
     }
     ok = __syncthreads_and(ok) != 0;
-    if (ok) chain8_finish(tr, vs, yin, bar, me, last, bw, x8 + (size_t)(f + r0) * R8, &flags[base + k]);
+    if (ok) chain8_finish<R>(tr, vs, yin, bar, me, last, bw, x8 + (size_t)(f + r0) * R, &flags[base + k]);
   }
   cluster_sync_all();
 }
@@ -733,9 +762,11 @@ __global__ void k_unpack8(int n, int nr, const double *x8, double *x) {
 }  // namespace
 
 bool solve8_configure(std::string &err) {
-  cudaError_t e = cudaFuncSetAttribute(k_fwd_chain8, cudaFuncAttributeMaxDynamicSharedMemorySize, CHAIN8_SMEM);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_bwd_chain8, cudaFuncAttributeMaxDynamicSharedMemorySize, CHAIN8_SMEM);
+  cudaError_t e = cudaSuccess;
+  for (auto k : {k_fwd_chain8<R8>, k_fwd_chain8<1>})
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, CHAIN8_SMEM);
+  for (auto k : {k_bwd_chain8<R8>, k_bwd_chain8<1>})
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, CHAIN8_SMEM);
   if (e != cudaSuccess) {
     err = std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(e);
     return false;
@@ -750,40 +781,47 @@ void launch_unpack8(int n, int nr, const double *x8, double *x, cudaStream_t st)
   k_unpack8<<<(unsigned)(((int64_t)n * R8 + 255) / 256), 256, 0, st>>>(n, nr, x8, x);
 }
 
-void launch_solve8(const DevSym &S, const SolvePlan &SP, const Solve8Dev &D, double *x8, double *c8,
-                   int l0, int l1, bool fwd, LaunchQueue &st) {
+template <int R>
+static void solve8_levels(const DevSym &S, const SolvePlan &SP, const Solve8Dev &D, double *x8, double *c8,
+                          int l0, int l1, bool fwd, LaunchQueue &st) {
   auto chain = [&](int off, int cnt) {
     const int grid = (cnt + CL - 1) / CL * CL;
     if (cnt <= 0) return;
     if (fwd)
-      launch_early(st, CL, k_fwd_chain8, grid, NT8, CHAIN8_SMEM, S, D.fchain + off, cnt, x8, c8, D.cptr, D.cidx,
+      launch_early(st, CL, k_fwd_chain8<R>, grid, NT8, CHAIN8_SMEM, S, D.fchain + off, cnt, x8, c8, D.cptr, D.cidx,
                    D.flags);
     else
-      launch_early(st, CL, k_bwd_chain8, grid, NT8, CHAIN8_SMEM, S, D.bchain + off, cnt, x8, D.flags);
+      launch_early(st, CL, k_bwd_chain8<R>, grid, NT8, CHAIN8_SMEM, S, D.bchain + off, cnt, x8, D.flags);
   };
   for (int l = l0; fwd && l < l1; ++l) {
     const int nw = SP.warp_off[l + 1] - SP.warp_off[l], ns = SP.level_off[l + 1] - SP.level_off[l];
     const int nc = SP.c8_off[l + 1] - SP.c8_off[l];
     if (nw > 0)
-      launch_early(st, 1, k_fwd_warp8, (nw + WN - 1) / WN, WN * 32, 0, S, D.warp_list + SP.warp_off[l], nw, x8,
+      launch_early(st, 1, k_fwd_warp8<R>, (nw + WN - 1) / WN, WN * 32, 0, S, D.warp_list + SP.warp_off[l], nw, x8,
                    c8, D.cptr, D.cidx);
     if (ns > 0)
-      launch_early(st, 1, k_fwd_small8, ns, NT8, SMALL8_SMEM, S, D.list + SP.level_off[l], x8, c8, D.cptr, D.cidx);
+      launch_early(st, 1, k_fwd_small8<R>, ns, NT8, SMALL8_SMEM, S, D.list + SP.level_off[l], x8, c8, D.cptr, D.cidx);
     chain(SP.chain_off[l], SP.chain_off[l + 1] - SP.chain_off[l]);
     if (nc > 0 && SP.c8_split[l])
-      launch_early(st, 1, k_contrib8_split, nc, CS_W * 32, 0, S, D.c8_tasks + SP.c8_off[l], x8, c8);
+      launch_early(st, 1, k_contrib8_split<R>, nc, CS_W * 32, 0, S, D.c8_tasks + SP.c8_off[l], x8, c8);
     else if (nc > 0)
-      launch_early(st, 1, k_contrib8, nc, NT8, 0, S, D.c8_tasks + SP.c8_off[l], x8, c8);
+      launch_early(st, 1, k_contrib8<R>, nc, NT8, 0, S, D.c8_tasks + SP.c8_off[l], x8, c8);
   }
   for (int l = l1 - 1; !fwd && l >= l0; --l) {
     const int nw = SP.warp_off[l + 1] - SP.warp_off[l], ns = SP.level_off[l + 1] - SP.level_off[l];
     const int ng = SP.g8_off[l + 1] - SP.g8_off[l];
-    if (ng > 0) launch_early(st, 1, k_gather8, ng, G8_W * 32, 0, S, D.g8_tasks + SP.g8_off[l], x8);
+    if (ng > 0) launch_early(st, 1, k_gather8<R>, ng, G8_W * 32, 0, S, D.g8_tasks + SP.g8_off[l], x8);
     chain(SP.chain_off[l], SP.chain_off[l + 1] - SP.chain_off[l]);
-    if (ns > 0) launch_early(st, 1, k_bwd_small8, ns, NT8, SMALL8_SMEM, S, D.list + SP.level_off[l], x8);
+    if (ns > 0) launch_early(st, 1, k_bwd_small8<R>, ns, NT8, SMALL8_SMEM, S, D.list + SP.level_off[l], x8);
     if (nw > 0)
-      launch_early(st, 1, k_bwd_warp8, (nw + WN - 1) / WN, WN * 32, 0, S, D.warp_list + SP.warp_off[l], nw, x8);
+      launch_early(st, 1, k_bwd_warp8<R>, (nw + WN - 1) / WN, WN * 32, 0, S, D.warp_list + SP.warp_off[l], nw, x8);
   }
+}
+
+void launch_solve8(const DevSym &S, const SolvePlan &SP, const Solve8Dev &D, double *x8, double *c8, int stride,
+                   int l0, int l1, bool fwd, LaunchQueue &st) {
+  if (stride == R8) solve8_levels<R8>(S, SP, D, x8, c8, l0, l1, fwd, st);
+  else solve8_levels<1>(S, SP, D, x8, c8, l0, l1, fwd, st);
 }
 
 }  // namespace swc
