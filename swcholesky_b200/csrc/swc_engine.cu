@@ -533,7 +533,7 @@ bool build_plan(int n, const int *c, const int *r, const int64_t *lC, const int 
   P.dense_toff.assign(supNo, -1);
   std::vector<std::vector<int>> by_level(nlev);
   for (int s = 0; s < supNo; ++s) by_level[level[s]].push_back(s);
-  int launches = 2;
+  int launches = 1;   // the status words
   for (int lv = 0; lv < nlev; ++lv) {
     Wave &W = P.waves[lv];
     W.small_off = (int)P.small_list.size();
@@ -647,13 +647,12 @@ bool build_plan(int n, const int *c, const int *r, const int64_t *lC, const int 
     } else {
       launches += (W.big_cnt > 0);
       for (int j = 0; j < maxnb; ++j)
-        launches += (W.panel_cnt[j] > 0) + (W.syrk_cnt[j] > 0) + (W.diag_cnt[j] > 0);
+        launches += (W.panel_cnt[j] > 0) + (W.syrk_nc[j] > 0) + (W.syrk_cnt[j] > W.syrk_nc[j]) + (W.diag_cnt[j] > 0);
     }
   }
   if (!P.persist_list.empty()) launches += 1;
   if (!P.tiny_list.empty()) launches += 1;
   P.launches = launches;   // + one per wave with update tiles (build_left_plan)
-  P.launches_scatter = launches;
 
   // ---- algorithmic work per kernel class (one factorization) ----
   {
@@ -769,7 +768,6 @@ bool build_left_plan(const int *Ls, const int *prunePtr, const int *pruneSet, co
     tiles.clear();
     W.upd_cnt = (int)P.upd_tasks.size() - W.upd_off;
     P.launches += W.upd_cnt > 0;
-    P.launches_scatter += W.upd_cnt > 0;
   }
   P.left = true;
   return true;
@@ -920,7 +918,6 @@ bool build_scatter_plan(int n, const int *Ls, const HostSym &H, const FrontPlan 
     for (const ScTile &t : P.sc_dense)
       if ((P.sc_used[t.d] & 3) != 3) { err = "internal: dense tile without its tensor maps"; return false; }
     // per level: larger K first (a shorter tail); one descendant's tiles stay together
-    int sc_launches = 0;
     for (int lv = 0; lv < nlev; ++lv) {
       std::vector<ScTile> &v = by_wave[lv];
       std::stable_sort(v.begin(), v.end(),
@@ -931,15 +928,7 @@ bool build_scatter_plan(int n, const int *Ls, const HostSym &H, const FrontPlan 
       P.waves[lv].scs_off = (int)P.sc_small.size();
       P.waves[lv].scs_cnt = (int)small_by_wave[lv].size();
       P.sc_small.insert(P.sc_small.end(), small_by_wave[lv].begin(), small_by_wave[lv].end());
-      sc_launches += !v.empty() + !small_by_wave[lv].empty();
     }
-    // one assemble launch up front instead of one per level; scatter instead of tile-owner
-    int asm_l = 0;
-    for (const Wave &W : P.waves) {
-      asm_l += W.asm_cnt > 0;
-      if (P.left) P.launches_scatter -= W.upd_cnt > 0;
-    }
-    P.launches_scatter += (asm_l > 0) - asm_l + sc_launches;
   return true;
 }
 
@@ -1482,7 +1471,6 @@ bool Engine::analyze(int n, const int *c, const int *r, const int64_t *lC, const
   // hold, the right-looking tables are checked) now
   if (!FP->ok && !build_left_plan(Ls, prunePtr, pruneSet, H, P, err)) return false;
   if (!FP->closed && !build_scatter_plan(n, Ls, H, FP.get(), P, tuning_, err)) return false;
-  if (FP->ok) P.launches = FP->launches;
 
   // ---- solve plan: levels of the supernodal etree, per-level task lists ----
   SolvePlan SP;
@@ -2082,6 +2070,11 @@ int Engine::factor_profiled(const double *values, bool values_on_device, int *in
   }
   for (auto &pe : prof) cudaEventDestroy(pe.second);
   return rc;
+}
+
+int Engine::launches_per_factor() const {
+  const bool front = front_ && front_->ok && (front_ready_ || !front_tried_);
+  return front ? front_->launches : plan_.launches;
 }
 
 int Engine::finish(int *info, std::string &err) {

@@ -207,8 +207,7 @@ struct Plan {
   double sc_flops = 0;               // executed flops of the tiles (128x128 blocks)
   int persist_smem = 0;
   bool left = false;               // the left-looking tiles are built (build_left_plan)
-  int launches = 0;  // kernel launches per factorization
-  int launches_scatter = 0;  // the same in the mixed modes with right-looking updates
+  int launches = 0;  // kernel launches per FP64 factorization, left-looking
   KernelStats work;  // algorithmic flops/bytes per kernel class
 };
 
@@ -428,10 +427,8 @@ class Engine {
   int nsuper() const { return nsuper_; }
   const Plan &plan() const { return plan_; }
   double *device_L() const { return dL_; }
-  // kernel launches of one factorization in the given mode
-  int launches_per_factor(int prec = 0) const {
-    return prec != 0 ? plan_.launches_scatter : plan_.launches;
-  }
+  // kernel launches of one FP64 factorization
+  int launches_per_factor() const;
 
   // Adjoint (swc_adjoint.cu), on the current factor; device pointers, grad has one entry
   // per stored nonzero of A.

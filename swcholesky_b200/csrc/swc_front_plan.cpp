@@ -241,7 +241,7 @@ void build_front_plan(int n, const int *c, const int *r, const int *Ls, const in
     for (const auto &it : items) pairs[end[t0 + it.first]++] = it.second;
   };
   F.waves.resize(nlev);
-  int launches = 2 + !P.big_list.empty();
+  int launches = 1 + !P.big_list.empty();
   for (int lv = 0; lv < nlev; ++lv) {
     FrontWave &W = F.waves[lv];
     W.small_off = (int)F.small_list.size();
