@@ -204,8 +204,9 @@ int swc_profile(swc_handle_t handle, const double *values, int values_on_device,
  * stats[0..19] = levels, kernel launches per factorization,
  * small-class supernodes, tiled-class supernodes, update tiles, update (tile, descendant)
  * pairs, TRSM tiles, SYRK tiles, then per kernel class (memset, small, assemble, update,
- * panel, syrk) the algorithmic flops [8..13] and DRAM bytes [14..19] of one
- * factorization.  No reference counterpart. */
+ * panel, syrk) the algorithmic flops [8..13] and DRAM bytes [14..19] of one FP64
+ * factorization (the update tiles and pairs are the left-looking kernels', which run where
+ * the multifrontal ones do not apply).  No reference counterpart. */
 int swc_plan_stats(int n, const int *c, const int *r, const size_t *lC, const int *Ls,
                    const size_t *Li_ptr, const int *blockSet, int supNo, const int *prunePtr,
                    const int *pruneSet, int plan, double *stats);

@@ -434,7 +434,10 @@ int swc_plan_stats(int n, const int *c, const int *r, const size_t *lC, const in
     return fail(SWC_INVALID_INPUT, err);
   if (!swc::check_front_plan(n, Ls, H, P, FP, err) || !swc::check_adjoint_plan(H, P, FP, err))
     return fail(SWC_INVALID_INPUT, err);
-  if (FP.ok) P.launches = FP.launches;
+  if (FP.ok) {
+    P.launches = FP.launches;
+    P.work = FP.work;
+  }
   swc::SolvePlan SP;
   swc::build_solve_plan(n, Ls, H, SP);
   if (!swc::check_solve_plan(n, Ls, H, SP, err)) return fail(SWC_INVALID_INPUT, err);

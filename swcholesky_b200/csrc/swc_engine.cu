@@ -769,7 +769,7 @@ bool build_left_plan(const int *Ls, const int *prunePtr, const int *pruneSet, co
     W.upd_cnt = (int)P.upd_tasks.size() - W.upd_off;
     P.launches += W.upd_cnt > 0;
   }
-  P.left = true;
+  P.left = P.update_work = true;
   return true;
 }
 
@@ -1824,7 +1824,7 @@ void Engine::launch_all(std::vector<std::pair<int, cudaEvent_t>> *prof, int prec
       mark(-1, cnt);
     };
     if (front) {
-      mark(K_ASSEMBLE, FWv->ext_cnt);
+      mark(K_UPDATE, FWv->ext_cnt);
       launch_front_extend(sym_, *front_dev_, d_fext_ + FWv->ext_off, d_fext_end_ + FWv->ext_off,
                           d_fext_pairs_, FWv->ext_cnt, LaunchQueue{st, behind});
       mark(-1, FWv->ext_cnt);
@@ -2049,8 +2049,10 @@ int Engine::factor_profiled(const double *values, bool values_on_device, int *in
   std::vector<std::pair<int, cudaEvent_t>> prof;
   launch_all(&prof, prec);
   int rc = finish(info, err);
+  const bool front = prec == 0 && front_ready_;
   std::string werr;
-  if (!plan_.left) {   // the update class's algorithmic work comes with its tiles
+  if (!front && !plan_.update_work) {   // the descendants' updates' work comes with their tiles
+    plan_.update_work = true;
     Plan w;
     w.waves = plan_.waves;
     w.big_list = plan_.big_list;
@@ -2059,7 +2061,7 @@ int Engine::factor_profiled(const double *values, bool values_on_device, int *in
       plan_.work.bytes[K_UPDATE] = w.work.bytes[K_UPDATE];
     }
   }
-  out = plan_.work;
+  out = front ? front_->work : plan_.work;
   for (int k = 0; k < K_NKINDS; ++k) { out.launches[k] = 0; out.ms[k] = 0; }
   for (size_t i = 0; i + 1 < prof.size(); i += 2) {
     float ms = 0;

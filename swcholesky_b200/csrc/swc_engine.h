@@ -164,7 +164,10 @@ struct Wave {
   int scs_off = 0, scs_cnt = 0; // the same level's small contributions
 };
 
-// Kernel classes, for per-kernel timing (profiled factorization) and flop accounting.
+// Kernel classes, for per-kernel timing (profiled factorization) and flop accounting.  K_SMALL: the
+// small supernodes whole; K_ASSEMBLE: A into the tiled panels; K_UPDATE: the descendants' updates of
+// those (multifrontal: the children's blocks added to them, and the contribution blocks formed by
+// tiles); K_PANEL, K_SYRK: their dense steps.
 enum KernelKind { K_MEMSET = 0, K_SMALL, K_ASSEMBLE, K_UPDATE, K_PANEL, K_SYRK, K_NKINDS };
 
 struct KernelStats {
@@ -208,7 +211,8 @@ struct Plan {
   int persist_smem = 0;
   bool left = false;               // the left-looking tiles are built (build_left_plan)
   int launches = 0;  // kernel launches per FP64 factorization, left-looking
-  KernelStats work;  // algorithmic flops/bytes per kernel class
+  KernelStats work;  // algorithmic flops/bytes per kernel class (left-looking)
+  bool update_work = false;   // K_UPDATE's are known
 };
 
 

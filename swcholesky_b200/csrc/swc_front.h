@@ -137,6 +137,8 @@ struct FrontPlan {
   std::vector<int> ext_end, sch_end;        // one past the last pair
   std::vector<int4> ext_pairs, sch_pairs;   // (child, a0, b0, na | nb << 16)
   int launches = 0;
+  KernelStats work;                // algorithmic flops (products; a child's entry added is not counted)
+                                   // and bytes per kernel class
 };
 
 // Derives the multifrontal plan of an analysed structure.  P.ok stays false, and the

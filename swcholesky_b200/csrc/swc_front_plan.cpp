@@ -312,6 +312,34 @@ void build_front_plan(int n, const int *c, const int *r, const int *Ls, const in
   for (int s : F.warp_list) F.warp_desc.push_back(desc(s, false));
   for (int s : F.cta_list) F.cta_desc.push_back(desc(s, false));
   for (int e : F.small_list) F.small_desc.push_back(desc(e < 0 ? ~e : e, e < 0));
+
+  // work: every product once, every entry of A, of L and of the blocks read or written once by the
+  // class that does it
+  F.work = P.work;
+  KernelStats &K = F.work;
+  K.flops[K_SMALL] = K.bytes[K_SMALL] = K.flops[K_UPDATE] = K.bytes[K_UPDATE] = 0.0;
+  std::vector<char> by_tiles(ns, 0);
+  for (int e : F.small_list)
+    if (e < 0) by_tiles[~e] = 1;
+  for (int s = 0; s < ns; ++s) {
+    const double w = width(s), rr = rows(s) - width(s);
+    const int own = tiled[s] || by_tiles[s] ? K_UPDATE : K_SMALL;   // who forms its block
+    if (!tiled[s]) {
+      K.flops[K_SMALL] += w * w * w / 3.0 + rr * w * w;
+      K.bytes[K_SMALL] += 8.0 * (w + rr) * w + 12.0 * (c[super[s + 1]] - c[super[s]]);
+    }
+    K.flops[own] += rr * (rr + 1.0) * w;
+    K.bytes[own] += 4.0 * rr * (rr + 1.0) + (own == K_UPDATE ? 8.0 * rr * w : 0.0);
+    for (int q = F.child_ptr[s]; q < F.child_ptr[s + 1]; ++q) {
+      const double rd = rows(F.child[q]) - width(F.child[q]), n1 = F.child_n1[F.child[q]], n2 = rd - n1;
+      K.bytes[tiled[s] ? K_UPDATE : K_SMALL] += 8.0 * (n1 * rd - n1 * (n1 - 1.0) / 2.0) + 4.0 * rd;
+      K.bytes[own] += 4.0 * n2 * (n2 + 1.0);
+    }
+  }
+  for (const int4 &t : F.ext_tasks) {   // tiles of tiled panels, read and written
+    const int nr = std::min(TB, rows(t.x) - t.y), nc = std::min(TB, width(t.x) - t.z);
+    K.bytes[K_UPDATE] += 16.0 * (t.y == t.z ? nr * nc - nc * (nc - 1) / 2 : nr * nc);
+  }
   F.ok = true;
 }
 
