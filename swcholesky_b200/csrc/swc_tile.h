@@ -64,9 +64,12 @@ constexpr int KC = 16;
 constexpr int MT = 128;               // threads of the tensor-core tile kernels
 constexpr int LDS = TB + 4;           // padded row of a staged k-slice: 64-bit fragment loads conflict-free
 constexpr int STAGE = 2 * KC * LDS;   // doubles per pipeline stage (A and B slices)
-// Tile launches that run beside the chain of diagonal blocks: one CTA per SM of three groups (its
-// shared memory keeps a second one out), so the SMs the launch leaves free stay free.
-constexpr int BG = 3, BG_SMEM = BG * 2 * STAGE * 8;
+// Tile launches that run beside the chain of diagonal blocks: one CTA per SM of three groups, so the
+// SMs the launch leaves free stay free.  It asks for more than half of an SM's 228 KB of shared memory
+// (1 KB of it per CTA is the system's), whatever its registers would allow; its stages need 102 KB.
+constexpr int SM_SMEM = 228 * 1024;
+constexpr int BG = 3, BG_SMEM = SM_SMEM / 2;
+static_assert(BG_SMEM >= BG * 2 * STAGE * 8 && 2 * (BG_SMEM + 1024) > SM_SMEM, "the stages fit, a second CTA does not");
 static_assert(MT == 2 * TB, "staging pattern: two threads per tile row");
 
 __device__ __forceinline__ void cp_async8(double *smem, const double *gmem, bool pred) {
