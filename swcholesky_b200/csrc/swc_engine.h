@@ -20,6 +20,9 @@ namespace swc {
 // the second factorization of a structure frees those left.  A block serves requests of 8/9 of its
 // size or more.  Not for use by several threads at once (an engine is not either).
 constexpr size_t KEEP_BYTES = (size_t)64 << 20;
+// Contribution blocks of at most this size are taken by the analysis, larger ones by the first FP64
+// factorization.
+constexpr size_t BLOCKS_AT_ONCE = (size_t)16 << 20;
 class DeviceMemory {
  public:
   ~DeviceMemory();
@@ -490,6 +493,7 @@ class Engine {
   bool swept_ = false;                         // and the adjoint's sweep
   bool prepare_tree(std::string &err);   // the tree's tables (also the adjoint's)
   bool prepare_front(std::string &err);
+  bool take_blocks();
   void drop_blocks();
   void release_front();
   size_t mirror_bytes() const { return sizeof(float) * (size_t)std::max<int64_t>(kmirror_len_, 8); }
