@@ -278,7 +278,6 @@ void Engine::release() {
   d_xk_ = d_xk16_ = nullptr;
   d_tmaps_ = nullptr;
   d_tc_pairs_ = d_syrk_pairs_ = nullptr;
-  d_syrk_end_ = nullptr;
   d_sc_tiles_ = nullptr;
   d_sc_small_ = nullptr;
   d_sc_dense_ = nullptr;
@@ -587,7 +586,6 @@ bool build_plan(int n, const int *c, const int *r, const int64_t *lC, const int 
         P.syrk_pairs.push_back(TcPair{s, r0, cc, (first * TB) | (kc << 16), low_bits(std::min(TB, m - r0)),
                                       low_bits(std::min(TB, w - cc))});
         P.syrk_tasks.push_back(make_int4(s, r0, cc, (int)P.syrk_tasks.size()));
-        P.syrk_end.push_back((int)P.syrk_tasks.size());
       };
       for (int s : big) {
         int w = super[s + 1] - super[s];
@@ -707,7 +705,6 @@ bool build_plan(int n, const int *c, const int *r, const int64_t *lC, const int 
       K.flops[K_SYRK] = K.bytes[K_SYRK] = 0.0;
     }
   }
-  H.xptr = xptr;
   H.dinv_off.assign(supNo, -1);
   H.ndinv = 0;
   for (int s : P.big_list) {
@@ -1522,7 +1519,6 @@ bool Engine::analyze(int n, const int *c, const int *r, const int64_t *lC, const
   up.add(d_panel_, P.panel_tasks.data(), P.panel_tasks.size());
   up.add(d_syrk_, P.syrk_tasks.data(), P.syrk_tasks.size());
   up.add(d_syrk_pairs_, P.syrk_pairs.data(), P.syrk_pairs.size());
-  up.add(d_syrk_end_, P.syrk_end.data(), P.syrk_end.size());
   up.add(d_dense_tasks_, P.dense_tasks.data(), P.dense_tasks.size());
   up.add(d_dense_toff_, P.dense_toff.data(), P.dense_toff.size());
   up.add(d_dinv_off_, H.dinv_off.data(), H.dinv_off.size());

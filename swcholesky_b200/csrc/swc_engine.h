@@ -59,7 +59,7 @@ class DeviceMemory {
   void give(void *p, bool keep);
 };
 
-// Host tables in one device block (the sources stay alive until commit).
+// Host tables in one device block, a copy each (the sources stay alive until commit).
 class TableUpload {
  public:
   template <typename T>
@@ -192,7 +192,6 @@ struct Plan {
   std::vector<int4> upd_pairs;     // (d, a0, b0, na | nb << 16)
   std::vector<TcPair> tc_pairs;    // the same pairs for the tcgen05 kernel (tile masks)
   std::vector<TcPair> syrk_pairs;  // per SYRK task: its product (s, r0, c0, step block)
-  std::vector<int> syrk_end;       // per SYRK task: one past its pair (its index + 1)
   std::vector<int2> panel_tasks;
   std::vector<int4> syrk_tasks;
   std::vector<int> diag_list;
@@ -538,7 +537,6 @@ class Engine {
   std::vector<int64_t> h_xk_;
   int64_t kmirror_len_ = 0;
   TcPair *d_tc_pairs_ = nullptr, *d_syrk_pairs_ = nullptr;
-  int *d_syrk_end_ = nullptr;
   ScTile *d_sc_tiles_ = nullptr;               // right-looking update tiles and their tables
   int2 *d_sc_small_ = nullptr;
   ScTile *d_sc_dense_ = nullptr;

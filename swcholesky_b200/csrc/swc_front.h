@@ -27,8 +27,8 @@
 
 namespace swc {
 
-// Fronts done by one warp: padded panel of at most FRONT_WARP_ELEMS doubles, at most
-// FRONT_WARP_R off-diagonal rows.
+// Fronts done by one warp: padded panel of at most FRONT_WARP_ELEMS doubles, at most FRONT_WARP_M
+// rows.
 constexpr int FRONT_WARP_ELEMS = 1280;
 constexpr int FRONT_WARP_M = 128;
 constexpr int FRONT_KIDS = 4;   // children whose row maps are held at a time
@@ -113,7 +113,7 @@ struct FrontWave {
 // FRONT_BG_STEPS), on all but FRONT_BG_RESERVE SMs, beside the chain of diagonal blocks (about
 // FRONT_STEP_US per 64 columns), where that chain is what the wave waits for: its dense products
 // at FRONT_FLOPS_US flops per us take at most 1.5 times as long.  Waves of few small fronts
-// gain (24 x 23 x 22 3-unknown grid 3249 -> 3138 us, 41 x 37 x 43 7-point grid 3072 -> 3027);
+// gain (24 x 23 x 22 3-unknown grid 3249 -> 3155 us, 41 x 37 x 43 7-point grid 3072 -> 3039);
 // with more work the launches only disturb each other (60^3: 14.6 -> 16.2 ms).
 constexpr int FRONT_BG_STEPS = 3, FRONT_BG_RESERVE = 40;
 constexpr double FRONT_STEP_US = 22.0, FRONT_FLOPS_US = 28e6;

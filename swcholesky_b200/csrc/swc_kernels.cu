@@ -864,10 +864,9 @@ __global__ void __launch_bounds__(MT, 4) k_trsm_step(DevSym S, const int2 *tasks
 
 // Trailing update of a step: task = (s, r0, c0, product index) with c0 >= (step+1)*64,
 // r0 >= c0; the product names the column blocks applied (the step's block, or a group of
-// blocks ending with it).  The diagonal tile of the next block is updated by the TRSM
-// launch of the step and factored by k_diag_step, which runs concurrently.  The tile just below
-// that one also goes to the place of its diagonal block's inverse in dinv (free until then),
-// unsolved, for the block's own solve of it.
+// blocks ending with it).  The next diagonal tile's update by the step's block is k_diag_step's,
+// which factors it beside this launch.  The tile just below that one also goes to the place of its
+// diagonal block's inverse in dinv (free until then), unsolved, for the block's own solve of it.
 constexpr int SYRK_SMEM = 2 * STAGE * 8;
 
 __global__ void __launch_bounds__(MT) k_syrk_step(DevSym S, const int4 *tasks, const TcPair *prod,

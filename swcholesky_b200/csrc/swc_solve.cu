@@ -200,7 +200,7 @@ __global__ void __launch_bounds__(CT, 2) k_fwd_contrib(DevSym S, const int2 *tas
 
 // Backward solve, level by level (root first):
 //   k_bwd_gather  tiled supernodes: x[f + j] := x[f + j] - sum_{a >= w} L(a, j) x[rows[a]] for
-//                 the columns j0..j0+15 of s (one warp per column, eight loads in flight per
+//                 the columns j0..j0+15 of s (one warp per column, GU loads in flight per
 //                 lane); the rows below are columns of ancestors, already solved.  Then
 //                 k_bwd_chain.
 //   k_bwd_small   small supernodes, one CTA each: the gather and L_ss^{-T}.
