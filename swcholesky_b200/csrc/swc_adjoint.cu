@@ -500,8 +500,11 @@ static int64_t place_adjoint(const std::vector<std::vector<int>> &waves, const s
   FrontArena A;
   std::vector<int> left(len.size());   // children not done yet
   for (size_t s = 0; s < len.size(); ++s) left[s] = F.child_ptr[s + 1] - F.child_ptr[s];
+  std::vector<int> order;
   for (const std::vector<int> &here : waves) {
-    for (int s : here) zoff[s] = A.take(len[s]);
+    order = here;   // the largest first: less is lost between them
+    std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return len[a] > len[b]; });
+    for (int s : order) zoff[s] = A.take(len[s]);
     for (int s : here) {
       if (F.child_ptr[s + 1] == F.child_ptr[s]) A.give(zoff[s], len[s]);
       const int p = parent[s];

@@ -20,7 +20,9 @@
 
 #include <cstdint>
 #include <map>
+#include <set>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "swc_engine.h"
@@ -65,7 +67,8 @@ inline int64_t front_memory_limit(int64_t xsize) {
   return 4 * xsize > floor ? 4 * xsize : floor;
 }
 
-// First-fit placement of blocks that live over a range of waves.
+// Best-fit placement of blocks that live over a range of waves, in logarithmic time (batches free and
+// place a hundred thousand small blocks level by level).
 class FrontArena {
  public:
   int64_t take(int64_t len);
@@ -73,7 +76,9 @@ class FrontArena {
   int64_t end() const { return end_; }
 
  private:
-  std::map<int64_t, int64_t> free_;
+  void put(int64_t at, int64_t len);
+  std::map<int64_t, int64_t> free_;                    // length by place
+  std::set<std::pair<int64_t, int64_t>> by_len_;       // (length, place)
   int64_t end_ = 0;
 };
 

@@ -44,32 +44,43 @@ bool prune_sets_complete(const int *Ls, const int *prunePtr, const int *pruneSet
 }  // namespace
 
 int64_t FrontArena::take(int64_t len) {
-  for (auto it = free_.begin(); it != free_.end(); ++it)
-    if (it->second >= len) {
-      const int64_t at = it->first, rest = it->second - len;
-      free_.erase(it);
-      if (rest) free_[at + len] = rest;
-      return at;
-    }
-  const int64_t at = end_;
-  end_ += len;
+  auto it = by_len_.lower_bound({len, 0});
+  if (it == by_len_.end()) {
+    const int64_t at = end_;
+    end_ += len;
+    return at;
+  }
+  const int64_t at = it->second, rest = it->first - len;
+  by_len_.erase(it);
+  free_.erase(at);
+  if (rest) put(at + len, rest);
   return at;
 }
 
+void FrontArena::put(int64_t at, int64_t len) {
+  free_[at] = len;
+  by_len_.insert({len, at});
+}
+
 void FrontArena::give(int64_t at, int64_t len) {
-  auto it = free_.emplace(at, len).first;
-  auto nx = std::next(it);
-  if (nx != free_.end() && it->first + it->second == nx->first) {
-    it->second += nx->second;
-    free_.erase(nx);
+  auto drop = [&](std::map<int64_t, int64_t>::iterator it) {
+    by_len_.erase({it->second, it->first});
+    return free_.erase(it);
+  };
+  auto nx = free_.lower_bound(at);
+  if (nx != free_.end() && at + len == nx->first) {
+    len += nx->second;
+    nx = drop(nx);
   }
-  if (it != free_.begin()) {
-    auto pv = std::prev(it);
-    if (pv->first + pv->second == it->first) {
-      pv->second += it->second;
-      free_.erase(it);
+  if (nx != free_.begin()) {
+    auto pv = std::prev(nx);
+    if (pv->first + pv->second == at) {
+      at = pv->first;
+      len += pv->second;
+      drop(pv);
     }
   }
+  put(at, len);
 }
 
 void build_front_plan(int n, const int *c, const int *r, const int *Ls, const int *prunePtr,
@@ -171,8 +182,11 @@ void build_front_plan(int n, const int *c, const int *r, const int *Ls, const in
   for (int s = 0; s < ns; ++s)
     if (walk(s) && len(s) && walk(parent[s])) A.give(F.cb_off[s], len(s));
   for (int lv = 0; lv < nlev; ++lv) {
+    std::vector<int> here;   // the largest first: less is lost between them
     for (int s : by_level[lv])
-      if (!walk(s) && len(s)) F.cb_off[s] = A.take(len(s));
+      if (!walk(s) && len(s)) here.push_back(s);
+    std::stable_sort(here.begin(), here.end(), [&](int a, int b) { return len(a) > len(b); });
+    for (int s : here) F.cb_off[s] = A.take(len(s));
     for (int s : by_level[lv])
       if (!walk(s))
         for (int q = F.child_ptr[s]; q < F.child_ptr[s + 1]; ++q)
