@@ -2261,12 +2261,12 @@ void Engine::run_solve(double *x, int nrhs) {
         cudaMemcpyAsync(xr, d_sx_, bytes, cudaMemcpyDeviceToDevice, stream_);
       }
     } else {
-      launch_pack8(n_, nr, xr, d_x8_, stream_);
+      launch_pack8(n_, nr, xr, d_x8_, 8, stream_);
       cudaGraphExec_t g = use_graph_ && solved_[1] ? solve_graph(true) : nullptr;
       solved_[1] = true;
       if (g) cudaGraphLaunch(g, stream_);
       else run_solve8(d_x8_, d_c8_, 8);
-      launch_unpack8(n_, nr, d_x8_, xr, stream_);
+      launch_unpack8(n_, nr, d_x8_, xr, 8, stream_);
     }
   }
 }
@@ -2367,7 +2367,7 @@ bool Engine::refine(const double *b, double *x, int nrhs, double tol, int maxit,
     for (int k = 0; nrhs > 1 && k < nrhs; k += 8) {
       const int nr = std::min(8, nrhs - k);
       const size_t at = (size_t)k * n_;
-      launch_pack8(n_, nr, xx + at, d_x8_, st);
+      launch_pack8(n_, nr, xx + at, d_x8_, 8, st);
       launch_spmv8(n_, d_csr_rp_, d_csr_ci_, d_csr_val_, d_x8_, b + at, r + at, nr, st);
     }
     if (nrhs == 1) launch_spmv(n_, d_csr_rp_, d_csr_ci_, d_csr_val_, xx, b, r, st);
@@ -2465,19 +2465,21 @@ bool Engine::solve_in_scratch(const double *b, double *x, int nrhs, double *scra
   if (x != b) e = cudaMemcpyAsync(x, b, sizeof(double) * n_ * nrhs, cudaMemcpyDeviceToDevice, st);
   if (e == cudaSuccess) e = cudaMemsetAsync(d_status_ + 2, 0, sizeof(int), st);
   if (e != cudaSuccess) { err = std::string("solve: ") + cudaGetErrorString(e); return false; }
-  // the groups and the kernels of run_solve; a group that the scratch cannot hold interleaved, with
-  // its contributions, goes one vector at a time through the same products
+  // the groups and the kernels of run_solve; where the scratch cannot hold eight vectors and their
+  // contributions, four, two or one at a time through the same products
+  int R = 8;
+  while (R > 1 && R * (cs + n_) > capacity) R /= 2;
   for (int r0 = 0; r0 < nrhs; r0 += 8) {
     const int nr = std::min(8, nrhs - r0);
-    double *xr = x + (size_t)r0 * n_, *x8 = scratch + 8 * cs;
     if (nr == 1) {
-      run_solve_with(xr, 1, scratch);
-    } else if (8 * (cs + n_) <= capacity) {
-      launch_pack8(n_, nr, xr, x8, st);
-      run_solve8(x8, scratch, 8);
-      launch_unpack8(n_, nr, x8, xr, st);
-    } else {
-      for (int r = 0; r < nr; ++r) run_solve8(xr + (size_t)r * n_, scratch, 1);
+      run_solve_with(x + (size_t)r0 * n_, 1, scratch);
+      continue;
+    }
+    for (int r = 0; r < nr; r += R) {
+      double *xr = x + (size_t)(r0 + r) * n_, *x8 = R > 1 ? scratch + R * cs : xr;
+      if (R > 1) launch_pack8(n_, std::min(R, nr - r), xr, x8, R, st);
+      run_solve8(x8, scratch, R);
+      if (R > 1) launch_unpack8(n_, std::min(R, nr - r), x8, xr, R, st);
     }
   }
   e = cudaStreamSynchronize(st);

@@ -319,10 +319,11 @@ struct Solve8Dev {
   int *flags;   // the chained blocks' counters, zeroed before the solve
 };
 bool solve8_configure(std::string &err);
-void launch_pack8(int n, int nr, const double *x, double *x8, cudaStream_t st);
-void launch_unpack8(int n, int nr, const double *x8, double *x, cudaStream_t st);
-// the levels l0 .. l1 - 1, forward or backward; stride 8, or 1: one plain vector in x8, its
-// contributions in c8, the same arithmetic
+// stride: 8, or 4, 2, 1 for as many vectors (x8 and the contributions c8 interleaved by it) with the
+// same arithmetic; the last is a plain vector
+void launch_pack8(int n, int nr, const double *x, double *x8, int stride, cudaStream_t st);
+void launch_unpack8(int n, int nr, const double *x8, double *x, int stride, cudaStream_t st);
+// the levels l0 .. l1 - 1, forward or backward
 void launch_solve8(const DevSym &S, const SolvePlan &SP, const Solve8Dev &D, double *x8, double *c8, int stride,
                    int l0, int l1, bool fwd, LaunchQueue &st);
 

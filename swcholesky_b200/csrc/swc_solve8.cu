@@ -13,13 +13,14 @@
 // their contributions in a second kernel.  Backward: the mirror image.
 //
 // A right-hand side's result does not depend on the others of its group, nor on its place among
-// them (a tensor-core product's columns are independent).  The kernels come with vectors R = 8 apart
-// and with R = 1, one plain vector in place of the interleaved ones and seven zero columns: the
-// same result bit for bit, for callers whose scratch has no room for eight.
+// them (a tensor-core product's columns are independent).  The kernels come with the vectors
+// interleaved by R = 8, and by 4, 2 and 1 (a plain vector) with zero columns for the others: the same
+// result bit for bit, for callers whose scratch has no room for eight.
 #include <cuda_runtime.h>
 
 #include <algorithm>
 #include <cstdint>
+#include <type_traits>
 
 #include "swc_chain.h"
 #include "swc_engine.h"
@@ -35,14 +36,14 @@ constexpr int NT8 = 256, W8 = NT8 / 32;
 // Right-hand side r of row i in vectors R apart; zero where there is none.
 template <int R>
 __device__ __forceinline__ double rhs_of(const double *x, int64_t i, int r) {
-  return R == R8 || r < R ? x[i * R + r] : 0.0;
+  return r < R ? x[i * R + r] : 0.0;
 }
 
 // Right-hand sides 2 kq, 2 kq + 1 of a row.
 template <int R>
 __device__ __forceinline__ void store_pair(double *row, int kq, double a, double b) {
-  if (R == R8) *reinterpret_cast<double2 *>(row + 2 * kq) = make_double2(a, b);
-  else if (kq == 0) row[0] = a;
+  if (R == 1 && kq == 0) row[0] = a;
+  if (R > 1 && 2 * kq < R) *reinterpret_cast<double2 *>(row + 2 * kq) = make_double2(a, b);
 }
 
 // v - sum of the contributions listed for column j, right-hand side r.
@@ -737,7 +738,8 @@ __global__ void __launch_bounds__(NT8, 1) k_bwd_chain8(DevSym S, const int2 *tas
       const double s0 = (acc[0][0] + acc[1][0]) + (acc[2][0] + acc[3][0]);
       const double s1 = (acc[0][1] + acc[1][1]) + (acc[2][1] + acc[3][1]);
       double2 v = make_double2(0.0, 0.0);
-      if (R == R8 && row < bw) v = *reinterpret_cast<const double2 *>(&x8[(size_t)(f + r0 + row) * R8 + 2 * kq]);
+      if (R > 1 && row < bw && 2 * kq < R)
+        v = *reinterpret_cast<const double2 *>(&x8[(size_t)(f + r0 + row) * R + 2 * kq]);
       if (R == 1 && row < bw && kq == 0) v.x = x8[f + r0 + row];
       *reinterpret_cast<double2 *>(vs + row * R8 + 2 * kq) = make_double2(v.x - s0, v.y - s1);
     }
@@ -747,25 +749,36 @@ __global__ void __launch_bounds__(NT8, 1) k_bwd_chain8(DevSym S, const int2 *tas
   cluster_sync_all();
 }
 
-// nr vectors of length n (leading dimension n) to the interleaved form, zeros beyond nr; and back.
+// nr vectors of length n (leading dimension n) to the form interleaved by R, zeros beyond nr; and back.
+template <int R>
 __global__ void k_pack8(int n, int nr, const double *x, double *x8) {
   const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int i = (int)(e >> 3), r = (int)(e & 7);
+  const int i = (int)(e / R), r = (int)(e % R);
   if (i < n) x8[e] = r < nr ? x[(size_t)r * n + i] : 0.0;
 }
+template <int R>
 __global__ void k_unpack8(int n, int nr, const double *x8, double *x) {
   const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int i = (int)(e >> 3), r = (int)(e & 7);
+  const int i = (int)(e / R), r = (int)(e % R);
   if (i < n && r < nr) x[(size_t)r * n + i] = x8[e];
+}
+
+// fn with the interleaving as a constant
+template <class F>
+void with_stride(int stride, F fn) {
+  if (stride == 8) fn(std::integral_constant<int, 8>());
+  else if (stride == 4) fn(std::integral_constant<int, 4>());
+  else if (stride == 2) fn(std::integral_constant<int, 2>());
+  else fn(std::integral_constant<int, 1>());
 }
 
 }  // namespace
 
 bool solve8_configure(std::string &err) {
   cudaError_t e = cudaSuccess;
-  for (auto k : {k_fwd_chain8<R8>, k_fwd_chain8<1>})
+  for (auto k : {k_fwd_chain8<8>, k_fwd_chain8<4>, k_fwd_chain8<2>, k_fwd_chain8<1>})
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, CHAIN8_SMEM);
-  for (auto k : {k_bwd_chain8<R8>, k_bwd_chain8<1>})
+  for (auto k : {k_bwd_chain8<8>, k_bwd_chain8<4>, k_bwd_chain8<2>, k_bwd_chain8<1>})
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, CHAIN8_SMEM);
   if (e != cudaSuccess) {
     err = std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(e);
@@ -774,11 +787,13 @@ bool solve8_configure(std::string &err) {
   return true;
 }
 
-void launch_pack8(int n, int nr, const double *x, double *x8, cudaStream_t st) {
-  k_pack8<<<(unsigned)(((int64_t)n * R8 + 255) / 256), 256, 0, st>>>(n, nr, x, x8);
+void launch_pack8(int n, int nr, const double *x, double *x8, int stride, cudaStream_t st) {
+  const unsigned grid = (unsigned)(((int64_t)n * stride + 255) / 256);
+  with_stride(stride, [&](auto R) { k_pack8<R.value><<<grid, 256, 0, st>>>(n, nr, x, x8); });
 }
-void launch_unpack8(int n, int nr, const double *x8, double *x, cudaStream_t st) {
-  k_unpack8<<<(unsigned)(((int64_t)n * R8 + 255) / 256), 256, 0, st>>>(n, nr, x8, x);
+void launch_unpack8(int n, int nr, const double *x8, double *x, int stride, cudaStream_t st) {
+  const unsigned grid = (unsigned)(((int64_t)n * stride + 255) / 256);
+  with_stride(stride, [&](auto R) { k_unpack8<R.value><<<grid, 256, 0, st>>>(n, nr, x8, x); });
 }
 
 template <int R>
@@ -820,8 +835,7 @@ static void solve8_levels(const DevSym &S, const SolvePlan &SP, const Solve8Dev 
 
 void launch_solve8(const DevSym &S, const SolvePlan &SP, const Solve8Dev &D, double *x8, double *c8, int stride,
                    int l0, int l1, bool fwd, LaunchQueue &st) {
-  if (stride == R8) solve8_levels<R8>(S, SP, D, x8, c8, l0, l1, fwd, st);
-  else solve8_levels<1>(S, SP, D, x8, c8, l0, l1, fwd, st);
+  with_stride(stride, [&](auto R) { solve8_levels<R.value>(S, SP, D, x8, c8, l0, l1, fwd, st); });
 }
 
 }  // namespace swc

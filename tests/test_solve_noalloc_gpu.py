@@ -1,6 +1,6 @@
 """swc_solve_noalloc gives the same result as swc_solve, bit for bit, at every number of right-hand
 sides it takes: counts around the groups of eight, and structures whose eight vectors and
-contributions fit its scratch interleaved and others whose do not (one vector at a time then)."""
+contributions fit its scratch interleaved and others of which it takes four, two or one at a time."""
 import ctypes
 
 import numpy as np
@@ -18,6 +18,7 @@ def structures():
     yield "plate", M.weighted_grid_2d(61, 47, shift=0.1, seed=1), M.nested_dissection((61, 47)), 1 << 30
     yield "plate_wide", M.weighted_grid_2d(201, 189, shift=0.1, seed=2), M.nested_dissection((201, 189)), 1 << 30
     yield "plate_crowded", M.weighted_grid_2d(330, 301, shift=0.1, seed=2), M.nested_dissection((330, 301)), 1 << 30
+    yield "plate_largest", M.weighted_grid_2d(410, 400, shift=0.1, seed=2), M.nested_dissection((410, 400)), 1 << 30
     yield "brick", M.laplacian_3d(20, 1e-2), M.nested_dissection((20, 20, 20)), 1 << 30
     yield "brick_large", M.laplacian_3d(31, 1e-2), M.nested_dissection((31, 31, 31)), 1 << 30
     yield "brick_capped", M.laplacian_3d(15, 1e-2), M.nested_dissection((15, 15, 15)), 70
