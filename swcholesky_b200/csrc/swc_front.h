@@ -67,8 +67,9 @@ inline int64_t front_memory_limit(int64_t xsize) {
   return 4 * xsize > floor ? 4 * xsize : floor;
 }
 
-// Best-fit placement of blocks that live over a range of waves, in logarithmic time (batches free and
-// place a hundred thousand small blocks level by level).
+// Placement of blocks that live over a range of waves: the first free place that fits while there are
+// FEW, then the smallest, in logarithmic time (batches free and place a hundred thousand small blocks
+// level by level; for small structures the index would cost more than it saves).
 class FrontArena {
  public:
   int64_t take(int64_t len);
@@ -76,9 +77,12 @@ class FrontArena {
   int64_t end() const { return end_; }
 
  private:
+  static constexpr size_t FEW = 256;
   void put(int64_t at, int64_t len);
+  std::map<int64_t, int64_t>::iterator drop(std::map<int64_t, int64_t>::iterator it);
   std::map<int64_t, int64_t> free_;                    // length by place
-  std::set<std::pair<int64_t, int64_t>> by_len_;       // (length, place)
+  std::set<std::pair<int64_t, int64_t>> by_len_;       // (length, place), once indexed_
+  bool indexed_ = false;
   int64_t end_ = 0;
 };
 

@@ -44,29 +44,39 @@ bool prune_sets_complete(const int *Ls, const int *prunePtr, const int *pruneSet
 }  // namespace
 
 int64_t FrontArena::take(int64_t len) {
-  auto it = by_len_.lower_bound({len, 0});
-  if (it == by_len_.end()) {
+  if (!indexed_ && free_.size() > FEW) {
+    for (const auto &f : free_) by_len_.insert({f.second, f.first});
+    indexed_ = true;
+  }
+  auto it = free_.begin();
+  if (indexed_) {
+    const auto fit = by_len_.lower_bound({len, 0});
+    it = fit == by_len_.end() ? free_.end() : free_.find(fit->second);
+  } else {
+    while (it != free_.end() && it->second < len) ++it;
+  }
+  if (it == free_.end()) {
     const int64_t at = end_;
     end_ += len;
     return at;
   }
-  const int64_t at = it->second, rest = it->first - len;
-  by_len_.erase(it);
-  free_.erase(at);
+  const int64_t at = it->first, rest = it->second - len;
+  drop(it);
   if (rest) put(at + len, rest);
   return at;
 }
 
 void FrontArena::put(int64_t at, int64_t len) {
-  free_[at] = len;
-  by_len_.insert({len, at});
+  free_.emplace(at, len);
+  if (indexed_) by_len_.insert({len, at});
+}
+
+std::map<int64_t, int64_t>::iterator FrontArena::drop(std::map<int64_t, int64_t>::iterator it) {
+  if (indexed_) by_len_.erase({it->second, it->first});
+  return free_.erase(it);
 }
 
 void FrontArena::give(int64_t at, int64_t len) {
-  auto drop = [&](std::map<int64_t, int64_t>::iterator it) {
-    by_len_.erase({it->second, it->first});
-    return free_.erase(it);
-  };
   auto nx = free_.lower_bound(at);
   if (nx != free_.end() && at + len == nx->first) {
     len += nx->second;
