@@ -33,7 +33,17 @@ namespace {
 constexpr int R8 = 8;
 constexpr int NT8 = 256, W8 = NT8 / 32;
 
-// Right-hand side r of row i in vectors R apart; zero where there is none.
+// Element e (row e / 8, right-hand side e % 8) in vectors interleaved by R: its place, and its value,
+// zero where there is none.
+template <int R>
+__device__ __forceinline__ int place8(int e) {
+  return R == R8 ? e : (e >> 3) * R + (e & 7);
+}
+template <int R>
+__device__ __forceinline__ double at8(const double *x, int e) {
+  return R == R8 || (e & 7) < R ? x[place8<R>(e)] : 0.0;
+}
+// Right-hand side r of row i; zero where there is none.
 template <int R>
 __device__ __forceinline__ double rhs_of(const double *x, int64_t i, int r) {
   return r < R ? x[i * R + r] : 0.0;
@@ -115,7 +125,7 @@ __global__ void __launch_bounds__(NT8) k_fwd_small8(DevSym S, const int *list, d
   stage_block(Ld, Ls, m, w);
   pdl_wait();
   for (int e = tid; e < w * R8; e += NT8)
-    v[e] = take_contribs<R>(c8, cptr, cidx, f + (e >> 3), e & 7, rhs_of<R>(y8, f + (e >> 3), e & 7));
+    v[e] = take_contribs<R>(c8, cptr, cidx, f + (e >> 3), e & 7, at8<R>(y8 + (size_t)f * R, e));
   __syncthreads();
   {
     const int i0 = lane, i1 = lane + 32;
@@ -137,7 +147,8 @@ __global__ void __launch_bounds__(NT8) k_fwd_small8(DevSym S, const int *list, d
     if (i1 < w) v[i1 * R8 + warp] = x1;
   }
   __syncthreads();
-  for (int e = tid; e < w * R; e += NT8) y8[(size_t)f * R + e] = v[e / R * R8 + e % R];
+  for (int e = tid; e < w * R8; e += NT8)
+    if ((e & 7) < R) y8[(size_t)f * R + place8<R>(e)] = v[e];
   double *out = c8 + (size_t)(rb - f) * R;
   for (int a0 = w + 8 * warp; a0 < m; a0 += 8 * W8) contrib_rows8<R>(Ls, m, w, a0, v, out);
 }
@@ -183,7 +194,7 @@ __global__ void __launch_bounds__(NT8) k_bwd_small8(DevSym S, const int *list, d
     double t = 0.0;
 #pragma unroll
     for (int q = 0; q < W8; ++q) t += part[q * SMALL_MAX_W * R8 + e];
-    v[e] = rhs_of<R>(x8, f + (e >> 3), e & 7) - t;
+    v[e] = at8<R>(x8 + (size_t)f * R, e) - t;
   }
   __syncthreads();
   stage_block(Ld, Ls, m, w);
@@ -207,7 +218,8 @@ __global__ void __launch_bounds__(NT8) k_bwd_small8(DevSym S, const int *list, d
     if (i1 < w) v[i1 * R8 + warp] = x1;
   }
   __syncthreads();
-  for (int e = tid; e < w * R; e += NT8) x8[(size_t)f * R + e] = v[e / R * R8 + e % R];
+  for (int e = tid; e < w * R8; e += NT8)
+    if ((e & 7) < R) x8[(size_t)f * R + place8<R>(e)] = v[e];
 }
 
 // ---- the small supernodes of crowded levels (w <= SOLVE_WARP_W), one warp each: lane (r, q)
@@ -429,7 +441,7 @@ __global__ void __launch_bounds__(CS_W * 32, 1) k_contrib8_split(DevSym S, const
     double t = 0.0;
 #pragma unroll
     for (int q = 0; q < CS_W; ++q) t += part[q][e];
-    c8[(size_t)((rb - f) + (a0 - w) + (e >> 3)) * R + (e & 7)] = t;
+    c8[(size_t)((rb - f) + (a0 - w)) * R + place8<R>(e)] = t;
   }
 }
 
@@ -487,7 +499,7 @@ __global__ void __launch_bounds__(G8_W * 32, 1) k_gather8(DevSym S, const int2 *
     double t = 0.0;
 #pragma unroll
     for (int q = 0; q < G8_W; ++q) t += part[q][e];
-    x8[(size_t)(f + j0 + (e >> 3)) * R + (e & 7)] -= t;
+    x8[(size_t)(f + j0) * R + place8<R>(e)] -= t;
   }
 }
 
@@ -583,7 +595,7 @@ __global__ void __launch_bounds__(NT8, 1) k_fwd_chain8(DevSym S, const int2 *tas
     for (int h = 0; h < BLK8 / NT8; ++h) {
       const int e = tid + h * NT8, row = e >> 3;
       vs[e] = row < bw ? take_contribs<R>(c8, cptr, cidx, f + r0 + row, e & 7,
-                                          rhs_of<R>(y8, f + r0 + row, e & 7)) : 0.0;
+                                          at8<R>(y8 + (size_t)(f + r0) * R, e)) : 0.0;
     }
     double acc[8][2];
 #pragma unroll
